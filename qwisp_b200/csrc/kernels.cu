@@ -1244,152 +1244,6 @@ __global__ void __launch_bounds__(128) k_gdn_core(GdnArgs a) {
         if (tid < 16) hist_out[(size_t)j * convDim + ch_v] = f2h(xval(idx, ch_v));
     }
 }
-// ---- segments of many rows (prompt chunks, verify rows): the same arithmetic in two kernels ----
-// k_gdn_prep   everything that does not depend on the state, for all rows side by side: conv + SiLU of every channel, the
-//              q/k norms and scales, decay and beta, the conv history the call leaves.  grid (Hk + Hv, M), 128 threads:
-//              CTAs [0, Hk) own a key head's q and k channels, CTAs [Hk, Hk + Hv) a value head's v channels and gates.
-// k_gdn_scan   the recurrence alone, rows of a segment in sequence, the operands of 32 rows at a time staged in shared
-//              memory by cp.async one chunk ahead.
-//              Same grid and state ownership as k_gdn_core.
-// Every value is formed by the same functions in the same order as in k_gdn_core, so the outputs and the state are
-// identical bit for bit; the split only removes the per-row latency chain (and the 16-fold recomputation of q / k).
-__global__ void __launch_bounds__(128) k_gdn_prep(GdnArgs a) {
-    __shared__ float red_s[8];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m = blockIdx.y;
-    const SegDesc seg = a.segs[a.row_seg[m]];
-    const int tt = m - seg.row0;
-    const int keyDim = a.Hk * GDN_DK, valDim = a.Hv * GDN_DV, convDim = 2 * keyDim + valDim;
-    const int side = a.tab.parity[seg.slot];
-    const __half* hist_in = a.tab.conv_hist + (size_t)seg.slot * a.tab.hist_stride_stream + (size_t)side * a.tab.hist_stride_side +
-                            (size_t)a.gdn_index * a.tab.hist_stride_layer;
-    __half* hist_out = a.tab.conv_hist + (size_t)seg.slot * a.tab.hist_stride_stream + (size_t)(side ^ 1) * a.tab.hist_stride_side +
-                       (size_t)a.gdn_index * a.tab.hist_stride_layer;
-    auto xval = [&](int idx, int ch) -> float {               // row idx of [hist(3) | rows of the segment]
-        if (idx < CONV_K - 1) return h2f(hist_in[(size_t)idx * convDim + ch]);
-        return h2f(a.inproj[(size_t)(seg.row0 + idx - (CONV_K - 1)) * a.ld + ch]);
-    };
-    auto conv = [&](int ch) -> float {
-        const float4 w = *reinterpret_cast<const float4*>(a.conv_w + (size_t)ch * 4);
-        return gdn_conv_silu(xval(tt + 0, ch), xval(tt + 1, ch), xval(tt + 2, ch), xval(tt + 3, ch), w);
-    };
-    const bool last = (tt == seg.nrows - 1);
-    if ((int)blockIdx.x < a.Hk) {
-        const int hk = blockIdx.x, ch_q = hk * GDN_DK + tid, ch_k = keyDim + hk * GDN_DK + tid;
-        const float qc = conv(ch_q), kc = conv(ch_k);
-        const float sq = warp_sum(qc * qc), sk = warp_sum(kc * kc);
-        if (lane == 0) { red_s[warp] = sq; red_s[4 + warp] = sk; }
-        __syncthreads();
-        const float iq = gdn_head_inv(red_s[0], red_s[1], red_s[2], red_s[3], a.eps);
-        const float ik = gdn_head_inv(red_s[4], red_s[5], red_s[6], red_s[7], a.eps);
-        a.qk[(size_t)m * 2 * keyDim + hk * GDN_DK + tid] = f2h(gdn_scale_q(qc, iq));              // exact: the value is an fp16 product
-        a.qk[(size_t)m * 2 * keyDim + keyDim + hk * GDN_DK + tid] = f2h(gdn_scale_k(kc, ik));
-        if (last)
-            for (int j = 0; j < CONV_K - 1; ++j) {
-                hist_out[(size_t)j * convDim + ch_q] = f2h(xval(seg.nrows + j, ch_q));
-                hist_out[(size_t)j * convDim + ch_k] = f2h(xval(seg.nrows + j, ch_k));
-            }
-    } else {
-        const int hv = blockIdx.x - a.Hk, ch_v = 2 * keyDim + hv * GDN_DV + tid;
-        a.vc[(size_t)m * valDim + hv * GDN_DV + tid] = f2h(conv(ch_v));                            // exact: conv + SiLU is rounded to fp16
-        if (tid == 0) {
-            const __half bh = a.inproj[(size_t)m * a.ld + convDim + valDim + hv];
-            const __half ah = a.inproj[(size_t)m * a.ld + convDim + valDim + a.Hv + hv];
-            float g, beta;
-            gdn_gate(bh, ah, a.A_log[hv], a.dt_bias[hv], g, beta);
-            a.gb[(size_t)m * a.Hv + hv] = make_float2(g, beta);
-        }
-        if (last)
-            for (int j = 0; j < CONV_K - 1; ++j) hist_out[(size_t)j * convDim + ch_v] = f2h(xval(seg.nrows + j, ch_v));
-    }
-}
-constexpr int GS_CH = 32;                                    // rows per staged chunk
-__device__ __forceinline__ void gs_cp16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void gs_cp8(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__global__ void __launch_bounds__(128) k_gdn_scan(GdnArgs a) {
-    // operands of 32 rows at a time, two buffers: q | k of the key head, the 16 v values of this CTA's state rows, (decay, beta)
-    __shared__ __align__(16) __half qk_s[2][GS_CH][2 * GDN_DK];
-    __shared__ __align__(16) __half v_s[2][GS_CH][16];
-    __shared__ __align__(8) float2 gb_s[2][GS_CH];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int dvt = blockIdx.x, hv = blockIdx.y;
-    const SegDesc seg = a.segs[blockIdx.z];
-    const int hk = hv / (a.Hv / a.Hk);
-    const int keyDim = a.Hk * GDN_DK, valDim = a.Hv * GDN_DV;
-    const int side = a.tab.parity[seg.slot];
-    const float* S_in = a.tab.gdn_state + (size_t)seg.slot * a.tab.state_stride_stream + (size_t)side * a.tab.state_stride_side +
-                        (size_t)a.gdn_index * a.tab.state_stride_layer + ((size_t)hv * GDN_DV + dvt * 16) * GDN_DK;
-    float* S_out = a.tab.gdn_state + (size_t)seg.slot * a.tab.state_stride_stream + (size_t)(side ^ 1) * a.tab.state_stride_side +
-                   (size_t)a.gdn_index * a.tab.state_stride_layer + ((size_t)hv * GDN_DV + dvt * 16) * GDN_DK;
-    float4 S[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) S[i] = *reinterpret_cast<const float4*>(S_in + (size_t)(warp * 4 + i) * GDN_DK + lane * 4);
-    auto stage = [&](int c, int b) {
-        const int t0 = c * GS_CH, n = min(GS_CH, seg.nrows - t0);
-        for (int i = tid; i < n * 32; i += 128) {                                    // q, k: 16 + 16 pieces of 16 bytes per row
-            const int r = i >> 5, p = i & 31;
-            const size_t row = (size_t)(seg.row0 + t0 + r);
-            gs_cp16(&qk_s[b][r][p * 8], a.qk + row * 2 * keyDim + (p < 16 ? 0 : keyDim) + hk * GDN_DK + (p & 15) * 8);
-        }
-        for (int i = tid; i < n * 2; i += 128) {
-            const int r = i >> 1, p = i & 1;
-            gs_cp16(&v_s[b][r][p * 8], a.vc + (size_t)(seg.row0 + t0 + r) * valDim + hv * GDN_DV + dvt * 16 + p * 8);
-        }
-        for (int i = tid; i < n; i += 128) gs_cp8(&gb_s[b][i], a.gb + (size_t)(seg.row0 + t0 + i) * a.Hv + hv);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    auto h4 = [](uint2 u) -> float4 {
-        const __half2 lo = *reinterpret_cast<const __half2*>(&u.x), hi = *reinterpret_cast<const __half2*>(&u.y);
-        const float2 a2 = __half22float2(lo), b2 = __half22float2(hi);
-        return make_float4(a2.x, a2.y, b2.x, b2.y);
-    };
-    const int nchunks = (seg.nrows + GS_CH - 1) / GS_CH;
-    stage(0, 0);
-    for (int c = 0; c < nchunks; ++c) {
-        const int b = c & 1;
-        if (c + 1 < nchunks) { stage(c + 1, b ^ 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-        else asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        const int t0 = c * GS_CH, n = min(GS_CH, seg.nrows - t0);
-        for (int r = 0; r < n; ++r) {
-            const float4 qq = h4(*reinterpret_cast<const uint2*>(&qk_s[b][r][lane * 4]));
-            const float4 kq = h4(*reinterpret_cast<const uint2*>(&qk_s[b][r][GDN_DK + lane * 4]));
-            const float4 vv = h4(*reinterpret_cast<const uint2*>(&v_s[b][r][warp * 4]));
-            const float2 gb = gb_s[b][r];
-            const float vs[4] = {vv.x, vv.y, vv.z, vv.w};
-            // the warp's four rows together: their two butterfly sums share shuffles (warp_sum4), same additions as gdn_row_step()
-            const float kvz = warp_sum4(gdn_decay_dot(S[0], gb.x, kq), gdn_decay_dot(S[1], gb.x, kq), gdn_decay_dot(S[2], gb.x, kq),
-                                        gdn_decay_dot(S[3], gb.x, kq), lane);
-            float op[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float kv = __shfl_sync(0xffffffffu, kvz, 8 * i);
-                const float delta = (vs[i] - kv) * gb.y;
-                op[i] = gdn_update_dot(S[i], kq, delta, qq);
-            }
-            const float oz = warp_sum4(op[0], op[1], op[2], op[3], lane);
-            if ((lane & 7) == 0)
-                a.y[(size_t)(seg.row0 + t0 + r) * valDim + hv * GDN_DV + dvt * 16 + warp * 4 + (lane >> 3)] = f2h(oz);
-        }
-        __syncthreads();                       // the buffer is refilled by the next iteration's stage()
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(S_out + (size_t)(warp * 4 + i) * GDN_DK + lane * 4) = S[i];
-}
-void launch_gdn_rows(const GdnArgs& a, int M, int nsegs, cudaStream_t st) {
-    {
-        ProfScope ps("k_gdn_prep", (double)M * (2 * a.Hk * GDN_DK + a.Hv * GDN_DV) * 4, st);
-        k_gdn_prep<<<dim3((unsigned)(a.Hk + a.Hv), (unsigned)M), 128, 0, st>>>(a);
-        COUNT_LAUNCH();
-    }
-    ProfScope ps("k_gdn_scan", (double)nsegs * a.Hv * GDN_DV * GDN_DK * 8, st);
-    k_gdn_scan<<<dim3(8, (unsigned)a.Hv, (unsigned)nsegs), 128, 0, st>>>(a);
-    COUNT_LAUNCH();
-}
 void launch_gdn_core(const GdnArgs& a, int nsegs, cudaStream_t st, bool pdl) {
     dim3 grid(8, a.Hv, nsegs);
     ProfScope ps("k_gdn_core", (double)nsegs * a.Hv * GDN_DV * GDN_DK * 8, st);

@@ -109,11 +109,12 @@ struct GdnArgs {
     StreamTable tab; int gdn_index;      // which GDN layer (index among GDN layers)
     const SegDesc* segs;
     __half* y;                           // [M][Hv*128]
-    // two-kernel form for segments of many rows: row -> segment, and the scratch between the kernels
+    // two-kernel form (gdn_rows.cu): row -> segment, and the scratch between the kernels
     const int* row_seg = nullptr;
-    __half* qk = nullptr;                // [M][2*Hk*128] normed, scaled q | k
-    __half* vc = nullptr;                // [M][Hv*128] conv + SiLU of v
-    float2* gb = nullptr;                // [M][Hv] (decay, beta)
+    float* qk = nullptr;                 // gdn_qk_floats(): normed, scaled k | q
+    unsigned char* vg = nullptr;         // gdn_vg_bytes(): conv + SiLU of v, (decay, beta)
+    int M = 0;                           // rows of the call (filled by the launcher)
+    unsigned* err = nullptr;
 };
 
 struct AttnArgs {
@@ -231,6 +232,7 @@ void launch_gdn_core(const GdnArgs& a, int nsegs, cudaStream_t st, bool pdl);
 // prefill-mode attention of one stream's chunk on the tensor cores (after launch_attn_prep); false: call not covered
 bool launch_attn_prefill(const AttnArgs& a, int nsegs, cudaStream_t st);
 void launch_gdn_rows(const GdnArgs& a, int M, int nsegs, cudaStream_t st);   // the same result by k_gdn_prep + k_gdn_scan (needs the scratch fields)
+size_t gdn_qk_floats(int Hk, int rows); size_t gdn_vg_bytes(int Hv, int rows);
 void launch_attn_prep(const AttnArgs& a, cudaStream_t st);
 // q/k prep (when every row is its stream's only row) + split-KV decode + merge in one launch; counters: M*KV zeros
 void launch_attn_fused(const AttnArgs& a, bool prep, unsigned* counters, cudaStream_t st, bool pdl);

@@ -734,24 +734,43 @@ bool launch_router_rows(const RouterArgs& a, cudaStream_t st) {
 }
 
 // ================================================================================ combine
-// grid (M), 256 threads:
+// grid (M, ceil(H / 2048)), 256 threads, 8 outputs a thread:
 // out/resid[m] (+)= sum_k fp16(d[m*topk + k] * score[m,k]) (ascending k) + sigmoid(sgl[m]) * shared[m]
 // (swift/Sources/QwispCore/SeedlessFusedVerify.swift:462-484, SeedlessMetalForward.swift:1024-1028)
+// Bound by latency: with one output and 2-byte loads per thread and step the eight steps of a thread were 8 dependent
+// round trips; all 16-byte loads of a thread are now in flight at once.
 __global__ void __launch_bounds__(256) k_moe_combine(const __half* dbuf, const __half* shared_rows, const __half* scores, const __half* sgl,
                                                      int H, int topk, __half* resid, __half* out) {
-    const int m = blockIdx.x;
-    for (int n = threadIdx.x; n < H; n += blockDim.x) {
-        __half acc = f2h(0.0f);
-        for (int k = 0; k < topk; ++k)
-            acc = hadd_rn(acc, hmul_rn(__ldcg(dbuf + (size_t)(m * topk + k) * H + n), scores[m * topk + k]));
-        const __half res = hadd_rn(acc, hmul_rn(sigmoid_h(sgl[m]), __ldcg(shared_rows + (size_t)m * H + n)));
-        if (resid) resid[(size_t)m * H + n] = hadd_rn(resid[(size_t)m * H + n], res);
-        else out[(size_t)m * H + n] = res;
+    const int m = blockIdx.x, n = (blockIdx.y * 256 + threadIdx.x) * 8;
+    if (n >= H) return;
+    const uint4 sh = __ldcg(reinterpret_cast<const uint4*>(shared_rows + (size_t)m * H + n));
+    uint4 rv = make_uint4(0, 0, 0, 0);
+    if (resid) rv = *reinterpret_cast<const uint4*>(resid + (size_t)m * H + n);
+    const __half* d0 = dbuf + (size_t)m * topk * H + n;
+    __half acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = f2h(0.0f);
+#pragma unroll 8
+    for (int k = 0; k < topk; ++k) {
+        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(d0 + (size_t)k * H));
+        const __half sc = scores[m * topk + k];
+        const __half* vh = reinterpret_cast<const __half*>(&v);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = hadd_rn(acc[i], hmul_rn(vh[i], sc));
     }
+    const __half gate = sigmoid_h(sgl[m]);
+    const __half* shh = reinterpret_cast<const __half*>(&sh);
+    __half* rh = reinterpret_cast<__half*>(&rv);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const __half res = hadd_rn(acc[i], hmul_rn(gate, shh[i]));
+        rh[i] = resid ? hadd_rn(rh[i], res) : res;
+    }
+    *reinterpret_cast<uint4*>((resid ? resid : out) + (size_t)m * H + n) = rv;
 }
 void launch_moe_combine(const __half* dbuf, const __half* shared_rows, const __half* scores, const __half* sgl, int M, int H, int topk,
                         __half* resid, __half* out, cudaStream_t st) {
-    profile_launch("k_moe_combine", st, [&] { k_moe_combine<<<M, 256, 0, st>>>(dbuf, shared_rows, scores, sgl, H, topk, resid, out); return 0; });
+    profile_launch("k_moe_combine", st, [&] { k_moe_combine<<<dim3((unsigned)M, (unsigned)((H + 2047) / 2048)), 256, 0, st>>>(dbuf, shared_rows, scores, sgl, H, topk, resid, out); return 0; });
 }
 
 }  // namespace sl

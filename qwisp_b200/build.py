@@ -6,7 +6,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 SO = os.path.join(HERE, "libseedless_b200.so")
-SOURCES = ["synth.cu", "kernels.cu", "step_persistent.cu", "ep_exchange.cu", "rows_kernels.cu", "gdn_rows.cu", "attn_prefill.cu", "sampler.cu", "gemm_tc.cu", "engine.cu"]
+SOURCES = ["synth.cu", "kernels.cu", "step_persistent.cu", "ep_exchange.cu", "rows_kernels.cu", "gdn_rows.cu", "state_io.cu", "attn_prefill.cu", "sampler.cu", "gemm_tc.cu", "engine.cu"]
 HEADERS = ["common.cuh", "gemv.cuh", "mixer_math.cuh", "route.cuh", "kernels.h", os.path.join("..", "..", "include", "seedless_b200.h")]
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-lineinfo",
@@ -41,7 +41,7 @@ def build(force=False, verbose=False):
             sys.stderr.write(out)
         if p.returncode != 0:
             raise RuntimeError("nvcc failed: " + " ".join(cmd))
-    link = [nvcc, "-shared", "-o", SO] + objs + ["-ccbin", "/usr/bin/g++", "-lcudart"]
+    link = [nvcc, "-shared", "-o", SO] + objs + ["-ccbin", "/usr/bin/g++", "-lcudart", "-lpthread"]
     subprocess.check_call(link)
     return SO
 

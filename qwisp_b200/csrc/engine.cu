@@ -69,7 +69,8 @@ struct sl_engine {
     int* inds = nullptr; MoeLists lists{};
     float *part_o = nullptr, *part_ml = nullptr, *pval = nullptr;
     int *pidx = nullptr, *out_tok = nullptr, *tok_in = nullptr, *hist = nullptr, *hist_pos = nullptr;
-    int *row_seg = nullptr, *row_off = nullptr, *row_pos = nullptr;
+    int *row_pos = nullptr;
+    int *desc = nullptr;            // a call's tokens and row / segment descriptors, one block (see row_seg_of); tok_in = its start
     unsigned* counters = nullptr; unsigned* tile_counters = nullptr; unsigned* att_counters = nullptr; unsigned* err_flag = nullptr; unsigned* err_host = nullptr; float* adj_buf = nullptr; int* samp_buf = nullptr; unsigned* slot_sync = nullptr; unsigned* router_groups = nullptr;
     bool use_route_in_experts = true;   // with the fused kernel: routing done by its CTAs (SL_FLAG_ROUTE_IN_ROUTER: by the router's last CTA)
     bool use_rows = true;           // calls with more than 8 rows use the many-row kernels (SL_FLAG_PASS_KERNELS turns it off)
@@ -82,10 +83,12 @@ struct sl_engine {
     void* ep_region = nullptr;        // this rank's exchange region (shared with the peers through CUDA IPC)
     void* ep_mapped[8] = {};          // peers' regions as mapped here
     int ep_layer_seq = 0;             // MoE layers enqueued so far in the step being built
-    SegDesc* segs = nullptr;
     int hist_cap = 0;
     // pinned staging
-    int* pin_i = nullptr; size_t pin_ints = 0;
+    int* pin_i = nullptr;           // host image of `desc`
+    bool pin_busy = false;          // an enqueued copy may still read pin_i
+    int* pin_out = nullptr;         // [pin_out_ints] page-locked: where tokens arrive
+    size_t pin_out_ints = 0;
     // streams
     StreamTable tab{};
     __half* kv_pool = nullptr;
@@ -105,6 +108,7 @@ struct sl_engine {
     bool ps_ok = false, use_persistent = false;
     PStepArgs ps{};
     uint32_t* ps_timeline = nullptr;
+    StateIoRing sio;                // slots of state save / restore
     bool poisoned = false, inject = false;
     std::string fault;
 };
@@ -275,6 +279,13 @@ int32_t build_layout(sl_engine* e) {
     return SL_OK;
 }
 
+// Layout of the descriptor block of an M-row call: tokens [M] | segment of each row [M] | row inside its segment [M] |
+// segments.  One copy brings all of it; the places depend on M alone, so a step graph (keyed by M) can hold them.
+size_t desc_ints(int R) { return (size_t)3 * R + 4 + (size_t)R * (sizeof(SegDesc) / sizeof(int)); }
+int* row_seg_of(int* desc, int M) { return desc + M; }
+int* row_off_of(int* desc, int M) { return desc + 2 * (size_t)M; }
+SegDesc* segs_of(int* desc, int M) { return reinterpret_cast<SegDesc*>(desc + (((size_t)3 * M + 3) & ~(size_t)3)); }
+
 int32_t build_runtime(sl_engine* e) {
     const sl_config& c = e->cfg;
     const int R = c.max_rows, H = e->H;
@@ -313,15 +324,13 @@ int32_t build_runtime(sl_engine* e) {
     if ((rc = dalloc(e, &e->pval, (size_t)R * (e->V / 16)))) return rc;
     if ((rc = dalloc(e, &e->pidx, (size_t)R * (e->V / 16)))) return rc;
     if ((rc = dalloc(e, &e->out_tok, (size_t)R))) return rc;
-    if ((rc = dalloc(e, &e->tok_in, (size_t)R))) return rc;
+    if ((rc = dalloc(e, &e->desc, desc_ints(R)))) return rc;
+    e->tok_in = e->desc;
     e->hist_cap = 1 << 16;
     if ((rc = dalloc(e, &e->hist, (size_t)e->hist_cap))) return rc;
     if ((rc = dalloc(e, &e->hist_pos, (size_t)1))) return rc;
-    if ((rc = dalloc(e, &e->row_seg, (size_t)R))) return rc;
-    if ((rc = dalloc(e, &e->row_off, (size_t)R))) return rc;
     if ((rc = dalloc(e, &e->row_pos, (size_t)R))) return rc;
     if ((rc = dalloc(e, &e->counters, (size_t)8))) return rc;
-    if ((rc = dalloc(e, &e->segs, (size_t)R))) return rc;
     if ((rc = dalloc(e, &e->lists.n_active, (size_t)1))) return rc;
     if ((rc = dalloc(e, &e->lists.slot_expert, (size_t)256))) return rc;
     if ((rc = dalloc(e, &e->lists.slot_off, (size_t)256))) return rc;
@@ -344,8 +353,9 @@ int32_t build_runtime(sl_engine* e) {
     if ((rc = dalloc(e, &e->att_counters, (size_t)R * c.attn_kv_heads))) return rc;
     CU(e, cudaMemset(e->att_counters, 0, (size_t)R * c.attn_kv_heads * sizeof(unsigned)));
     CU(e, cudaMemset(e->hist_pos, 0, sizeof(int)));
-    e->pin_ints = (size_t)R * 8 + 64;
-    CU(e, cudaMallocHost(&e->pin_i, e->pin_ints * sizeof(int)));
+    CU(e, cudaMallocHost(&e->pin_i, desc_ints(R) * sizeof(int)));
+    e->pin_out_ints = R > 4096 ? (size_t)R : 4096;
+    CU(e, cudaMallocHost(&e->pin_out, e->pin_out_ints * sizeof(int)));
     // stream tables
     const int S = c.max_streams;
     StreamTable& t = e->tab;
@@ -431,7 +441,7 @@ int32_t setup_persistent(sl_engine* e) {
     a.geom = g; a.layers = dl; a.n_layers = (int)host.size();
     a.embed = e->embed; a.final_norm = e->final_norm; a.lm_head = e->r_lm_head;
     a.eps = c.rms_eps; a.theta = c.rope_theta;
-    a.tab = e->tab; a.segs = e->segs; a.kv_pool = e->kv_pool; a.n_attn_layers = e->n_attn > 0 ? e->n_attn : 1; a.page_size = c.kv_page_size; a.nsplit = NSPLIT;
+    a.tab = e->tab; a.segs = segs_of(e->desc, 1); a.kv_pool = e->kv_pool; a.n_attn_layers = e->n_attn > 0 ? e->n_attn : 1; a.page_size = c.kv_page_size; a.nsplit = NSPLIT;
     a.tok_in = e->tok_in; a.out_tok = e->out_tok; a.hist = e->hist; a.hist_pos = e->hist_pos; a.hist_cap = e->hist_cap;
     // exchange lines of a layer (16 bytes carry 4 halves): residual stream in, in-projection out, mixer out,
     // residual stream after the mixer, router logits (one per half line) + shared-gate logit, SwiGLU rows; the
@@ -637,8 +647,8 @@ void enqueue_mixer(sl_engine* e, const LayerW& L, const __half* rows, const __ha
     }
     if (!L.is_attn) {
         GdnArgs g{}; g.inproj = e->inproj; g.ld = e->gdn_in; g.conv_w = L.conv_w; g.A_log = L.A_log; g.dt_bias = L.dt_bias;
-        g.Hk = c.gdn_k_heads; g.Hv = c.gdn_v_heads; g.eps = c.rms_eps; g.tab = e->tab; g.gdn_index = L.type_index; g.segs = e->segs; g.y = e->mix;
-        g.row_seg = e->row_seg; g.qk = e->gdn_qk; g.vg = e->gdn_vg; g.err = e->err_flag;
+        g.Hk = c.gdn_k_heads; g.Hv = c.gdn_v_heads; g.eps = c.rms_eps; g.tab = e->tab; g.gdn_index = L.type_index; g.segs = segs_of(e->desc, M); g.y = e->mix;
+        g.row_seg = row_seg_of(e->desc, M); g.qk = e->gdn_qk; g.vg = e->gdn_vg; g.err = e->err_flag;
         // segments of many rows: the state-independent part for all rows side by side, then the bare recurrence (same bits)
         if (e->use_rows && M >= 16) launch_gdn_rows(g, M, nsegs, st);
         else launch_gdn_core(g, nsegs, st, e->use_pdl);
@@ -647,7 +657,7 @@ void enqueue_mixer(sl_engine* e, const LayerW& L, const __half* rows, const __ha
     } else {
         AttnArgs a{}; a.inproj = e->inproj; a.ld = e->attn_in; a.q_norm = L.q_norm; a.k_norm = L.k_norm; a.NH = c.attn_heads; a.KV = c.attn_kv_heads;
         a.eps = c.rms_eps; a.theta = c.rope_theta; a.tab = e->tab; a.attn_index = L.type_index; a.n_attn_layers = e->n_attn > 0 ? e->n_attn : 1;
-        a.page_size = c.kv_page_size; a.kv_pool = e->kv_pool; a.segs = e->segs; a.row_seg = e->row_seg; a.row_off = e->row_off;
+        a.page_size = c.kv_page_size; a.kv_pool = e->kv_pool; a.segs = segs_of(e->desc, M); a.row_seg = row_seg_of(e->desc, M); a.row_off = row_off_of(e->desc, M);
         a.row_pos_override = row_pos_override; a.qrot = e->qrot; a.part_o = e->part_o; a.part_ml = e->part_ml; a.nsplit = NSPLIT; a.gated = e->mix; a.M = M;
         // a row that is its stream's only row in this call can make its own q/K/V inside the attention kernel;
         // several rows of one stream need every row's K/V in the arena before any of them attends
@@ -681,7 +691,7 @@ void enqueue_step(sl_engine* e, int M, int nsegs, HeadMode head, bool want_logit
         d.logits = want_logits ? e->logits : nullptr; d.pval = e->pval; d.pidx = e->pidx; d.out_tok = e->out_tok; d.counter = e->counters + 0;
         launch_dense(PRO_RMSNORM, EPI_ARGMAX, d, st, e->use_pdl);
     }
-    StepEndArgs se{}; se.tab = e->tab; se.segs = e->segs; se.nsegs = nsegs; se.M = M;
+    StepEndArgs se{}; se.tab = e->tab; se.segs = segs_of(e->desc, M); se.nsegs = nsegs; se.M = M;
     se.out_tok = (head == HEAD_ARGMAX || head == HEAD_LOGITS) ? e->out_tok : nullptr;
     se.tok_in = e->tok_in; se.hist = e->hist; se.hist_pos = e->hist_pos; se.hist_cap = e->hist_cap;
     launch_step_end(se, st);
@@ -697,33 +707,24 @@ int32_t ensure_pages(sl_stream* s, int new_len) {
     if (need <= have) return SL_OK;
     if ((int)e->free_pages.size() < need - have) return SL_ERR_CAPACITY;
     for (int i = have; i < need; ++i) { s->pages.push_back(e->free_pages.back()); e->free_pages.pop_back(); }
-    CU(e, cudaMemcpyAsync(e->tab.page_table + (size_t)s->slot * e->tab.max_pages + have, s->pages.data() + have,
-                          (size_t)(need - have) * sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    // the source is pageable host memory owned by the stream object: make the copy complete before it can change
-    CU(e, cudaStreamSynchronize(e->stream));
+    launch_set_pages(e->tab.page_table + (size_t)s->slot * e->tab.max_pages + have, s->pages.data() + have, need - have, e->stream);
     return SL_OK;
 }
 
 // upload tokens (optional) and row / segment descriptors for a call
 int32_t upload_descs(sl_engine* e, const std::vector<SegDesc>& segs, const int32_t* tokens, int M) {
-    CU(e, cudaStreamSynchronize(e->stream));    // the pinned staging area may still feed an earlier copy
+    if (e->pin_busy) CU(e, cudaStreamSynchronize(e->stream));    // the staging area may still feed an earlier copy
     int* pin = e->pin_i;
-    size_t off = 0;
-    int* p_tok = pin + off; off += M;
-    int* p_seg = pin + off; off += M;
-    int* p_off = pin + off; off += M;
-    SegDesc* p_sd = reinterpret_cast<SegDesc*>(pin + off);
+    int *p_seg = row_seg_of(pin, M), *p_off = row_off_of(pin, M);
+    SegDesc* p_sd = segs_of(pin, M);
     for (size_t si = 0; si < segs.size(); ++si) {
         p_sd[si] = segs[si];
         for (int r = 0; r < segs[si].nrows; ++r) { p_seg[segs[si].row0 + r] = (int)si; p_off[segs[si].row0 + r] = r; }
     }
-    if (tokens) {
-        memcpy(p_tok, tokens, (size_t)M * sizeof(int));
-        CU(e, cudaMemcpyAsync(e->tok_in, p_tok, (size_t)M * sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    }
-    CU(e, cudaMemcpyAsync(e->row_seg, p_seg, (size_t)M * sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    CU(e, cudaMemcpyAsync(e->row_off, p_off, (size_t)M * sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    CU(e, cudaMemcpyAsync(e->segs, p_sd, segs.size() * sizeof(SegDesc), cudaMemcpyHostToDevice, e->stream));
+    if (tokens) memcpy(pin, tokens, (size_t)M * sizeof(int));
+    const size_t from = tokens ? 0 : (size_t)M, to = (size_t)((int*)(p_sd + segs.size()) - pin);
+    e->pin_busy = true;
+    CU(e, cudaMemcpyAsync(e->desc + from, pin + from, (to - from) * sizeof(int), cudaMemcpyHostToDevice, e->stream));
     return SL_OK;
 }
 
@@ -760,6 +761,7 @@ int32_t enqueue_decode_step(sl_engine* e, int rows) {
 
 int32_t sync_check(sl_engine* e) {
     CU(e, cudaStreamSynchronize(e->stream));
+    e->pin_busy = false;
     CU(e, cudaGetLastError());
     // a kernel that gave up a bounded wait went on with whatever it had: the results of this call are not to be trusted
     if (e->err_host && *(volatile unsigned*)e->err_host) {
@@ -767,6 +769,16 @@ int32_t sync_check(sl_engine* e) {
         snprintf(msg, sizeof msg, "a kernel gave up a bounded wait (code %u): results discarded", *(volatile unsigned*)e->err_host);
         return poison_msg(e, msg);
     }
+    return SL_OK;
+}
+
+// n ints from the device to the caller, by way of page-locked memory when they fit (a copy to pageable memory takes several
+// times as long to set up; having the step's last kernel store them in host memory itself made every step 10 us longer)
+int32_t collect_ints(sl_engine* e, const int* dev, int n, int32_t* out) {
+    const bool staged = (size_t)n <= e->pin_out_ints;
+    CU(e, cudaMemcpyAsync(staged ? e->pin_out : out, dev, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+    int32_t rc = sync_check(e); if (rc) return rc;
+    if (staged) memcpy(out, e->pin_out, (size_t)n * sizeof(int));
     return SL_OK;
 }
 
@@ -803,7 +815,9 @@ int32_t sl_engine_destroy(sl_engine* e) {
     cudaDeviceSynchronize();
     for (auto& g : e->graphs) cudaGraphExecDestroy(g.second);
     for (void* p : e->allocs) cudaFree(p);
+    e->sio.destroy();
     if (e->pin_i) cudaFreeHost(e->pin_i);
+    if (e->pin_out) cudaFreeHost(e->pin_out);
     if (e->err_host) cudaFreeHost(e->err_host);
     if (e->own_stream) cudaStreamDestroy(e->own_stream);
     cudaGetLastError();
@@ -1101,8 +1115,7 @@ int32_t sl_step_argmax(sl_stream* s, const int32_t* tokens, int32_t M, int32_t* 
     if (!s || !out_tokens) return SL_ERR_INVALID;
     sl_engine* e = s->e;
     int32_t rc = run_single(s, tokens, M, HEAD_ARGMAX, false); if (rc) return rc;
-    CU(e, cudaMemcpyAsync(out_tokens, e->out_tok, (size_t)M * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-    return sync_check(e);
+    return collect_ints(e, e->out_tok, M, out_tokens);
 }
 int32_t sl_step_logits(sl_stream* s, const int32_t* tokens, int32_t M, uint16_t* out_logits_f16) {
     if (!s || !out_logits_f16) return SL_ERR_INVALID;
@@ -1176,8 +1189,7 @@ int32_t sl_chained_collect(sl_stream* s, int32_t K, int32_t* out_tokens) {
     sl_engine* e = s->e;
     int32_t rc = guard(e); if (rc) return rc;
     if (K > e->hist_cap) return SL_ERR_INVALID;
-    CU(e, cudaMemcpyAsync(out_tokens, e->hist, (size_t)K * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-    return sync_check(e);
+    return collect_ints(e, e->hist, K, out_tokens);
 }
 int32_t sl_chained_step_argmax(sl_stream* s, int32_t first, int32_t K, int32_t* out_tokens) {
     if (first < 0) return SL_ERR_INVALID;
@@ -1203,8 +1215,7 @@ int32_t sl_batch_step_argmax(sl_engine* e, sl_stream* const* streams, const int3
     e->ep_step = false;
     if (rc) return rc;
     for (int b = 0; b < B; ++b) { streams[b]->kv_len += 1; streams[b]->parity ^= 1; streams[b]->calls += 1; }
-    CU(e, cudaMemcpyAsync(out_tokens, e->out_tok, (size_t)B * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-    return sync_check(e);
+    return collect_ints(e, e->out_tok, B, out_tokens);
 }
 
 // ---- expert-parallel decode (no counterpart in the reference, which runs on one GPU) ----
@@ -1266,12 +1277,12 @@ int32_t sl_ep_init(sl_engine* e, int32_t rank, int32_t world, const uint8_t* id1
 }
 
 // ---- snapshot / rollback ----
+// (the values travel as kernel arguments: no host memory to keep alive, nothing to wait for)
 static int32_t push_len_parity(sl_stream* s) {
     sl_engine* e = s->e;
-    int v[2] = {s->kv_len, s->parity};
-    CU(e, cudaMemcpyAsync(e->tab.kv_len + s->slot, &v[0], sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    CU(e, cudaMemcpyAsync(e->tab.parity + s->slot, &v[1], sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    return sync_check(e);
+    launch_set_len_parity(e->tab, s->slot, s->kv_len, s->parity, e->stream);
+    CU(e, cudaGetLastError());
+    return SL_OK;
 }
 int32_t sl_snapshot(sl_stream* s, sl_snap* out) {
     if (!s || !out) return SL_ERR_INVALID;
@@ -1338,44 +1349,22 @@ int32_t sl_state_size(sl_stream* s, uint64_t* nbytes) {
     *nbytes = n;
     return SL_OK;
 }
-// copy positions [0,len) of (layer, K|V, head) between the paged arena and a contiguous host run
-static int32_t kv_copy(sl_stream* s, int attn_index, int which, int kvh, int len, uint8_t* host, bool to_host) {
+static StateIoArgs state_io_args(sl_stream* s, int len) {
     sl_engine* e = s->e; const sl_config& c = e->cfg;
-    size_t page_elems = (size_t)e->n_attn * 2 * c.attn_kv_heads * c.kv_page_size * ATT_D;
-    for (int p0 = 0; p0 < len; p0 += c.kv_page_size) {
-        int n = len - p0 < c.kv_page_size ? len - p0 : c.kv_page_size;
-        __half* dev = e->kv_pool + (size_t)s->pages[p0 / c.kv_page_size] * page_elems +
-                      (((size_t)attn_index * 2 + which) * c.attn_kv_heads + kvh) * c.kv_page_size * ATT_D;
-        uint8_t* hp = host + (size_t)p0 * ATT_D * 2;
-        if (to_host) CU(e, cudaMemcpyAsync(hp, dev, (size_t)n * ATT_D * 2, cudaMemcpyDeviceToHost, e->stream));
-        else CU(e, cudaMemcpyAsync(dev, hp, (size_t)n * ATT_D * 2, cudaMemcpyHostToDevice, e->stream));
-    }
-    return SL_OK;
+    StateIoArgs a{};
+    a.n_layers = c.n_layers; a.attn_every = c.attn_every; a.n_attn = e->n_attn; a.kv_heads = c.attn_kv_heads; a.page_size = c.kv_page_size; a.len = len;
+    a.hist_words = (uint32_t)(e->tab.hist_stride_layer / 2); a.state_words = (uint32_t)e->tab.state_stride_layer;
+    a.state = cur_state(s); a.hist = cur_hist(s); a.kv_pool = e->kv_pool; a.pages = e->tab.page_table + (size_t)s->slot * e->tab.max_pages;
+    return a;
 }
 int32_t sl_state_save(sl_stream* s, void* buf, uint64_t nbytes) {
     if (!s || !buf) return SL_ERR_INVALID;
-    sl_engine* e = s->e; const sl_config& c = e->cfg;
+    sl_engine* e = s->e;
     int32_t rc = guard(e); if (rc) return rc;
     uint64_t need; sl_state_size(s, &need);
     if (nbytes < need) return SL_ERR_CAPACITY;
-    uint8_t* p = (uint8_t*)buf;
-    auto u32 = [&](uint32_t v) { memcpy(p, &v, 4); p += 4; };
-    u32(0x31535751u); u32(1); u32((uint32_t)c.n_layers);
-    for (const LayerW& L : e->layers) {
-        if (L.is_attn) {
-            u32(1); u32(c.attn_kv_heads); u32(ATT_D); u32(s->kv_len);
-            for (int which = 0; which < 2; ++which)
-                for (int hh = 0; hh < c.attn_kv_heads; ++hh) {
-                    if ((rc = kv_copy(s, L.type_index, which, hh, s->kv_len, p, true))) return rc;
-                    p += (size_t)s->kv_len * ATT_D * 2;
-                }
-        } else {
-            size_t cc = e->tab.hist_stride_layer, sc = e->tab.state_stride_layer;
-            u32(2); u32((uint32_t)cc); u32((uint32_t)sc);
-            CU(e, cudaMemcpyAsync(p, cur_hist(s) + (size_t)L.type_index * cc, cc * 2, cudaMemcpyDeviceToHost, e->stream)); p += cc * 2;
-            CU(e, cudaMemcpyAsync(p, cur_state(s) + (size_t)L.type_index * sc, sc * 4, cudaMemcpyDeviceToHost, e->stream)); p += sc * 4;
-        }
-    }
+    const int err = state_io(e->sio, state_io_args(s, s->kv_len), true, (uint8_t*)buf, need, e->stream);
+    if (err) return poison(e, "sl_state_save", (cudaError_t)err);
     return sync_check(e);
 }
 int32_t sl_state_restore(sl_stream* s, const void* buf, uint64_t nbytes) {
@@ -1408,25 +1397,11 @@ int32_t sl_state_restore(sl_stream* s, const void* buf, uint64_t nbytes) {
     if (len < 0) len = 0;
     if ((rc = ensure_pages(s, len))) return rc;
     // pass 2: copy
-    off = 12;
-    for (const LayerW& L : e->layers) {
-        off += 4;
-        if (L.is_attn) {
-            off += 12;
-            for (int which = 0; which < 2; ++which)
-                for (int hh = 0; hh < c.attn_kv_heads; ++hh) {
-                    if ((rc = kv_copy(s, L.type_index, which, hh, len, const_cast<uint8_t*>(b + off), false))) return rc;
-                    off += (size_t)len * ATT_D * 2;
-                }
-        } else {
-            size_t cc = e->tab.hist_stride_layer, sc = e->tab.state_stride_layer;
-            off += 8;
-            CU(e, cudaMemcpyAsync(cur_hist(s) + (size_t)L.type_index * cc, b + off, cc * 2, cudaMemcpyHostToDevice, e->stream)); off += cc * 2;
-            CU(e, cudaMemcpyAsync(cur_state(s) + (size_t)L.type_index * sc, b + off, sc * 4, cudaMemcpyHostToDevice, e->stream)); off += sc * 4;
-        }
-    }
+    const int err = state_io(e->sio, state_io_args(s, len), false, const_cast<uint8_t*>(b), nbytes, e->stream);
+    if (err) return poison(e, "sl_state_restore", (cudaError_t)err);
     s->kv_len = len;
-    return push_len_parity(s);
+    if ((rc = push_len_parity(s))) return rc;
+    return sync_check(e);
 }
 
 // ---- single operators ----

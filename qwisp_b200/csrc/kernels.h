@@ -250,6 +250,25 @@ void profile_launch(const char* tag, cudaStream_t st, const std::function<int()>
 void profile_start();
 int profile_report(char* buf, size_t cap);
 
+// ---- stream state <-> host blob (state_io.cu) ----
+struct StateIoArgs {
+    int n_layers, attn_every, n_attn, kv_heads, page_size, len;
+    uint32_t hist_words, state_words;       // 4-byte words of one GDN layer's conv history / state
+    float* state; __half* hist;             // current side of the stream, GDN layers in order
+    __half* kv_pool; const int* pages;      // the stream's page table row (device)
+};
+struct StateIoRing {                        // page-locked slots and their device counterparts, made at the first use
+    uint8_t *pinned = nullptr, *dev = nullptr;
+    cudaEvent_t done[16] = {};
+    int init();
+    void destroy();
+};
+// copies the whole blob out of (save) or into the stream's caches; when it returns, a save is complete in `host` and a
+// restore has read all of `host` (its device work may still be in flight on st).  0 or a cudaError_t.
+int state_io(StateIoRing& ring, const StateIoArgs& a, bool save, uint8_t* host, size_t bytes, cudaStream_t st);
+void launch_set_pages(int* dst, const int* pages, int n, cudaStream_t st);     // dst[i] = pages[i]; pages (host) is read before the call returns
+void launch_set_len_parity(const StreamTable& tab, int slot, int len, int parity, cudaStream_t st);
+
 // synthetic data + quantiser (synth.cu)
 uint64_t tensor_seed(uint64_t base_seed, const char* name);
 void launch_synth_f16(uint64_t tseed, int64_t n, float mean, float std, __half* out, cudaStream_t st);

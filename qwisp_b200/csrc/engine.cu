@@ -25,6 +25,7 @@ namespace {
 constexpr int NSPLIT = 64;          // KV splits of the decode attention
 
 struct Tensor { void* ptr; size_t bytes; };
+struct StepGraph { cudaGraphExec_t exec = nullptr; int kernels = 0, eager_runs = 0; uint64_t used = 0; };   // kernels: inside the graph, so that replays are counted
 
 struct LayerW {
     bool is_attn = false;
@@ -94,10 +95,8 @@ struct sl_engine {
     __half* kv_pool = nullptr;
     std::vector<int> free_pages;
     std::vector<int> free_slots;
-    // decode graphs keyed by rows (each segment one row)
-    std::map<int, cudaGraphExec_t> graphs;
-    std::map<int, int> graph_kernels;   // kernels inside each captured step (so replays are counted too)
-    std::map<int, int> eager_runs;
+    std::map<uint64_t, StepGraph> graphs;      // by shape, see enqueue_call
+    uint64_t graph_clock = 0;
     bool use_graph = true;
     bool use_prefetch = false;      // L2 prefetch of the weights later kernels read (SL_FLAG_L2_PREFETCH); slower now that
                                     // every kernel starts its own weight copies ahead of the launch wait
@@ -520,9 +519,9 @@ void pf_q4(PfList& pf, int i, const Q4R& q, size_t max_bytes = (size_t)48 << 20)
 // xq / sxq (optional): also leave the normed rows in the prepared form of the many-row expert kernels; returns true if it did.
 bool enqueue_router(sl_engine* e, const RouterArgs& ra, int M, bool pdl, __half* xq = nullptr, float* sxq = nullptr) {
     cudaStream_t st = e->stream;
-    // (expert-parallel calls take this path from 2 rows on: its routing kernel spreads the dispatch over CTAs and warps)
+    // From 2 rows on: the one-kernel router ends in one CTA that routes and groups everything (33 us at 4 rows, 9 at one).
     // (prefill mode takes it for ANY row count: which kernels run must not depend on how a prompt is cut into calls)
-    if ((M > 8 || e->hybrid || (ra.epd.sig.world > 0 && M > 1)) && e->use_rows && !ra.no_route && e->E <= 256 && ra.norm_w && ra.ldh == e->H) {
+    if ((M > 1 || e->hybrid) && e->use_rows && !ra.no_route && e->E <= 256 && ra.norm_w && ra.ldh == e->H) {
         const bool ep = ra.epd.sig.world > 0;
         if (ep) launch_final_norm_ep(ra.h, ra.norm_w, ra.eps, M, e->H, ra.p, ra.epd, st);     // the rows leave for the peers here
         else launch_final_norm(ra.h, ra.norm_w, ra.eps, M, e->H, ra.p, st, xq, sxq);
@@ -600,7 +599,7 @@ void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half
     ra.no_route = (fused && e->use_route_in_experts) ? 1 : 0;
     ea.route_here = ra.no_route;
     const bool tc_experts = e->hybrid && e->E <= 256 && e->use_rows;      // prefill mode: for any row count (chunk-split invariance)
-    const bool rows_experts = !tc_experts && M > 8 && e->E <= 256 && e->use_rows;
+    const bool rows_experts = !tc_experts && M > 1 && e->E <= 256 && e->use_rows;
     const bool prepared = enqueue_router(e, ra, M, e->use_pdl, rows_experts ? e->xq_p : nullptr, e->sx_p);
     if (fused && launch_expert_fused(ea, st, e->use_pdl)) return;                      // one launch for gate/up + down
     if (tc_experts) {
@@ -612,7 +611,7 @@ void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half
         }
         ea.tile_counter = e->tile_counters;
     }
-    if (rows_experts || (tc_experts && M > 8)) {
+    if (rows_experts || (tc_experts && M > 1)) {
         // many rows: the normed rows are prepared once (by the norm kernel when it ran), the experts run without CTA-wide
         // barriers, the combine is its own kernel
         if (!prepared) launch_rows_prep_plain(e->p, e->H, M, e->H, e->xq_p, e->sx_p, st);
@@ -728,36 +727,49 @@ int32_t upload_descs(sl_engine* e, const std::vector<SegDesc>& segs, const int32
     return SL_OK;
 }
 
-// decode-shaped steps (every segment one row) replay a CUDA graph after the first eager run
-int32_t enqueue_decode_step(sl_engine* e, int rows) {
+// Strict calls of few rows replay a CUDA graph from the second call of their shape on (the first runs eagerly, so that
+// one-time set-up is outside the capture): a step is hundreds of launches, and a replay spends neither the host's time on
+// them nor the gaps between them.  The shape is (rows, segments, head); descriptors live where the rows alone decide.
+// At most GRAPH_CAP graphs are kept, the least recently used one goes.
+constexpr int GRAPH_MAX_ROWS = 64;
+constexpr size_t GRAPH_CAP = 64;
+int32_t enqueue_call(sl_engine* e, int rows, int nsegs, HeadMode head, bool want_logits) {
     // a single stream's decode step: one launch of the step kernel does the whole token
-    if (rows == 1 && !e->ep_step && e->ps_ok && e->use_persistent) {
+    if (rows == 1 && head == HEAD_ARGMAX && !want_logits && !e->hybrid && !e->ep_step && e->ps_ok && e->use_persistent) {
         profile_launch("k_step_persistent", e->stream, [&] { return launch_step_persistent(e->ps, e->stream); });
         CU(e, cudaGetLastError());
         return SL_OK;
     }
     // (expert-parallel steps contain no collective -- the exchange is this library's own kernels over peer memory --
     // so they are captured like any other step)
-    if (!e->use_graph) { enqueue_step(e, rows, rows, HEAD_ARGMAX, false); return e->poisoned ? SL_ERR_CUDA : SL_OK; }
-    const int key = rows | (e->ep_step ? (1 << 24) : 0);
-    auto it = e->graphs.find(key);
-    if (it == e->graphs.end()) {
-        if (e->eager_runs[key]++ == 0) { enqueue_step(e, rows, rows, HEAD_ARGMAX, false); return SL_OK; }
-        cudaGraph_t graph = nullptr; cudaGraphExec_t exec = nullptr;
+    if (!e->use_graph || e->hybrid || rows > GRAPH_MAX_ROWS) { enqueue_step(e, rows, nsegs, head, want_logits); return e->poisoned ? SL_ERR_CUDA : SL_OK; }
+    const uint64_t key = (uint64_t)rows | (uint64_t)nsegs << 16 | (uint64_t)head << 32 | (uint64_t)want_logits << 40 | (uint64_t)e->ep_step << 41;
+    StepGraph& g = e->graphs[key];
+    g.used = ++e->graph_clock;
+    if (!g.exec) {
+        if (g.eager_runs++ == 0) { enqueue_step(e, rows, nsegs, head, want_logits); return e->poisoned ? SL_ERR_CUDA : SL_OK; }
+        if (e->graphs.size() > GRAPH_CAP) {
+            auto old = e->graphs.end();
+            for (auto it = e->graphs.begin(); it != e->graphs.end(); ++it) if (it->first != key && (old == e->graphs.end() || it->second.used < old->second.used)) old = it;
+            CU(e, cudaStreamSynchronize(e->stream));               // it may still be running
+            if (old->second.exec) cudaGraphExecDestroy(old->second.exec);
+            e->graphs.erase(old);
+        }
+        cudaGraph_t graph = nullptr;
         CU(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
         const int64_t before = kernel_launch_count();
-        enqueue_step(e, rows, rows, HEAD_ARGMAX, false);
-        e->graph_kernels[key] = (int)(kernel_launch_count() - before);
-        count_launches(-(int64_t)e->graph_kernels[key]);          // the capture itself launched nothing
+        enqueue_step(e, rows, nsegs, head, want_logits);
+        g.kernels = (int)(kernel_launch_count() - before);
+        count_launches(-(int64_t)g.kernels);                       // the capture itself launched nothing
         CU(e, cudaStreamEndCapture(e->stream, &graph));
-        CU(e, cudaGraphInstantiate(&exec, graph, 0));
+        CU(e, cudaGraphInstantiate(&g.exec, graph, 0));
         cudaGraphDestroy(graph);
-        it = e->graphs.emplace(key, exec).first;
     }
-    CU(e, cudaGraphLaunch(it->second, e->stream));
-    count_launches(e->graph_kernels[key]);
+    CU(e, cudaGraphLaunch(g.exec, e->stream));
+    count_launches(g.kernels);
     return SL_OK;
 }
+int32_t enqueue_decode_step(sl_engine* e, int rows) { return enqueue_call(e, rows, rows, HEAD_ARGMAX, false); }
 
 int32_t sync_check(sl_engine* e) {
     CU(e, cudaStreamSynchronize(e->stream));
@@ -795,8 +807,7 @@ int32_t run_single(sl_stream* s, const int32_t* tokens, int M, HeadMode head, bo
     }
     std::vector<SegDesc> segs{SegDesc{s->slot, 0, M, 0}};
     if ((rc = upload_descs(e, segs, tokens, M))) return rc;
-    if (M == 1 && head == HEAD_ARGMAX && !want_logits) { if ((rc = enqueue_decode_step(e, 1))) return rc; }
-    else enqueue_step(e, M, 1, head, want_logits);
+    if ((rc = enqueue_call(e, M, 1, head, want_logits))) return rc;
     s->kv_len += M; s->parity ^= 1; s->calls += 1;
     return SL_OK;
 }
@@ -813,7 +824,7 @@ int32_t sl_engine_destroy(sl_engine* e) {
     if (e->ep_comm && g_nccl.ok) { cudaStreamSynchronize(e->stream); g_nccl.CommDestroy((ncclComm_t)e->ep_comm); e->ep_comm = nullptr; }
     for (int d = 0; d < 8; ++d) if (e->ep_mapped[d]) { cudaIpcCloseMemHandle(e->ep_mapped[d]); e->ep_mapped[d] = nullptr; }
     cudaDeviceSynchronize();
-    for (auto& g : e->graphs) cudaGraphExecDestroy(g.second);
+    for (auto& g : e->graphs) if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
     for (void* p : e->allocs) cudaFree(p);
     e->sio.destroy();
     if (e->pin_i) cudaFreeHost(e->pin_i);
@@ -984,8 +995,8 @@ int32_t sl_engine_create_synthetic(const sl_config* cfg, const sl_synth_spec* sy
 int32_t sl_engine_set_cuda_stream(sl_engine* e, void* cuda_stream) {
     if (!e) return SL_ERR_INVALID;
     cudaStreamSynchronize(e->stream);
-    for (auto& g : e->graphs) cudaGraphExecDestroy(g.second);    // graphs are tied to the stream they were captured on
-    e->graphs.clear(); e->eager_runs.clear();
+    for (auto& g : e->graphs) if (g.second.exec) cudaGraphExecDestroy(g.second.exec);    // graphs are tied to the stream they were captured on
+    e->graphs.clear();
     e->stream = cuda_stream ? (cudaStream_t)cuda_stream : e->own_stream;
     return SL_OK;
 }

@@ -288,30 +288,15 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_expert_umma(ExpertArgs a) {
     constexpr int NT = XT_NT;
     __shared__ __align__(8) uint64_t s_bar[TC_STAGES];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_base[260];
+    __shared__ SlotTable s_tab;
     __shared__ int s_srow[NT], s_dst[NT];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2;
     const int K = DOWN ? a.I : a.H, G = K >> 6, GP = G >> 1;
     const int ntiles = DOWN ? a.H / 16 : a.I / 8;                       // tiles of 16 weight rows per expert
     const int NRT = (ntiles + 7) / 8;                                   // groups of 128 weight rows
     const int npair = a.M * a.topk;
-    const int n_active = *a.lists.n_active;
     const int nshared = a.M_shared >= 0 ? a.M_shared : a.M;
-    if (warp == 0) {                                                    // (slot, block) prefix, as in k_expert_rows
-        int run = 0;
-        for (int j0 = 0; j0 <= n_active; j0 += 32) {
-            const int j = j0 + lane;
-            int nb = 0;
-            if (j < n_active) nb = (a.lists.slot_cnt[j] + NT - 1) / NT;
-            else if (j == n_active) nb = (nshared + NT - 1) / NT;
-            int inc = nb;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) { const int o = __shfl_up_sync(0xffffffffu, inc, d); if (lane >= d) inc += o; }
-            if (j <= n_active) s_base[j] = run + inc - nb;
-            run += __shfl_sync(0xffffffffu, inc, 31);
-        }
-        if (lane == 0) s_base[n_active + 1] = run;
-    }
+    const int n_active = slot_table(s_tab, a.lists, NT, nshared);
     if (tid == 0) { for (int i = 0; i < TC_STAGES; ++i) mbar_init(&s_bar[i], 1); mbar_fence_init(); }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&s_tmem)), "r"((uint32_t)NT) : "memory");
@@ -321,24 +306,22 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_expert_umma(ExpertArgs a) {
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = s_tmem;
-    const int total = s_base[n_active + 1] * NRT;
+    const int total = s_tab.base[n_active + 1] * NRT;
     int cb = 0;                                                          // commits made so far on each stage's barrier (same in every thread)
     bool failed = false;
     for (int item = blockIdx.x; item < total && !failed; item += gridDim.x) {
         const int sb = item / NRT, rt = item - sb * NRT;
-        int lo = 0, hi = n_active;
-        while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (s_base[mid] <= sb) lo = mid; else hi = mid - 1; }
-        const int j = lo, blk = sb - s_base[j];
+        const int j = slot_of(s_tab, n_active, sb), blk = sb - s_tab.base[j];
         const bool shared = (j == n_active);
-        const int cnt = shared ? nshared : a.lists.slot_cnt[j];
-        const int e = shared ? 0 : a.lists.slot_expert[j];
+        const int cnt = shared ? nshared : s_tab.cnt[j];
+        const int e = shared ? 0 : s_tab.expert[j];
         const Q4R& q = DOWN ? (shared ? a.sh_down : a.down) : (shared ? a.sh_gu : a.gu);
         if (tid < NT) {
             const int ridx = blk * NT + tid;
             int dst = -1, srow = -1;
             if (ridx < cnt) {
                 if (shared) { dst = npair + ridx; srow = DOWN ? dst : a.shared_row0 + ridx; }
-                else { const int pr = a.lists.pairs[a.lists.slot_off[j] + ridx]; dst = pr; srow = DOWN ? pr : pr / a.topk; }
+                else { const int pr = a.lists.pairs[s_tab.off[j] + ridx]; dst = pr; srow = DOWN ? pr : pr / a.topk; }
             }
             s_srow[tid] = srow; s_dst[tid] = dst;
         }

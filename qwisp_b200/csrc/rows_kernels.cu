@@ -14,10 +14,7 @@
 //   k_gemv_rows      dense projection: a CTA of 8 warps = 8 tiles x (8*RG rows); the rows' slice of 256 inputs is staged in
 //                    shared memory (cp.async, two buffers) and shared by the warps; each warp streams its tile's slices
 //                    from global memory two slices ahead.
-//   k_expert_rows    routed + shared experts grouped by expert: persistent CTAs of 16 consumer warps + 1 producer warp.
-//                    The producer gathers the rows of the next (expert, row block) into a ring of shared-memory stages with
-//                    bulk copies (mbarrier full / empty), the consumers each own one tile over the whole K -- no CTA-wide
-//                    barrier between experts, which is what bounded the pass kernels when every expert has one or two rows.
+//   k_expert_rows    routed + shared experts grouped by expert: every warp walks tiles of its CTA's run on its own.
 //   k_moe_combine    weighted sum of a row's top-k expert rows in ascending k + shared expert + residual.
 #include "kernels.h"
 #include "gemv.cuh"
@@ -80,11 +77,12 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
 // Wait of the expert kernel's ring, bounded in TIME (~50 ms): the first wait of a CTA that runs out raises the CTA's
-// abort word, and every later wait of that CTA gives up at once, so a stall costs one timeout per CTA, not one per item.
+// abort word, and every later wait of that CTA gives up at once, so a stall costs one timeout per CTA, not one per block.
 constexpr long long XR_TIMEOUT = 100000000ll;                 // cycles
 __device__ __forceinline__ bool xr_wait(uint64_t* bar, uint32_t parity, volatile int* abort_word) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -236,210 +234,213 @@ bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st) {
 }
 
 // ================================================================================ experts
-// A work item is (expert slot, block of 8 rows, group of 16 tiles); items are numbered slot-major, tile group fastest, so
-// neighbouring CTAs read neighbouring weights and the same rows.  Slot n_active is the shared expert (all rows).
-constexpr int XR_CONS = 16;                  // consumer warps = tiles per item
-constexpr int XR_THREADS = (XR_CONS + 1) * 32;
-struct XrStage {                             // one ring stage in shared memory
-    __half* xs;                              // [8][K + 8]
-    float* sxs;                              // [8][K/64 + 4]
-    float* craw;                             // down: [8][K/8] chunk sums as written by the gate/up kernel
-    int* info;                               // [0..7] destination rows (-1: none), [8] expert, [9] shared, [10] tile group
+// Work: (expert slot, block of 8 of its rows) x tiles of 16 weight rows, block-major; slot n_active is the shared expert
+// (all rows).  A CTA per multiprocessor takes an equal, contiguous run of the tiles (one to three blocks at decode sizes)
+// and its 24 consumer warps walk that run, a tile over the whole K each.  A producer warp gathers the rows of the next block
+// into a ring of shared-memory stages with bulk copies (mbarrier full / empty): no CTA-wide barrier between experts, which
+// is what bounded the pass kernels when every expert has one or two rows.
+// Bound: instruction issue first (the 4-bit expansion is about 150 of the 260 instructions that a slice of 16 x 256 weights
+// needs), the weight stream second.  So: as many warps as the registers allow (six per sub-partition; four left 40 % of
+// the issue slots empty), whole runs instead of items of 16 tiles (seven rounds for the work of 6.2), and a slice's weights
+// by 16-byte asynchronous copies two slices ahead (110 KB per SM in flight; bulk copies of 2 KB arrive later; rows
+// straight from L1 instead of staged: eight lines per load, 89 us for gate/up).  Batch of 64 (event times, 4.5 us of
+// them the events'): gate/up 73.6 -> 67.7 us, down 53.4 -> 43.3; 7 rows: 27.0 -> 23.0, 18.9 -> 18.8.
+constexpr int XR_WARPS = 24;
+constexpr int XR_DEPTH = 2;                   // slices in a warp's ring
+constexpr int XR_UNIT = 2048 + 256;           // bytes of a slice of a tile: nibbles, then scales and biases
+constexpr int XR_BLOCKS = 64;                 // most (slot, block) entries of a CTA's run
+constexpr int XR_THREADS = (XR_WARPS + 1) * 32;
+struct XrBlock { int expert; int src[8], dst[8]; };   // expert -1: the shared one; src, dst -1: no row
+struct XrStage {                              // the rows of a block in shared memory
+    __half* xs;                               // [8][K + 8]
+    float* sxs;                               // [8][K/64 + 4]
+    float* craw;                              // down: [8][K/8] chunk sums as written by the gate/up kernel
 };
 template <bool DOWN>
-__host__ __device__ inline size_t xr_stage_bytes(int K) {
-    size_t b = (size_t)8 * (K + 8) * 2 + (size_t)8 * (K / 64 + 4) * 4 + 16 * 4;
-    if (DOWN) b += (size_t)8 * (K / 8) * 4;
-    return (b + 15) & ~(size_t)15;
-}
-template <bool DOWN>
+__host__ __device__ constexpr size_t xr_stage_bytes(int K) { return (size_t)8 * (K + 8) * 2 + (size_t)8 * (K / 64 + 4) * 4 + (DOWN ? (size_t)8 * (K / 8) * 4 : 0); }
 __device__ __forceinline__ XrStage xr_carve(unsigned char* base, int K) {
     XrStage s;
     s.xs = reinterpret_cast<__half*>(base); base += (size_t)8 * (K + 8) * 2;
     s.sxs = reinterpret_cast<float*>(base); base += (size_t)8 * (K / 64 + 4) * 4;
-    s.craw = reinterpret_cast<float*>(base); if (DOWN) base += (size_t)8 * (K / 8) * 4;
-    s.info = reinterpret_cast<int*>(base);
+    s.craw = reinterpret_cast<float*>(base);
     return s;
 }
-// grid: one CTA per multiprocessor; dynamic shared memory: nstages stages
-template <bool DOWN>
-__global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int nstages) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int s_base[260];                                  // first (slot, block) index of every slot; [n_active + 1] = total
+// S: slices of K
+template <bool DOWN, int S>
+__global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int lg_tiles, int nstages) {
+    extern __shared__ __align__(16) unsigned char smem[];        // weight rings, then nstages stages
     __shared__ __align__(8) uint64_t s_full[8], s_empty[8], s_raw[8];
-    __shared__ int s_sig; __shared__ int s_abort;
+    __shared__ SlotTable s_tab;
+    __shared__ XrBlock s_blk[XR_BLOCKS];
+    __shared__ int s_sig, s_abort;
+    constexpr int K = S << 8, G64 = K >> 6, SXS = G64 + 4, XS = K + 8;
+    constexpr size_t stage_bytes = xr_stage_bytes<DOWN>(K);
+    unsigned char* stages = smem + (size_t)XR_WARPS * XR_DEPTH * XR_UNIT;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, t = lane & 3;
-    const int K = DOWN ? a.I : a.H;
-    const int slices = K >> 8, G64 = K >> 6, SXS = G64 + 4, XS = K + 8;
-    const int ntiles = DOWN ? a.H / 16 : a.I / 8;
-    const int NTG = (ntiles + XR_CONS - 1) / XR_CONS;
-    const int npair = a.M * a.topk;
-    const int n_active = *a.lists.n_active;
+    const int ntiles = 1 << lg_tiles, npair = a.M * a.topk;
     const int nshared = a.M_shared >= 0 ? a.M_shared : a.M;
-    const size_t stage_bytes = xr_stage_bytes<DOWN>(K);
-    // ---- (slot, block) prefix: warp 0 scans the slot counts in chunks of 32
-    if (warp == 0) {
-        int run = 0;
-        for (int j0 = 0; j0 <= n_active; j0 += 32) {
-            const int j = j0 + lane;
-            int nb = 0;
-            if (j < n_active) nb = (a.lists.slot_cnt[j] + 7) >> 3;
-            else if (j == n_active) nb = (nshared + 7) >> 3;
-            int inc = nb;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) { const int o = __shfl_up_sync(0xffffffffu, inc, d); if (lane >= d) inc += o; }
-            if (j <= n_active) s_base[j] = run + inc - nb;
-            run += __shfl_sync(0xffffffffu, inc, 31);
-        }
-        if (lane == 0) s_base[n_active + 1] = run;
-    }
     if (tid == 0) {
         s_abort = 0;
-        for (int i = 0; i < nstages; ++i) { mbar_init(&s_full[i], DOWN ? 1 : 8); mbar_init(&s_empty[i], XR_CONS); mbar_init(&s_raw[i], 8); }
+        for (int i = 0; i < nstages; ++i) { mbar_init(&s_full[i], DOWN ? 1 : 8); mbar_init(&s_empty[i], XR_WARPS); mbar_init(&s_raw[i], 8); }
         mbar_fence_init();
     }
+    const int n_active = slot_table(s_tab, a.lists, 8, nshared);
     __syncthreads();
-    const int total = s_base[n_active + 1] * NTG;
-    // (slot, block) index -> slot: the last j with s_base[j] <= sb
-    auto slot_of = [&](int sb) {
-        int lo = 0, hi = n_active;
-        while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (s_base[mid] <= sb) lo = mid; else hi = mid - 1; }
-        return lo;
-    };
-    bool failed = false;
+    const long total = (long)s_tab.base[n_active + 1] << lg_tiles;
+    const int lo = (int)(total * blockIdx.x / gridDim.x), hi = (int)(total * (blockIdx.x + 1) / gridDim.x);
+    const int b0 = lo >> lg_tiles, nb = hi > lo ? ((hi - 1) >> lg_tiles) - b0 + 1 : 0;
+    for (int i = tid; i < nb * 8; i += XR_THREADS) {           // the rows of the run's blocks
+        const int sb = b0 + (i >> 3), j = slot_of(s_tab, n_active, sb), first = (sb - s_tab.base[j]) * 8, ridx = first + (i & 7);
+        const bool shared = (j == n_active);
+        const bool have = ridx < (shared ? nshared : s_tab.cnt[j]);
+        int dst = -1, src = -1;
+        if (have && shared) { dst = npair + ridx; src = DOWN ? dst : a.shared_row0 + ridx; }
+        else if (have) { dst = a.lists.pairs[s_tab.off[j] + ridx]; src = DOWN ? dst : dst / a.topk; }
+        XrBlock& b = s_blk[i >> 3];
+        b.src[i & 7] = src; b.dst[i & 7] = dst;
+        if ((i & 7) == 0) b.expert = shared ? -1 : s_tab.expert[j];
+    }
+    __syncthreads();
     unsigned fail_code = 0;          // which wait ran out: 16 producer/empty, 32 producer/chunk sums, 64 consumer/full
-    if (warp == XR_CONS) {
-        // ------------------------------------------------------------ producer
-        int k = 0;
-        for (int item = blockIdx.x; item < total; item += gridDim.x, ++k) {
+    if (warp == XR_WARPS) {
+        // ------------------------------------------------------------ producer: the rows of the run's blocks, stage after stage
+        for (int k = 0; k < nb; ++k) {
             const int stg = k % nstages, use = k / nstages;
-            const XrStage S = xr_carve<DOWN>(smem + (size_t)stg * stage_bytes, K);
-            if (use > 0 && !xr_wait(&s_empty[stg], (uint32_t)((use - 1) & 1), &s_abort)) { failed = true; fail_code |= 16u; break; }
-            const int sb = item / NTG, tg = item - sb * NTG;
-            const int j = slot_of(sb), blk = sb - s_base[j];
-            const bool shared = (j == n_active);
-            const int cnt = shared ? nshared : a.lists.slot_cnt[j];
+            const XrStage St = xr_carve(stages + (size_t)stg * stage_bytes, K);
+            if (use > 0 && !xr_wait(&s_empty[stg], (uint32_t)((use - 1) & 1), &s_abort)) { fail_code |= 16u; break; }
             if (lane < 8) {
-                const int ridx = blk * 8 + lane;
-                int dst = -1, srow = 0;
-                if (ridx < cnt) {
-                    if (shared) { dst = npair + ridx; srow = DOWN ? dst : a.shared_row0 + ridx; }
-                    else { const int pr = a.lists.pairs[a.lists.slot_off[j] + ridx]; dst = pr; srow = DOWN ? pr : pr / a.topk; }
-                }
-                S.info[lane] = dst;
-                if (lane == 0) { S.info[8] = shared ? 0 : a.lists.slot_expert[j]; S.info[9] = shared ? 1 : 0; S.info[10] = tg; }
                 uint64_t* bar = DOWN ? &s_raw[stg] : &s_full[stg];
-                if (dst >= 0) {
-                    const __half* xsrc = (DOWN ? a.hbuf : a.xq) + (size_t)srow * K;
-                    if (DOWN) {
-                        mbar_expect_tx(bar, (uint32_t)(K * 2 + (K / 8) * 4));
-                        bulk_g2s(S.xs + (size_t)lane * XS, xsrc, (uint32_t)K * 2, bar);
-                        bulk_g2s(S.craw + (size_t)lane * (K / 8), a.csum + (size_t)srow * (K / 8), (uint32_t)(K / 8) * 4, bar);
-                    } else {
-                        mbar_expect_tx(bar, (uint32_t)(K * 2 + G64 * 4));
-                        bulk_g2s(S.xs + (size_t)lane * XS, xsrc, (uint32_t)K * 2, bar);
-                        bulk_g2s(S.sxs + (size_t)lane * SXS, a.sxq + (size_t)srow * G64, (uint32_t)G64 * 4, bar);
-                    }
-                } else {
-                    mbar_arrive(bar);
-                }
+                const int src = s_blk[k].src[lane];
+                if (src >= 0) {
+                    const __half* xsrc = (DOWN ? a.hbuf : a.xq) + (size_t)src * K;
+                    constexpr uint32_t sums = (DOWN ? K / 8 : G64) * 4;
+                    mbar_expect_tx(bar, (uint32_t)(K * 2) + sums);
+                    bulk_g2s(St.xs + (size_t)lane * XS, xsrc, (uint32_t)K * 2, bar);
+                    if (DOWN) bulk_g2s(St.craw + (size_t)lane * (K / 8), a.csum + (size_t)src * (K / 8), sums, bar);
+                    else bulk_g2s(St.sxs + (size_t)lane * SXS, a.sxq + (size_t)src * G64, sums, bar);
+                } else mbar_arrive(bar);                              // (a column without a row keeps what was there: nobody reads its result)
             }
             if (DOWN) {
-                // group sums from the chunk sums: eight chunk sums combined in the butterfly order of rows_store()
-                if (!xr_wait(&s_raw[stg], (uint32_t)(use & 1), &s_abort)) { failed = true; fail_code |= 32u; break; }
+                // group sums from the chunk sums: eight of them combined in the butterfly order of rows_store()
+                if (!xr_wait(&s_raw[stg], (uint32_t)(use & 1), &s_abort)) { fail_code |= 32u; break; }
                 for (int i = lane; i < 8 * G64; i += 32) {
                     const int row = i / G64, g = i - row * G64;
-                    const float* c = S.craw + (size_t)row * (K / 8) + g * 8;
-                    const float4 lo = *reinterpret_cast<const float4*>(c), hi = *reinterpret_cast<const float4*>(c + 4);
-                    const float e = __fadd_rn(__fadd_rn(lo.x, hi.x), __fadd_rn(lo.z, hi.z));       // (s0 + s4) + (s2 + s6)
-                    const float o = __fadd_rn(__fadd_rn(lo.y, hi.y), __fadd_rn(lo.w, hi.w));       // (s1 + s5) + (s3 + s7)
-                    S.sxs[(size_t)row * SXS + g] = __fadd_rn(e, o);
+                    const float* c = St.craw + (size_t)row * (K / 8) + g * 8;
+                    const float4 lo4 = *reinterpret_cast<const float4*>(c), hi4 = *reinterpret_cast<const float4*>(c + 4);
+                    const float e = __fadd_rn(__fadd_rn(lo4.x, hi4.x), __fadd_rn(lo4.z, hi4.z));       // (s0 + s4) + (s2 + s6)
+                    const float o = __fadd_rn(__fadd_rn(lo4.y, hi4.y), __fadd_rn(lo4.w, hi4.w));       // (s1 + s5) + (s3 + s7)
+                    St.sxs[(size_t)row * SXS + g] = __fadd_rn(e, o);
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&s_full[stg]);
             }
         }
     } else {
-        // ------------------------------------------------------------ consumers: warp = one tile of the item's group
-        const Q4R& qr = DOWN ? a.down : a.gu;
-        const Q4R& qs = DOWN ? a.sh_down : a.sh_gu;
-        const size_t wstep = q4r_w_uint4(K), sstep = q4r_s_uint4(K);
-        auto tile_ptrs = [&](int item, const uint4*& wt, const uint4*& stl, bool& valid) {
-            const int sb = item / NTG, tg = item - sb * NTG;
-            const int j = slot_of(sb);
-            const bool shared = (j == n_active);
-            const int tile = tg * XR_CONS + warp;
-            valid = tile < ntiles;
-            const Q4R& q = shared ? qs : qr;
-            const size_t T = (size_t)(shared ? 0 : a.lists.slot_expert[j]) * ntiles + (valid ? tile : 0);
-            wt = q.wr + T * wstep; stl = q.sr + T * sstep;
-        };
-        SliceRegs cur, nxt;
-        const uint4 *wt = nullptr, *stl = nullptr, *wt_n = nullptr, *stl_n = nullptr;
-        bool valid = false, valid_n = false;
-        if ((int)blockIdx.x < total) { tile_ptrs(blockIdx.x, wt, stl, valid); if (valid) load_slice(cur, wt, stl, 0, lane); }
-        int k = 0;
-        for (int item = blockIdx.x; item < total; item += gridDim.x, ++k) {
-            const int stg = k % nstages, use = k / nstages;
-            const XrStage S = xr_carve<DOWN>(smem + (size_t)stg * stage_bytes, K);
-            const int item_n = item + gridDim.x;
-            if (item_n < total) tile_ptrs(item_n, wt_n, stl_n, valid_n); else valid_n = false;
-            if (!xr_wait(&s_full[stg], (uint32_t)(use & 1), &s_abort)) { failed = true; fail_code |= 64u; break; }
-            float tot[1][4] = {{0.f, 0.f, 0.f, 0.f}};
+    // ---------------------------------------------------------------- consumers
+    unsigned char* ring = smem + (size_t)warp * XR_DEPTH * XR_UNIT;
+    const size_t wstep = q4r_w_uint4(K), sstep = q4r_s_uint4(K);
+    // nibbles and scales of tile task `i` (nullptr past the run's end)
+    auto tile_of = [&](int i, const uint4*& w, const uint4*& sc) {
+        w = nullptr; sc = nullptr;
+        if (i >= hi) return;
+        const int e = s_blk[(i >> lg_tiles) - b0].expert;
+        const Q4R& q = DOWN ? (e < 0 ? a.sh_down : a.down) : (e < 0 ? a.sh_gu : a.gu);
+        const size_t T = ((size_t)max(e, 0) << lg_tiles) + (i & (ntiles - 1));
+        w = q.wr + T * wstep; sc = q.sr + T * sstep;
+    };
+    auto request = [&](int slot, const uint4* w, const uint4* sc, int s) {      // slice s of a tile into a ring slot: one copy group
+        if (w) {
+            uint4* d = reinterpret_cast<uint4*>(ring + slot * XR_UNIT);
+            const uint4* p = w + s * 128 + lane;
+            cp_async16(d + lane, p); cp_async16(d + lane + 32, p + 32); cp_async16(d + lane + 64, p + 64); cp_async16(d + lane + 96, p + 96);
+            if (lane < 16) cp_async16(d + 128 + lane, sc + s * 16 + lane);
+        }
+        cp_async_commit();
+    };
+    constexpr int NB = XR_DEPTH > S ? XR_DEPTH / S : 1;           // tiles the ring holds at least the start of
+    const uint4 *w0, *c0, *wn, *cn;                               // this tile, and the one whose slices are requested ahead
+    tile_of(lo + warp, w0, c0);
+    if (S >= XR_DEPTH) { request(0, w0, c0, 0); request(1, w0, c0, 1); }
+    else { request(0, w0, c0, 0); tile_of(lo + warp + XR_WARPS, wn, cn); request(1, wn, cn, 0); }
+    int odd = 0, cur = 0;                                         // cur: the block whose stage this warp holds
+    bool here = false;                                            // its rows have arrived
 #pragma unroll 1
-            for (int s = 0; s < slices; ++s) {
-                if (s + 1 < slices) { if (valid) load_slice(nxt, wt, stl, s + 1, lane); }
-                else if (valid_n) load_slice(nxt, wt_n, stl_n, 0, lane);
-                if (valid) {
-                    float accS[1][4] = {{0.f, 0.f, 0.f, 0.f}}, accB[1][4] = {{0.f, 0.f, 0.f, 0.f}};
-                    compute_rows<1>(cur, S.xs + s * 256, XS, S.sxs + s * 4, SXS, r, t, accS, accB);
-                    add_slice<1>(tot, accS, accB);
-                }
-                cur = nxt;
-            }
-            if (valid) {
-                const int tile = S.info[10] * XR_CONS + warp;
-                if (DOWN) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int dst = S.info[2 * t + (i & 1)];
-                        if (dst >= 0) {
-                            __half* rowp = a.dbuf + (size_t)dst * a.H;
-                            if (a.ep_pairs_per_rank > 0 && dst < npair) {       // routed pair in expert-parallel mode: the owner's buffer
-                                const int own = dst / a.ep_pairs_per_rank;
-                                rowp = a.peer_dbuf[own] + (size_t)(dst - own * a.ep_pairs_per_rank) * a.H;
-                            }
-                            rowp[tile * 16 + r + 8 * (i >> 1)] = f2h(tot[0][i]);
-                        }
-                    }
-                } else {
-                    // SwiGLU of (gate row r, up row r) per column; the 8 outputs of a column (lanes with the same t) form one
-                    // 8-chunk of the down projection's input: stored in the paired order with its chunk sum
-#pragma unroll
-                    for (int jc = 0; jc < 2; ++jc) {
-                        const __half hv = swiglu_h(f2h(tot[0][jc]), f2h(tot[0][2 + jc]));
-                        const unsigned hb = __half_as_ushort(hv);
-                        unsigned v[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) v[i] = __shfl_sync(0xffffffffu, hb, i * 4 + t);
-                        const int dst = S.info[2 * t + jc];
-                        if (r == 0 && dst >= 0) {
-                            const uint4 nat = make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
-                            const uint4 prd = make_uint4(v[0] | (v[4] << 16), v[1] | (v[5] << 16), v[2] | (v[6] << 16), v[3] | (v[7] << 16));
-                            *reinterpret_cast<uint4*>(a.hbuf + (size_t)dst * a.I + tile * 8) = prd;
-                            a.csum[(size_t)dst * (a.I / 8) + tile] = sum8_f32(nat);
-                        }
-                    }
-                }
-            }
+    for (int i = lo + warp; i < hi; i += XR_WARPS) {
+        tile_of(i + NB * XR_WARPS, wn, cn);
+        const int bi = (i >> lg_tiles) - b0, tile = i & (ntiles - 1);
+        const XrBlock& b = s_blk[bi];
+        if (bi != cur) {                                          // done with the stages of the blocks before
             __syncwarp();
-            if (lane == 0) mbar_arrive(&s_empty[stg]);
-            wt = wt_n; stl = stl_n; valid = valid_n;
+            if (lane == 0) for (int u = cur; u < bi; ++u) mbar_arrive(&s_empty[u % nstages]);
+            cur = bi; here = false;
+        }
+        if (!here && !xr_wait(&s_full[bi % nstages], (uint32_t)((bi / nstages) & 1), &s_abort)) { fail_code |= 64u; break; }
+        here = true;
+        const XrStage St = xr_carve(stages + (size_t)(bi % nstages) * stage_bytes, K);
+        const __half* xp = St.xs + (size_t)r * XS + 16 * t;
+        const float *sx0 = St.sxs + 2 * t * SXS, *sx1 = sx0 + SXS;
+        float tot[1][4] = {{0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const int slot = S >= XR_DEPTH ? s % XR_DEPTH : odd;
+            XRegs xr;
+            const float4 sa = *reinterpret_cast<const float4*>(sx0 + s * 4), sb = *reinterpret_cast<const float4*>(sx1 + s * 4);
+            xr.sx[0] = make_float2(sa.x, sb.x); xr.sx[1] = make_float2(sa.y, sb.y); xr.sx[2] = make_float2(sa.z, sb.z); xr.sx[3] = make_float2(sa.w, sb.w);
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                xr.x[2 * g] = *reinterpret_cast<const uint4*>(xp + s * 256 + 64 * g);
+                xr.x[2 * g + 1] = *reinterpret_cast<const uint4*>(xp + s * 256 + 64 * g + 8);
+            }
+            cp_async_wait<XR_DEPTH - 1>();
+            __syncwarp();                                         // every lane's part of the slice is there
+            SliceRegs rg;
+            load_slice_smem(rg, reinterpret_cast<const uint4*>(ring + slot * XR_UNIT), reinterpret_cast<const uint4*>(ring + slot * XR_UNIT + 2048), lane);
+            float accS[1][4] = {{0.f, 0.f, 0.f, 0.f}}, accB[1][4] = {{0.f, 0.f, 0.f, 0.f}};
+            compute_slice_x(rg, xr, accS[0], accB[0]);
+            add_slice<1>(tot, accS, accB);
+            __syncwarp();                                         // every lane has read the slot: it may be filled again
+            if (S > XR_DEPTH && s + XR_DEPTH < S) request(slot, w0, c0, s + XR_DEPTH);
+            else request(slot, wn, cn, S > XR_DEPTH ? s + XR_DEPTH - S : s);
+        }
+        w0 = wn; c0 = cn; odd ^= 1;
+        if (DOWN) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int dst = b.dst[2 * t + (u & 1)];
+                if (dst >= 0) {
+                    __half* rowp = a.dbuf + (size_t)dst * a.H;
+                    if (a.ep_pairs_per_rank > 0 && dst < npair) {       // routed pair in expert-parallel mode: the owner's buffer
+                        const int own = dst / a.ep_pairs_per_rank;
+                        rowp = a.peer_dbuf[own] + (size_t)(dst - own * a.ep_pairs_per_rank) * a.H;
+                    }
+                    rowp[tile * 16 + r + 8 * (u >> 1)] = f2h(tot[0][u]);
+                }
+            }
+        } else {
+            // SwiGLU of (gate row r, up row r) per column; the 8 outputs of a column (lanes with the same t) form one
+            // 8-chunk of the down projection's input: stored in the paired order with its chunk sum
+#pragma unroll
+            for (int jc = 0; jc < 2; ++jc) {
+                const __half hv = swiglu_h(f2h(tot[0][jc]), f2h(tot[0][2 + jc]));
+                const unsigned hb = __half_as_ushort(hv);
+                unsigned v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] = __shfl_sync(0xffffffffu, hb, u * 4 + t);
+                const int dst = b.dst[2 * t + jc];
+                if (r == 0 && dst >= 0) {
+                    const uint4 nat = make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
+                    const uint4 prd = make_uint4(v[0] | (v[4] << 16), v[1] | (v[5] << 16), v[2] | (v[6] << 16), v[3] | (v[7] << 16));
+                    *reinterpret_cast<uint4*>(a.hbuf + (size_t)dst * a.I + tile * 8) = prd;
+                    a.csum[(size_t)dst * (a.I / 8) + tile] = sum8_f32(nat);
+                }
+            }
         }
     }
-    if (failed && a.err && lane == 0) atomicOr(a.err, fail_code | (DOWN ? 8u : 4u));
-    __syncthreads();
-    if (s_abort) {                             // bulk copies this CTA started may still be landing in its shared memory: outlast them
+    __syncwarp();
+    if (lane == 0) for (int u = cur; u < nb; ++u) mbar_arrive(&s_empty[u % nstages]);      // (also of blocks in which this warp had no tile)
+    }
+    if (fail_code && a.err && lane == 0) atomicOr(a.err, fail_code | (DOWN ? 8u : 4u));
+    if (fail_code) {                           // bulk copies this CTA started may still be landing in its shared memory: outlast them
         const long long t0 = clock64();
         while (clock64() - t0 < 200000ll) { }
     }
@@ -458,23 +459,35 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
             st_release_sys(a.ep_sig.flags[tid] + 8 + a.ep_sig.rank, ep_seq(a.ep_sig.ctr, a.ep_sig.layer, 1));
     }
 }
-template <bool DOWN>
+template <bool DOWN, int S>
 static bool launch_expert_rows_t(const ExpertArgs& a, cudaStream_t st) {
-    const int K = DOWN ? a.I : a.H;
-    if (K % 256 || K > 4096 || !a.csum || (!DOWN && (!a.xq || !a.sxq))) return false;
-    const size_t sb = xr_stage_bytes<DOWN>(K);
-    int nstages = (int)((size_t)(190 * 1024) / sb);
+    const int ntiles = DOWN ? a.H / 16 : a.I / 8, grid = sm_count();
+    int lg = 0; while ((1 << lg) < ntiles) ++lg;
+    const long pairs = (long)a.M * a.topk, blocks = pairs / 8 + (pairs < 256 ? pairs : 256) + a.M / 8 + 1;    // at most one partial block per expert
+    const size_t ring = (size_t)XR_WARPS * XR_DEPTH * XR_UNIT, sb = xr_stage_bytes<DOWN>(S << 8);
+    int nstages = (int)(((size_t)216 * 1024 - ring) / sb);
     if (nstages > 8) nstages = 8;
-    if (nstages < 2) return false;
-    const size_t smem = sb * nstages;
+    if ((1 << lg) != ntiles || blocks / grid + 2 > XR_BLOCKS || nstages < 1) return false;
+    const size_t smem = ring + sb * nstages;
     static bool configured = false;
-    if (!configured) { cudaFuncSetAttribute(k_expert_rows<DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); configured = true; }
-    const int grid = sm_count();
-    profile_launch(DOWN ? "k_expert_rows_down" : "k_expert_rows_gateup", st, [&] { k_expert_rows<DOWN><<<grid, XR_THREADS, smem, st>>>(a, nstages); return 0; });
+    if (!configured) { cudaFuncSetAttribute(k_expert_rows<DOWN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
+    profile_launch(DOWN ? "k_expert_rows_down" : "k_expert_rows_gateup", st, [&] { k_expert_rows<DOWN, S><<<grid, XR_THREADS, smem, st>>>(a, lg, nstages); return 0; });
     return true;
 }
-bool launch_expert_rows_gateup(const ExpertArgs& a, cudaStream_t st) { return launch_expert_rows_t<false>(a, st); }
-bool launch_expert_rows_down(const ExpertArgs& a, cudaStream_t st) { return launch_expert_rows_t<true>(a, st); }
+template <bool DOWN>
+static bool launch_expert_rows_d(const ExpertArgs& a, cudaStream_t st) {
+    if (!a.csum || (!DOWN && (!a.xq || !a.sxq))) return false;
+    switch (DOWN ? a.I : a.H) {
+        case 256: return launch_expert_rows_t<DOWN, 1>(a, st);
+        case 512: return launch_expert_rows_t<DOWN, 2>(a, st);
+        case 1024: return launch_expert_rows_t<DOWN, 4>(a, st);
+        case 2048: return launch_expert_rows_t<DOWN, 8>(a, st);
+        case 4096: return launch_expert_rows_t<DOWN, 16>(a, st);
+        default: return false;
+    }
+}
+bool launch_expert_rows_gateup(const ExpertArgs& a, cudaStream_t st) { return launch_expert_rows_d<false>(a, st); }
+bool launch_expert_rows_down(const ExpertArgs& a, cudaStream_t st) { return launch_expert_rows_d<true>(a, st); }
 
 // ================================================================================ router for many rows
 // k_router_rows   logits of all rows: a CTA keeps 8 router rows (or the shared gate) in registers and walks the row

@@ -1,6 +1,6 @@
 // gemm_tc.cu -- 4-bit group-64 GEMM for many activation rows ("F2": prompt chunks in prefill mode) on the 5th-generation
-// tensor cores: tcgen05.mma (kind::f16) issued by one thread, operands in shared memory described by matrix
-// descriptors, the accumulator in tensor memory (TMEM), read back once with tcgen05.ld.
+// tensor cores: tcgen05.mma (kind::f16) issued by one thread, the expanded weights and the accumulator in tensor memory
+// (TMEM), the activations in shared memory.
 //
 //   y[t, n] (+)= sum_k x[t, k] * fp16(scale[n, k/64] * q[n, k] + bias[n, k/64])
 //
@@ -10,180 +10,132 @@
 // this is not bit-identical to the GEMV family, but every token column is independent of the others and K is walked in
 // a fixed order, so results do not depend on how many rows share a call or on how a prompt is cut into calls.
 //
-// A CTA of 256 threads owns 128 weight rows (8 tiles of the fragment-major layout, one per warp) and NT activation rows.
-// Four shared-memory stages rotate over the K groups of 64 inputs; per group
-//   B  the NT x 64 activations go global -> shared memory by cp.async (16-byte pieces, no registers), issued TWO groups
-//      ahead into the stage whose MMAs of four groups ago have completed;
-//   A  each warp dequantises its tile's fragment register (16 nibbles of two weight rows; scale and bias applied with one
-//      fp16x2 multiply-add per pair; halves put back in natural order) into the stage -- the register was loaded two
-//      groups ahead;
-//   two groups share one cp.async.wait_group + fence.proxy.async + barrier, after which one thread issues eight MMAs
-//   (M=128, N=NT, K=16) that accumulate into the NT TMEM columns and commits them to a stage mbarrier.
-// Operand tiles are K-major with the 128-byte swizzle (an unswizzled layout ran the same MMAs several times slower).
+// One kernel, k_tc, serves the dense projections (DenseWork) and the grouped experts (ExpertWork): persistent CTAs, one
+// per multiprocessor, walk a run of items of 128 weight rows x NT activation rows over the whole K, 128 inputs a stage.
+// The warps have roles and meet only at mbarriers:
+//   mma        1 warp: waits for a full stage, issues its eight MMAs (M=128, N=NT, K=16), commits them to the stage's
+//             "empty" barrier.  It is warp 0: the other warps keep the issue slots busy;
+//   load       4 warps: the NT x 128 activations of the stage, 16-byte asynchronous copies that count themselves in at
+//             the stage's "full" barrier;
+//   dequant   16 warps: a warp owns one 16-row tile of the item and every second stage; its fragments are loaded two of
+//             its stages ahead (across items), turned into MMA order by two shuffles per word pair, expanded to fp16 (scale
+//             and bias by one fp16x2 multiply-add per pair) and stored to the A operand in TMEM;
+//   epilogue   4 warps: read the finished accumulator while the next item accumulates in the other half of its TMEM.
+// The first form (256 threads that all loaded, expanded, synchronised and waited in turn, one pair of groups ahead)
+// spent 2.5 us on a pair of groups whose MMAs take 0.3: every pair paid the latency of its weights and of its rows.
+// With roles but the A operand in shared memory, writing and reading it took most of that memory's bandwidth.
 #include "kernels.h"
 #include "gemv.cuh"
 
 namespace sl {
 
-constexpr int TC_ROWS = 128;      // weight rows per CTA (UMMA M)
+constexpr int TC_ROWS = 128;      // weight rows per item (UMMA M)
+constexpr int TC_LD = 4, TC_EPI = 4, TC_DQ = 16;                            // warps of each role (+ 1 for the MMAs)
+constexpr int TC_EPI0 = 4, TC_DQ0 = 8;                                      // first warp of the role (load: 1, 2, 3 and the last)
+constexpr int TC_THREADS = (1 + TC_LD + TC_EPI + TC_DQ) * 32;
 
-// Operand tiles in shared memory: K-major, 128-byte swizzle.  A row holds the 64 halves of one K group (128 bytes); 8 rows
-// form a 1024-byte atom inside which the 16-byte chunk index is XORed with the row index (conflict-free for the threads
-// that fill it and for the tensor core that reads it); atoms of further rows follow at 1024-byte steps.  Tiles start on
-// 1024-byte boundaries.
-__device__ __forceinline__ unsigned char* tc_at(unsigned char* tile, int row, int chunk) {
-    return tile + ((size_t)(row >> 3) << 10) + ((row & 7) << 7) + (((chunk ^ row) & 7) << 4);
-}
+// Activation tiles in shared memory: K-major, 128-byte swizzle.  A row holds 64 halves (128 bytes); 8 rows form a 1024-byte
+// atom inside which the 16-byte chunk index is XORed with the row index (conflict-free for the threads that fill it and for
+// the tensor core that reads it; an unswizzled layout ran the same MMAs several times slower); atoms of further rows follow
+// at 1024-byte steps.  Tiles start on 1024-byte boundaries.
+__device__ __forceinline__ uint32_t tc_off(int row, int chunk) { return ((uint32_t)(row >> 3) << 10) + ((row & 7) << 7) + (((chunk ^ row) & 7) << 4); }
 __device__ __forceinline__ uint64_t umma_desc_sw128(const void* smem_ptr) {
     // shared-memory matrix descriptor: start address; leading byte offset 1 (unused by swizzled K-major layouts); stride
     // byte offset 1024 (between 8-row atoms); all without their 4 low bits; descriptor version 1; layout type 2 = 128-byte swizzle
     const uint64_t addr = (uint64_t)(smem_u32(smem_ptr) >> 4) & 0x3FFFull;
     return addr | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+// D (TMEM) (+)= A (TMEM, 8 columns = 16 halves of K per lane) * B (shared memory)
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        :: "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        :: "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t r[32]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t r[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr) : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+// 16 lanes x 32 columns.  Registers 4c .. 4c+3 of lane 4r + t: (row r, columns 8c + 2t, + 1), (row r + 8, the same columns)
+__device__ __forceinline__ void tmem_st16x256(uint32_t taddr, const uint32_t v[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 :: "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+                    "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void tc_arrive(uint64_t* b) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory"); }
 
-// Short wait on a stage barrier: non-blocking polls (the MMAs it waits for take a few hundred nanoseconds; a blocking
-// try_wait may park the warp for longer than that), bounded like every wait.
-__device__ __forceinline__ bool tc_wait(uint64_t* b, uint32_t parity) {
-    for (int i = 0; i < (1 << 24); ++i) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(smem_u32(b)), "r"(parity) : "memory");
-        if (ok) return true;
+// Bounded wait of a role.  The first that runs out (seconds) raises the CTA's abort word; every later wait of the CTA then
+// gives up at once, so the roles leave their loops one after another.
+__device__ __forceinline__ bool tc_wait(uint64_t* b, uint32_t parity, volatile int* abort_word) {
+    if (mbar_try_wait(b, parity)) return true;
+    for (int i = 0; i < (1 << 22); ++i) {
+        if (mbar_try_wait(b, parity)) return true;
+        if ((i & 255) == 255 && *abort_word) return false;
     }
+    *abort_word = 1;
     return false;
 }
-// ---- pieces of a K group shared by the dense and the grouped-expert kernels ----
-constexpr int TC_STAGES = 4;
-constexpr int TC_THREADS = 256;
-// fragment register of one 16-row tile (wv: nibbles of rows A_r / B_r, sv: their scales and biases for the pair of groups)
-// -> fp16 weights, natural order, in the A stage
-__device__ __forceinline__ void tc_dequant_A(unsigned char* sA, int tl, int r, int t, int g, uint4 wv, uint4 sv, bool valid) {
-    uint4 o[4] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-    if (valid) {
-        const uint32_t sa = (g & 1) ? sv.z : sv.x, sb = (g & 1) ? sv.w : sv.y;         // (scale, bias) of rows A_r and B_r
-        const __half2 hA = *reinterpret_cast<const __half2*>(&sa), hB = *reinterpret_cast<const __half2*>(&sb);
-        const __half2 sA2 = __half2half2(__low2half(hA)), bA2 = __half2half2(__high2half(hA));
-        const __half2 sB2 = __half2half2(__low2half(hB)), bB2 = __half2half2(__high2half(hB));
-        const uint32_t words[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-        for (int wi = 0; wi < 4; ++wi) {
-            uint32_t d[4], w[4];
-            dequant8(words[wi], d);                                    // (q0,q4) (q1,q5) (q2,q6) (q3,q7)
-            const __half2 sc = (wi < 2) ? sA2 : sB2, bi = (wi < 2) ? bA2 : bB2;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const __half2 wq = __hfma2(*reinterpret_cast<const __half2*>(&d[j]), sc, bi);
-                w[j] = *reinterpret_cast<const uint32_t*>(&wq);
-            }
-            o[wi].x = __byte_perm(w[0], w[1], 0x5410);                 // (w0, w1)
-            o[wi].y = __byte_perm(w[2], w[3], 0x5410);                 // (w2, w3)
-            o[wi].z = __byte_perm(w[0], w[1], 0x7632);                 // (w4, w5)
-            o[wi].w = __byte_perm(w[2], w[3], 0x7632);                 // (w6, w7)
-        }
-    }
-    const int rowA = tl * 16 + r;                                     // row A_r of the tile; B_r is 8 rows further (the next atom)
-    *reinterpret_cast<uint4*>(tc_at(sA, rowA, 2 * t)) = o[0];
-    *reinterpret_cast<uint4*>(tc_at(sA, rowA, 2 * t + 1)) = o[1];
-    *reinterpret_cast<uint4*>(tc_at(sA, rowA + 8, 2 * t)) = o[2];
-    *reinterpret_cast<uint4*>(tc_at(sA, rowA + 8, 2 * t + 1)) = o[3];
+
+// ---- one K group (64 inputs) of a 16-row tile: fragment register -> A operand
+// Lane 4r + t holds inputs 16t .. 16t + 15 of rows A_r and B_r = r + 8 (two words each); the MMA wants inputs 16c .. 16c + 15
+// in column block c, of which this lane stores 4t .. 4t + 3.  So the four lanes of a quad transpose a 4 x 4 matrix of
+// 16-bit items (4 nibbles): a shuffle with lane ^ 2 and one with lane ^ 1 per row.
+struct TcQuad { bool hi; bool odd; uint32_t own, send; };                   // what a lane needs to know for it
+__device__ __forceinline__ TcQuad tc_quad(int t) {
+    // after the first exchange lanes 0, 1 hold (blocks t, t + 2) in (keep, got), lanes 2, 3 (blocks t, t - 2); the byte selectors
+    // pick this lane's halves (even lanes the low ones, odd lanes the high ones) resp. its neighbour's, lower block first
+    TcQuad q; q.hi = t >= 2; q.odd = (t & 1) != 0;
+    const uint32_t lo = q.hi ? 0x1054u : 0x5410u, up = q.hi ? 0x3276u : 0x7632u;
+    q.own = q.odd ? up : lo; q.send = q.odd ? lo : up;
+    return q;
 }
-// piece idx of the B stage: token = 8 * (idx / 64) + idx % 8, chunk = (idx / 8) % 8 -- the 8 lanes of a quarter warp write
-// into the 8 rows of one atom (distinct swizzled chunks) and read 4 x 64 contiguous bytes per token row
-__device__ __forceinline__ void tc_piece(int idx, int& n, int& c) { n = ((idx >> 6) << 3) + (idx & 7); c = (idx >> 3) & 7; }
-__device__ __forceinline__ void tc_cp16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+// words of one row -> e: items of blocks 0 | 2, o: items of blocks 1 | 3
+__device__ __forceinline__ void tc_transpose(const TcQuad& q, uint32_t x, uint32_t y, uint32_t& e, uint32_t& o) {
+    const uint32_t keep = q.hi ? y : x, got = __shfl_xor_sync(0xffffffffu, q.hi ? x : y, 2);
+    const uint32_t own = __byte_perm(keep, got, q.own), nb = __shfl_xor_sync(0xffffffffu, __byte_perm(keep, got, q.send), 1);
+    e = q.odd ? nb : own; o = q.odd ? own : nb;
 }
-__device__ __forceinline__ void tc_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// The K loop of one output tile.  load_a(g, wv, sv): this warp's fragment register of group g; b_src(n): global address
-// of token row n's first input, or nullptr (the row stays zero).  cb: commits made on the barriers of stages 1 and 3 by
-// earlier tiles of this CTA (a tile adds G/4 to each; G is a multiple of 4); advanced here.  Returns false if a wait ran out.
-template <int NT, class LoadA, class BSrc>
-__device__ __forceinline__ bool tc_mainloop(unsigned char* smem, uint64_t* s_bar, int& cb, uint32_t tmem_base, int G, bool tvalid,
-                                            LoadA load_a, BSrc b_src) {
-    constexpr int A_BYTES = TC_ROWS * 128, B_BYTES = NT * 128, STAGE = A_BYTES + B_BYTES, NB = NT * 8 / TC_THREADS;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, t = lane & 3;
-    const uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(TC_ROWS >> 4) << 24);   // f32 accumulate, f16 x f16, K-major both
-    bool ok = true;
-    // this thread's pieces of the B tile: source row pointer (or null) and offset inside a stage
-    const __half* bsrc[NB]; uint32_t boff[NB];
+// two items -> the halves of block `c` (low item) and c + 2 (high item), scaled
+__device__ __forceinline__ void tc_expand(uint32_t w, __half2 sc, __half2 bi, uint32_t* c0, uint32_t* c2) {
+    uint32_t d[4], v[4];
+    dequant8(w, d);                                                          // (n0 of the low item, n0 of the high one), (n1, n1), ...
 #pragma unroll
-    for (int h = 0; h < NB; ++h) {
-        int n, c; tc_piece(tid + TC_THREADS * h, n, c);
-        const __half* p = b_src(n);
-        bsrc[h] = p ? p + c * 8 : nullptr;
-        boff[h] = (uint32_t)(tc_at(smem + A_BYTES, n, c) - smem);
-        if (!p) {
-#pragma unroll
-            for (int s = 0; s < TC_STAGES; ++s) *reinterpret_cast<uint4*>(smem + (size_t)s * STAGE + boff[h]) = make_uint4(0, 0, 0, 0);
-        }
+    for (int j = 0; j < 4; ++j) {
+        const __half2 h = __hfma2(*reinterpret_cast<const __half2*>(&d[j]), sc, bi);
+        v[j] = *reinterpret_cast<const uint32_t*>(&h);
     }
-    auto issue_b = [&](int g) {
-        unsigned char* st = smem + (size_t)(g % TC_STAGES) * STAGE;
-#pragma unroll
-        for (int h = 0; h < NB; ++h) if (bsrc[h]) tc_cp16(st + boff[h], bsrc[h] + g * 64);
-    };
-    uint4 wv0, sv0, wv1, sv1;                                              // fragment registers of groups g and g + 1
-    if (tvalid) { load_a(0, wv0, sv0); load_a(1, wv1, sv1); }
-    issue_b(0); issue_b(1);
-    tc_cp_commit();
-    // Two groups per barrier: B of the NEXT pair is requested first (its stages were last read by the MMAs of the pair
-    // before this one), then both A tiles of this pair are dequantised, then one wait + fence + barrier and eight MMAs.
-    for (int g = 0; g < G; g += 2) {                                       // G is a multiple of 4 (K is a multiple of 256)
-        const int s0 = g % TC_STAGES, s1 = s0 + 1;
-        unsigned char* sA0 = smem + (size_t)s0 * STAGE;
-        unsigned char* sA1 = smem + (size_t)s1 * STAGE;
-        if (g + 2 < G) {
-            // stages (g + 2) % 4 and (g + 3) % 4 were used by groups g - 2 and g - 1: their commit is the one on stage (g + 3) % 4
-            const int s3 = (g + 3) % TC_STAGES;
-            if (g >= 2 && !tc_wait(&s_bar[s3], (uint32_t)((cb + (g + 3) / TC_STAGES - 1) & 1))) ok = false;
-            issue_b(g + 2); issue_b(g + 3);
-        }
-        tc_cp_commit();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        tc_dequant_A(sA0, warp, r, t, g, wv0, sv0, tvalid);
-        tc_dequant_A(sA1, warp, r, t, g + 1, wv1, sv1, tvalid);
-        if (tvalid && g + 2 < G) { load_a(g + 2, wv0, sv0); load_a(g + 3, wv1, sv1); }
-        asm volatile("cp.async.wait_group 1;" ::: "memory");               // B of this pair has landed (the next pair may be in flight)
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {
-                unsigned char* sA = (ks < 4) ? sA0 : sA1;
-                const uint64_t da = umma_desc_sw128(sA + (ks & 3) * 32), db = umma_desc_sw128(sA + A_BYTES + (ks & 3) * 32);
-                umma_f16(tmem_base, da, db, idesc, (g > 0 || ks > 0) ? 1u : 0u);
-            }
-            umma_commit(&s_bar[s1]);                                       // one commit per pair, on the odd stage's barrier
-        }
-    }
-    // the last commit covers every MMA issued before it
-    cb += G / TC_STAGES;                                                   // commits so far on the barriers of stages 1 and 3
-    if (!tc_wait(&s_bar[(G - 1) % TC_STAGES], (uint32_t)((cb - 1) & 1))) ok = false;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    return ok;
+    c0[0] = __byte_perm(v[0], v[1], 0x5410); c0[1] = __byte_perm(v[2], v[3], 0x5410);
+    c2[0] = __byte_perm(v[0], v[1], 0x7632); c2[1] = __byte_perm(v[2], v[3], 0x7632);
 }
+// s2: (scale, bias) of rows A_r and B_r; taddr: the tile's lanes, the group's first column
+__device__ __forceinline__ void tc_group_A(const TcQuad& q, uint4 wv, uint32_t sa, uint32_t sb, uint32_t taddr) {
+    const __half2 hA = *reinterpret_cast<const __half2*>(&sa), hB = *reinterpret_cast<const __half2*>(&sb);
+    uint32_t v[16], e, o;
+    tc_transpose(q, wv.x, wv.y, e, o);
+    tc_expand(e, __half2half2(__low2half(hA)), __half2half2(__high2half(hA)), v, v + 8);
+    tc_expand(o, __half2half2(__low2half(hA)), __half2half2(__high2half(hA)), v + 4, v + 12);
+    tc_transpose(q, wv.z, wv.w, e, o);
+    tc_expand(e, __half2half2(__low2half(hB)), __half2half2(__high2half(hB)), v + 2, v + 10);
+    tc_expand(o, __half2half2(__low2half(hB)), __half2half2(__high2half(hB)), v + 6, v + 14);
+    tmem_st16x256(taddr, v);
+}
+
+// ================================================================================ the two kinds of work
+// Items are numbered (rows block, 128 weight rows), weight rows fastest; a CTA walks a contiguous run of them, so most
+// steps stay inside a block.  A work type gives the weights of a tile of an item (moved along by a cursor), the place of a
+// block's activation rows (halves from base(), 32 bits: at most 17k rows of 4096), and the epilogue.
+constexpr uint32_t TC_NO_ROW = 0xffffffffu;
+struct TcTile { const uint4 *w, *s; int blk, rt; };   // fragment-major nibbles and scales of a tile (nullptr: none) of weight-row group rt
 
 struct GemmTcArgs {
     Q4R q; int N, K, M;
@@ -192,190 +144,371 @@ struct GemmTcArgs {
     int add_to_y;                    // y += result (residual) instead of y = result
     unsigned* err;
 };
-
+// Dense projection: a block is a token tile.
 template <int NT>
-__global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_umma(GemmTcArgs a) {
-    extern __shared__ __align__(1024) unsigned char smem_raw[];         // 4 stages x [A: 128 rows x 128 B][B: NT tokens x 128 B]
-    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // tiles start on 1024-byte boundaries
-    __shared__ __align__(8) uint64_t s_bar[TC_STAGES];
-    __shared__ uint32_t s_tmem;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int row0 = blockIdx.x * TC_ROWS, t0 = blockIdx.y * NT;
-    const int nt = min(NT, a.M - t0);
-    const int G = a.K >> 6, GP = G >> 1;
-    const int ntiles = a.N >> 4;
-    if (tid == 0) { for (int i = 0; i < TC_STAGES; ++i) mbar_init(&s_bar[i], 1); mbar_fence_init(); }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&s_tmem)), "r"((uint32_t)NT) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+struct DenseWork {
+    using Args = GemmTcArgs;
+    static constexpr bool STRIDED = true;                                   // rows of a block lie stride() halves apart
+    struct Shared {};
+    const Args& a;
+    int NRT;                                                                // weight-row groups
+    __device__ DenseWork(const Args& args, Shared&) : a(args), NRT((args.N + TC_ROWS - 1) / TC_ROWS) {}
+    __device__ int items() const { return NRT * ((a.M + NT - 1) / NT); }
+    __device__ int inputs() const { return a.K; }
+    __device__ unsigned* err() const { return a.err; }
+    __device__ bool has_tile(int rt, int tl) const { return rt * 8 + tl < a.N >> 4; }
+    __device__ TcTile tile(int blk, int rt, int tl) const {
+        const int T = rt * 8 + tl, GP = a.K >> 7;
+        if (!has_tile(rt, tl)) return {nullptr, nullptr, blk, rt};          // (a matrix whose rows are not a multiple of 128)
+        return {a.q.wr + (size_t)T * GP * 64, a.q.sr + (size_t)T * GP * 8, blk, rt};
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = s_tmem;
-    const int T = (row0 >> 4) + warp;                                  // this warp's tile
-    const bool tvalid = T < ntiles;                                    // (the last CTA of a matrix whose rows are not a multiple of 128)
-    const int r = lane >> 2;
-    int cb = 0;
-    bool failed = !tc_mainloop<NT>(smem, s_bar, cb, tmem_base, G, tvalid,
-        [&](int g, uint4& wv, uint4& sv) {
-            wv = ldg_nc_u4(a.q.wr + ((size_t)T * GP + (g >> 1)) * 64 + (g & 1) * 32 + lane);
-            sv = ldg_nc_u4(a.q.sr + ((size_t)T * GP + (g >> 1)) * 8 + r);
-        },
-        [&](int n) -> const __half* { return n < nt ? a.x + (size_t)(t0 + n) * a.ldx : nullptr; });
-    failed = __syncthreads_or(failed ? 1 : 0) != 0;
-    if (failed && a.err && tid == 0) atomicOr(a.err, 1u);
-    if (!failed) {
-        // accumulator lane = weight row of the CTA; warps w and w + 4 share a lane quarter and split the token columns
-        const int row = row0 + (warp & 3) * 32 + lane;
-        const int cbeg = (warp >> 2) * (NT / 2);
-        for (int c0 = cbeg; c0 < cbeg + NT / 2; c0 += 32) {
-            if (c0 >= nt) break;
-            uint32_t dreg[32];
-            tmem_ld32(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, dreg);
+    __device__ const __half* base() const { return a.x; }
+    __device__ uint32_t stride() const { return (uint32_t)a.ldx; }
+    __device__ uint32_t row(int blk, int n) const { return blk * NT + n < a.M ? (uint32_t)(blk * NT + n) * (uint32_t)a.ldx : TC_NO_ROW; }
+    struct Epi {};
+    // quarter: accumulator lanes 32 * quarter ..; taddr: the item's columns in TMEM; release() once they have been read
+    template <class Release>
+    __device__ void epilogue(Epi&, int blk, int rt, int quarter, int lane, uint32_t taddr, Release release) const {
+        const int row = rt * TC_ROWS + quarter * 32 + lane, t0 = blk * NT, nt = min(NT, a.M - t0);
+#pragma unroll 1
+        for (int c0 = 0; c0 < nt; c0 += 16) {
+            uint32_t d[16];
+            tmem_ld16(taddr + (uint32_t)c0, d);
+            if (c0 + 16 >= nt) release();
             if (row < a.N) {
+                __half* y = a.y + (size_t)(t0 + c0) * a.ldy + row;
+                __half old[16];
+                if (a.add_to_y) {                                           // sixteen residual values in flight at a time
 #pragma unroll
-                for (int n = 0; n < 32; ++n) {
+                    for (int n = 0; n < 16; ++n) if (c0 + n < nt) old[n] = y[(size_t)n * a.ldy];
+                }
+#pragma unroll
+                for (int n = 0; n < 16; ++n)
                     if (c0 + n < nt) {
-                        const size_t idx = (size_t)(t0 + c0 + n) * a.ldy + row;
-                        __half val = f2h(__uint_as_float(dreg[n]));
-                        if (a.add_to_y) val = hadd_rn(a.y[idx], val);
-                        a.y[idx] = val;
+                        const __half v = f2h(__uint_as_float(d[n]));
+                        y[(size_t)n * a.ldy] = a.add_to_y ? hadd_rn(old[n], v) : v;
                     }
+            }
+        }
+    }
+};
+// Routed + shared experts of a prompt chunk: a block is up to NT rows of one expert slot, gathered through the pair lists.
+// gate/up: the epilogue applies SwiGLU to (gate row r, up row r) of a paired tile -- they sit 8 accumulator lanes apart --
+// and stores the SwiGLU rows in natural order; down: the pair's output row.
+template <bool DOWN, int NT>
+struct ExpertWork {
+    using Args = ExpertArgs;
+    static constexpr bool STRIDED = false;
+    struct Shared { SlotTable tab; int dst[2][NT]; };
+    const Args& a;
+    Shared& sh;
+    int n_active, K, ntiles, NRT, npair, nshared;
+    __device__ ExpertWork(const Args& args, Shared& s) : a(args), sh(s) {
+        K = DOWN ? a.I : a.H;
+        ntiles = DOWN ? a.H / 16 : a.I / 8;                                 // tiles of 16 weight rows per expert
+        NRT = (ntiles + 7) / 8;                                             // groups of 128 weight rows
+        npair = a.M * a.topk;
+        nshared = a.M_shared >= 0 ? a.M_shared : a.M;
+        n_active = slot_table(sh.tab, a.lists, NT, nshared);
+        __syncthreads();
+    }
+    __device__ int items() const { return sh.tab.base[n_active + 1] * NRT; }
+    __device__ int inputs() const { return K; }
+    __device__ unsigned* err() const { return a.err; }
+    __device__ bool has_tile(int rt, int tl) const { return rt * 8 + tl < ntiles; }
+    __device__ TcTile tile(int blk, int rt, int tl) const {
+        if (!has_tile(rt, tl)) return {nullptr, nullptr, blk, rt};
+        const int j = slot_of(sh.tab, n_active, blk);
+        const bool shared = (j == n_active);
+        const Q4R& q = DOWN ? (shared ? a.sh_down : a.down) : (shared ? a.sh_gu : a.gu);
+        const size_t T = (size_t)(shared ? 0 : sh.tab.expert[j]) * ntiles + rt * 8 + tl;
+        return {q.wr + T * (K >> 7) * 64, q.sr + T * (K >> 7) * 8, blk, rt};
+    }
+    // row n of a block: its pair id (shared expert: npair + row), or -1
+    __device__ int pair_of(int blk, int n) const {
+        const int j = slot_of(sh.tab, n_active, blk), i = (blk - sh.tab.base[j]) * NT + n;
+        if (j == n_active) return i < nshared ? npair + i : -1;
+        return i < sh.tab.cnt[j] ? a.lists.pairs[sh.tab.off[j] + i] : -1;
+    }
+    __device__ const __half* base() const { return DOWN ? a.hbuf : a.p; }
+    __device__ uint32_t stride() const { return 0; }
+    __device__ uint32_t row(int blk, int n) const {
+        const int p = pair_of(blk, n);
+        if (p < 0) return TC_NO_ROW;
+        return (uint32_t)(DOWN ? p : (p >= npair ? a.shared_row0 + p - npair : p / a.topk)) * (uint32_t)K;
+    }
+    struct Epi { int blk = -1, buf = 0, count = 0; };                       // the block whose rows are listed in sh.dst[buf]
+    template <class Release>
+    __device__ void epilogue(Epi& e, int blk, int rt, int quarter, int lane, uint32_t taddr, Release release) const {
+        const int i = quarter * 32 + lane;
+        if (blk != e.blk) {
+            e.blk = blk; e.buf ^= 1;
+            for (int n = i; n < NT; n += TC_EPI * 32) sh.dst[e.buf][n] = pair_of(blk, n);
+            const int j = slot_of(sh.tab, n_active, blk);
+            e.count = min(NT, (j == n_active ? nshared : sh.tab.cnt[j]) - (blk - sh.tab.base[j]) * NT);
+            asm volatile("bar.sync 1, 128;" ::: "memory");                  // the epilogue warps: the list is there
+        }
+        const int* dsts = sh.dst[e.buf];
+        const int i16 = i & 15, etile = rt * 8 + (i >> 4);
+        const bool up = i16 >= 8, have = etile < ntiles;
+        __half* out = DOWN ? a.dbuf + (size_t)rt * TC_ROWS + i : a.hbuf + etile * 8 + (i16 & 7);
+#pragma unroll 1
+        for (int c0 = 0; c0 < e.count; c0 += 16) {
+            uint32_t d[16];
+            tmem_ld16(taddr + (uint32_t)c0, d);
+            if (c0 + 16 >= e.count) release();
+            if (DOWN) {
+#pragma unroll
+                for (int n = 0; n < 16; ++n) {
+                    const int dst = dsts[c0 + n];
+                    if (dst >= 0 && have) out[(size_t)dst * a.H] = f2h(__uint_as_float(d[n]));
+                }
+            } else {
+                // two columns at a time: the gate lane finishes the first, the up lane the second; each sends what the other lacks
+#pragma unroll
+                for (int n = 0; n < 16; n += 2) {
+                    const uint32_t other = __shfl_xor_sync(0xffffffffu, up ? d[n] : d[n + 1], 8);
+                    const float g = __uint_as_float(up ? other : d[n]), u = __uint_as_float(up ? d[n + 1] : other);
+                    const __half v = swiglu_h(f2h(g), f2h(u));
+                    const int dst = dsts[c0 + n + (up ? 1 : 0)];
+                    if (dst >= 0 && have) out[(size_t)dst * a.I] = v;
                 }
             }
         }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"((uint32_t)NT) : "memory");
-}
+};
 
-template <int NT>
-static int launch_gemm_tc_t(const GemmTcArgs& a, cudaStream_t st) {
-    constexpr size_t smem = (size_t)TC_STAGES * (TC_ROWS * 128 + NT * 128) + 1024;
+// ================================================================================ the kernel
+// ST: stages (even); U: stages' fragments a dequant warp has in flight (K / 256 is a multiple of it)
+// TMEM columns: [2][NT] accumulators, [ST][64] A operands
+template <class W, int NT, int ST, int U>
+__global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];             // ST stages x [2 groups][NT rows x 128 B]
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // tiles start on 1024-byte boundaries
+    constexpr int TILE = NT * 128, STAGE = 2 * TILE;
+    static_assert(2 * NT + ST * 64 <= 512 && ST % 2 == 0, "tensor memory");
+    __shared__ __align__(8) uint64_t s_full[ST], s_empty[ST], s_acc_full[2], s_acc_empty[2];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_abort;
+    __shared__ typename W::Shared s_work;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        s_abort = 0;
+        for (int i = 0; i < ST; ++i) { mbar_init(&s_full[i], TC_DQ / 2 + TC_LD * 32); mbar_init(&s_empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&s_acc_full[i], 1); mbar_init(&s_acc_empty[i], TC_EPI); }
+        mbar_fence_init();
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&s_tmem)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    W work(a, s_work);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem;
+    const int items = work.items(), KS = work.inputs() >> 7, NRT = work.NRT;              // KS: stages per item (even)
+    const int lo = (int)((long)items * blockIdx.x / gridDim.x), hi = (int)((long)items * (blockIdx.x + 1) / gridDim.x);
+    const int blk0 = lo / NRT, rt0 = lo - blk0 * NRT;
+    bool ok = true;
+    if (warp == 0) {
+        // ------------------------------------------------------------ mma: one lane, with as few instructions per stage as can be
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(TC_ROWS >> 4) << 24);   // f32 accumulate, f16 x f16, K-major B
+        if (lane == 0) {
+            const uint64_t db0 = umma_desc_sw128(smem);
+            const uint32_t ta0 = tmem + 2 * NT;
+            uint64_t db = db0; uint32_t ta = ta0;                           // (the address field counts 16 bytes: a K step of 16 halves is 2)
+            int st = 0; uint32_t ph = 0;
+            for (int k = 0; k < hi - lo && ok; ++k) {
+                if (k >= 2) ok = tc_wait(&s_acc_empty[k & 1], (uint32_t)(((k >> 1) - 1) & 1), &s_abort);
+                tc_fence_after();
+                const uint32_t acc = tmem + (uint32_t)((k & 1) * NT);
+#pragma unroll 1
+                for (int s = 0; s < KS; ++s) {
+                    if (!tc_wait(&s_full[st], ph, &s_abort)) { ok = false; break; }
+                    tc_fence_after();
+                    tc_fence_proxy();                                       // the rows other threads' asynchronous copies wrote are operand data now
+                    umma_f16_ts(acc, ta, db, idesc, s > 0 ? 1u : 0u);
+#pragma unroll
+                    for (int j = 1; j < 8; ++j) umma_f16_ts(acc, ta + j * 8, db + (j >> 2) * (TILE >> 4) + (j & 3) * 2, idesc, 1u);
+                    umma_commit(&s_empty[st]);
+                    db += STAGE >> 4; ta += 64;
+                    if (++st == ST) { st = 0; ph ^= 1u; db = db0; ta = ta0; }
+                }
+                umma_commit(&s_acc_full[k & 1]);
+            }
+        }
+        __syncwarp();
+    } else if (warp >= TC_DQ0 && warp < TC_DQ0 + TC_DQ) {
+        // ------------------------------------------------------------ dequant: tile tl of every item, stages par, par + 2, ...
+        // (a warp reaches the TMEM lanes 32 * (warp % 4) ..: two tiles)
+        const int d = warp - TC_DQ0, par = d >> 3, half = (d >> 2) & 1, tl = (d & 3) * 2 + half, r = lane >> 2;
+        const TcQuad quad = tc_quad(lane & 3);
+        const uint32_t ta = tmem + 2 * NT + ((uint32_t)((d & 3) * 32 + half * 16) << 16);
+        uint4 w0[U], w1[U], sv[U];
+        int f_left = hi - lo, f_s = 0;                                      // the fetch cursor (f_s counts this warp's stages of an item)
+        TcTile ft = f_left > 0 ? work.tile(blk0, rt0, tl) : TcTile{nullptr, nullptr, 0, 0};
+        auto fetch = [&](uint4& a0, uint4& a1, uint4& sc) {
+            if (ft.w) {
+                const uint4* p = ft.w + f_s * 128 + par * 64 + lane;
+                a0 = ldg_nc_u4(p); a1 = ldg_nc_u4(p + 32);
+                sc = ldg_nc_u4(ft.s + f_s * 16 + par * 8 + r);
+            }
+            if (++f_s == KS >> 1) {
+                f_s = 0;
+                if (--f_left <= 0) ft.w = nullptr;
+                else if (ft.rt + 1 == NRT) ft = work.tile(ft.blk + 1, 0, tl);
+                else if (ft.w && work.has_tile(ft.rt + 1, tl)) { ft.w += KS * 512; ft.s += KS * 64; ++ft.rt; }      // eight tiles on
+                else { ft.w = nullptr; ++ft.rt; }
+            }
+        };
+#pragma unroll
+        for (int u = 0; u < U; ++u) fetch(w0[u], w1[u], sv[u]);
+        int st = par, rt = rt0; uint32_t ph = 1;                            // parity of the stage's "empty" (a fresh barrier passes at 1)
+        for (int k = 0; k < hi - lo && ok; ++k) {
+            const bool valid = work.has_tile(rt, tl);
+            if (++rt == NRT) rt = 0;
+#pragma unroll 1
+            for (int s = 0; s < KS >> 1 && ok; s += U) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    ok = tc_wait(&s_empty[st], ph, &s_abort) && ok;
+                    if (valid) {                                            // (of a tile the matrix does not have the outputs are not stored)
+                        tc_fence_after();
+                        tc_group_A(quad, w0[u], sv[u].x, sv[u].y, ta + st * 64);
+                        tc_group_A(quad, w1[u], sv[u].z, sv[u].w, ta + st * 64 + 32);
+                    }
+                    fetch(w0[u], w1[u], sv[u]);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) tc_arrive(&s_full[st]);
+                    st += 2; if (st >= ST) { st -= ST; ph ^= 1u; }
+                }
+            }
+        }
+    } else if (warp < TC_EPI0 || warp >= TC_DQ0) {
+        // ------------------------------------------------------------ load: the activation rows of every stage
+        constexpr int NP = NT / 16;                                         // rows of a stage per thread, 2 pieces of 16 bytes each
+        const int lt = (warp < TC_EPI0 ? warp - 1 : 3) * 32 + lane;
+        // the 8 lanes of a quarter warp write into the 8 rows of one atom (distinct swizzled chunks) and read 4 x 64 contiguous
+        // bytes per row
+        const int n0 = ((lt >> 6) << 3) + (lt & 7), chunk = (lt >> 3) & 7;  // rows n0 + 16 h, the same chunk of both groups
+        const uint32_t off0 = smem_u32(smem) + tc_off(n0, chunk);
+        const __half* base = work.base() + chunk * 8;
+        uint32_t src[W::STRIDED ? 1 : NP];                                  // row places (strided: of the first row)
+        int st = 0; uint32_t ph = 1;
+        int blk = blk0, rt = rt0, held = -1, have = 0;                      // held: the block whose row places are in src; have: its rows (strided)
+        for (int k = 0; k < hi - lo && ok; ++k) {
+            if (blk != held) {
+                held = blk;
+                if (W::STRIDED) {
+                    src[0] = work.row(blk, n0); have = 0;
+                    for (int h = 0; h < NP; ++h) have += work.row(blk, n0 + 16 * h) != TC_NO_ROW;
+                } else {
+#pragma unroll
+                    for (int h = 0; h < NP; ++h) src[W::STRIDED ? 0 : h] = work.row(blk, n0 + 16 * h);
+                }
+            }
+            if (++rt == NRT) { rt = 0; ++blk; }
+#pragma unroll 1
+            for (int s = 0; s < KS && ok; ++s) {
+                ok = tc_wait(&s_empty[st], ph, &s_abort) && ok;
+                const uint32_t B = off0 + (uint32_t)st * STAGE;
+                auto copy = [&](int h, const __half* p) {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(B + 2048u * h), "l"(p) : "memory");
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(B + TILE + 2048u * h), "l"(p + 64) : "memory");
+                };
+                // (a row the item does not have keeps what was there: its column is not stored)
+                if (W::STRIDED) {
+                    const __half* p = base + src[0] + s * 128;
+#pragma unroll 4
+                    for (int h = 0; h < NP; ++h, p += (size_t)16 * work.stride()) if (h < have) copy(h, p);
+                } else {
+#pragma unroll
+                    for (int h = 0; h < NP; ++h) {
+                        const uint32_t o = src[W::STRIDED ? 0 : h];
+                        if (o != TC_NO_ROW) copy(h, base + o + s * 128);
+                    }
+                }
+                // the barrier counts this thread in when its copies have landed: nobody waits for them here
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&s_full[st])) : "memory");
+                if (++st == ST) { st = 0; ph ^= 1u; }
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        // ------------------------------------------------------------ epilogue
+        typename W::Epi epi;
+        const int quarter = warp - TC_EPI0;
+        int blk = blk0, rt = rt0;
+        for (int k = 0; k < hi - lo && ok; ++k) {
+            ok = tc_wait(&s_acc_full[k & 1], (uint32_t)((k >> 1) & 1), &s_abort);
+            tc_fence_after();
+            if (ok) work.epilogue(epi, blk, rt, quarter, lane, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((k & 1) * NT), [&] {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) tc_arrive(&s_acc_empty[k & 1]);
+            });
+            if (++rt == NRT) { rt = 0; ++blk; }
+        }
+    }
+    if (!ok) {                                 // MMAs of this CTA may still be running: outlast them before TMEM is given back
+        if (work.err() && lane == 0) atomicOr(work.err(), 1u);
+        const long long c0 = clock64();
+        while (clock64() - c0 < 200000ll) { }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512u) : "memory");
+}
+template <class W, int NT, int ST, int U>
+static int launch_tc_t(const typename W::Args& a, int grid, cudaStream_t st) {
+    constexpr size_t smem = (size_t)ST * NT * 256 + 1024;
     static bool configured = false;
     if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(k_gemm_umma<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t err = cudaFuncSetAttribute(k_tc<W, NT, ST, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (err != cudaSuccess) return (int)err;
         configured = true;
     }
-    dim3 grid((unsigned)((a.N + TC_ROWS - 1) / TC_ROWS), (unsigned)((a.M + NT - 1) / NT));
-    k_gemm_umma<NT><<<grid, TC_THREADS, smem, st>>>(a);
+    k_tc<W, NT, ST, U><<<grid, TC_THREADS, smem, st>>>(a);
     return (int)cudaGetLastError();
 }
-
+template <int NT, int ST>
+static int launch_gemm_tc_t(const GemmTcArgs& a, cudaStream_t st) {
+    const int items = ((a.N + TC_ROWS - 1) / TC_ROWS) * ((a.M + NT - 1) / NT), grid = items < sm_count() ? items : sm_count();
+    if (a.K % 512 == 0) return launch_tc_t<DenseWork<NT>, NT, ST, 2>(a, grid, st);
+    return launch_tc_t<DenseWork<NT>, NT, ST, 1>(a, grid, st);
+}
 int launch_gemm_tc(const Q4R& q, int N, int K, int M, const __half* x, int ldx, __half* y, int ldy, bool add_to_y, unsigned* err, cudaStream_t st) {
     if (N % 16 || K % 256) return -1;
     GemmTcArgs a{q, N, K, M, x, ldx, y, ldy, add_to_y ? 1 : 0, err};
-    // the token tile is a scheduling choice only: a token's column never interacts with another's
-    return M <= 64 ? launch_gemm_tc_t<64>(a, st) : launch_gemm_tc_t<256>(a, st);
+    // The token tile is a scheduling choice only (a token's column never interacts with another's).  An item's time is the
+    // larger of its MMAs and of the expansion of its weights (whatever the tile: about equal at 128 tokens), and a
+    // multiprocessor does ceil(items / multiprocessors) of them: the cheapest sum, the wider tile on a tie.
+    const long row_tiles = (N + TC_ROWS - 1) / TC_ROWS;
+    const int nts[3] = {128, 64, 32}, cost[3] = {320, 260, 260};
+    int best = 0; long best_cost = 0;
+    for (int i = 0; i < 3; ++i) {
+        const long items = row_tiles * ((M + nts[i] - 1) / nts[i]), c = (items + sm_count() - 1) / sm_count() * cost[i];
+        if (i == 0 || c < best_cost) { best = i; best_cost = c; }
+    }
+    if (best == 0) return launch_gemm_tc_t<128, 4>(a, st);
+    if (best == 1) return launch_gemm_tc_t<64, 6>(a, st);
+    return launch_gemm_tc_t<32, 6>(a, st);
 }
 
-// ================================================================================ grouped experts (prefill mode)
-// Routed + shared experts of a prompt chunk on the same tensor-core pipeline: a work item is (expert slot, block of up to 64
-// of its rows, 128 weight rows = 8 tiles); the block's rows are gathered through the pair lists into the B stage, the
-// expert's weights are dequantised once per 64 rows.  Items are numbered slot-major, weight-row group fastest; persistent
-// CTAs walk them.  gate/up: the epilogue applies SwiGLU to (gate row r, up row r) of a paired tile -- they sit 8
-// accumulator lanes apart -- and stores the SwiGLU rows in natural order; down: the pair's output row.
-// Prefill-mode numerics (dequantised fp16 weights, one f32 accumulator per output over the whole K); a token's column
-// never interacts with another's, so the result does not depend on which rows share a block.
-constexpr int XT_NT = 64;
-template <bool DOWN>
-__global__ void __launch_bounds__(TC_THREADS, 2) k_expert_umma(ExpertArgs a) {
-    extern __shared__ __align__(1024) unsigned char smem_raw[];         // 4 stages x [A 16 KB][B 8 KB]
-    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    constexpr int NT = XT_NT;
-    __shared__ __align__(8) uint64_t s_bar[TC_STAGES];
-    __shared__ uint32_t s_tmem;
-    __shared__ SlotTable s_tab;
-    __shared__ int s_srow[NT], s_dst[NT];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2;
-    const int K = DOWN ? a.I : a.H, G = K >> 6, GP = G >> 1;
-    const int ntiles = DOWN ? a.H / 16 : a.I / 8;                       // tiles of 16 weight rows per expert
-    const int NRT = (ntiles + 7) / 8;                                   // groups of 128 weight rows
-    const int npair = a.M * a.topk;
-    const int nshared = a.M_shared >= 0 ? a.M_shared : a.M;
-    const int n_active = slot_table(s_tab, a.lists, NT, nshared);
-    if (tid == 0) { for (int i = 0; i < TC_STAGES; ++i) mbar_init(&s_bar[i], 1); mbar_fence_init(); }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&s_tmem)), "r"((uint32_t)NT) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = s_tmem;
-    const int total = s_tab.base[n_active + 1] * NRT;
-    int cb = 0;                                                          // commits made so far on each stage's barrier (same in every thread)
-    bool failed = false;
-    for (int item = blockIdx.x; item < total && !failed; item += gridDim.x) {
-        const int sb = item / NRT, rt = item - sb * NRT;
-        const int j = slot_of(s_tab, n_active, sb), blk = sb - s_tab.base[j];
-        const bool shared = (j == n_active);
-        const int cnt = shared ? nshared : s_tab.cnt[j];
-        const int e = shared ? 0 : s_tab.expert[j];
-        const Q4R& q = DOWN ? (shared ? a.sh_down : a.down) : (shared ? a.sh_gu : a.gu);
-        if (tid < NT) {
-            const int ridx = blk * NT + tid;
-            int dst = -1, srow = -1;
-            if (ridx < cnt) {
-                if (shared) { dst = npair + ridx; srow = DOWN ? dst : a.shared_row0 + ridx; }
-                else { const int pr = a.lists.pairs[s_tab.off[j] + ridx]; dst = pr; srow = DOWN ? pr : pr / a.topk; }
-            }
-            s_srow[tid] = srow; s_dst[tid] = dst;
-        }
-        __syncthreads();
-        const __half* xbase = DOWN ? a.hbuf : a.p;
-        const int tile = rt * 8 + warp;
-        const bool tvalid = tile < ntiles;
-        const size_t Tt = (size_t)e * ntiles + (tvalid ? tile : 0);
-        failed = !tc_mainloop<NT>(smem, s_bar, cb, tmem_base, G, tvalid,
-            [&](int g, uint4& wv, uint4& sv) {
-                wv = ldg_nc_u4(q.wr + (Tt * GP + (g >> 1)) * 64 + (g & 1) * 32 + lane);
-                sv = ldg_nc_u4(q.sr + (Tt * GP + (g >> 1)) * 8 + r);
-            },
-            [&](int n) -> const __half* { const int srow = s_srow[n]; return srow >= 0 ? xbase + (size_t)srow * K : nullptr; });
-        failed = __syncthreads_or(failed ? 1 : 0) != 0;
-        if (!failed) {
-            const int i = (warp & 3) * 32 + lane;                        // accumulator lane = weight row inside the 128
-            const int i16 = i & 15, tl = i >> 4, etile = rt * 8 + tl;
-            const int c0 = (warp >> 2) * (NT / 2);                       // warps w and w + 4 split the token columns
-            uint32_t dreg[32];
-            tmem_ld32(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, dreg);
-#pragma unroll
-            for (int n = 0; n < 32; ++n) {
-                const float v = __uint_as_float(dreg[n]);
-                const int dst = s_dst[c0 + n];
-                if (DOWN) {
-                    if (dst >= 0 && etile < ntiles) a.dbuf[(size_t)dst * a.H + (size_t)rt * TC_ROWS + i] = f2h(v);
-                } else {
-                    const float other = __shfl_xor_sync(0xffffffffu, v, 8);               // the up row of this gate row
-                    if (dst >= 0 && etile < ntiles && i16 < 8) a.hbuf[(size_t)dst * a.I + etile * 8 + i16] = swiglu_h(f2h(v), f2h(other));
-                }
-            }
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();                                                 // accumulator, stages and row lists may be reused
-    }
-    if (failed && a.err && tid == 0) atomicOr(a.err, 1u);
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"((uint32_t)NT) : "memory");
-}
+constexpr int XT_NT = 64;            // rows of an expert's block: a 1024-token chunk gives an expert about 32
 template <bool DOWN>
 static bool launch_expert_tc_t(const ExpertArgs& a, cudaStream_t st) {
     const int K = DOWN ? a.I : a.H;
     if (K % 256 || a.ep_pairs_per_rank > 0) return false;              // (expert-parallel calls keep the row kernels)
-    constexpr size_t smem = (size_t)TC_STAGES * (TC_ROWS * 128 + XT_NT * 128) + 1024;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(k_expert_umma<DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
-        configured = true;
-    }
-    const int grid = 2 * sm_count();                                    // 97 KB of shared memory and 64 TMEM columns per CTA: two fit a multiprocessor
-    profile_launch(DOWN ? "k_expert_umma_down" : "k_expert_umma_gateup", st, [&] { k_expert_umma<DOWN><<<grid, TC_THREADS, smem, st>>>(a); return 0; });
-    return true;
+    int rc = 0;
+    profile_launch(DOWN ? "k_expert_umma_down" : "k_expert_umma_gateup", st, [&] {
+        rc = K % 512 == 0 ? launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, 2>(a, sm_count(), st) : launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, 1>(a, sm_count(), st);
+        return rc;
+    });
+    return rc == 0;
 }
 bool launch_expert_tc_gateup(const ExpertArgs& a, cudaStream_t st) { return launch_expert_tc_t<false>(a, st); }
 bool launch_expert_tc_down(const ExpertArgs& a, cudaStream_t st) { return launch_expert_tc_t<true>(a, st); }

@@ -23,7 +23,10 @@
 //   epilogue   4 warps: read the finished accumulator while the next item accumulates in the other half of its TMEM.
 // The first form (256 threads that all loaded, expanded, synchronised and waited in turn, one pair of groups ahead)
 // spent 2.5 us on a pair of groups whose MMAs take 0.3: every pair paid the latency of its weights and of its rows.
-// With roles but the A operand in shared memory, writing and reading it took most of that memory's bandwidth.
+// With roles but the A operand in shared memory, writing and reading it took most of that memory's bandwidth, and an MMA
+// warp that branched on its lane number needed 1200 cycles a stage to compute addresses: uniform code needs 700.
+// 1024-token chunk of the 2048 / 512 / 256-expert geometry (event times): experts 223 + 138 -> 158 + 109 us, dense
+// 105 -> 51; bound now by the issue of the expansion (ALU 60 % busy), tensor pipe 22 to 39 %.
 #include "kernels.h"
 #include "gemv.cuh"
 
@@ -68,6 +71,11 @@ __device__ __forceinline__ void tmem_st16x256(uint32_t taddr, const uint32_t v[1
     asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
                  :: "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
                     "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
 }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -291,7 +299,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     __shared__ typename W::Shared s_work;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // (the shuffle tells the compiler that it is uniform)
     if (tid == 0) {
         s_abort = 0;
         for (int i = 0; i < ST; ++i) { mbar_init(&s_full[i], TC_DQ / 2 + TC_LD * 32); mbar_init(&s_empty[i], 1); }
@@ -306,39 +314,40 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
     const int items = work.items(), KS = work.inputs() >> 7, NRT = work.NRT;              // KS: stages per item (even)
     const int lo = (int)((long)items * blockIdx.x / gridDim.x), hi = (int)((long)items * (blockIdx.x + 1) / gridDim.x);
     const int blk0 = lo / NRT, rt0 = lo - blk0 * NRT;
     bool ok = true;
     if (warp == 0) {
-        // ------------------------------------------------------------ mma: one lane, with as few instructions per stage as can be
+        // ------------------------------------------------------------ mma
+        // The whole warp walks the stages, so that addresses and descriptors stay in uniform registers; one elected lane issues.
         const uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(TC_ROWS >> 4) << 24);   // f32 accumulate, f16 x f16, K-major B
-        if (lane == 0) {
-            const uint64_t db0 = umma_desc_sw128(smem);
-            const uint32_t ta0 = tmem + 2 * NT;
-            uint64_t db = db0; uint32_t ta = ta0;                           // (the address field counts 16 bytes: a K step of 16 halves is 2)
-            int st = 0; uint32_t ph = 0;
-            for (int k = 0; k < hi - lo && ok; ++k) {
-                if (k >= 2) ok = tc_wait(&s_acc_empty[k & 1], (uint32_t)(((k >> 1) - 1) & 1), &s_abort);
-                tc_fence_after();
-                const uint32_t acc = tmem + (uint32_t)((k & 1) * NT);
+        const uint64_t db0 = umma_desc_sw128(smem);
+        const uint32_t ta0 = tmem + 2 * NT;
+        int st = 0; uint32_t ph = 0;
+        for (int k = 0; k < hi - lo && ok; ++k) {
+            if (k >= 2) ok = tc_wait(&s_acc_empty[k & 1], (uint32_t)(((k >> 1) - 1) & 1), &s_abort);
+            tc_fence_after();
+            const uint32_t acc = tmem + (uint32_t)((k & 1) * NT);
 #pragma unroll 1
-                for (int s = 0; s < KS; ++s) {
-                    if (!tc_wait(&s_full[st], ph, &s_abort)) { ok = false; break; }
-                    tc_fence_after();
-                    tc_fence_proxy();                                       // the rows other threads' asynchronous copies wrote are operand data now
+            for (int s = 0; s < KS; ++s) {
+                if (!tc_wait(&s_full[st], ph, &s_abort)) { ok = false; break; }
+                tc_fence_after();
+                tc_fence_proxy();                                           // the rows other threads' asynchronous copies wrote are operand data now
+                const uint64_t db = db0 + (uint32_t)(st * (STAGE >> 4));    // (the address field counts 16 bytes: a K step of 16 halves is 2)
+                const uint32_t ta = ta0 + st * 64;
+                if (tc_elect()) {
                     umma_f16_ts(acc, ta, db, idesc, s > 0 ? 1u : 0u);
 #pragma unroll
                     for (int j = 1; j < 8; ++j) umma_f16_ts(acc, ta + j * 8, db + (j >> 2) * (TILE >> 4) + (j & 3) * 2, idesc, 1u);
                     umma_commit(&s_empty[st]);
-                    db += STAGE >> 4; ta += 64;
-                    if (++st == ST) { st = 0; ph ^= 1u; db = db0; ta = ta0; }
+                    if (s == KS - 1) umma_commit(&s_acc_full[k & 1]);
                 }
-                umma_commit(&s_acc_full[k & 1]);
+                __syncwarp();
+                if (++st == ST) { st = 0; ph ^= 1u; }
             }
         }
-        __syncwarp();
     } else if (warp >= TC_DQ0 && warp < TC_DQ0 + TC_DQ) {
         // ------------------------------------------------------------ dequant: tile tl of every item, stages par, par + 2, ...
         // (a warp reaches the TMEM lanes 32 * (warp % 4) ..: two tiles)

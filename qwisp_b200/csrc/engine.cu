@@ -61,7 +61,7 @@ struct sl_engine {
     const __half *embed = nullptr, *final_norm = nullptr;
     Q4W lm_head; Q4R r_lm_head;
     // scratch (sized by max_rows)
-    __half *h = nullptr, *p = nullptr, *inproj = nullptr, *mix = nullptr, *rlogits = nullptr, *sgl = nullptr, *scores = nullptr;
+    __half *h = nullptr, *h2 = nullptr, *p = nullptr, *inproj = nullptr, *mix = nullptr, *rlogits = nullptr, *sgl = nullptr, *scores = nullptr;
     __half *hbuf = nullptr, *dbuf = nullptr, *normed = nullptr, *qrot = nullptr, *opx = nullptr, *opy = nullptr;
     // many-row kernels: prepared rows of a dense projection / of the experts' input, their group sums, chunk sums of the SwiGLU rows
     __half *xq = nullptr, *xq_p = nullptr; float *sxq = nullptr, *sx_p = nullptr, *csum = nullptr;
@@ -295,6 +295,7 @@ int32_t build_runtime(sl_engine* e) {
     size_t mix_w = (size_t)(e->valDim > e->attn_out ? e->valDim : e->attn_out);
     size_t prow = (size_t)R * e->topk + R;
     if ((rc = dalloc(e, &e->h, (size_t)R * H))) return rc;
+    if ((rc = dalloc(e, &e->h2, (size_t)H))) return rc;      // one-row steps: the residual row alternates between the two
     if ((rc = dalloc(e, &e->p, (size_t)R * H))) return rc;
     if ((rc = dalloc(e, &e->normed, (size_t)R * (e->valDim > H ? e->valDim : H)))) return rc;   // also the gated-norm rows of prefill mode
     {
@@ -577,7 +578,8 @@ int32_t enqueue_moe_ep(sl_engine* e, const LayerW& L, RouterArgs ra, int M, __ha
 }
 
 // next: the layer after L (nullptr after the last one, where the lm_head follows)
-void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half* rows, int ld, bool apply_norm, int M, __half* resid, __half* plain_out) {
+// defer (optional): where the combine may be left to the next layer's in-projection, it is, and *defer says what it needs
+void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half* rows, int ld, bool apply_norm, int M, __half* resid, __half* plain_out, MoeRow* defer = nullptr) {
     cudaStream_t st = e->stream;
     RouterArgs ra{}; ra.h = rows; ra.ldh = ld; ra.norm_w = apply_norm ? L.post_norm : nullptr; ra.eps = e->cfg.rms_eps;
     ra.router = L.router; ra.shared_gate = L.shared_gate; ra.M = M; ra.H = e->H; ra.E = e->E;
@@ -598,6 +600,12 @@ void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half
     // batch-1 decode: the router stops at the logits and the fused expert kernel's CTAs route the row themselves
     ra.no_route = (fused && e->use_route_in_experts) ? 1 : 0;
     ea.route_here = ra.no_route;
+    if (defer && fused && ea.route_here) {
+        // (a last-arriver combine at the end of the expert kernel was 3 us of fence, ticket and L2 round trips per layer; the
+        // in-projection's CTAs each do the whole row's instead, in 0.6 us, while they wait for nothing else)
+        ea.resid = nullptr; ea.out = nullptr;
+        *defer = MoeRow{e->dbuf, e->scores, e->sgl, e->topk, nullptr};
+    }
     const bool tc_experts = e->hybrid && e->E <= 256 && e->use_rows;      // prefill mode: for any row count (chunk-split invariance)
     const bool rows_experts = !tc_experts && M > 1 && e->E <= 256 && e->use_rows;
     const bool prepared = enqueue_router(e, ra, M, e->use_pdl, rows_experts ? e->xq_p : nullptr, e->sx_p);
@@ -628,14 +636,15 @@ void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half
 
 // mixer of one layer: input rows are normed inside (norm_w != nullptr) or already normed
 void enqueue_mixer(sl_engine* e, const LayerW& L, const __half* rows, const __half* norm_w, int M, int nsegs,
-                   __half* resid, __half* plain_out, const int* row_pos_override) {
+                   __half* resid, __half* plain_out, const int* row_pos_override, const MoeRow* pending = nullptr) {
     cudaStream_t st = e->stream;
     const sl_config& c = e->cfg;
     DenseArgs d{}; d.err = e->err_flag; d.norm_scratch = e->normed; d.xq = e->use_rows ? e->xq : nullptr; d.sxq = e->sxq; d.q = L.r_in; d.N = (int)L.in_proj.N; d.K = e->H; d.M = M;
     d.x = rows; d.ldx = e->H; d.nw = norm_w; d.eps = c.rms_eps; d.y = e->inproj; d.ldy = (int)L.in_proj.N;
     if (e->use_prefetch) pf_q4(d.pf, 0, L.r_out);
     d.tc = e->hybrid;
-    launch_dense(norm_w ? PRO_RMSNORM : PRO_PLAIN, EPI_STORE, d, st, e->use_pdl);
+    if (pending) d.moe = *pending;                             // rows: the residual before the last block's combine; resid: where it is kept after it
+    launch_dense(pending ? PRO_MOERMS : (norm_w ? PRO_RMSNORM : PRO_PLAIN), EPI_STORE, d, st, e->use_pdl);
     DenseArgs o{};
     o.err = e->err_flag; o.q = L.r_out; o.N = e->H; o.K = L.out_proj.K; o.M = M;
     o.eps = c.rms_eps; o.y = resid ? resid : plain_out; o.ldy = e->H; o.tc = e->hybrid; o.norm_scratch = e->normed; o.xq = e->use_rows ? e->xq : nullptr; o.sxq = e->sxq;
@@ -677,16 +686,23 @@ void enqueue_step(sl_engine* e, int M, int nsegs, HeadMode head, bool want_logit
     cudaStream_t st = e->stream;
     e->ep_layer_seq = 0;
     launch_embed(e->embed, e->tok_in, M, e->H, e->V, e->h, st);
+    __half* h = e->h;                                          // the residual rows
+    MoeRow moe;                                                // a one-row step's last MoE block, not yet combined (moe.d set)
     for (size_t li = 0; li < e->layers.size(); ++li) {
         const LayerW& L = e->layers[li];
-        enqueue_mixer(e, L, e->h, L.in_norm, M, nsegs, e->h, nullptr, nullptr);
-        enqueue_moe(e, L, li + 1 < e->layers.size() ? &e->layers[li + 1] : nullptr, e->h, e->H, true, M, e->h, nullptr);
+        const LayerW* next = li + 1 < e->layers.size() ? &e->layers[li + 1] : nullptr;
+        const __half* rows = h;
+        const MoeRow* pending = moe.d ? &moe : nullptr;
+        if (pending) { h = (h == e->h) ? e->h2 : e->h; moe.out = h; }
+        enqueue_mixer(e, L, rows, L.in_norm, M, nsegs, h, nullptr, nullptr, pending);
+        moe = MoeRow{};
+        enqueue_moe(e, L, next, h, e->H, true, M, h, nullptr, next && M == 1 && !e->hybrid && !e->ep_step ? &moe : nullptr);
     }
     if (head == HEAD_NORMED) {
-        launch_final_norm(e->h, e->final_norm, e->cfg.rms_eps, M, e->H, e->normed, st);
+        launch_final_norm(h, e->final_norm, e->cfg.rms_eps, M, e->H, e->normed, st);
     } else if (head == HEAD_ARGMAX || head == HEAD_LOGITS) {
         DenseArgs d{}; d.q = e->r_lm_head; d.N = e->V; d.K = e->H; d.M = M;
-        d.x = e->h; d.ldx = e->H; d.nw = e->final_norm; d.eps = e->cfg.rms_eps;
+        d.x = h; d.ldx = e->H; d.nw = e->final_norm; d.eps = e->cfg.rms_eps;
         d.logits = want_logits ? e->logits : nullptr; d.pval = e->pval; d.pidx = e->pidx; d.out_tok = e->out_tok; d.counter = e->counters + 0;
         launch_dense(PRO_RMSNORM, EPI_ARGMAX, d, st, e->use_pdl);
     }

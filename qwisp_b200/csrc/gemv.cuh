@@ -27,7 +27,9 @@
 
 namespace sl {
 
-enum { PRO_PLAIN = 0, PRO_RMSNORM = 1, PRO_NORMGATE = 2, PRO_NORMGATE32 = 3 };   // NORMGATE32: gated norm with an f32 weight
+// NORMGATE32: gated norm with an f32 weight; MOERMS: one row whose MoE block is still to be combined (see moe_combine8), then RMSNorm
+enum { PRO_PLAIN = 0, PRO_RMSNORM = 1, PRO_NORMGATE = 2, PRO_NORMGATE32 = 3, PRO_MOERMS = 4 };
+__host__ __device__ constexpr bool pro_is_rms(int pro) { return pro == PRO_RMSNORM || pro == PRO_MOERMS; }
 __host__ __device__ constexpr bool pro_is_normgate(int pro) { return pro == PRO_NORMGATE || pro == PRO_NORMGATE32; }
 enum { EPI_STORE = 0, EPI_RESID = 1, EPI_SWIGLU = 2, EPI_ARGMAX = 3 };
 
@@ -87,6 +89,9 @@ __device__ __forceinline__ void rows_store(__half* xq_row, float* sx_row, int k0
 // The first two units of a warp are requested by stage_issue and held in registers, so a kernel
 // can put those loads in flight early and do other set-up before it needs them; further units
 // (more than two rows, or K = 4096 with two) are loaded where they are used.
+// A row's MoE block before the combine: its top_k expert rows and the shared expert's, the gates, the shared-gate logit;
+// out: where the row after the combine is kept (written by one CTA)
+struct MoeRow { const __half* d = nullptr; const __half* scores = nullptr; const __half* sgl = nullptr; int topk = 0; __half* out = nullptr; };
 struct StageSrc {
     const __half* x; int ldx;        // rows (plain) / residual stream (rmsnorm) / y (normgate)
     const int* rows;                 // optional row list (shared memory), else rows row0, row0+1, ...
@@ -94,6 +99,7 @@ struct StageSrc {
     const __half* z; int ldz;        // gate input of the gated norm
     float eps;
     const float* nw32 = nullptr;     // gated norm only: f32 norm weight (the norm then runs in f32, see stage_finish)
+    MoeRow moe;                      // PRO_MOERMS
 };
 struct StageRegs { uint4 a[2], b[2], c[2]; };   // activations, norm weights, gate inputs of the first two units
 
@@ -180,7 +186,7 @@ template <int PRO>
 __device__ __forceinline__ void stage_finish(const StageRegs& sr, const XStage& st, const StageSrc& s, int row0, int mr, int K) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int lgc = 31 - __clz(K >> 8), chunks = 1 << lgc, units = mr << lgc;
-    if (PRO == PRO_RMSNORM) {
+    if (pro_is_rms(PRO)) {
         for (int j = 0, u = warp; u < units; ++j, u += nw) {
             const int col = u >> lgc, ch = u & (chunks - 1);
             const uint4 v = (j == 0) ? sr.a[0] : ((j == 1) ? sr.a[1] : stage_load(s, row0, col, (ch << 8) + lane * 8));
@@ -195,10 +201,13 @@ __device__ __forceinline__ void stage_finish(const StageRegs& sr, const XStage& 
         uint4 o;
         if (PRO == PRO_PLAIN) {
             o = v;
-        } else if (PRO == PRO_RMSNORM) {
-            float tot = 0.f;
-            for (int c = 0; c < chunks; ++c) tot += st.part[col * 16 + c];
-            float inv = __frsqrt_rn(__fadd_rn(__fdiv_rn(tot, (float)K), s.eps));
+        } else if (pro_is_rms(PRO)) {
+            float pc[16], tot = 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) *reinterpret_cast<float4*>(pc + 4 * c) = *reinterpret_cast<const float4*>(st.part + col * 16 + 4 * c);
+#pragma unroll
+            for (int c = 0; c < 16; ++c) if (c < chunks) tot += pc[c];
+            float inv = __frsqrt_rn(__fadd_rn(__fmul_rn(tot, 1.0f / (float)K), s.eps));       // (K is a power of two: the quotient, exactly)
             const uint4 wv = (j == 0) ? sr.b[0] : ((j == 1) ? sr.b[1] : *reinterpret_cast<const uint4*>(s.nw + k0));
             o = rms_apply8(v, wv, inv);
         } else {
@@ -209,6 +218,33 @@ __device__ __forceinline__ void stage_finish(const StageRegs& sr, const XStage& 
         }
         store_staged(st, col, k0, o, lane);
     }
+}
+// 8 consecutive outputs of a row's MoE block on top of the residual row h: fp16 weighted sum in ascending k
+// (SeedlessFusedVerify.swift:462-471) + sigmoid(gate logit) * shared (:474-484) + residual (SeedlessMetalForward.swift:1024-1028).
+// Every step is one correctly rounded fp16 operation, as in the other forms of the combine.
+__device__ __forceinline__ uint4 moe_combine8(const MoeRow& m, uint4 h, int H, int k0, int lane) {
+    uint4 d[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) if (k < m.topk) d[k] = __ldcg(reinterpret_cast<const uint4*>(m.d + (size_t)k * H + k0));
+    const uint4 sh = __ldcg(reinterpret_cast<const uint4*>(m.d + (size_t)m.topk * H + k0));
+    const unsigned sc = lane < m.topk ? (unsigned)__half_as_ushort(__ldcg(m.scores + lane)) : 0u;
+    const __half2 gate = __half2half2(sigmoid_h(__ldcg(m.sgl)));
+    __half2 acc[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i] = __float2half2_rn(0.0f);
+#pragma unroll
+    for (int k = 0; k < 16; ++k)
+        if (k < m.topk) {
+            const __half2 w = __half2half2(__ushort_as_half((unsigned short)__shfl_sync(0xffffffffu, sc, k)));
+            const __half2* dk = reinterpret_cast<const __half2*>(&d[k]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[i] = __hadd2_rn(acc[i], __hmul2_rn(dk[i], w));
+        }
+    __half2* hh = reinterpret_cast<__half2*>(&h);
+    const __half2* s2 = reinterpret_cast<const __half2*>(&sh);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) hh[i] = __hadd2_rn(hh[i], __hadd2_rn(acc[i], __hmul2_rn(gate, s2[i])));
+    return h;
 }
 // whole-prologue forms for kernels that have nothing to overlap with the loads
 __device__ __forceinline__ void stage_plain(const XStage& st, const __half* x, int ldx, int row0, int mr, int K) {

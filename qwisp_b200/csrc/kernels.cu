@@ -112,6 +112,11 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) k_gemv(DenseArgs a) 
     pdl_wait();
     pdl_launch_dependents();
     stage_issue<PRO>(sregs, src, row0, mr, a.K);
+    if (PRO == PRO_MOERMS && (warp << 8) < a.K) {             // (one row: a warp has one 256-wide chunk at most)
+        const int k0 = (warp << 8) + lane * 8;
+        sregs.a[0] = moe_combine8(a.moe, sregs.a[0], a.K, k0, lane);
+        if (blockIdx.x == 0) *reinterpret_cast<uint4*>(a.moe.out + k0) = sregs.a[0];
+    }
     // the residual value this thread will add in the epilogue (first epilogue iteration) is final already:
     // request it now instead of at the end of the kernel
     __half resid0 = f2h(0.0f);
@@ -406,6 +411,7 @@ gemv_path:
     SL_CASE(PRO_PLAIN, EPI_STORE)
     SL_CASE(PRO_PLAIN, EPI_RESID)
     SL_CASE(PRO_RMSNORM, EPI_STORE)
+    SL_CASE(PRO_MOERMS, EPI_STORE)
     SL_CASE(PRO_NORMGATE, EPI_RESID)
     SL_CASE(PRO_NORMGATE, EPI_STORE)
     SL_CASE(PRO_NORMGATE32, EPI_RESID)
@@ -969,9 +975,9 @@ __global__ void __launch_bounds__(512, 1) k_expert_fused(ExpertArgs a) {
         wstage_copy(ws2, q2.wr, q2.sr, ((size_t)e * nt2 + (size_t)blockIdx.x * TPC2) << lg2, nvu2, UD);
     };
     if (issuer) { wstage_init(ws1, UG); wstage_init(ws2, UD); }
-    __shared__ float s_rbuf[512 + 32];
-    __shared__ int s_inds[16];
+    __shared__ float s_rbuf[256];
     __shared__ __half s_scores[16];
+    const bool deferred = !a.resid && !a.out;                  // the combine is left to the next kernel (moe_combine8)
     const bool shared = (y == (int)gridDim.y - 1);             // one row: its top_k experts are distinct, slot k = k-th choice
     if (shared && issuer) issue(true, 0);
     pdl_wait();
@@ -981,14 +987,22 @@ __global__ void __launch_bounds__(512, 1) k_expert_fused(ExpertArgs a) {
         // all CTAs) instead of the router kernel ending in a one-CTA routing tail that all CTAs would wait for.
         // The last warp does it (it stages no activations) and starts this slot's weight copies straight away,
         // while the other warps stage the activation row; the barrier after the staging publishes the scores.
-        if (warp == 15) {
-            route_row_warp(a.rlogits, a.E, a.topk, s_inds, s_scores, s_rbuf, lane);
-            __syncwarp();
-            if (!shared && lane == 0) issue(false, s_inds[y]);
-            if (blockIdx.x == 0 && y == 0 && lane < a.topk) { a.inds_out[lane] = s_inds[lane]; a.scores_out[lane] = s_scores[lane]; }
+        // The gates are needed at the combine: by all CTAs when the last one of a tile group combines here, else by the next
+        // kernel, for which a CTA of the shared expert makes them (its weights were on their way before the wait).
+        const bool writer = shared && blockIdx.x == 0;
+        if (warp == 15 && (!shared || !deferred || writer)) {
+            const uint4 raw = route_load<false>(a.rlogits, a.E, lane);
+            const int my_id = route_select(raw, a.E, a.topk, lane);
+            __syncwarp();                                      // (lane 0 initialised the barriers)
+            if (!shared && lane == y) issue(false, my_id);
+            if (!deferred || writer) {
+                const __half g = route_gate(raw, my_id, a.E, a.topk, s_rbuf, lane);
+                if (lane < a.topk) s_scores[lane] = g;
+                if (writer && lane < a.topk) { a.inds_out[lane] = my_id; a.scores_out[lane] = g; }
+            }
         }
     } else {
-        if ((int)threadIdx.x < a.topk) { s_inds[threadIdx.x] = a.lists.slot_expert[threadIdx.x]; s_scores[threadIdx.x] = a.scores[threadIdx.x]; }
+        if ((int)threadIdx.x < a.topk) s_scores[threadIdx.x] = a.scores[threadIdx.x];
         if (!shared && issuer) issue(false, a.lists.slot_expert[y]);
     }
     const int dst = shared ? npair : y;                        // row of hbuf / dbuf (pair id k, or top_k for the shared expert)
@@ -1069,6 +1083,7 @@ __global__ void __launch_bounds__(512, 1) k_expert_fused(ExpertArgs a) {
             if (tile2 < nt2) a.dbuf[(size_t)dst * a.H + tile2 * 16 + row] = f2h(tile_sum(red, tl2, sl2, row, 0));
         }
     }
+    if (deferred) return;
     // what the combine needs besides the other CTAs' results is fetched before the ticket, so the CTA that
     // turns out to be last only waits for the expert outputs (column i of the group per thread; TPC2*16 <= 512)
     const int ncols = min(TPC2 * 16, a.H - (int)blockIdx.x * TPC2 * 16);
@@ -1148,12 +1163,13 @@ void launch_expert_down(const ExpertArgs& a, int nslots, cudaStream_t st, bool p
 // Gated-delta-net core: causal conv1d + SiLU, q/k l2-style norm + scale, beta / decay, the
 // recurrent state update and readout, for all rows of a segment in sequence.
 // (conv: SeedlessFusedVerify.swift:634-663; prep: :839-938; recurrence: GatedDelta.swift:63-124)
-// grid (8 dv-tiles of 16, Hv, nsegs), 128 threads.  The fp32 state tile [16 dv][128 dk] of this
+// grid (8 dv-tiles of 16, Hv, nsegs), 192 threads: four warps hold the state, one makes v, one the gates (a chain of
+// logarithms and exponentials as long as the convolutions).  The fp32 state tile [16 dv][128 dk] of this
 // CTA lives in registers for the whole call: read once from the current ping-pong side, written
 // once to the other side.  Conv history likewise goes from one side to the other.
 // ============================================================================================
-__global__ void __launch_bounds__(128) k_gdn_core(GdnArgs a) {
-    __shared__ float q_s[128], k_s[128], v_s[16];
+__global__ void __launch_bounds__(192) k_gdn_core(GdnArgs a) {
+    __shared__ __align__(16) float q_s[128], k_s[128]; __shared__ float v_s[16];
     __shared__ float red_s[8]; __shared__ float gb_s[2];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int dvt = blockIdx.x, hv = blockIdx.y;
@@ -1173,11 +1189,12 @@ __global__ void __launch_bounds__(128) k_gdn_core(GdnArgs a) {
     // the state was written a whole step ago: loaded ahead of the programmatic-launch wait
     float4 S[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) S[i] = *reinterpret_cast<const float4*>(S_in + (size_t)(warp * 4 + i) * GDN_DK + lane * 4);
+    for (int i = 0; i < 4; ++i) if (warp < 4) S[i] = *reinterpret_cast<const float4*>(S_in + (size_t)(warp * 4 + i) * GDN_DK + lane * 4);
     // also ahead of the wait: conv weights, decay parameters (cold in HBM once per token) and the three
     // history rows of this thread's channels (written a step ago)
-    const int ch_q = hk * GDN_DK + tid, ch_k = keyDim + hk * GDN_DK + tid;
+    const int ch_q = hk * GDN_DK + (tid & 127), ch_k = keyDim + hk * GDN_DK + (tid & 127);
     const int ch_v = 2 * keyDim + hv * GDN_DV + dvt * 16 + (tid & 15);
+    const bool vmaker = warp == 4 && lane < 16;
     const float4 wq = *reinterpret_cast<const float4*>(a.conv_w + (size_t)ch_q * 4);
     const float4 wk = *reinterpret_cast<const float4*>(a.conv_w + (size_t)ch_k * 4);
     const float4 wv = *reinterpret_cast<const float4*>(a.conv_w + (size_t)ch_v * 4);
@@ -1194,7 +1211,7 @@ __global__ void __launch_bounds__(128) k_gdn_core(GdnArgs a) {
 
     auto xval = [&](int idx, int ch) -> float {               // row idx of [hist(3) | rows of the segment]
         if (idx < CONV_K - 1) {
-            const float* hsel = (ch == ch_q) ? hq : ((ch == ch_k) ? hkk : hvv);
+            const float* hsel = (ch == ch_v) ? hvv : ((ch == ch_k) ? hkk : hq);
             return (idx == 0) ? hsel[0] : ((idx == 1) ? hsel[1] : hsel[2]);
         }
         return h2f(a.inproj[(size_t)(seg.row0 + idx - (CONV_K - 1)) * a.ld + ch]);
@@ -1204,51 +1221,54 @@ __global__ void __launch_bounds__(128) k_gdn_core(GdnArgs a) {
     };
     for (int tt = 0; tt < seg.nrows; ++tt) {
         const int row = seg.row0 + tt;
-        float qc = conv(tt, ch_q, wq), kc = conv(tt, ch_k, wk);
-        if (tid < 16) v_s[tid] = conv(tt, ch_v, wv);
-        float sq = warp_sum(qc * qc), sk = warp_sum(kc * kc);
-        if (lane == 0) { red_s[warp] = sq; red_s[4 + warp] = sk; }
-        if (tid == 0) {
-            __half bh = a.inproj[(size_t)row * a.ld + convDim + a.Hv * GDN_DV + hv];
-            __half ah = a.inproj[(size_t)row * a.ld + convDim + a.Hv * GDN_DV + a.Hv + hv];
+        if (warp < 4) {
+            const float qc = conv(tt, ch_q, wq), kc = conv(tt, ch_k, wk);
+            q_s[tid] = qc; k_s[tid] = kc;
+            const float sq = warp_sum(qc * qc), sk = warp_sum(kc * kc);
+            if (lane == 0) { red_s[warp] = sq; red_s[4 + warp] = sk; }
+        } else if (vmaker) {
+            v_s[lane] = conv(tt, ch_v, wv);
+        } else if (tid == 160) {
+            const __half bh = a.inproj[(size_t)row * a.ld + convDim + a.Hv * GDN_DV + hv];
+            const __half ah = a.inproj[(size_t)row * a.ld + convDim + a.Hv * GDN_DV + a.Hv + hv];
             gdn_gate(bh, ah, A_log_h, dt_bias_h, gb_s[0], gb_s[1]);
         }
         __syncthreads();
-        float iq = gdn_head_inv(red_s[0], red_s[1], red_s[2], red_s[3], a.eps);
-        float ik = gdn_head_inv(red_s[4], red_s[5], red_s[6], red_s[7], a.eps);
-        q_s[tid] = gdn_scale_q(qc, iq);
-        k_s[tid] = gdn_scale_k(kc, ik);
-        __syncthreads();
-        const float g = gb_s[0], beta = gb_s[1];
-        const float4 kq = *reinterpret_cast<const float4*>(k_s + lane * 4);
-        const float4 qq = *reinterpret_cast<const float4*>(q_s + lane * 4);
+        if (warp < 4) {
+            const float iq = gdn_head_inv(red_s[0], red_s[1], red_s[2], red_s[3], a.eps);
+            const float ik = gdn_head_inv(red_s[4], red_s[5], red_s[6], red_s[7], a.eps);
+            const float g = gb_s[0], beta = gb_s[1];
+            float4 kq = *reinterpret_cast<const float4*>(k_s + lane * 4), qq = *reinterpret_cast<const float4*>(q_s + lane * 4);
+            kq = make_float4(gdn_scale_k(kq.x, ik), gdn_scale_k(kq.y, ik), gdn_scale_k(kq.z, ik), gdn_scale_k(kq.w, ik));
+            qq = make_float4(gdn_scale_q(qq.x, iq), gdn_scale_q(qq.y, iq), gdn_scale_q(qq.z, iq), gdn_scale_q(qq.w, iq));
+            float o[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float4 s = S[i];
-            const float o = gdn_row_step(s, g, kq, qq, v_s[warp * 4 + i], beta);
-            S[i] = s;
-            if (lane == 0) a.y[(size_t)row * (a.Hv * GDN_DV) + hv * GDN_DV + dvt * 16 + warp * 4 + i] = f2h(o);
+            for (int i = 0; i < 4; ++i) { float4 s = S[i]; o[i] = gdn_row_step(s, g, kq, qq, v_s[warp * 4 + i], beta); S[i] = s; }
+            if (lane == 0) {
+                __half2* y = reinterpret_cast<__half2*>(a.y + (size_t)row * (a.Hv * GDN_DV) + hv * GDN_DV + dvt * 16 + warp * 4);
+                y[0] = __halves2half2(f2h(o[0]), f2h(o[1])); y[1] = __halves2half2(f2h(o[2]), f2h(o[3]));
+            }
         }
-        __syncthreads();
+        if (tt + 1 < seg.nrows) __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(S_out + (size_t)(warp * 4 + i) * GDN_DK + lane * 4) = S[i];
+    for (int i = 0; i < 4; ++i) if (warp < 4) *reinterpret_cast<float4*>(S_out + (size_t)(warp * 4 + i) * GDN_DK + lane * 4) = S[i];
     // new conv history = last three rows of [hist | rows]; q/k channels by one CTA per key head
-    const bool owner_qk = (dvt == 0) && (hv % (a.Hv / a.Hk) == 0);
+    const bool owner_qk = warp < 4 && (dvt == 0) && (hv % (a.Hv / a.Hk) == 0);
     for (int j = 0; j < CONV_K - 1; ++j) {
         int idx = seg.nrows + j;
         if (owner_qk) {
             hist_out[(size_t)j * convDim + ch_q] = f2h(xval(idx, ch_q));
             hist_out[(size_t)j * convDim + ch_k] = f2h(xval(idx, ch_k));
         }
-        if (tid < 16) hist_out[(size_t)j * convDim + ch_v] = f2h(xval(idx, ch_v));
+        if (vmaker) hist_out[(size_t)j * convDim + ch_v] = f2h(xval(idx, ch_v));
     }
 }
 void launch_gdn_core(const GdnArgs& a, int nsegs, cudaStream_t st, bool pdl) {
     dim3 grid(8, a.Hv, nsegs);
     ProfScope ps("k_gdn_core", (double)nsegs * a.Hv * GDN_DV * GDN_DK * 8, st);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid; cfg.blockDim = dim3(128); cfg.stream = st;
+    cfg.gridDim = grid; cfg.blockDim = dim3(192); cfg.stream = st;
     cudaLaunchAttribute attr[1];
     set_pdl(cfg, attr, pdl);
     GdnArgs copy = a;

@@ -24,6 +24,7 @@ struct DenseArgs {
     __half* logits;                                              // optional [M][N] (argmax epilogue)
     float* pval; int* pidx; int* out_tok; unsigned* counter;     // argmax partials / result / ticket
     PfList pf;                                                   // weights of later kernels to pull into L2
+    MoeRow moe;                                                  // PRO_MOERMS: x is the residual row before the last MoE block's combine
 };
 
 // what a kernel needs to raise this rank's flags at its peers (world == 0: not expert-parallel)

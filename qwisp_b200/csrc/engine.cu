@@ -53,6 +53,7 @@ struct sl_engine {
     int H = 0, E = 0, I = 0, topk = 0, V = 0;
     int keyDim = 0, valDim = 0, convDim = 0, gdn_in = 0, attn_in = 0, attn_out = 0;
     int n_gdn = 0, n_attn = 0;
+    int call_keys = 0;              // most keys of a row of the call being enqueued; 0 inside a graph, which outlives the length
     bool hybrid = false;            // set for the duration of a prefill-mode call: dense projections on the tensor-core GEMM
     cudaStream_t own_stream = nullptr, stream = nullptr;
     std::map<std::string, Tensor> tensors;
@@ -666,7 +667,7 @@ void enqueue_mixer(sl_engine* e, const LayerW& L, const __half* rows, const __ha
         AttnArgs a{}; a.inproj = e->inproj; a.ld = e->attn_in; a.q_norm = L.q_norm; a.k_norm = L.k_norm; a.NH = c.attn_heads; a.KV = c.attn_kv_heads;
         a.eps = c.rms_eps; a.theta = c.rope_theta; a.tab = e->tab; a.attn_index = L.type_index; a.n_attn_layers = e->n_attn > 0 ? e->n_attn : 1;
         a.page_size = c.kv_page_size; a.kv_pool = e->kv_pool; a.segs = segs_of(e->desc, M); a.row_seg = row_seg_of(e->desc, M); a.row_off = row_off_of(e->desc, M);
-        a.row_pos_override = row_pos_override; a.qrot = e->qrot; a.part_o = e->part_o; a.part_ml = e->part_ml; a.nsplit = NSPLIT; a.gated = e->mix; a.M = M;
+        a.row_pos_override = row_pos_override; a.qrot = e->qrot; a.part_o = e->part_o; a.part_ml = e->part_ml; a.nsplit = NSPLIT; a.gated = e->mix; a.M = M; a.max_keys = e->call_keys;
         // a row that is its stream's only row in this call can make its own q/K/V inside the attention kernel;
         // several rows of one stream need every row's K/V in the arena before any of them attends
         // (prefill mode always prepares first and runs the tiled kernel, whatever the row count: chunk-split invariance)
@@ -823,7 +824,10 @@ int32_t run_single(sl_stream* s, const int32_t* tokens, int M, HeadMode head, bo
     }
     std::vector<SegDesc> segs{SegDesc{s->slot, 0, M, 0}};
     if ((rc = upload_descs(e, segs, tokens, M))) return rc;
-    if ((rc = enqueue_call(e, M, 1, head, want_logits))) return rc;
+    e->call_keys = M > GRAPH_MAX_ROWS ? s->kv_len + M : 0;
+    rc = enqueue_call(e, M, 1, head, want_logits);
+    e->call_keys = 0;
+    if (rc) return rc;
     s->kv_len += M; s->parity ^= 1; s->calls += 1;
     return SL_OK;
 }

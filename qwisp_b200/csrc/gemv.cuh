@@ -223,23 +223,29 @@ __device__ __forceinline__ void stage_finish(const StageRegs& sr, const XStage& 
 // (SeedlessFusedVerify.swift:462-471) + sigmoid(gate logit) * shared (:474-484) + residual (SeedlessMetalForward.swift:1024-1028).
 // Every step is one correctly rounded fp16 operation, as in the other forms of the combine.
 __device__ __forceinline__ uint4 moe_combine8(const MoeRow& m, uint4 h, int H, int k0, int lane) {
-    uint4 d[16];
+    uint4 d[8];                                           // (eight rows at a time: top_k is 8, more go round again)
 #pragma unroll
-    for (int k = 0; k < 16; ++k) if (k < m.topk) d[k] = __ldcg(reinterpret_cast<const uint4*>(m.d + (size_t)k * H + k0));
+    for (int k = 0; k < 8; ++k) if (k < m.topk) d[k] = __ldcg(reinterpret_cast<const uint4*>(m.d + (size_t)k * H + k0));
     const uint4 sh = __ldcg(reinterpret_cast<const uint4*>(m.d + (size_t)m.topk * H + k0));
     const unsigned sc = lane < m.topk ? (unsigned)__half_as_ushort(__ldcg(m.scores + lane)) : 0u;
     const __half2 gate = __half2half2(sigmoid_h(__ldcg(m.sgl)));
     __half2 acc[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i] = __float2half2_rn(0.0f);
+    for (int kb = 0; kb < m.topk; kb += 8) {
+        if (kb > 0) {
 #pragma unroll
-    for (int k = 0; k < 16; ++k)
-        if (k < m.topk) {
-            const __half2 w = __half2half2(__ushort_as_half((unsigned short)__shfl_sync(0xffffffffu, sc, k)));
-            const __half2* dk = reinterpret_cast<const __half2*>(&d[k]);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[i] = __hadd2_rn(acc[i], __hmul2_rn(dk[i], w));
+            for (int k = 0; k < 8; ++k) if (kb + k < m.topk) d[k] = __ldcg(reinterpret_cast<const uint4*>(m.d + (size_t)(kb + k) * H + k0));
         }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (kb + k < m.topk) {
+                const __half2 w = __half2half2(__ushort_as_half((unsigned short)__shfl_sync(0xffffffffu, sc, kb + k)));
+                const __half2* dk = reinterpret_cast<const __half2*>(&d[k]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[i] = __hadd2_rn(acc[i], __hmul2_rn(dk[i], w));
+            }
+    }
     __half2* hh = reinterpret_cast<__half2*>(&h);
     const __half2* s2 = reinterpret_cast<const __half2*>(&sh);
 #pragma unroll
@@ -353,6 +359,39 @@ __device__ __forceinline__ void load_xregs(XRegs& xr, const XStage& st, int slic
         xr.x[2 * g] = make_uint4(0, 0, 0, 0); xr.x[2 * g + 1] = make_uint4(0, 0, 0, 0);
         if (n < mr) { xr.x[2 * g] = *reinterpret_cast<const uint4*>(xp + 64 * g); xr.x[2 * g + 1] = *reinterpret_cast<const uint4*>(xp + 64 * g + 8); }
         xr.sx[g] = *reinterpret_cast<const float2*>(st.sxs + (slice * 4 + g) * 8 + 2 * t);
+    }
+}
+// The slice's weights expanded ahead of the activations: fp16 integers as MMA operands; scales and biases as loaded
+struct SliceA { uint32_t a[4][16]; uint4 sc[2]; };
+__device__ __forceinline__ void expand_slice(SliceA& e, const uint4* w_unit, const uint4* s_unit, int lane) {
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        const uint4 wv = w_unit[lane + 32 * g];
+        dequant8(wv.x, e.a[g]); dequant8(wv.z, e.a[g] + 4); dequant8(wv.y, e.a[g] + 8); dequant8(wv.w, e.a[g] + 12);
+    }
+    e.sc[0] = s_unit[lane >> 2]; e.sc[1] = s_unit[8 + (lane >> 2)];
+}
+// what remains of compute_slice() then (same operations)
+__device__ __forceinline__ void compute_expanded(const SliceA& e, const XStage& st, int slice, int n, int t, int mr, float accS[4], float accB[4]) {
+    const __half* xp = st.xs + (size_t)n * st.stride + slice * 256 + 16 * t;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        uint4 X0 = make_uint4(0, 0, 0, 0), X1 = make_uint4(0, 0, 0, 0);
+        if (n < mr) { X0 = *reinterpret_cast<const uint4*>(xp + 64 * g); X1 = *reinterpret_cast<const uint4*>(xp + 64 * g + 8); }
+        const float2 sx2 = *reinterpret_cast<const float2*>(st.sxs + (slice * 4 + g) * 8 + 2 * t);
+        const uint32_t* a = e.a[g];
+        float c[4];
+        mma_f16_z(c, a[0], a[4], a[1], a[5], X0.x, X0.y);
+        mma_f16(c, a[2], a[6], a[3], a[7], X0.z, X0.w);
+        mma_f16(c, a[8], a[12], a[9], a[13], X1.x, X1.y);
+        mma_f16(c, a[10], a[14], a[11], a[15], X1.z, X1.w);
+        const uint4 sv = e.sc[g >> 1];
+        const uint32_t sa_ba = (g & 1) ? sv.z : sv.x, sb_bb = (g & 1) ? sv.w : sv.y;
+        const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&sa_ba)), fb = __half22float2(*reinterpret_cast<const __half2*>(&sb_bb));
+        accS[0] = fmaf(fa.x, c[0], accS[0]); accS[1] = fmaf(fa.x, c[1], accS[1]);
+        accS[2] = fmaf(fb.x, c[2], accS[2]); accS[3] = fmaf(fb.x, c[3], accS[3]);
+        accB[0] = fmaf(fa.y, sx2.x, accB[0]); accB[1] = fmaf(fa.y, sx2.y, accB[1]);
+        accB[2] = fmaf(fb.y, sx2.x, accB[2]); accB[3] = fmaf(fb.y, sx2.y, accB[3]);
     }
 }
 // One slice (4 groups) of a 16-row tile.

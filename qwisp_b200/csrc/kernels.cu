@@ -1038,12 +1038,20 @@ __global__ void __launch_bounds__(512, 1) k_expert_fused(ExpertArgs a) {
         }
     }
     // ---- the CTAs of this slot meet: every tile group's part of the SwiGLU row is in hbuf ----
-    __threadfence();
     __syncthreads();
+    SliceA ex;                                                 // this warp's unit of the down projection, expanded meanwhile
+    if (threadIdx.x == 0) {
+        unsigned* arrive = a.slot_sync + y;
+        // (release: the CTA's stores, ordered before it by the barrier, are visible to whoever acquires the count)
+        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(arrive), "r"(1u) : "memory");
+    }
+    if (UD == 1 && warp < nvu2) {
+        if (!mbar_wait_bounded(ws2.bar, 0) && a.err && lane == 0) atomicOr(a.err, 1u);
+        expand_slice(ex, ws2.w + (size_t)warp * 128, ws2.s + (size_t)warp * 16, lane);
+    }
     if (threadIdx.x == 0) {
         unsigned* arrive = a.slot_sync + y;
         unsigned* leave = a.slot_sync + gridDim.y + y;
-        atomicAdd(arrive, 1u);
         bool ok = false;
         for (int spin = 0; spin < (1 << 22); ++spin) {
             unsigned v;
@@ -1062,6 +1070,14 @@ __global__ void __launch_bounds__(512, 1) k_expert_fused(ExpertArgs a) {
         stage_issue<PRO_PLAIN>(sregs, src, dst, 1, a.I);
         stage_finish<PRO_PLAIN>(sregs, st, src, dst, 1, a.I);
         __syncthreads();
+        if (UD == 1) {
+            if (warp < nvu2) {
+                float accS[4] = {0.f, 0.f, 0.f, 0.f}, accB[4] = {0.f, 0.f, 0.f, 0.f}, v[4];
+                compute_expanded(ex, st, warp & (sl2 - 1), r, t, 1, accS, accB);
+                finish_acc4(accS, accB, t, v);
+                store_partial(red, warp, lane, v);
+            }
+        } else {
         XRegs xr;
         load_xregs(xr, st, warp & (sl2 - 1), r, t, 1);
 #pragma unroll 1
@@ -1076,6 +1092,7 @@ __global__ void __launch_bounds__(512, 1) k_expert_fused(ExpertArgs a) {
                 finish_acc4(accS, accB, t, v);
                 store_partial(red, u, lane, v);
             }
+        }
         }
         __syncthreads();
         for (int i = threadIdx.x; i < TPC2 * 16; i += blockDim.x) {
@@ -1372,13 +1389,15 @@ __device__ __forceinline__ uint4 norm_rope_head(const __half* src, const __half*
     }
     return o;
 }
-// grid (nsplit, KV heads, M), 256 threads, dynamic shared memory 8*8*256 floats.
+// grid (nsplit, KV heads, M), 512 threads, dynamic shared memory 8*8*256 floats.  Warp w takes the split's keys w % 8,
+// w % 8 + 8, ... for the four query heads of group w / 8: half the work per key and half the registers of one warp for all
+// eight heads, twice the warps (a CTA fills a multiprocessor's registers either way).
 // prep != 0 (every row is the only row of its stream in this launch): each CTA norms and rotates its
 // 8 query heads itself, and the CTA whose key range holds the row's own position also makes that
 // position's K and V, stores them in the arena and uses them from shared memory.  prep == 0: q and
 // the arena were written by k_attn_prep.  Either way the CTA that finishes last for a (row, kv head)
 // merges the splits, normalises, rounds to fp16 and applies the sigmoid output gate.
-__global__ void __launch_bounds__(256) k_attn_fused(AttnArgs a, int prep, unsigned* counters) {
+__global__ void __launch_bounds__(512, 1) k_attn_fused(AttnArgs a, int prep, unsigned* counters) {
     extern __shared__ __align__(16) float sm_acc[];           // [8 warps][8 heads][256]
     __shared__ float sm_m[8][ATT_G], sm_l[8][ATT_G];
     __shared__ __align__(16) __half sq[ATT_G][ATT_D];
@@ -1386,7 +1405,7 @@ __global__ void __launch_bounds__(256) k_attn_fused(AttnArgs a, int prep, unsign
     __shared__ int s_last;
     __shared__ float s_cs[32], s_sn[32];
     const int split = blockIdx.x, kvh = blockIdx.y, m = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kw = warp & 7, g0 = (warp >> 3) * 4;
     // Ahead of the programmatic-launch wait: everything that does not depend on this step's in-projection.
     // Stream lengths and page tables were written before the step; with prep != 0 every position below the
     // row's own was stored in an earlier step, so the warp's first keys and values can already be in flight.
@@ -1399,7 +1418,7 @@ __global__ void __launch_bounds__(256) k_attn_fused(AttnArgs a, int prep, unsign
     const bool own = prep && (pos_m >= p0) && (pos_m < p1);
     const __half* rowp = a.inproj + (size_t)m * a.ld;
     uint4 kcur = make_uint4(0, 0, 0, 0), vcur = make_uint4(0, 0, 0, 0);
-    const int first = p0 + warp;
+    const int first = p0 + kw;
     const bool early_kv = prep && first < p1 && first != pos_m;
     if (early_kv) {
         kcur = reinterpret_cast<const uint4*>(kv_ptr(a, slot, first, 0, kvh))[lane];
@@ -1410,36 +1429,34 @@ __global__ void __launch_bounds__(256) k_attn_fused(AttnArgs a, int prep, unsign
     pdl_launch_dependents();
     if (prep) {
         __syncthreads();                                      // the rotation table
+        if (warp < ATT_G) {
         uint4 qo = norm_rope_head_tab(reinterpret_cast<const uint4*>(rowp + (size_t)(kvh * ATT_G + warp) * 2 * ATT_D)[lane], a.q_norm, a.eps, s_cs, s_sn, lane);
         reinterpret_cast<uint4*>(sq[warp])[lane] = qo;
-        if (own && warp == 1) {
+        }
+        if (own && warp == 8) {
             uint4 ko = norm_rope_head_tab(reinterpret_cast<const uint4*>(rowp + a.NH * 2 * ATT_D + kvh * ATT_D)[lane], a.k_norm, a.eps, s_cs, s_sn, lane);
             reinterpret_cast<uint4*>(sk)[lane] = ko;
             reinterpret_cast<uint4*>(kv_ptr(a, slot, pos_m, 0, kvh))[lane] = ko;
         }
-        if (own && warp == 2) {
+        if (own && warp == 9) {
             uint4 vo = reinterpret_cast<const uint4*>(rowp + a.NH * 2 * ATT_D + a.KV * ATT_D + kvh * ATT_D)[lane];
             reinterpret_cast<uint4*>(sv)[lane] = vo;
             reinterpret_cast<uint4*>(kv_ptr(a, slot, pos_m, 1, kvh))[lane] = vo;
         }
-    } else {
+    } else if (warp < ATT_G) {
         reinterpret_cast<uint4*>(sq[warp])[lane] = reinterpret_cast<const uint4*>(a.qrot + ((size_t)m * a.NH + kvh * ATT_G + warp) * ATT_D)[lane];
     }
     __syncthreads();
     const float scale = 0.0625f;                              // 256^-0.5
-    float q[ATT_G][8];
+    float q[4][8], acc[4][8];
 #pragma unroll
-    for (int g = 0; g < ATT_G; ++g) {
-        uint4 qv = reinterpret_cast<const uint4*>(sq[g])[lane];
+    for (int g = 0; g < 4; ++g) {
+        uint4 qv = reinterpret_cast<const uint4*>(sq[g0 + g])[lane];
         const __half* qh = reinterpret_cast<const __half*>(&qv);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) q[g][i] = scale * h2f(qh[i]);
+        for (int i = 0; i < 8; ++i) { q[g][i] = scale * h2f(qh[i]); acc[g][i] = 0.f; }
     }
-    float mx[ATT_G], l[ATT_G], acc[ATT_G][8];
-#pragma unroll
-    for (int g = 0; g < ATT_G; ++g) { mx[g] = -INFINITY; l[g] = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc[g][i] = 0.f; }
+    float mx = -INFINITY, l = 0.f;                            // of head g0 + lane / 8
     // keys of this warp: first, first + 8, ...; the next key's K and V are requested before the current one is used
     auto load_kv = [&](int pos, uint4& kk, uint4& vv) {
         if (own && pos == pos_m) { kk = reinterpret_cast<const uint4*>(sk)[lane]; vv = reinterpret_cast<const uint4*>(sv)[lane]; }
@@ -1457,41 +1474,39 @@ __global__ void __launch_bounds__(256) k_attn_fused(AttnArgs a, int prep, unsign
         float kf[8], vf[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) { kf[i] = h2f(kh[i]); vf[i] = h2f(vh[i]); }
-#pragma unroll
-        for (int g = 0; g < ATT_G; ++g) attn_key_step(q[g], kf, vf, mx[g], l[g], acc[g]);
+        attn_key_step4(q, kf, vf, mx, l, acc, lane);
         kcur = knext; vcur = vnext;
     }
     // ---- merge the 8 warps: all heads at once through shared memory ----
-    if (lane == 0) {
-#pragma unroll
-        for (int g = 0; g < ATT_G; ++g) { sm_m[warp][g] = mx[g]; sm_l[warp][g] = l[g]; }
-    }
+    if ((lane & 7) == 0) { sm_m[kw][g0 + (lane >> 3)] = mx; sm_l[kw][g0 + (lane >> 3)] = l; }
     __syncthreads();
 #pragma unroll
-    for (int g = 0; g < ATT_G; ++g) {
+    for (int gi = 0; gi < 4; ++gi) {
+        const int g = g0 + gi;
         float m8[8];
 #pragma unroll
         for (int w = 0; w < 8; ++w) m8[w] = sm_m[w][g];
-        const float gm = attn_warps_max(m8);
-        float f = (mx[g] == -INFINITY) ? 0.f : __expf(mx[g] - gm);
-        float4 lo = make_float4(acc[g][0] * f, acc[g][1] * f, acc[g][2] * f, acc[g][3] * f);
-        float4 hi = make_float4(acc[g][4] * f, acc[g][5] * f, acc[g][6] * f, acc[g][7] * f);
-        float4* dst = reinterpret_cast<float4*>(sm_acc + ((size_t)warp * ATT_G + g) * ATT_D + lane * 8);
+        const float gm = attn_warps_max(m8), mine = sm_m[kw][g];
+        float f = (mine == -INFINITY) ? 0.f : __expf(mine - gm);
+        float4 lo = make_float4(acc[gi][0] * f, acc[gi][1] * f, acc[gi][2] * f, acc[gi][3] * f);
+        float4 hi = make_float4(acc[gi][4] * f, acc[gi][5] * f, acc[gi][6] * f, acc[gi][7] * f);
+        float4* dst = reinterpret_cast<float4*>(sm_acc + ((size_t)kw * ATT_G + g) * ATT_D + lane * 8);
         dst[0] = lo; dst[1] = hi;
     }
     __syncthreads();
     {
-        const int d = threadIdx.x;                            // 256 threads = 256 dims
+        const int d = threadIdx.x & 255;                      // 512 threads = 256 dims of two halves of the heads
         float* po = a.part_o + (((size_t)m * a.NH + kvh * ATT_G) * a.nsplit + split) * ATT_D;
 #pragma unroll
-        for (int g = 0; g < ATT_G; ++g) {
+        for (int gi = 0; gi < 4; ++gi) {
+            const int g = g0 + gi;
             float o = 0.f;
 #pragma unroll
             for (int w = 0; w < 8; ++w) o += sm_acc[((size_t)w * ATT_G + g) * ATT_D + d];
             po[(size_t)g * a.nsplit * ATT_D + d] = o;
         }
-        if (d < ATT_G) {
-            const int g = d;
+        if (threadIdx.x < ATT_G) {
+            const int g = threadIdx.x;
             float m8[8], l8[8];
             for (int w = 0; w < 8; ++w) { m8[w] = sm_m[w][g]; l8[w] = sm_l[w][g]; }
             const float gm = attn_warps_max(m8);
@@ -1502,7 +1517,7 @@ __global__ void __launch_bounds__(256) k_attn_fused(AttnArgs a, int prep, unsign
     }
     // ---- the CTA that finishes last for this (row, kv head) merges the splits ----
     // (the output gate of this warp's head does not depend on the other CTAs: fetched before the ticket)
-    const uint4 gvv = reinterpret_cast<const uint4*>(rowp + (size_t)(kvh * ATT_G + warp) * 2 * ATT_D + ATT_D)[lane];
+    const uint4 gvv = reinterpret_cast<const uint4*>(rowp + (size_t)(kvh * ATT_G + kw) * 2 * ATT_D + ATT_D)[lane];
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1512,7 +1527,7 @@ __global__ void __launch_bounds__(256) k_attn_fused(AttnArgs a, int prep, unsign
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    {
+    if (warp < ATT_G) {
         const int g = warp, h = kvh * ATT_G + g;
         const float* po = a.part_o + ((size_t)m * a.NH + h) * a.nsplit * ATT_D;
         const float* pml = a.part_ml + ((size_t)m * a.NH + h) * a.nsplit * 2;
@@ -1528,8 +1543,8 @@ void launch_attn_fused(const AttnArgs& a, bool prep, unsigned* counters, cudaStr
     const size_t smem = (size_t)8 * ATT_G * ATT_D * sizeof(float);
     if (!configured) { cudaFuncSetAttribute(k_attn_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)a.nsplit, (unsigned)a.KV, (unsigned)a.M);
-    cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.gridDim = dim3((unsigned)(a.max_keys > 0 && a.max_keys < 32 * a.nsplit ? (a.max_keys + 31) / 32 : a.nsplit), (unsigned)a.KV, (unsigned)a.M);
+    cfg.blockDim = dim3(512); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute attr[1];
     set_pdl(cfg, attr, pdl);
     AttnArgs copy = a; int p = prep ? 1 : 0;

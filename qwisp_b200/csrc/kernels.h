@@ -130,6 +130,7 @@ struct AttnArgs {
     __half* qrot;                        // [M][NH][256]
     float* part_o; float* part_ml;       // split partials
     int nsplit;
+    int max_keys = 0;                    // most keys of a row, where the host knows it (0: not): no CTAs for splits that cannot exist
     __half* gated;                       // [M][NH*256]
     int M;
 };

@@ -116,6 +116,42 @@ __device__ __forceinline__ void attn_key_step(const float q[8], const float kf[8
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = fmaf(acc[i], factor, es * vf[i]);
 }
+// Butterfly sums of FOUR values per lane at once: the additions are those of four warp_sum() calls (partners at lane
+// distance 16, 8, 4, 2, 1, in that order; an addition's operands may be swapped, which changes nothing), but the first
+// two levels hand each value to a different quarter of the warp, so 6 shuffles do the work of 20.  On return the lanes
+// 8i .. 8i+7 hold the total of value i.
+__device__ __forceinline__ float warp_sum4(float a, float b, float c, float d, int lane) {
+    const bool hi = (lane & 16) != 0;
+    const float r0 = __shfl_xor_sync(0xffffffffu, hi ? a : c, 16), r1 = __shfl_xor_sync(0xffffffffu, hi ? b : d, 16);
+    const float x = (hi ? c : a) + r0, y = (hi ? d : b) + r1;           // lanes < 16: values a, b; lanes >= 16: c, d
+    const bool b3 = (lane & 8) != 0;
+    float z = (b3 ? y : x) + __shfl_xor_sync(0xffffffffu, b3 ? x : y, 8);
+    z += __shfl_xor_sync(0xffffffffu, z, 4);
+    z += __shfl_xor_sync(0xffffffffu, z, 2);
+    z += __shfl_xor_sync(0xffffffffu, z, 1);
+    return z;
+}
+// attn_key_step() for four query heads at once: lanes 8i .. 8i+7 keep head i's maximum and normaliser (mx, l) and make its
+// two exponentials, which every lane then fetches for its dims
+__device__ __forceinline__ void attn_key_step4(const float q[4][8], const float kf[8], const float vf[8], float& mx, float& l, float acc[4][8], int lane) {
+    float sc[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        sc[g] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sc[g] = fmaf(q[g][i], kf[i], sc[g]);
+    }
+    const float s = warp_sum4(sc[0], sc[1], sc[2], sc[3], lane);
+    const float nm = fmaxf(mx, s);
+    const float factor = __expf(mx - nm), es = __expf(s - nm);
+    mx = nm; l = fmaf(l, factor, es);
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        const float fg = __shfl_sync(0xffffffffu, factor, 8 * g), eg = __shfl_sync(0xffffffffu, es, 8 * g);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[g][i] = fmaf(acc[g][i], fg, eg * vf[i]);
+    }
+}
 // merge of the 8 key-warps of a split for one head: the maximum, and the rescaled normaliser
 __device__ __forceinline__ float attn_warps_max(const float m8[8]) {
     float gm = -INFINITY;
@@ -148,12 +184,19 @@ __device__ __forceinline__ uint4 attn_merge_splits(int used, int lane, uint4 gvv
     for (int j = 0; j < 2; ++j) { fv[j] = (msv[j] == -INFINITY) ? 0.f : __expf(msv[j] - gm); tot += lsv[j] * fv[j]; }
     tot = warp_sum(tot);
     float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int sp = 0; sp < used; ++sp) {
-        float f = __shfl_sync(0xffffffffu, (sp < 32) ? fv[0] : fv[1], sp & 31);
-        float4 x0, x1;
-        ld_o(sp, x0, x1);
-        o[0] = fmaf(x0.x, f, o[0]); o[1] = fmaf(x0.y, f, o[1]); o[2] = fmaf(x0.z, f, o[2]); o[3] = fmaf(x0.w, f, o[3]);
-        o[4] = fmaf(x1.x, f, o[4]); o[5] = fmaf(x1.y, f, o[5]); o[6] = fmaf(x1.z, f, o[6]); o[7] = fmaf(x1.w, f, o[7]);
+    for (int s0 = 0; s0 < used; s0 += 8) {                // eight splits' partials in flight at a time, added in ascending order
+        float4 x0[8], x1[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) if (s0 + i < used) ld_o(s0 + i, x0[i], x1[i]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int sp = s0 + i;
+            const float f = __shfl_sync(0xffffffffu, (sp < 32) ? fv[0] : fv[1], sp & 31);
+            if (sp < used) {
+                o[0] = fmaf(x0[i].x, f, o[0]); o[1] = fmaf(x0[i].y, f, o[1]); o[2] = fmaf(x0[i].z, f, o[2]); o[3] = fmaf(x0[i].w, f, o[3]);
+                o[4] = fmaf(x1[i].x, f, o[4]); o[5] = fmaf(x1[i].y, f, o[5]); o[6] = fmaf(x1[i].z, f, o[6]); o[7] = fmaf(x1[i].w, f, o[7]);
+            }
+        }
     }
     const __half* gh = reinterpret_cast<const __half*>(&gvv);
     uint4 outv; __half* oh = reinterpret_cast<__half*>(&outv);

@@ -351,8 +351,8 @@ int32_t build_runtime(sl_engine* e) {
     CU(e, cudaHostAlloc((void**)&e->err_host, 4 * sizeof(unsigned), cudaHostAllocMapped));
     memset(e->err_host, 0, 4 * sizeof(unsigned));
     CU(e, cudaHostGetDevicePointer((void**)&e->err_flag, e->err_host, 0));
-    if ((rc = dalloc(e, &e->att_counters, (size_t)R * c.attn_kv_heads))) return rc;
-    CU(e, cudaMemset(e->att_counters, 0, (size_t)R * c.attn_kv_heads * sizeof(unsigned)));
+    if ((rc = dalloc(e, &e->att_counters, (size_t)R * c.attn_kv_heads * 2))) return rc;
+    CU(e, cudaMemset(e->att_counters, 0, (size_t)R * c.attn_kv_heads * 2 * sizeof(unsigned)));
     CU(e, cudaMemset(e->hist_pos, 0, sizeof(int)));
     CU(e, cudaMallocHost(&e->pin_i, desc_ints(R) * sizeof(int)));
     e->pin_out_ints = R > 4096 ? (size_t)R : 4096;

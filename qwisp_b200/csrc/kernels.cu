@@ -1389,23 +1389,24 @@ __device__ __forceinline__ uint4 norm_rope_head(const __half* src, const __half*
     }
     return o;
 }
-// grid (nsplit, KV heads, M), 512 threads, dynamic shared memory 8*8*256 floats.  Warp w takes the split's keys w % 8,
-// w % 8 + 8, ... for the four query heads of group w / 8: half the work per key and half the registers of one warp for all
-// eight heads, twice the warps (a CTA fills a multiprocessor's registers either way).
+// grid (nsplit, KV heads * 2, M), 256 threads, dynamic shared memory 8*4*256 floats.  A CTA takes four of the kv head's
+// eight query heads, warp w the split's keys w, w + 8, ...: two CTAs fit a multiprocessor (one warp for all eight heads
+// needs 200 registers, so that one CTA's merge had nothing to run beside it).
 // prep != 0 (every row is the only row of its stream in this launch): each CTA norms and rotates its
 // 8 query heads itself, and the CTA whose key range holds the row's own position also makes that
 // position's K and V, stores them in the arena and uses them from shared memory.  prep == 0: q and
 // the arena were written by k_attn_prep.  Either way the CTA that finishes last for a (row, kv head)
 // merges the splits, normalises, rounds to fp16 and applies the sigmoid output gate.
-__global__ void __launch_bounds__(512, 1) k_attn_fused(AttnArgs a, int prep, unsigned* counters) {
-    extern __shared__ __align__(16) float sm_acc[];           // [8 warps][8 heads][256]
-    __shared__ float sm_m[8][ATT_G], sm_l[8][ATT_G];
-    __shared__ __align__(16) __half sq[ATT_G][ATT_D];
+__global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, unsigned* counters) {
+    extern __shared__ __align__(16) float sm_acc[];           // [8 warps][4 heads][256]
+    constexpr int HG = 4;                                     // query heads of a CTA
+    __shared__ float sm_m[8][HG], sm_l[8][HG];
+    __shared__ __align__(16) __half sq[HG][ATT_D];
     __shared__ __align__(16) __half sk[ATT_D], sv[ATT_D];
     __shared__ int s_last;
     __shared__ float s_cs[32], s_sn[32];
-    const int split = blockIdx.x, kvh = blockIdx.y, m = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kw = warp & 7, g0 = (warp >> 3) * 4;
+    const int split = blockIdx.x, kvh = blockIdx.y >> 1, h0 = blockIdx.y * HG, m = blockIdx.z;      // h0: first query head
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Ahead of the programmatic-launch wait: everything that does not depend on this step's in-projection.
     // Stream lengths and page tables were written before the step; with prep != 0 every position below the
     // row's own was stored in an earlier step, so the warp's first keys and values can already be in flight.
@@ -1418,7 +1419,7 @@ __global__ void __launch_bounds__(512, 1) k_attn_fused(AttnArgs a, int prep, uns
     const bool own = prep && (pos_m >= p0) && (pos_m < p1);
     const __half* rowp = a.inproj + (size_t)m * a.ld;
     uint4 kcur = make_uint4(0, 0, 0, 0), vcur = make_uint4(0, 0, 0, 0);
-    const int first = p0 + kw;
+    const int first = p0 + warp;
     const bool early_kv = prep && first < p1 && first != pos_m;
     if (early_kv) {
         kcur = reinterpret_cast<const uint4*>(kv_ptr(a, slot, first, 0, kvh))[lane];
@@ -1429,34 +1430,34 @@ __global__ void __launch_bounds__(512, 1) k_attn_fused(AttnArgs a, int prep, uns
     pdl_launch_dependents();
     if (prep) {
         __syncthreads();                                      // the rotation table
-        if (warp < ATT_G) {
-        uint4 qo = norm_rope_head_tab(reinterpret_cast<const uint4*>(rowp + (size_t)(kvh * ATT_G + warp) * 2 * ATT_D)[lane], a.q_norm, a.eps, s_cs, s_sn, lane);
+        if (warp < HG) {
+        uint4 qo = norm_rope_head_tab(reinterpret_cast<const uint4*>(rowp + (size_t)(h0 + warp) * 2 * ATT_D)[lane], a.q_norm, a.eps, s_cs, s_sn, lane);
         reinterpret_cast<uint4*>(sq[warp])[lane] = qo;
         }
-        if (own && warp == 8) {
+        if (own && warp == 4) {
             uint4 ko = norm_rope_head_tab(reinterpret_cast<const uint4*>(rowp + a.NH * 2 * ATT_D + kvh * ATT_D)[lane], a.k_norm, a.eps, s_cs, s_sn, lane);
             reinterpret_cast<uint4*>(sk)[lane] = ko;
-            reinterpret_cast<uint4*>(kv_ptr(a, slot, pos_m, 0, kvh))[lane] = ko;
+            if (!(blockIdx.y & 1)) reinterpret_cast<uint4*>(kv_ptr(a, slot, pos_m, 0, kvh))[lane] = ko;
         }
-        if (own && warp == 9) {
+        if (own && warp == 5) {
             uint4 vo = reinterpret_cast<const uint4*>(rowp + a.NH * 2 * ATT_D + a.KV * ATT_D + kvh * ATT_D)[lane];
             reinterpret_cast<uint4*>(sv)[lane] = vo;
-            reinterpret_cast<uint4*>(kv_ptr(a, slot, pos_m, 1, kvh))[lane] = vo;
+            if (!(blockIdx.y & 1)) reinterpret_cast<uint4*>(kv_ptr(a, slot, pos_m, 1, kvh))[lane] = vo;
         }
-    } else if (warp < ATT_G) {
-        reinterpret_cast<uint4*>(sq[warp])[lane] = reinterpret_cast<const uint4*>(a.qrot + ((size_t)m * a.NH + kvh * ATT_G + warp) * ATT_D)[lane];
+    } else if (warp < HG) {
+        reinterpret_cast<uint4*>(sq[warp])[lane] = reinterpret_cast<const uint4*>(a.qrot + ((size_t)m * a.NH + h0 + warp) * ATT_D)[lane];
     }
     __syncthreads();
     const float scale = 0.0625f;                              // 256^-0.5
-    float q[4][8], acc[4][8];
+    float q[HG][8], acc[HG][8];
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        uint4 qv = reinterpret_cast<const uint4*>(sq[g0 + g])[lane];
+    for (int g = 0; g < HG; ++g) {
+        uint4 qv = reinterpret_cast<const uint4*>(sq[g])[lane];
         const __half* qh = reinterpret_cast<const __half*>(&qv);
 #pragma unroll
         for (int i = 0; i < 8; ++i) { q[g][i] = scale * h2f(qh[i]); acc[g][i] = 0.f; }
     }
-    float mx = -INFINITY, l = 0.f;                            // of head g0 + lane / 8
+    float mx = -INFINITY, l = 0.f;                            // of head h0 + lane / 8
     // keys of this warp: first, first + 8, ...; the next key's K and V are requested before the current one is used
     auto load_kv = [&](int pos, uint4& kk, uint4& vv) {
         if (own && pos == pos_m) { kk = reinterpret_cast<const uint4*>(sk)[lane]; vv = reinterpret_cast<const uint4*>(sv)[lane]; }
@@ -1478,57 +1479,55 @@ __global__ void __launch_bounds__(512, 1) k_attn_fused(AttnArgs a, int prep, uns
         kcur = knext; vcur = vnext;
     }
     // ---- merge the 8 warps: all heads at once through shared memory ----
-    if ((lane & 7) == 0) { sm_m[kw][g0 + (lane >> 3)] = mx; sm_l[kw][g0 + (lane >> 3)] = l; }
+    if ((lane & 7) == 0) { sm_m[warp][lane >> 3] = mx; sm_l[warp][lane >> 3] = l; }
     __syncthreads();
 #pragma unroll
-    for (int gi = 0; gi < 4; ++gi) {
-        const int g = g0 + gi;
+    for (int g = 0; g < HG; ++g) {
         float m8[8];
 #pragma unroll
         for (int w = 0; w < 8; ++w) m8[w] = sm_m[w][g];
-        const float gm = attn_warps_max(m8), mine = sm_m[kw][g];
+        const float gm = attn_warps_max(m8), mine = sm_m[warp][g];
         float f = (mine == -INFINITY) ? 0.f : __expf(mine - gm);
-        float4 lo = make_float4(acc[gi][0] * f, acc[gi][1] * f, acc[gi][2] * f, acc[gi][3] * f);
-        float4 hi = make_float4(acc[gi][4] * f, acc[gi][5] * f, acc[gi][6] * f, acc[gi][7] * f);
-        float4* dst = reinterpret_cast<float4*>(sm_acc + ((size_t)kw * ATT_G + g) * ATT_D + lane * 8);
+        float4 lo = make_float4(acc[g][0] * f, acc[g][1] * f, acc[g][2] * f, acc[g][3] * f);
+        float4 hi = make_float4(acc[g][4] * f, acc[g][5] * f, acc[g][6] * f, acc[g][7] * f);
+        float4* dst = reinterpret_cast<float4*>(sm_acc + ((size_t)warp * HG + g) * ATT_D + lane * 8);
         dst[0] = lo; dst[1] = hi;
     }
     __syncthreads();
     {
-        const int d = threadIdx.x & 255;                      // 512 threads = 256 dims of two halves of the heads
-        float* po = a.part_o + (((size_t)m * a.NH + kvh * ATT_G) * a.nsplit + split) * ATT_D;
+        const int d = threadIdx.x;                            // 256 threads = 256 dims
+        float* po = a.part_o + (((size_t)m * a.NH + h0) * a.nsplit + split) * ATT_D;
 #pragma unroll
-        for (int gi = 0; gi < 4; ++gi) {
-            const int g = g0 + gi;
+        for (int g = 0; g < HG; ++g) {
             float o = 0.f;
 #pragma unroll
-            for (int w = 0; w < 8; ++w) o += sm_acc[((size_t)w * ATT_G + g) * ATT_D + d];
+            for (int w = 0; w < 8; ++w) o += sm_acc[((size_t)w * HG + g) * ATT_D + d];
             po[(size_t)g * a.nsplit * ATT_D + d] = o;
         }
-        if (threadIdx.x < ATT_G) {
+        if (threadIdx.x < HG) {
             const int g = threadIdx.x;
             float m8[8], l8[8];
             for (int w = 0; w < 8; ++w) { m8[w] = sm_m[w][g]; l8[w] = sm_l[w][g]; }
             const float gm = attn_warps_max(m8);
             const float ls = attn_warps_lsum(m8, l8, gm);
-            float* pml = a.part_ml + (((size_t)m * a.NH + kvh * ATT_G + g) * a.nsplit + split) * 2;
+            float* pml = a.part_ml + (((size_t)m * a.NH + h0 + g) * a.nsplit + split) * 2;
             pml[0] = gm; pml[1] = ls;
         }
     }
     // ---- the CTA that finishes last for this (row, kv head) merges the splits ----
     // (the output gate of this warp's head does not depend on the other CTAs: fetched before the ticket)
-    const uint4 gvv = reinterpret_cast<const uint4*>(rowp + (size_t)(kvh * ATT_G + kw) * 2 * ATT_D + ATT_D)[lane];
+    const uint4 gvv = reinterpret_cast<const uint4*>(rowp + (size_t)(h0 + (warp & 3)) * 2 * ATT_D + ATT_D)[lane];
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned ticket = atomicAdd(counters + m * a.KV + kvh, 1u);
+        unsigned ticket = atomicAdd(counters + m * gridDim.y + blockIdx.y, 1u);
         s_last = (ticket == (unsigned)used - 1) ? 1 : 0;
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    if (warp < ATT_G) {
-        const int g = warp, h = kvh * ATT_G + g;
+    if (warp < HG) {
+        const int h = h0 + warp;
         const float* po = a.part_o + ((size_t)m * a.NH + h) * a.nsplit * ATT_D;
         const float* pml = a.part_ml + ((size_t)m * a.NH + h) * a.nsplit * 2;
         const uint4 outv = attn_merge_splits(used, lane, gvv,
@@ -1536,15 +1535,15 @@ __global__ void __launch_bounds__(512, 1) k_attn_fused(AttnArgs a, int prep, uns
             [&](int sp) { return __ldcg(reinterpret_cast<const float2*>(pml) + sp); });
         reinterpret_cast<uint4*>(a.gated + ((size_t)m * a.NH + h) * ATT_D)[lane] = outv;
     }
-    if (threadIdx.x == 0) counters[m * a.KV + kvh] = 0u;
+    if (threadIdx.x == 0) counters[m * gridDim.y + blockIdx.y] = 0u;
 }
 void launch_attn_fused(const AttnArgs& a, bool prep, unsigned* counters, cudaStream_t st, bool pdl) {
     static bool configured = false;
-    const size_t smem = (size_t)8 * ATT_G * ATT_D * sizeof(float);
+    const size_t smem = (size_t)8 * 4 * ATT_D * sizeof(float);
     if (!configured) { cudaFuncSetAttribute(k_attn_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(a.max_keys > 0 && a.max_keys < 32 * a.nsplit ? (a.max_keys + 31) / 32 : a.nsplit), (unsigned)a.KV, (unsigned)a.M);
-    cfg.blockDim = dim3(512); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.gridDim = dim3((unsigned)(a.max_keys > 0 && a.max_keys < 32 * a.nsplit ? (a.max_keys + 31) / 32 : a.nsplit), (unsigned)a.KV * 2, (unsigned)a.M);
+    cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute attr[1];
     set_pdl(cfg, attr, pdl);
     AttnArgs copy = a; int p = prep ? 1 : 0;

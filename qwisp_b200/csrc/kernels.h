@@ -270,7 +270,7 @@ bool launch_attn_prefill(const AttnArgs& a, int nsegs, cudaStream_t st);
 void launch_gdn_rows(const GdnArgs& a, int M, int nsegs, cudaStream_t st);   // the same result by k_gdn_prep + k_gdn_scan (needs the scratch fields)
 size_t gdn_qk_floats(int Hk, int rows); size_t gdn_vg_bytes(int Hv, int rows);
 void launch_attn_prep(const AttnArgs& a, cudaStream_t st);
-// q/k prep (when every row is its stream's only row) + split-KV decode + merge in one launch; counters: M*KV zeros
+// q/k prep (when every row is its stream's only row) + split-KV decode + merge in one launch; counters: 2*M*KV zeros
 void launch_attn_fused(const AttnArgs& a, bool prep, unsigned* counters, cudaStream_t st, bool pdl);
 void launch_step_end(const StepEndArgs& a, cudaStream_t st);
 // xq / sxq (optional): the normed rows also in the prepared form of the many-row kernels

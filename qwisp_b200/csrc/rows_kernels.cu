@@ -18,6 +18,7 @@
 //   k_moe_combine    weighted sum of a row's top-k expert rows in ascending k + shared expert + residual.
 #include "kernels.h"
 #include "gemv.cuh"
+#include "mixer_math.cuh"
 #include "route.cuh"
 
 namespace sl {
@@ -571,6 +572,100 @@ __global__ void __launch_bounds__(256, 2) k_router_rows(RouterArgs a) {
         __syncthreads();                       // the buffer is refilled by the next iteration's stage()
     }
 }
+// The fp16 router for H <= 2048.  Bound by instruction issue: with one expert per warp and halves in registers and shared
+// memory every multiply-add came with two conversions (131 us at 512 rows).  Here a warp keeps TWO router rows as f32
+// registers, the rows of a group are converted once per CTA, and two rows run side by side: four independent chains of
+// the same multiply-adds in the same order.  gr: rows of a group (fewer for short calls, so that more CTAs share the work).
+template <int NB>
+__global__ void __launch_bounds__(256, 1) k_router_rows2(RouterArgs a, int gr) {
+    extern __shared__ __align__(16) unsigned char smem[];                   // [2][gr][H] halves, [gr][NB][2][128] f32
+    constexpr int H = NB * 256;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    __half* raw = reinterpret_cast<__half*>(smem);
+    float* xf = reinterpret_cast<float*>(smem + (size_t)2 * gr * H * 2);
+    const bool tail = (blockIdx.x == gridDim.x - 1);                        // the shared gate: warp w takes row w of a group
+    const int e0 = blockIdx.x * 16 + warp * 2;
+    float w[2][NB * 8];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const bool ok = tail ? j == 0 : e0 + j < a.E;
+        const __half* wrow = tail ? a.shared_gate : a.router + (size_t)(e0 + j) * H;
+#pragma unroll
+        for (int kb = 0; kb < NB; ++kb) {
+            const uint4 v = ok ? *reinterpret_cast<const uint4*>(wrow + kb * 256 + lane * 8) : make_uint4(0, 0, 0, 0);
+            const __half* vh = reinterpret_cast<const __half*>(&v);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[j][kb * 8 + i] = h2f(vh[i]);
+        }
+    }
+    const int ngroups = (a.M + gr - 1) / gr;
+    auto stage = [&](int rg, int b) {
+        const int mr = min(gr, a.M - rg * gr);
+        for (int i = tid; i < mr * (H / 8); i += 256)
+            cp_async16(raw + (size_t)b * gr * H + (size_t)i * 8, a.h + ((size_t)rg * gr + i / (H / 8)) * a.ldh + (size_t)(i % (H / 8)) * 8);
+        cp_async_commit();
+    };
+    auto dots = [&](const float* x0, const float* x1, float& a00, float& a01, float& a10, float& a11) {
+        a00 = 0.f; a01 = 0.f; a10 = 0.f; a11 = 0.f;                         // aRE: row R, expert E
+#pragma unroll
+        for (int kb = 0; kb < NB; ++kb) {
+            float p[8], q[8];
+            *reinterpret_cast<float4*>(p) = *reinterpret_cast<const float4*>(x0 + kb * 256 + lane * 4);
+            *reinterpret_cast<float4*>(p + 4) = *reinterpret_cast<const float4*>(x0 + kb * 256 + 128 + lane * 4);
+            *reinterpret_cast<float4*>(q) = *reinterpret_cast<const float4*>(x1 + kb * 256 + lane * 4);
+            *reinterpret_cast<float4*>(q + 4) = *reinterpret_cast<const float4*>(x1 + kb * 256 + 128 + lane * 4);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                a00 = fmaf(p[i], w[0][kb * 8 + i], a00); a01 = fmaf(p[i], w[1][kb * 8 + i], a01);
+                a10 = fmaf(q[i], w[0][kb * 8 + i], a10); a11 = fmaf(q[i], w[1][kb * 8 + i], a11);
+            }
+        }
+    };
+    int it = 0;
+    if ((int)blockIdx.y < ngroups) stage(blockIdx.y, 0);
+    for (int rg = blockIdx.y; rg < ngroups; rg += gridDim.y, ++it) {
+        const int b = it & 1;
+        if (rg + (int)gridDim.y < ngroups) { stage(rg + gridDim.y, b ^ 1); cp_async_wait<1>(); } else cp_async_wait<0>();
+        __syncthreads();
+        const int m0 = rg * gr, mr = min(gr, a.M - m0);
+        for (int i = tid; i < mr * (H / 8); i += 256) {                     // 8 inputs: 4 into each plane of their 256-wide block
+            const uint4 v = *reinterpret_cast<const uint4*>(raw + (size_t)b * gr * H + (size_t)i * 8);
+            const __half2* h = reinterpret_cast<const __half2*>(&v);
+            const float2 f0 = __half22float2(h[0]), f1 = __half22float2(h[1]), f2 = __half22float2(h[2]), f3 = __half22float2(h[3]);
+            float* d = xf + (size_t)(i >> 5) * 256 + (i & 31) * 4;
+            *reinterpret_cast<float4*>(d) = make_float4(f0.x, f0.y, f1.x, f1.y);
+            *reinterpret_cast<float4*>(d + 128) = make_float4(f2.x, f2.y, f3.x, f3.y);
+        }
+        __syncthreads();
+        if (tail) {
+            if (warp < mr) {
+                float d, x, y, z;
+                dots(xf + (size_t)warp * H, xf + (size_t)warp * H, d, x, y, z);
+                d = warp_sum(d);
+                if (lane == 0) a.sgl[m0 + warp] = f2h(d);
+            }
+        } else if (e0 < a.E) {
+            for (int c = 0; c < mr; c += 2) {
+                const int c1 = min(c + 1, mr - 1);
+                float a00, a01, a10, a11;
+                dots(xf + (size_t)c * H, xf + (size_t)c1 * H, a00, a01, a10, a11);
+                const float s = warp_sum4(a00, a01, a10, a11, lane);
+                const int row = m0 + c + (lane >> 4), e = e0 + ((lane >> 3) & 1);
+                if ((lane & 7) == 0 && row < m0 + mr && e < a.E) a.logits[(size_t)row * a.E + e] = f2h(s);
+            }
+        }
+    }
+}
+template <int NB>
+static void launch_router_rows2(const RouterArgs& a, cudaStream_t st) {
+    const int gx = (a.E + 15) / 16 + 1, want = sm_count() / gx > 0 ? sm_count() / gx : 1;
+    int gr = 2; while (gr < 8 && gr * want < a.M) gr *= 2;
+    const int ngroups = (a.M + gr - 1) / gr, gy = ngroups < want ? ngroups : want;
+    const size_t smem = (size_t)gr * NB * 256 * 8;
+    static bool configured = false;
+    if (!configured) { cudaFuncSetAttribute(k_router_rows2<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * NB * 256 * 8); configured = true; }
+    profile_launch("k_router_rows", st, [&] { k_router_rows2<NB><<<dim3((unsigned)gx, (unsigned)gy), 256, smem, st>>>(a, gr); return 0; });
+}
 // grid (ceil(M / 8)), 256 threads: one warp per row.  Expert-parallel: grid (M), one row per CTA.
 __global__ void __launch_bounds__(256) k_route_rows(RouterArgs a) {
     __shared__ float s_route[8][512 + 32];
@@ -642,81 +737,79 @@ __global__ void __launch_bounds__(256) k_route_rows(RouterArgs a) {
     }
 }
 // Prefill mode: the fp16 router logits as a small tensor-core GEMM (mma.sync m16n8k16, f32 accumulators): a CTA of 4 warps
-// computes 64 rows x 64 experts, K in chunks of 64 through two cp.async buffers (16-byte pieces swizzled by the row).
+// computes 32 rows x 32 experts, K in chunks of 128 through three cp.async stages (16-byte pieces swizzled by the row).
+// Bound by latency: 64 x 64 tiles left 12 CTAs at 129 rows and 64 at 1024, with one chunk of 64 in flight and the
+// shared-gate rows of a tile in one CTA.
 // Not the bit pattern of the strict router (the f32 sums run in MMA order), but a row's logits depend on that row only
 // and K is walked in a fixed order, so they do not depend on how a prompt is cut into calls.  The shared-gate logit is a
 // plain warp dot (the strict order) done by the CTAs of the first expert tile.
 __device__ __forceinline__ void rt_ldsm_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(smem_u32(p)));
 }
-__device__ __forceinline__ __half* rt_at(__half* base, int row, int chunk) { return base + row * 64 + ((chunk ^ (row & 7)) << 3); }   // rows of 64 halves
+constexpr int RT_K = 128, RT_T = 32, RT_ST = 3;               // inputs per chunk, rows / experts per CTA, stages
+__device__ __forceinline__ __half* rt_at(__half* base, int row, int chunk) { return base + row * RT_K + ((chunk ^ (row & 7)) << 3); }   // rows of 128 halves
 __global__ void __launch_bounds__(128) k_router_mma(RouterArgs a) {
-    __shared__ __align__(128) __half As[2][64 * 64], Bs[2][64 * 64];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * 64, e0 = blockIdx.y * 64;
-    const int rows = min(64, a.M - m0), cols = min(64, a.E - e0);
-    auto stage = [&](int kc, int b) {
-        for (int i = tid; i < 64 * 8; i += 128) {
-            const int r = i >> 3, c = i & 7;
-            if (r < rows) cp_async16(rt_at(As[b], r, c), a.h + (size_t)(m0 + r) * a.ldh + kc * 64 + c * 8);
-            else *reinterpret_cast<uint4*>(rt_at(As[b], r, c)) = make_uint4(0, 0, 0, 0);
-            if (r < cols) cp_async16(rt_at(Bs[b], r, c), a.router + (size_t)(e0 + r) * a.H + kc * 64 + c * 8);
-            else *reinterpret_cast<uint4*>(rt_at(Bs[b], r, c)) = make_uint4(0, 0, 0, 0);
+    __shared__ __align__(128) __half sm[RT_ST][2][RT_T * RT_K];               // 48 KB: [stage][rows | experts]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wr = warp >> 1, wc = warp & 1;
+    const int m0 = blockIdx.x * RT_T, e0 = blockIdx.y * RT_T;
+    const int rows = min(RT_T, a.M - m0), cols = min(RT_T, a.E - e0);
+    auto stage = [&](int kc) {
+        __half *As = sm[kc % RT_ST][0], *Bs = sm[kc % RT_ST][1];
+        for (int i = tid; i < RT_T * (RT_K / 8); i += 128) {
+            const int r = i / (RT_K / 8), c = i % (RT_K / 8);
+            if (r < rows) cp_async16(rt_at(As, r, c), a.h + (size_t)(m0 + r) * a.ldh + kc * RT_K + c * 8);
+            else *reinterpret_cast<uint4*>(rt_at(As, r, c)) = make_uint4(0, 0, 0, 0);
+            if (r < cols) cp_async16(rt_at(Bs, r, c), a.router + (size_t)(e0 + r) * a.H + kc * RT_K + c * 8);
+            else *reinterpret_cast<uint4*>(rt_at(Bs, r, c)) = make_uint4(0, 0, 0, 0);
         }
-        cp_async_commit();
     };
-    float acc[8][4];
-#pragma unroll
-    for (int n = 0; n < 8; ++n) { acc[n][0] = 0.f; acc[n][1] = 0.f; acc[n][2] = 0.f; acc[n][3] = 0.f; }
-    const int nk = a.H >> 6;
-    stage(0, 0);
+    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    const int nk = a.H / RT_K;
+    for (int kc = 0; kc < RT_ST - 1; ++kc) { if (kc < nk) stage(kc); cp_async_commit(); }
     for (int kc = 0; kc < nk; ++kc) {
-        const int b = kc & 1;
-        if (kc + 1 < nk) { stage(kc + 1, b ^ 1); cp_async_wait<1>(); } else cp_async_wait<0>();
-        __syncthreads();
+        cp_async_wait<RT_ST - 2>();
+        __syncthreads();                       // chunk kc is here, and everyone is done with the chunk whose stage is refilled now
+        if (kc + RT_ST - 1 < nk) stage(kc + RT_ST - 1);
+        cp_async_commit();
+        __half *As = sm[kc % RT_ST][0], *Bs = sm[kc % RT_ST][1];
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-            uint32_t a0, a1, a2, a3;
-            rt_ldsm_x4(a0, a1, a2, a3, rt_at(As[b], warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, ks * 2 + (lane >> 4)));
-#pragma unroll
-            for (int np = 0; np < 4; ++np) {
-                uint32_t b0, b1, b2, b3;
-                const int mi = lane >> 3;
-                rt_ldsm_x4(b0, b1, b2, b3, rt_at(Bs[b], (np * 2 + (mi >> 1)) * 8 + (lane & 7), ks * 2 + (mi & 1)));
-                mma_f16(acc[np * 2], a0, a1, a2, a3, b0, b1);
-                mma_f16(acc[np * 2 + 1], a0, a1, a2, a3, b2, b3);
-            }
+        for (int ks = 0; ks < RT_K / 16; ++ks) {
+            uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
+            const int mi = lane >> 3;
+            rt_ldsm_x4(a0, a1, a2, a3, rt_at(As, wr * 16 + (lane & 7) + (mi & 1) * 8, ks * 2 + (lane >> 4)));
+            rt_ldsm_x4(b0, b1, b2, b3, rt_at(Bs, wc * 16 + (mi >> 1) * 8 + (lane & 7), ks * 2 + (mi & 1)));
+            mma_f16(acc[0], a0, a1, a2, a3, b0, b1);
+            mma_f16(acc[1], a0, a1, a2, a3, b2, b3);
         }
-        __syncthreads();
     }
 #pragma unroll
-    for (int n = 0; n < 8; ++n)
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int r = warp * 16 + (lane >> 2) + 8 * (i >> 1), c = n * 8 + 2 * (lane & 3) + (i & 1);
+            const int r = wr * 16 + (lane >> 2) + 8 * (i >> 1), c = wc * 16 + n * 8 + 2 * (lane & 3) + (i & 1);
             if (r < rows && c < cols) a.logits[(size_t)(m0 + r) * a.E + e0 + c] = f2h(acc[n][i]);
         }
-    if (blockIdx.y == 0) {                     // shared-gate logit of the CTA's rows: lane l owns 8 inputs of every 256-wide block
-        for (int r = warp; r < rows; r += 4) {
-            const __half* xrow = a.h + (size_t)(m0 + r) * a.ldh;
-            float s = 0.f;
-            for (int kb = 0; kb < (a.H >> 8); ++kb) {
-                const uint4 xv = *reinterpret_cast<const uint4*>(xrow + kb * 256 + lane * 8);
-                const uint4 wv = *reinterpret_cast<const uint4*>(a.shared_gate + kb * 256 + lane * 8);
-                const __half* xh = reinterpret_cast<const __half*>(&xv);
-                const __half* wh = reinterpret_cast<const __half*>(&wv);
+    // shared-gate logits, the rows dealt to the expert tiles: lane l owns 8 inputs of every 256-wide block
+    for (int r = blockIdx.y + warp * gridDim.y; r < rows; r += 4 * gridDim.y) {
+        const __half* xrow = a.h + (size_t)(m0 + r) * a.ldh;
+        float s = 0.f;
+#pragma unroll 8
+        for (int kb = 0; kb < (a.H >> 8); ++kb) {
+            const uint4 xv = *reinterpret_cast<const uint4*>(xrow + kb * 256 + lane * 8);
+            const uint4 wv = *reinterpret_cast<const uint4*>(a.shared_gate + kb * 256 + lane * 8);
+            const __half* xh = reinterpret_cast<const __half*>(&xv);
+            const __half* wh = reinterpret_cast<const __half*>(&wv);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) s = fmaf(h2f(xh[i]), h2f(wh[i]), s);
-            }
-            s = warp_sum(s);
-            if (lane == 0) a.sgl[m0 + r] = f2h(s);
+            for (int i = 0; i < 8; ++i) s = fmaf(h2f(xh[i]), h2f(wh[i]), s);
         }
+        s = warp_sum(s);
+        if (lane == 0) a.sgl[m0 + r] = f2h(s);
     }
 }
 // prefill mode, fp16 router: logits on the tensor cores, then the routing / pair-list kernel.  false: not covered.
 bool launch_router_mma(const RouterArgs& a, cudaStream_t st) {
     if (a.E > 256 || a.H % 256 || a.norm_w || a.router_q8 || a.sg_q8) return false;
-    const dim3 grid((unsigned)((a.M + 63) / 64), (unsigned)((a.E + 63) / 64));
+    const dim3 grid((unsigned)((a.M + RT_T - 1) / RT_T), (unsigned)((a.E + RT_T - 1) / RT_T));
     profile_launch("k_router_mma", st, [&] { k_router_mma<<<grid, 128, 0, st>>>(a); return 0; });
     profile_launch("k_route_rows", st, [&] { k_route_rows<<<a.epd.sig.world > 0 ? a.M : (a.M + 7) / 8, 256, 0, st>>>(a); return 0; });
     return true;
@@ -737,7 +830,10 @@ bool launch_router_rows(const RouterArgs& a, cudaStream_t st) {
     int gy = (2 * sm_count() + gx - 1) / gx; if (gy > ngroups) gy = ngroups; if (gy < 1) gy = 1;
     const dim3 grid((unsigned)gx, (unsigned)gy);
     const bool q8 = a.router_q8 != nullptr;
-    profile_launch("k_router_rows", st, [&] {
+    if (!q8 && a.H == 512) launch_router_rows2<2>(a, st);
+    else if (!q8 && a.H == 1024) launch_router_rows2<4>(a, st);
+    else if (!q8 && a.H == 2048) launch_router_rows2<8>(a, st);
+    else profile_launch("k_router_rows", st, [&] {
         if (q8) k_router_rows<true><<<grid, 256, smem, st>>>(a); else k_router_rows<false><<<grid, 256, smem, st>>>(a);
         return 0;
     });

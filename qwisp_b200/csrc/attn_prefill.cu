@@ -57,6 +57,8 @@ __global__ void __launch_bounds__(128) k_attn_prefill(AttnArgs a) {
     const int rows = min(AP_BM, a.M - m0);
     const int pos_last = pos0 + m0 + rows - 1;
     const int ntiles = pos_last / AP_BN + 1;
+    pdl_wait();
+    pdl_launch_dependents();
     // ---- the query tile and the first key tile
     for (int i = tid; i < AP_BM * 32; i += 128) {
         const int r = i >> 5, c = i & 31;
@@ -194,13 +196,13 @@ __global__ void __launch_bounds__(128) k_attn_prefill(AttnArgs a) {
     }
 }
 // Needs: one segment, page_size a multiple of 32, NH = ATT_G * KV.  Returns false when the call is not covered.
-bool launch_attn_prefill(const AttnArgs& a, int nsegs, cudaStream_t st) {
+bool launch_attn_prefill(const AttnArgs& a, int nsegs, cudaStream_t st, bool pdl) {
     if (nsegs != 1 || a.page_size % AP_BN || a.NH != ATT_G * a.KV || a.row_pos_override) return false;
     const size_t smem = (size_t)(AP_BM * ATT_D + 2 * 2 * AP_BN * ATT_D) * sizeof(__half);
     static bool configured = false;
     if (!configured) { cudaFuncSetAttribute(k_attn_prefill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
     const dim3 grid((unsigned)((a.M + AP_BM - 1) / AP_BM), (unsigned)a.NH);
-    profile_launch("k_attn_prefill", st, [&] { k_attn_prefill<<<grid, 128, smem, st>>>(a); return 0; });
+    profile_launch("k_attn_prefill", st, [&] { return launch_pdl(pdl, k_attn_prefill, grid, 128, smem, st, a); });
     return true;
 }
 

@@ -526,10 +526,10 @@ bool enqueue_router(sl_engine* e, const RouterArgs& ra, int M, bool pdl, __half*
     if ((M > 1 || e->hybrid) && e->use_rows && !ra.no_route && e->E <= 256 && ra.norm_w && ra.ldh == e->H) {
         const bool ep = ra.epd.sig.world > 0;
         if (ep) launch_final_norm_ep(ra.h, ra.norm_w, ra.eps, M, e->H, ra.p, ra.epd, st);     // the rows leave for the peers here
-        else launch_final_norm(ra.h, ra.norm_w, ra.eps, M, e->H, ra.p, st, xq, sxq);
+        else launch_final_norm(ra.h, ra.norm_w, ra.eps, M, e->H, ra.p, st, pdl, xq, sxq);
         RouterArgs rb = ra; rb.h = ra.p; rb.ldh = e->H; rb.norm_w = nullptr; rb.ep_rows_sent = ep ? 1 : 0;
-        if (e->hybrid && launch_router_mma(rb, st)) return xq != nullptr;
-        if (launch_router_rows(rb, st)) return xq != nullptr;
+        if (e->hybrid && launch_router_mma(rb, st, pdl)) return xq != nullptr;
+        if (launch_router_rows(rb, st, pdl)) return xq != nullptr;
         // not covered: the one-kernel router norms the rows again from the original input
     }
     launch_router(ra, st, pdl);
@@ -566,9 +566,9 @@ int32_t enqueue_moe_ep(sl_engine* e, const LayerW& L, RouterArgs ra, int M, __ha
     const int nslots = T * topk < local_e ? T * topk : local_e;
     bool rows_done = false;
     if (T > 8 && local_e <= 256 && e->use_rows && T <= e->cfg.max_rows) {
-        launch_rows_prep_plain(P.pbuf[r], H, T, H, e->xq_p, e->sx_p, st);
+        launch_rows_prep_plain(P.pbuf[r], H, T, H, e->xq_p, e->sx_p, st, false);
         ea.xq = e->xq_p; ea.sxq = e->sx_p; ea.csum = e->csum;
-        rows_done = launch_expert_rows_gateup(ea, st) && launch_expert_rows_down(ea, st);
+        rows_done = launch_expert_rows_gateup(ea, st, false) && launch_expert_rows_down(ea, st, false);
     }
     if (!rows_done) {
         launch_expert_gateup(ea, nslots, st, false);
@@ -609,13 +609,14 @@ void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half
     }
     const bool tc_experts = e->hybrid && e->E <= 256 && e->use_rows;      // prefill mode: for any row count (chunk-split invariance)
     const bool rows_experts = !tc_experts && M > 1 && e->E <= 256 && e->use_rows;
-    const bool prepared = enqueue_router(e, ra, M, e->use_pdl, rows_experts ? e->xq_p : nullptr, e->sx_p);
-    if (fused && launch_expert_fused(ea, st, e->use_pdl)) return;                      // one launch for gate/up + down
+    const bool pdl = e->use_pdl;
+    const bool prepared = enqueue_router(e, ra, M, pdl, rows_experts ? e->xq_p : nullptr, e->sx_p);
+    if (fused && launch_expert_fused(ea, st, pdl)) return;                      // one launch for gate/up + down
     if (tc_experts) {
         // prefill mode: grouped GEMMs on the tensor cores, then the combine kernel
         ea.tile_counter = nullptr;
-        if (launch_expert_tc_gateup(ea, st) && launch_expert_tc_down(ea, st)) {
-            launch_moe_combine(e->dbuf, e->dbuf + (size_t)M * e->topk * e->H, e->scores, e->sgl, M, e->H, e->topk, resid, plain_out, st);
+        if (launch_expert_tc_gateup(ea, st, pdl) && launch_expert_tc_down(ea, st, pdl)) {
+            launch_moe_combine(e->dbuf, e->dbuf + (size_t)M * e->topk * e->H, e->scores, e->sgl, M, e->H, e->topk, resid, plain_out, st, pdl);
             return;
         }
         ea.tile_counter = e->tile_counters;
@@ -623,29 +624,30 @@ void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half
     if (rows_experts || (tc_experts && M > 1)) {
         // many rows: the normed rows are prepared once (by the norm kernel when it ran), the experts run without CTA-wide
         // barriers, the combine is its own kernel
-        if (!prepared) launch_rows_prep_plain(e->p, e->H, M, e->H, e->xq_p, e->sx_p, st);
+        if (!prepared) launch_rows_prep_plain(e->p, e->H, M, e->H, e->xq_p, e->sx_p, st, pdl);
         ea.xq = e->xq_p; ea.sxq = e->sx_p; ea.csum = e->csum; ea.tile_counter = nullptr;
-        if (launch_expert_rows_gateup(ea, st) && launch_expert_rows_down(ea, st)) {
-            launch_moe_combine(e->dbuf, e->dbuf + (size_t)M * e->topk * e->H, e->scores, e->sgl, M, e->H, e->topk, resid, plain_out, st);
+        if (launch_expert_rows_gateup(ea, st, pdl) && launch_expert_rows_down(ea, st, pdl)) {
+            launch_moe_combine(e->dbuf, e->dbuf + (size_t)M * e->topk * e->H, e->scores, e->sgl, M, e->H, e->topk, resid, plain_out, st, pdl);
             return;
         }
         ea.tile_counter = e->tile_counters;
     }
-    launch_expert_gateup(ea, nslots, st, e->use_pdl);
-    launch_expert_down(ea, nslots, st, e->use_pdl);
+    launch_expert_gateup(ea, nslots, st, pdl);
+    launch_expert_down(ea, nslots, st, pdl);
 }
 
 // mixer of one layer: input rows are normed inside (norm_w != nullptr) or already normed
 void enqueue_mixer(sl_engine* e, const LayerW& L, const __half* rows, const __half* norm_w, int M, int nsegs,
                    __half* resid, __half* plain_out, const int* row_pos_override, const MoeRow* pending = nullptr) {
     cudaStream_t st = e->stream;
+    const bool pdl = e->use_pdl;
     const sl_config& c = e->cfg;
     DenseArgs d{}; d.err = e->err_flag; d.norm_scratch = e->normed; d.xq = e->use_rows ? e->xq : nullptr; d.sxq = e->sxq; d.q = L.r_in; d.N = (int)L.in_proj.N; d.K = e->H; d.M = M;
     d.x = rows; d.ldx = e->H; d.nw = norm_w; d.eps = c.rms_eps; d.y = e->inproj; d.ldy = (int)L.in_proj.N;
     if (e->use_prefetch) pf_q4(d.pf, 0, L.r_out);
     d.tc = e->hybrid;
     if (pending) d.moe = *pending;                             // rows: the residual before the last block's combine; resid: where it is kept after it
-    launch_dense(pending ? PRO_MOERMS : (norm_w ? PRO_RMSNORM : PRO_PLAIN), EPI_STORE, d, st, e->use_pdl);
+    launch_dense(pending ? PRO_MOERMS : (norm_w ? PRO_RMSNORM : PRO_PLAIN), EPI_STORE, d, st, pdl);
     DenseArgs o{};
     o.err = e->err_flag; o.q = L.r_out; o.N = e->H; o.K = L.out_proj.K; o.M = M;
     o.eps = c.rms_eps; o.y = resid ? resid : plain_out; o.ldy = e->H; o.tc = e->hybrid; o.norm_scratch = e->normed; o.xq = e->use_rows ? e->xq : nullptr; o.sxq = e->sxq;
@@ -659,10 +661,10 @@ void enqueue_mixer(sl_engine* e, const LayerW& L, const __half* rows, const __ha
         g.Hk = c.gdn_k_heads; g.Hv = c.gdn_v_heads; g.eps = c.rms_eps; g.tab = e->tab; g.gdn_index = L.type_index; g.segs = segs_of(e->desc, M); g.y = e->mix;
         g.row_seg = row_seg_of(e->desc, M); g.qk = e->gdn_qk; g.vg = e->gdn_vg; g.err = e->err_flag;
         // segments of many rows: the state-independent part for all rows side by side, then the bare recurrence (same bits)
-        if (e->use_rows && M >= 16) launch_gdn_rows(g, M, nsegs, st);
-        else launch_gdn_core(g, nsegs, st, e->use_pdl);
+        if (e->use_rows && M >= 16) launch_gdn_rows(g, M, nsegs, st, pdl);
+        else launch_gdn_core(g, nsegs, st, pdl);
         o.x = e->mix; o.ldx = e->valDim; o.nw = L.gdn_norm; o.nw32 = L.gdn_norm32; o.z = e->inproj + e->convDim; o.ldz = e->gdn_in;
-        launch_dense(L.gdn_norm32 ? PRO_NORMGATE32 : PRO_NORMGATE, resid ? EPI_RESID : EPI_STORE, o, st, e->use_pdl);
+        launch_dense(L.gdn_norm32 ? PRO_NORMGATE32 : PRO_NORMGATE, resid ? EPI_RESID : EPI_STORE, o, st, pdl);
     } else {
         AttnArgs a{}; a.inproj = e->inproj; a.ld = e->attn_in; a.q_norm = L.q_norm; a.k_norm = L.k_norm; a.NH = c.attn_heads; a.KV = c.attn_kv_heads;
         a.eps = c.rms_eps; a.theta = c.rope_theta; a.tab = e->tab; a.attn_index = L.type_index; a.n_attn_layers = e->n_attn > 0 ? e->n_attn : 1;
@@ -673,12 +675,12 @@ void enqueue_mixer(sl_engine* e, const LayerW& L, const __half* rows, const __ha
         // (prefill mode always prepares first and runs the tiled kernel, whatever the row count: chunk-split invariance)
         const bool tiled = e->hybrid && nsegs == 1 && row_pos_override == nullptr && c.kv_page_size % 32 == 0;
         const bool self_prep = !tiled && (M == nsegs) && (row_pos_override == nullptr || M == 1);
-        if (!self_prep) launch_attn_prep(a, st);
+        if (!self_prep) launch_attn_prep(a, st, pdl);
         // prefill mode, one stream's chunk: the keys are walked once for 64 rows at a time on the tensor cores
-        if (!(tiled && launch_attn_prefill(a, nsegs, st)))
-            launch_attn_fused(a, self_prep, e->att_counters, st, e->use_pdl && self_prep);
+        if (!(tiled && launch_attn_prefill(a, nsegs, st, pdl)))
+            launch_attn_fused(a, self_prep, e->att_counters, st, pdl);
         o.x = e->mix; o.ldx = e->attn_out;
-        launch_dense(PRO_PLAIN, resid ? EPI_RESID : EPI_STORE, o, st, e->use_pdl);
+        launch_dense(PRO_PLAIN, resid ? EPI_RESID : EPI_STORE, o, st, pdl);
     }
 }
 
@@ -700,7 +702,7 @@ void enqueue_step(sl_engine* e, int M, int nsegs, HeadMode head, bool want_logit
         enqueue_moe(e, L, next, h, e->H, true, M, h, nullptr, next && M == 1 && !e->hybrid && !e->ep_step ? &moe : nullptr);
     }
     if (head == HEAD_NORMED) {
-        launch_final_norm(h, e->final_norm, e->cfg.rms_eps, M, e->H, e->normed, st);
+        launch_final_norm(h, e->final_norm, e->cfg.rms_eps, M, e->H, e->normed, st, e->use_pdl);
     } else if (head == HEAD_ARGMAX || head == HEAD_LOGITS) {
         DenseArgs d{}; d.q = e->r_lm_head; d.N = e->V; d.K = e->H; d.M = M;
         d.x = h; d.ldx = e->H; d.nw = e->final_norm; d.eps = e->cfg.rms_eps;
@@ -1480,7 +1482,7 @@ int32_t sl_op_qmm4_tc_device(const void* x_dev, const void* wr_dev, const void* 
     if (M <= 0 || N <= 0 || K <= 0 || N % 16 || !k_ok(K)) return SL_ERR_INVALID;
     if (!device_ok()) return SL_ERR_NO_DEVICE;
     Q4R q{}; q.wr = (const uint4*)wr_dev; q.sr = (const uint4*)sr_dev; q.tiles = N / 16; q.K = K;
-    int err = launch_gemm_tc(q, N, K, M, (const __half*)x_dev, K, (__half*)y_dev, N, false, nullptr, (cudaStream_t)cuda_stream);
+    int err = launch_gemm_tc(q, N, K, M, (const __half*)x_dev, K, (__half*)y_dev, N, false, nullptr, (cudaStream_t)cuda_stream, false);
     return err == 0 ? SL_OK : SL_ERR_CUDA;
 }
 int32_t sl_op_qmm4(const uint16_t* x, const uint32_t* w, const uint16_t* sc, const uint16_t* bi, int32_t M, int32_t K, int32_t N, uint16_t* y) {

@@ -28,6 +28,8 @@ __global__ void __launch_bounds__(128) k_gdn_prep(GdnArgs a) {
     __shared__ float red_s[R][8];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.y * R, nr = min(R, a.M - m0);
+    pdl_wait();
+    pdl_launch_dependents();
     const SegDesc seg = a.segs[a.row_seg[m0]];
     const int t0 = m0 - seg.row0;
     const int keyDim = a.Hk * GDN_DK, valDim = a.Hv * GDN_DV, convDim = 2 * keyDim + valDim;
@@ -264,13 +266,14 @@ static void launch_scan_t(const GdnArgs& a, int nsegs, cudaStream_t st) {
     if (!configured) { cudaFuncSetAttribute(k_gdn_scan<CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
     profile_launch("k_gdn_scan", st, [&] { k_gdn_scan<CH><<<dim3(4, (unsigned)a.Hv, (unsigned)nsegs), 128, smem, st>>>(a); return 0; });
 }
-void launch_gdn_rows(const GdnArgs& in, int M, int nsegs, cudaStream_t st) {
+void launch_gdn_rows(const GdnArgs& in, int M, int nsegs, cudaStream_t st, bool pdl) {
     GdnArgs a = in; a.M = M;
     profile_launch("k_gdn_prep", st, [&] {
-        if (nsegs == 1) k_gdn_prep<8><<<dim3((unsigned)(a.Hk + a.Hv), (unsigned)((M + 7) / 8)), 128, 0, st>>>(a);
-        else k_gdn_prep<1><<<dim3((unsigned)(a.Hk + a.Hv), (unsigned)M), 128, 0, st>>>(a);
-        return 0;
+        if (nsegs == 1) return launch_pdl(pdl, k_gdn_prep<8>, dim3((unsigned)(a.Hk + a.Hv), (unsigned)((M + 7) / 8)), 128, 0, st, a);
+        return launch_pdl(pdl, k_gdn_prep<1>, dim3((unsigned)(a.Hk + a.Hv), (unsigned)M), 128, 0, st, a);
     });
+    // (the scan is an ordinary launch: started early, its CTAs went to the multiprocessors that k_gdn_prep had left free,
+    // several to one, and 17 rows took 7 us longer)
     // one row per segment (batched decode): the state's traffic is the time, small buffers leave room for more CTAs per SM
     if (M == nsegs) launch_scan_t<1>(a, nsegs, st);
     else launch_scan_t<32>(a, nsegs, st);

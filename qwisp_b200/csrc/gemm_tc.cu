@@ -217,6 +217,7 @@ struct ExpertWork {
         NRT = (ntiles + 7) / 8;                                             // groups of 128 weight rows
         npair = a.M * a.topk;
         nshared = a.M_shared >= 0 ? a.M_shared : a.M;
+        pdl_wait();                                                         // (the lists)
         n_active = slot_table(sh.tab, a.lists, NT, nshared);
         __syncthreads();
     }
@@ -314,6 +315,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_launch_dependents();
     const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
     const int items = work.items(), KS = work.inputs() >> 7, NRT = work.NRT;              // KS: stages per item (even)
     const int lo = (int)((long)items * blockIdx.x / gridDim.x), hi = (int)((long)items * (blockIdx.x + 1) / gridDim.x);
@@ -398,6 +400,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         }
     } else if (warp < TC_EPI0 || warp >= TC_DQ0) {
         // ------------------------------------------------------------ load: the activation rows of every stage
+        pdl_wait();
         constexpr int NP = NT / 16;                                         // rows of a stage per thread, 2 pieces of 16 bytes each
         const int lt = (warp < TC_EPI0 ? warp - 1 : 3) * 32 + lane;
         // the 8 lanes of a quarter warp write into the 8 rows of one atom (distinct swizzled chunks) and read 4 x 64 contiguous
@@ -448,6 +451,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
         // ------------------------------------------------------------ epilogue
+        pdl_wait();                                                         // (residual rows, and rows that the kernel before may still read)
         typename W::Epi epi;
         const int quarter = warp - TC_EPI0;
         int blk = blk0, rt = rt0;
@@ -472,7 +476,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512u) : "memory");
 }
 template <class W, int NT, int ST, int U>
-static int launch_tc_t(const typename W::Args& a, int grid, cudaStream_t st) {
+static int launch_tc_t(const typename W::Args& a, int grid, cudaStream_t st, bool pdl) {
     constexpr size_t smem = (size_t)ST * NT * 256 + 1024;
     static bool configured = false;
     if (!configured) {
@@ -480,16 +484,15 @@ static int launch_tc_t(const typename W::Args& a, int grid, cudaStream_t st) {
         if (err != cudaSuccess) return (int)err;
         configured = true;
     }
-    k_tc<W, NT, ST, U><<<grid, TC_THREADS, smem, st>>>(a);
-    return (int)cudaGetLastError();
+    return launch_pdl(pdl, k_tc<W, NT, ST, U>, dim3((unsigned)grid), TC_THREADS, smem, st, a);
 }
 template <int NT, int ST>
-static int launch_gemm_tc_t(const GemmTcArgs& a, cudaStream_t st) {
+static int launch_gemm_tc_t(const GemmTcArgs& a, cudaStream_t st, bool pdl) {
     const int items = ((a.N + TC_ROWS - 1) / TC_ROWS) * ((a.M + NT - 1) / NT), grid = items < sm_count() ? items : sm_count();
-    if (a.K % 512 == 0) return launch_tc_t<DenseWork<NT>, NT, ST, 2>(a, grid, st);
-    return launch_tc_t<DenseWork<NT>, NT, ST, 1>(a, grid, st);
+    if (a.K % 512 == 0) return launch_tc_t<DenseWork<NT>, NT, ST, 2>(a, grid, st, pdl);
+    return launch_tc_t<DenseWork<NT>, NT, ST, 1>(a, grid, st, pdl);
 }
-int launch_gemm_tc(const Q4R& q, int N, int K, int M, const __half* x, int ldx, __half* y, int ldy, bool add_to_y, unsigned* err, cudaStream_t st) {
+int launch_gemm_tc(const Q4R& q, int N, int K, int M, const __half* x, int ldx, __half* y, int ldy, bool add_to_y, unsigned* err, cudaStream_t st, bool pdl) {
     if (N % 16 || K % 256) return -1;
     GemmTcArgs a{q, N, K, M, x, ldx, y, ldy, add_to_y ? 1 : 0, err};
     // The token tile is a scheduling choice only (a token's column never interacts with another's).  An item's time is the
@@ -502,24 +505,24 @@ int launch_gemm_tc(const Q4R& q, int N, int K, int M, const __half* x, int ldx, 
         const long items = row_tiles * ((M + nts[i] - 1) / nts[i]), c = (items + sm_count() - 1) / sm_count() * cost[i];
         if (i == 0 || c < best_cost) { best = i; best_cost = c; }
     }
-    if (best == 0) return launch_gemm_tc_t<128, 4>(a, st);
-    if (best == 1) return launch_gemm_tc_t<64, 6>(a, st);
-    return launch_gemm_tc_t<32, 6>(a, st);
+    if (best == 0) return launch_gemm_tc_t<128, 4>(a, st, pdl);
+    if (best == 1) return launch_gemm_tc_t<64, 6>(a, st, pdl);
+    return launch_gemm_tc_t<32, 6>(a, st, pdl);
 }
 
 constexpr int XT_NT = 64;            // rows of an expert's block: a 1024-token chunk gives an expert about 32
 template <bool DOWN>
-static bool launch_expert_tc_t(const ExpertArgs& a, cudaStream_t st) {
+static bool launch_expert_tc_t(const ExpertArgs& a, cudaStream_t st, bool pdl) {
     const int K = DOWN ? a.I : a.H;
     if (K % 256 || a.ep_pairs_per_rank > 0) return false;              // (expert-parallel calls keep the row kernels)
     int rc = 0;
     profile_launch(DOWN ? "k_expert_umma_down" : "k_expert_umma_gateup", st, [&] {
-        rc = K % 512 == 0 ? launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, 2>(a, sm_count(), st) : launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, 1>(a, sm_count(), st);
+        rc = K % 512 == 0 ? launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, 2>(a, sm_count(), st, pdl) : launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, 1>(a, sm_count(), st, pdl);
         return rc;
     });
     return rc == 0;
 }
-bool launch_expert_tc_gateup(const ExpertArgs& a, cudaStream_t st) { return launch_expert_tc_t<false>(a, st); }
-bool launch_expert_tc_down(const ExpertArgs& a, cudaStream_t st) { return launch_expert_tc_t<true>(a, st); }
+bool launch_expert_tc_gateup(const ExpertArgs& a, cudaStream_t st, bool pdl) { return launch_expert_tc_t<false>(a, st, pdl); }
+bool launch_expert_tc_down(const ExpertArgs& a, cudaStream_t st, bool pdl) { return launch_expert_tc_t<true>(a, st, pdl); }
 
 }  // namespace sl

@@ -355,6 +355,8 @@ __global__ void __launch_bounds__(256) k_normgate_rows(const __half* y, int ldy,
                                                        float eps, int M, int K, __half* out) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunks = K >> 8;
     const long u = (long)blockIdx.x * 8 + warp;
+    pdl_wait();
+    pdl_launch_dependents();
     if (u >= (long)M * chunks) return;
     const int row = (int)(u / chunks), k0 = ((int)(u % chunks) << 8) + lane * 8;
     const uint4 v = __ldcg(reinterpret_cast<const uint4*>(y + (size_t)row * ldy + k0));
@@ -362,11 +364,11 @@ __global__ void __launch_bounds__(256) k_normgate_rows(const __half* y, int ldy,
     const uint4 wv = *reinterpret_cast<const uint4*>(nw + (k0 & 127));
     *reinterpret_cast<uint4*>(out + (size_t)row * K + k0) = normgate8<PRO>(v, zv, wv, nw32, k0, eps);
 }
-static void launch_normgate_rows(int pro, const DenseArgs& a, cudaStream_t st) {
+static void launch_normgate_rows(int pro, const DenseArgs& a, cudaStream_t st, bool pdl) {
     ProfScope ps("k_normgate_rows", (double)a.M * a.K * 6, st);
     const unsigned grid = (unsigned)(((long)a.M * (a.K >> 8) + 7) / 8);
-    if (pro == PRO_NORMGATE32) k_normgate_rows<PRO_NORMGATE32><<<grid, 256, 0, st>>>(a.x, a.ldx, a.z, a.ldz, a.nw, a.nw32, a.eps, a.M, a.K, a.norm_scratch);
-    else k_normgate_rows<PRO_NORMGATE><<<grid, 256, 0, st>>>(a.x, a.ldx, a.z, a.ldz, a.nw, a.nw32, a.eps, a.M, a.K, a.norm_scratch);
+    launch_pdl(pdl, pro == PRO_NORMGATE32 ? k_normgate_rows<PRO_NORMGATE32> : k_normgate_rows<PRO_NORMGATE>, dim3(grid), 256, 0, st,
+               a.x, a.ldx, a.z, a.ldz, a.nw, a.nw32, a.eps, a.M, a.K, a.norm_scratch);
     COUNT_LAUNCH();
 }
 
@@ -385,21 +387,21 @@ void launch_dense(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pd
         const __half* x = a.x; int ldx = a.ldx;
         if (pro == PRO_RMSNORM) {
             if (a.ldx != a.K) goto gemv_path;                  // the row kernel reads dense rows
-            launch_final_norm(a.x, a.nw, a.eps, a.M, a.K, a.norm_scratch, st);
+            launch_final_norm(a.x, a.nw, a.eps, a.M, a.K, a.norm_scratch, st, pdl);
             x = a.norm_scratch; ldx = a.K;
         } else if (pro_is_normgate(pro)) {
-            launch_normgate_rows(pro, a, st);
+            launch_normgate_rows(pro, a, st, pdl);
             x = a.norm_scratch; ldx = a.K;
         }
         {
             ProfScope ps("k_gemm_umma", (double)a.N * a.K * 0.5625 + (double)a.M * (a.K + a.N) * 2, st);
-            launch_gemm_tc(a.q, a.N, a.K, a.M, x, ldx, a.y, a.ldy, epi == EPI_RESID, a.err, st);
+            launch_gemm_tc(a.q, a.N, a.K, a.M, x, ldx, a.y, a.ldy, epi == EPI_RESID, a.err, st, pdl);
             COUNT_LAUNCH();
         }
         return;
     }
 gemv_path:
-    if (a.M > ROWS_PER_PASS && launch_dense_rows(pro, epi, a, st)) return;
+    if (a.M > ROWS_PER_PASS && launch_dense_rows(pro, epi, a, st, pdl)) return;
     const GemvPlan pl = gemv_plan(a.K, epi == EPI_SWIGLU ? a.N / 8 : a.N / 16, 1, sm_count());
 #define SL_CASE(P, E)                                                                                       \
     if (pro == P && epi == E) {                                                                             \
@@ -505,6 +507,8 @@ __device__ __forceinline__ void block_rmsnorm_row(const __half* src, const __hal
 }
 __global__ void k_final_norm(const __half* h, const __half* w, float eps, int H, __half* out, __half* xq, float* sxq) {
     __shared__ float sm8[8];
+    pdl_wait();
+    pdl_launch_dependents();
     block_rmsnorm_row(h + (size_t)blockIdx.x * H, w, eps, H, out + (size_t)blockIdx.x * H, sm8, false, make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0),
                       xq ? xq + (size_t)blockIdx.x * H : nullptr, sxq ? sxq + (size_t)blockIdx.x * (H >> 6) : nullptr);
 }
@@ -521,9 +525,9 @@ __global__ void k_final_norm_ep(const __half* h, const __half* w, float eps, int
             *reinterpret_cast<uint4*>(epd.pbuf[d] + ((size_t)epd.sig.rank * M + m) * H + k) = v;
     }
 }
-void launch_final_norm(const __half* h, const __half* w, float eps, int M, int H, __half* out, cudaStream_t st, __half* xq, float* sxq) {
+void launch_final_norm(const __half* h, const __half* w, float eps, int M, int H, __half* out, cudaStream_t st, bool pdl, __half* xq, float* sxq) {
     ProfScope ps("k_final_norm", (double)M * H * 4, st);
-    k_final_norm<<<M, 256, 0, st>>>(h, w, eps, H, out, xq, sxq);
+    launch_pdl(pdl, k_final_norm, dim3((unsigned)M), 256, 0, st, h, w, eps, H, out, xq, sxq);
     COUNT_LAUNCH();
 }
 void launch_final_norm_ep(const __half* h, const __half* w, float eps, int M, int H, __half* out, const EpDispatch& epd, cudaStream_t st) {
@@ -1304,6 +1308,8 @@ __global__ void __launch_bounds__(32) k_attn_prep(AttnArgs a) {
     const int m = blockIdx.y, hidx = blockIdx.x, lane = threadIdx.x;
     const int slot = a.segs[a.row_seg[m]].slot;
     const int pos = row_position(a, m);
+    pdl_wait();
+    pdl_launch_dependents();
     const __half* rowp = a.inproj + (size_t)m * a.ld;
     if (hidx >= a.NH + a.KV) {                               // V copy
         int kvh = hidx - a.NH - a.KV;
@@ -1348,10 +1354,10 @@ __global__ void __launch_bounds__(32) k_attn_prep(AttnArgs a) {
     if (isq) reinterpret_cast<uint4*>(a.qrot + ((size_t)m * a.NH + hidx) * ATT_D)[lane] = o;
     else reinterpret_cast<uint4*>(kv_ptr(a, slot, pos, 0, hidx - a.NH))[lane] = o;
 }
-void launch_attn_prep(const AttnArgs& a, cudaStream_t st) {
+void launch_attn_prep(const AttnArgs& a, cudaStream_t st, bool pdl) {
     dim3 grid(a.NH + 2 * a.KV, a.M);
     ProfScope ps("k_attn_prep", 0.0, st);
-    k_attn_prep<<<grid, 32, 0, st>>>(a);
+    launch_pdl(pdl, k_attn_prep, grid, 32, 0, st, a);
     COUNT_LAUNCH();
 }
 

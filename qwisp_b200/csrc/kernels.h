@@ -231,20 +231,20 @@ int launch_step_persistent(const PStepArgs& a, cudaStream_t st);   // cooperativ
 
 void launch_dense(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl);
 // many-row forms (more than 8 rows per call); the bool launchers return false when the shape is not covered
-bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st);
-void launch_rows_prep_plain(const __half* x, int ldx, int M, int K, __half* xq, float* sxq, cudaStream_t st);
+bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl);
+void launch_rows_prep_plain(const __half* x, int ldx, int M, int K, __half* xq, float* sxq, cudaStream_t st, bool pdl);
 // prefill mode: the experts of a prompt chunk as grouped GEMMs on the tensor cores (pair lists as built by the router); hbuf in natural order
-bool launch_expert_tc_gateup(const ExpertArgs& a, cudaStream_t st);
-bool launch_expert_tc_down(const ExpertArgs& a, cudaStream_t st);
+bool launch_expert_tc_gateup(const ExpertArgs& a, cudaStream_t st, bool pdl);
+bool launch_expert_tc_down(const ExpertArgs& a, cudaStream_t st, bool pdl);
 // router for many rows: a.h holds rows that are already normed; logits kernel + routing / pair lists kernel
-bool launch_router_rows(const RouterArgs& a, cudaStream_t st);
-bool launch_router_mma(const RouterArgs& a, cudaStream_t st);    // prefill mode, fp16 router: logits on the tensor cores
-bool launch_expert_rows_gateup(const ExpertArgs& a, cudaStream_t st);
-bool launch_expert_rows_down(const ExpertArgs& a, cudaStream_t st);
+bool launch_router_rows(const RouterArgs& a, cudaStream_t st, bool pdl);
+bool launch_router_mma(const RouterArgs& a, cudaStream_t st, bool pdl);    // prefill mode, fp16 router: logits on the tensor cores
+bool launch_expert_rows_gateup(const ExpertArgs& a, cudaStream_t st, bool pdl);
+bool launch_expert_rows_down(const ExpertArgs& a, cudaStream_t st, bool pdl);
 void launch_moe_combine(const __half* dbuf, const __half* shared_rows, const __half* scores, const __half* sgl, int M, int H, int topk,
-                        __half* resid, __half* out, cudaStream_t st);
+                        __half* resid, __half* out, cudaStream_t st, bool pdl);
 // many-row GEMM on tcgen05 tensor cores with the accumulator in tensor memory (N % 16 == 0, K % 256 == 0); 0 or an error code
-int launch_gemm_tc(const Q4R& q, int N, int K, int M, const __half* x, int ldx, __half* y, int ldy, bool add_to_y, unsigned* err, cudaStream_t st);
+int launch_gemm_tc(const Q4R& q, int N, int K, int M, const __half* x, int ldx, __half* y, int ldy, bool add_to_y, unsigned* err, cudaStream_t st, bool pdl);
 // speculative-sampling rows on fp16 logits [M][V]: categorical draw, draw without the draft token, accept flag
 void launch_sample_rows(const __half* logits, const float* adj /*[V] added to every row, or nullptr*/, const int* draft, int* samp_full, int* samp_resid, int* accept, int M, int V,
                         float invT, float top_p, uint32_t seed_lo, uint32_t seed_hi, uint32_t base_pos, cudaStream_t st);
@@ -266,15 +266,15 @@ void launch_ep_combine(const EpPeers& P, const __half* shared_rows, const __half
 void launch_ep_step_end(unsigned* ctr, cudaStream_t st);
 void launch_gdn_core(const GdnArgs& a, int nsegs, cudaStream_t st, bool pdl);
 // prefill-mode attention of one stream's chunk on the tensor cores (after launch_attn_prep); false: call not covered
-bool launch_attn_prefill(const AttnArgs& a, int nsegs, cudaStream_t st);
-void launch_gdn_rows(const GdnArgs& a, int M, int nsegs, cudaStream_t st);   // the same result by k_gdn_prep + k_gdn_scan (needs the scratch fields)
+bool launch_attn_prefill(const AttnArgs& a, int nsegs, cudaStream_t st, bool pdl);
+void launch_gdn_rows(const GdnArgs& a, int M, int nsegs, cudaStream_t st, bool pdl);   // the same result by k_gdn_prep + k_gdn_scan (needs the scratch fields)
 size_t gdn_qk_floats(int Hk, int rows); size_t gdn_vg_bytes(int Hv, int rows);
-void launch_attn_prep(const AttnArgs& a, cudaStream_t st);
+void launch_attn_prep(const AttnArgs& a, cudaStream_t st, bool pdl);
 // q/k prep (when every row is its stream's only row) + split-KV decode + merge in one launch; counters: 2*M*KV zeros
 void launch_attn_fused(const AttnArgs& a, bool prep, unsigned* counters, cudaStream_t st, bool pdl);
 void launch_step_end(const StepEndArgs& a, cudaStream_t st);
 // xq / sxq (optional): the normed rows also in the prepared form of the many-row kernels
-void launch_final_norm(const __half* h, const __half* w, float eps, int M, int H, __half* out, cudaStream_t st, __half* xq = nullptr, float* sxq = nullptr);
+void launch_final_norm(const __half* h, const __half* w, float eps, int M, int H, __half* out, cudaStream_t st, bool pdl, __half* xq = nullptr, float* sxq = nullptr);
 // expert-parallel: the normed rows also go into every rank's gather buffer (RouterArgs::ep_rows_sent then tells the routing kernel)
 void launch_final_norm_ep(const __half* h, const __half* w, float eps, int M, int H, __half* out, const EpDispatch& epd, cudaStream_t st);
 void launch_wait_probe(unsigned* err, cudaStream_t st);   // test hook: a bounded wait that runs out sets bit 2 of *err
@@ -283,6 +283,17 @@ void count_launch();
 void count_launches(int64_t n);
 // run `fn` (one kernel launch) between the profiling events of `tag` when profiling is on, and count it
 void profile_launch(const char* tag, cudaStream_t st, const std::function<int()>& fn);
+// k<<<grid, threads, smem, st>>>(args...); pdl: as a programmatic dependent launch (k waits for its predecessor itself)
+template <class... P, class... A>
+inline int launch_pdl(bool pdl, void (*k)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    if (pdl) { cfg.attrs = attr; cfg.numAttrs = 1; }
+    return (int)cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
 void profile_start();
 int profile_report(char* buf, size_t cap);
 

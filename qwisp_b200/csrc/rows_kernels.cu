@@ -37,6 +37,8 @@ __global__ void __launch_bounds__(512) k_rows_prep(RowsPrepArgs a) {
     __shared__ float part[16];
     const int row = blockIdx.x, ch = threadIdx.x >> 5, lane = threadIdx.x & 31, chunks = a.K >> 8;
     const int k0 = (ch << 8) + lane * 8;
+    pdl_wait();
+    pdl_launch_dependents();
     const uint4 v = __ldcg(reinterpret_cast<const uint4*>(a.x + (size_t)row * a.ldx + k0));
     uint4 o;
     if (PRO == PRO_PLAIN) {
@@ -56,19 +58,18 @@ __global__ void __launch_bounds__(512) k_rows_prep(RowsPrepArgs a) {
     }
     rows_store(a.xq + (size_t)row * a.K, a.sxq + (size_t)row * (a.K >> 6), k0, o, lane);
 }
-static void launch_rows_prep_args(int pro, const RowsPrepArgs& a, int M, cudaStream_t st) {
+static void launch_rows_prep_args(int pro, const RowsPrepArgs& a, int M, cudaStream_t st, bool pdl) {
     const unsigned threads = (unsigned)(a.K >> 8) * 32u;
     profile_launch("k_rows_prep", st, [&] {
-        if (pro == PRO_PLAIN) k_rows_prep<PRO_PLAIN><<<M, threads, 0, st>>>(a);
-        else if (pro == PRO_RMSNORM) k_rows_prep<PRO_RMSNORM><<<M, threads, 0, st>>>(a);
-        else if (pro == PRO_NORMGATE) k_rows_prep<PRO_NORMGATE><<<M, threads, 0, st>>>(a);
-        else k_rows_prep<PRO_NORMGATE32><<<M, threads, 0, st>>>(a);
-        return 0;
+        if (pro == PRO_PLAIN) return launch_pdl(pdl, k_rows_prep<PRO_PLAIN>, dim3((unsigned)M), threads, 0, st, a);
+        if (pro == PRO_RMSNORM) return launch_pdl(pdl, k_rows_prep<PRO_RMSNORM>, dim3((unsigned)M), threads, 0, st, a);
+        if (pro == PRO_NORMGATE) return launch_pdl(pdl, k_rows_prep<PRO_NORMGATE>, dim3((unsigned)M), threads, 0, st, a);
+        return launch_pdl(pdl, k_rows_prep<PRO_NORMGATE32>, dim3((unsigned)M), threads, 0, st, a);
     });
 }
-void launch_rows_prep_plain(const __half* x, int ldx, int M, int K, __half* xq, float* sxq, cudaStream_t st) {
+void launch_rows_prep_plain(const __half* x, int ldx, int M, int K, __half* xq, float* sxq, cudaStream_t st, bool pdl) {
     RowsPrepArgs p{x, ldx, nullptr, nullptr, nullptr, 0, 0.f, K, xq, sxq};
-    launch_rows_prep_args(PRO_PLAIN, p, M, st);
+    launch_rows_prep_args(PRO_PLAIN, p, M, st, pdl);
 }
 
 // ================================================================================ shared compute
@@ -174,7 +175,9 @@ __global__ void __launch_bounds__(256, RG == 1 ? 2 : 1) k_gemv_rows(RowsDenseArg
         cp_async_commit();
     };
     SliceRegs cur, n1, n2;                                    // this slice and the next two (weights stream two slices ahead)
-    if (active) { load_slice(cur, wt, stl, 0, lane); if (slices > 1) load_slice(n1, wt, stl, 1, lane); }
+    if (active) { load_slice(cur, wt, stl, 0, lane); if (slices > 1) load_slice(n1, wt, stl, 1, lane); }      // weights: ahead of the programmatic-launch wait
+    pdl_wait();
+    pdl_launch_dependents();
     stage(0, 0);
     float tot[RG][4];
 #pragma unroll
@@ -213,24 +216,24 @@ __global__ void __launch_bounds__(256, RG == 1 ? 2 : 1) k_gemv_rows(RowsDenseArg
         }
 }
 template <int EPI, int RG>
-static void launch_gemv_rows_t(const RowsDenseArgs& a, cudaStream_t st) {
+static void launch_gemv_rows_t(const RowsDenseArgs& a, cudaStream_t st, bool pdl) {
     const size_t smem = (size_t)2 * 8 * RG * RD_XS * 2 + (size_t)2 * 8 * RG * 4 * 4;
     static bool configured = false;
     if (!configured) { cudaFuncSetAttribute(k_gemv_rows<EPI, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
     const dim3 grid((unsigned)(((a.N >> 4) + 7) / 8), (unsigned)((a.M + 8 * RG - 1) / (8 * RG)));
-    profile_launch(EPI == EPI_RESID ? "k_gemv_rows_outproj" : "k_gemv_rows_inproj", st, [&] { k_gemv_rows<EPI, RG><<<grid, 256, smem, st>>>(a); return 0; });
+    profile_launch(EPI == EPI_RESID ? "k_gemv_rows_outproj" : "k_gemv_rows_inproj", st, [&] { return launch_pdl(pdl, k_gemv_rows<EPI, RG>, grid, 256, smem, st, a); });
 }
 // dense projection of M > 8 rows: prologue rows, then the tile kernel.  Returns false when the shape is not covered.
-bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st) {
+bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl) {
     if (!a.xq || !a.sxq || a.K % 256 || a.K > 4096 || a.N % 16 || (epi != EPI_STORE && epi != EPI_RESID)) return false;
     RowsPrepArgs p{a.x, a.ldx, a.nw, a.nw32, a.z, a.ldz, a.eps, a.K, a.xq, a.sxq};
-    launch_rows_prep_args(pro, p, a.M, st);
+    launch_rows_prep_args(pro, p, a.M, st, pdl);
     RowsDenseArgs d{a.q, a.N, a.K, a.M, a.xq, a.sxq, a.y, a.ldy};
     // 32 rows per CTA (weights dequantised once per 32 rows) when that still fills the device, else 8
     const long ctas4 = (long)(((a.N >> 4) + 7) / 8) * ((a.M + 31) / 32);
     const bool rg4 = ctas4 >= sm_count();
-    if (epi == EPI_RESID) { if (rg4) launch_gemv_rows_t<EPI_RESID, 4>(d, st); else launch_gemv_rows_t<EPI_RESID, 1>(d, st); }
-    else { if (rg4) launch_gemv_rows_t<EPI_STORE, 4>(d, st); else launch_gemv_rows_t<EPI_STORE, 1>(d, st); }
+    if (epi == EPI_RESID) { if (rg4) launch_gemv_rows_t<EPI_RESID, 4>(d, st, pdl); else launch_gemv_rows_t<EPI_RESID, 1>(d, st, pdl); }
+    else { if (rg4) launch_gemv_rows_t<EPI_STORE, 4>(d, st, pdl); else launch_gemv_rows_t<EPI_STORE, 1>(d, st, pdl); }
     return true;
 }
 
@@ -285,6 +288,8 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
         for (int i = 0; i < nstages; ++i) { mbar_init(&s_full[i], DOWN ? 1 : 8); mbar_init(&s_empty[i], XR_WARPS); mbar_init(&s_raw[i], 8); }
         mbar_fence_init();
     }
+    if (!DOWN) pdl_wait();                                      // the lists (down: they were there before gate/up started)
+    pdl_launch_dependents();
     const int n_active = slot_table(s_tab, a.lists, 8, nshared);
     __syncthreads();
     const long total = (long)s_tab.base[n_active + 1] << lg_tiles;
@@ -305,6 +310,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
     unsigned fail_code = 0;          // which wait ran out: 16 producer/empty, 32 producer/chunk sums, 64 consumer/full
     if (warp == XR_WARPS) {
         // ------------------------------------------------------------ producer: the rows of the run's blocks, stage after stage
+        if (DOWN) pdl_wait();                                  // the gate/up kernel's rows
         for (int k = 0; k < nb; ++k) {
             const int stg = k % nstages, use = k / nstages;
             const XrStage St = xr_carve(stages + (size_t)stg * stage_bytes, K);
@@ -461,7 +467,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
     }
 }
 template <bool DOWN, int S>
-static bool launch_expert_rows_t(const ExpertArgs& a, cudaStream_t st) {
+static bool launch_expert_rows_t(const ExpertArgs& a, cudaStream_t st, bool pdl) {
     const int ntiles = DOWN ? a.H / 16 : a.I / 8, grid = sm_count();
     int lg = 0; while ((1 << lg) < ntiles) ++lg;
     const long pairs = (long)a.M * a.topk, blocks = pairs / 8 + (pairs < 256 ? pairs : 256) + a.M / 8 + 1;    // at most one partial block per expert
@@ -472,23 +478,23 @@ static bool launch_expert_rows_t(const ExpertArgs& a, cudaStream_t st) {
     const size_t smem = ring + sb * nstages;
     static bool configured = false;
     if (!configured) { cudaFuncSetAttribute(k_expert_rows<DOWN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
-    profile_launch(DOWN ? "k_expert_rows_down" : "k_expert_rows_gateup", st, [&] { k_expert_rows<DOWN, S><<<grid, XR_THREADS, smem, st>>>(a, lg, nstages); return 0; });
+    profile_launch(DOWN ? "k_expert_rows_down" : "k_expert_rows_gateup", st, [&] { return launch_pdl(pdl, k_expert_rows<DOWN, S>, dim3((unsigned)grid), XR_THREADS, smem, st, a, lg, nstages); });
     return true;
 }
 template <bool DOWN>
-static bool launch_expert_rows_d(const ExpertArgs& a, cudaStream_t st) {
+static bool launch_expert_rows_d(const ExpertArgs& a, cudaStream_t st, bool pdl) {
     if (!a.csum || (!DOWN && (!a.xq || !a.sxq))) return false;
     switch (DOWN ? a.I : a.H) {
-        case 256: return launch_expert_rows_t<DOWN, 1>(a, st);
-        case 512: return launch_expert_rows_t<DOWN, 2>(a, st);
-        case 1024: return launch_expert_rows_t<DOWN, 4>(a, st);
-        case 2048: return launch_expert_rows_t<DOWN, 8>(a, st);
-        case 4096: return launch_expert_rows_t<DOWN, 16>(a, st);
+        case 256: return launch_expert_rows_t<DOWN, 1>(a, st, pdl);
+        case 512: return launch_expert_rows_t<DOWN, 2>(a, st, pdl);
+        case 1024: return launch_expert_rows_t<DOWN, 4>(a, st, pdl);
+        case 2048: return launch_expert_rows_t<DOWN, 8>(a, st, pdl);
+        case 4096: return launch_expert_rows_t<DOWN, 16>(a, st, pdl);
         default: return false;
     }
 }
-bool launch_expert_rows_gateup(const ExpertArgs& a, cudaStream_t st) { return launch_expert_rows_d<false>(a, st); }
-bool launch_expert_rows_down(const ExpertArgs& a, cudaStream_t st) { return launch_expert_rows_d<true>(a, st); }
+bool launch_expert_rows_gateup(const ExpertArgs& a, cudaStream_t st, bool pdl) { return launch_expert_rows_d<false>(a, st, pdl); }
+bool launch_expert_rows_down(const ExpertArgs& a, cudaStream_t st, bool pdl) { return launch_expert_rows_d<true>(a, st, pdl); }
 
 // ================================================================================ router for many rows
 // k_router_rows   logits of all rows: a CTA keeps 8 router rows (or the shared gate) in registers and walks the row
@@ -531,6 +537,8 @@ __global__ void __launch_bounds__(256, 2) k_router_rows(RouterArgs a) {
         cp_async_commit();
     };
     int it = 0;
+    pdl_wait();
+    pdl_launch_dependents();
     if ((int)blockIdx.y < ngroups) stage(blockIdx.y, 0);
     for (int rg = blockIdx.y; rg < ngroups; rg += gridDim.y, ++it) {
         const int b = it & 1;
@@ -622,6 +630,8 @@ __global__ void __launch_bounds__(256, 1) k_router_rows2(RouterArgs a, int gr) {
         }
     };
     int it = 0;
+    pdl_wait();
+    pdl_launch_dependents();
     if ((int)blockIdx.y < ngroups) stage(blockIdx.y, 0);
     for (int rg = blockIdx.y; rg < ngroups; rg += gridDim.y, ++it) {
         const int b = it & 1;
@@ -657,14 +667,14 @@ __global__ void __launch_bounds__(256, 1) k_router_rows2(RouterArgs a, int gr) {
     }
 }
 template <int NB>
-static void launch_router_rows2(const RouterArgs& a, cudaStream_t st) {
+static void launch_router_rows2(const RouterArgs& a, cudaStream_t st, bool pdl) {
     const int gx = (a.E + 15) / 16 + 1, want = sm_count() / gx > 0 ? sm_count() / gx : 1;
     int gr = 2; while (gr < 8 && gr * want < a.M) gr *= 2;
     const int ngroups = (a.M + gr - 1) / gr, gy = ngroups < want ? ngroups : want;
     const size_t smem = (size_t)gr * NB * 256 * 8;
     static bool configured = false;
     if (!configured) { cudaFuncSetAttribute(k_router_rows2<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * NB * 256 * 8); configured = true; }
-    profile_launch("k_router_rows", st, [&] { k_router_rows2<NB><<<dim3((unsigned)gx, (unsigned)gy), 256, smem, st>>>(a, gr); return 0; });
+    profile_launch("k_router_rows", st, [&] { return launch_pdl(pdl, k_router_rows2<NB>, dim3((unsigned)gx, (unsigned)gy), 256, smem, st, a, gr); });
 }
 // grid (ceil(M / 8)), 256 threads: one warp per row.  Expert-parallel: grid (M), one row per CTA.
 __global__ void __launch_bounds__(256) k_route_rows(RouterArgs a) {
@@ -672,6 +682,8 @@ __global__ void __launch_bounds__(256) k_route_rows(RouterArgs a) {
     __shared__ int s_cnt[256], s_off[256], s_slot[256], s_cur[256], s_wsum[8], s_wact[8];
     __shared__ int s_last;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_wait();
+    pdl_launch_dependents();
     if (a.epd.sig.world > 0) {
         // expert-parallel (grid = M, one row per CTA): warp 0 routes the row, then warp w stores the normed row and its
         // routing indices into rank w's gather buffers over peer memory; the CTA that finishes last raises this rank's
@@ -764,6 +776,8 @@ __global__ void __launch_bounds__(128) k_router_mma(RouterArgs a) {
         }
     };
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    pdl_wait();
+    pdl_launch_dependents();
     const int nk = a.H / RT_K;
     for (int kc = 0; kc < RT_ST - 1; ++kc) { if (kc < nk) stage(kc); cp_async_commit(); }
     for (int kc = 0; kc < nk; ++kc) {
@@ -807,16 +821,16 @@ __global__ void __launch_bounds__(128) k_router_mma(RouterArgs a) {
     }
 }
 // prefill mode, fp16 router: logits on the tensor cores, then the routing / pair-list kernel.  false: not covered.
-bool launch_router_mma(const RouterArgs& a, cudaStream_t st) {
+bool launch_router_mma(const RouterArgs& a, cudaStream_t st, bool pdl) {
     if (a.E > 256 || a.H % 256 || a.norm_w || a.router_q8 || a.sg_q8) return false;
     const dim3 grid((unsigned)((a.M + RT_T - 1) / RT_T), (unsigned)((a.E + RT_T - 1) / RT_T));
-    profile_launch("k_router_mma", st, [&] { k_router_mma<<<grid, 128, 0, st>>>(a); return 0; });
-    profile_launch("k_route_rows", st, [&] { k_route_rows<<<a.epd.sig.world > 0 ? a.M : (a.M + 7) / 8, 256, 0, st>>>(a); return 0; });
+    profile_launch("k_router_mma", st, [&] { return launch_pdl(pdl, k_router_mma, grid, 128, 0, st, a); });
+    profile_launch("k_route_rows", st, [&] { return launch_pdl(pdl, k_route_rows, dim3((unsigned)(a.epd.sig.world > 0 ? a.M : (a.M + 7) / 8)), 256, 0, st, a); });
     return true;
 }
 
 // rows already normed in a.h (ldh); E <= 256.  Returns false when the shape is not covered.
-bool launch_router_rows(const RouterArgs& a, cudaStream_t st) {
+bool launch_router_rows(const RouterArgs& a, cudaStream_t st, bool pdl) {
     if (a.E > 256 || a.H % 256 || a.H > 4096 || a.norm_w) return false;
     const size_t smem = (size_t)2 * 8 * a.H * 2;
     static bool configured = false;
@@ -830,15 +844,14 @@ bool launch_router_rows(const RouterArgs& a, cudaStream_t st) {
     int gy = (2 * sm_count() + gx - 1) / gx; if (gy > ngroups) gy = ngroups; if (gy < 1) gy = 1;
     const dim3 grid((unsigned)gx, (unsigned)gy);
     const bool q8 = a.router_q8 != nullptr;
-    if (!q8 && a.H == 512) launch_router_rows2<2>(a, st);
-    else if (!q8 && a.H == 1024) launch_router_rows2<4>(a, st);
-    else if (!q8 && a.H == 2048) launch_router_rows2<8>(a, st);
+    if (!q8 && a.H == 512) launch_router_rows2<2>(a, st, pdl);
+    else if (!q8 && a.H == 1024) launch_router_rows2<4>(a, st, pdl);
+    else if (!q8 && a.H == 2048) launch_router_rows2<8>(a, st, pdl);
     else profile_launch("k_router_rows", st, [&] {
-        if (q8) k_router_rows<true><<<grid, 256, smem, st>>>(a); else k_router_rows<false><<<grid, 256, smem, st>>>(a);
-        return 0;
+        return launch_pdl(pdl, q8 ? k_router_rows<true> : k_router_rows<false>, grid, 256, smem, st, a);
     });
     const int route_grid = a.epd.sig.world > 0 ? a.M : ngroups;
-    profile_launch("k_route_rows", st, [&] { k_route_rows<<<route_grid, 256, 0, st>>>(a); return 0; });
+    profile_launch("k_route_rows", st, [&] { return launch_pdl(pdl, k_route_rows, dim3((unsigned)route_grid), 256, 0, st, a); });
     return true;
 }
 
@@ -851,6 +864,8 @@ bool launch_router_rows(const RouterArgs& a, cudaStream_t st) {
 __global__ void __launch_bounds__(256) k_moe_combine(const __half* dbuf, const __half* shared_rows, const __half* scores, const __half* sgl,
                                                      int H, int topk, __half* resid, __half* out) {
     const int m = blockIdx.x, n = (blockIdx.y * 256 + threadIdx.x) * 8;
+    pdl_wait();
+    pdl_launch_dependents();
     if (n >= H) return;
     const uint4 sh = __ldcg(reinterpret_cast<const uint4*>(shared_rows + (size_t)m * H + n));
     uint4 rv = make_uint4(0, 0, 0, 0);
@@ -878,8 +893,10 @@ __global__ void __launch_bounds__(256) k_moe_combine(const __half* dbuf, const _
     *reinterpret_cast<uint4*>((resid ? resid : out) + (size_t)m * H + n) = rv;
 }
 void launch_moe_combine(const __half* dbuf, const __half* shared_rows, const __half* scores, const __half* sgl, int M, int H, int topk,
-                        __half* resid, __half* out, cudaStream_t st) {
-    profile_launch("k_moe_combine", st, [&] { k_moe_combine<<<dim3((unsigned)M, (unsigned)((H + 2047) / 2048)), 256, 0, st>>>(dbuf, shared_rows, scores, sgl, H, topk, resid, out); return 0; });
+                        __half* resid, __half* out, cudaStream_t st, bool pdl) {
+    profile_launch("k_moe_combine", st, [&] {
+        return launch_pdl(pdl, k_moe_combine, dim3((unsigned)M, (unsigned)((H + 2047) / 2048)), 256, 0, st, dbuf, shared_rows, scores, sgl, H, topk, resid, out);
+    });
 }
 
 }  // namespace sl

@@ -96,27 +96,35 @@ __device__ __forceinline__ bool xr_wait(uint64_t* bar, uint32_t parity, volatile
     }
 }
 
-// One slice (4 groups of 64 inputs) of a 16-row tile against 8*RG staged rows.
-// xs: the slice's activations of staged row 0 (paired order), rows xstride halves apart; sxs: group sums of staged
-// row 0 for the slice's 4 groups, rows sxstride floats apart.  acc[q]: (row A, col 2t), (A, 2t+1), (B, 2t), (B, 2t+1)
-// of row group q.  The order of operations per column is that of compute_slice_x().
+constexpr int XR_DEPTH = 2;                   // slices in a warp's ring
+constexpr int XR_UNIT = 2048 + 256;           // bytes of a slice of a tile: nibbles, then scales and biases
+// slice s of a tile (nibbles w, scales sc) into a ring slot of the calling warp
+__device__ __forceinline__ void ring_request(unsigned char* slot, const uint4* w, const uint4* sc, int s, int lane) {
+    uint4* d = reinterpret_cast<uint4*>(slot);
+    const uint4* p = w + s * 128 + lane;
+    cp_async16(d + lane, p); cp_async16(d + lane + 32, p + 32); cp_async16(d + lane + 64, p + 64); cp_async16(d + lane + 96, p + 96);
+    if (lane < 16) cp_async16(d + 128 + lane, sc + s * 16 + lane);
+}
+// One slice (4 groups of 64 inputs) of a 16-row tile, in a ring slot, against 8*RG staged rows.
+// xp: the slice's activations of this lane's row of group 0 (row r, paired order, + 16 t), rows xstride halves apart; sxp: the
+// group sums [group][row] of the slice, at column 2t, groups sxstride floats apart.  acc[q]: (row A, col 2t), (A, 2t+1),
+// (B, 2t), (B, 2t+1) of row group q.  The order of operations per column is that of compute_slice_x().
 template <int RG>
-__device__ __forceinline__ void compute_rows(const SliceRegs& rg, const __half* xs, int xstride, const float* sxs, int sxstride,
-                                             int r, int t, float accS[RG][4], float accB[RG][4]) {
+__device__ __forceinline__ void compute_rows(const unsigned char* slot, const __half* xp, int xstride, const float* sxp, int sxstride,
+                                             int lane, float accS[RG][4], float accB[RG][4]) {
+    const uint4* w = reinterpret_cast<const uint4*>(slot);
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-        const uint4 wv = rg.w[g];
+        const uint4 wv = w[g * 32 + lane];
         uint32_t a0[4], b0[4], a1[4], b1[4];
         dequant8(wv.x, a0); dequant8(wv.z, b0); dequant8(wv.y, a1); dequant8(wv.w, b1);
-        const uint4 sv = rg.sc[g >> 1];
-        const uint32_t sa_ba = (g & 1) ? sv.z : sv.x, sb_bb = (g & 1) ? sv.w : sv.y;
-        const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&sa_ba));
-        const float2 fb = __half22float2(*reinterpret_cast<const __half2*>(&sb_bb));
+        const uint2 sv = *reinterpret_cast<const uint2*>(slot + 2048 + (g >> 1) * 128 + (lane >> 2) * 16 + (g & 1) * 8);
+        const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&sv.x));
+        const float2 fb = __half22float2(*reinterpret_cast<const __half2*>(&sv.y));
 #pragma unroll
         for (int q = 0; q < RG; ++q) {
-            const __half* xp = xs + (size_t)(q * 8 + r) * xstride + 64 * g + 16 * t;
-            const uint4 X0 = *reinterpret_cast<const uint4*>(xp), X1 = *reinterpret_cast<const uint4*>(xp + 8);
-            const float sx0 = sxs[(q * 8 + 2 * t) * sxstride + g], sx1 = sxs[(q * 8 + 2 * t + 1) * sxstride + g];
+            const uint4 X0 = *reinterpret_cast<const uint4*>(xp + (size_t)q * 8 * xstride + 64 * g), X1 = *reinterpret_cast<const uint4*>(xp + (size_t)q * 8 * xstride + 64 * g + 8);
+            const float2 sx = *reinterpret_cast<const float2*>(sxp + g * sxstride + q * 8);
             float c[4];
             mma_f16_z(c, a0[0], b0[0], a0[1], b0[1], X0.x, X0.y);
             mma_f16(c, a0[2], b0[2], a0[3], b0[3], X0.z, X0.w);
@@ -124,8 +132,8 @@ __device__ __forceinline__ void compute_rows(const SliceRegs& rg, const __half* 
             mma_f16(c, a1[2], b1[2], a1[3], b1[3], X1.z, X1.w);
             accS[q][0] = fmaf(fa.x, c[0], accS[q][0]); accS[q][1] = fmaf(fa.x, c[1], accS[q][1]);
             accS[q][2] = fmaf(fb.x, c[2], accS[q][2]); accS[q][3] = fmaf(fb.x, c[3], accS[q][3]);
-            accB[q][0] = fmaf(fa.y, sx0, accB[q][0]); accB[q][1] = fmaf(fa.y, sx1, accB[q][1]);
-            accB[q][2] = fmaf(fb.y, sx0, accB[q][2]); accB[q][3] = fmaf(fb.y, sx1, accB[q][3]);
+            accB[q][0] = fmaf(fa.y, sx.x, accB[q][0]); accB[q][1] = fmaf(fa.y, sx.y, accB[q][1]);
+            accB[q][2] = fmaf(fb.y, sx.x, accB[q][2]); accB[q][3] = fmaf(fb.y, sx.y, accB[q][3]);
         }
     }
 }
@@ -144,84 +152,104 @@ struct RowsDenseArgs {
     const __half* xq; const float* sxq;  // prepared rows
     __half* y; int ldy;
 };
-constexpr int RD_XS = 256 + 8;           // halves per staged row of one slice (16 bytes of skew: conflict-free B loads)
-// grid (ceil(tiles / 8), ceil(M / (8*RG))), 256 threads
-template <int EPI, int RG>
-__global__ void __launch_bounds__(256, RG == 1 ? 2 : 1) k_gemv_rows(RowsDenseArgs a) {
+// grid (CTAs of a block, blocks of 8*RG rows), NW warps: the CTA holds its block's rows over the whole K in shared memory and
+// its warps walk an equal run of the tiles of 16 weight rows, each warp with its own ring of slices.
+template <int RG, int NW>
+__host__ __device__ constexpr size_t rd_smem(int K) { return (size_t)NW * XR_DEPTH * XR_UNIT + (size_t)8 * RG * (K + 8) * 2 + (size_t)(K >> 6) * (8 * RG + 2) * 4; }
+template <int EPI, int RG, int NW>
+__global__ void __launch_bounds__(NW * 32, 1) k_gemv_rows(RowsDenseArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int NR = 8 * RG;
-    __half* xs = reinterpret_cast<__half*>(smem);                               // [2][NR][RD_XS]
-    float* sxs = reinterpret_cast<float*>(smem + (size_t)2 * NR * RD_XS * 2);    // [2][NR][4]
+    constexpr int NR = 8 * RG, SXS = NR + 2;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, t = lane & 3;
-    const int slices = a.K >> 8, G64 = a.K >> 6, ntiles = a.N >> 4;
-    const int tile = blockIdx.x * 8 + warp;
-    const bool active = tile < ntiles;
+    const int slices = a.K >> 8, G64 = a.K >> 6, ntiles = a.N >> 4, XS = a.K + 8;      // 16 bytes of skew: conflict-free loads
+    unsigned char* ring = smem + (size_t)warp * XR_DEPTH * XR_UNIT;
+    __half* xs = reinterpret_cast<__half*>(smem + (size_t)NW * XR_DEPTH * XR_UNIT);    // [NR][K + 8]
+    float* sxs = reinterpret_cast<float*>(xs + (size_t)NR * XS);                       // [K/64][NR + 2]
     const int row0 = blockIdx.y * NR, nrows = min(NR, a.M - row0);
-    const uint4* wt = a.q.wr + (size_t)tile * q4r_w_uint4(a.K);
-    const uint4* stl = a.q.sr + (size_t)tile * q4r_s_uint4(a.K);
-    auto stage = [&](int s, int b) {
-        __half* xb = xs + (size_t)b * NR * RD_XS;
-        for (int i = tid; i < NR * 32; i += 256) {
-            const int row = i >> 5, c = i & 31;
-            __half* dst = xb + (size_t)row * RD_XS + c * 8;
-            if (row < nrows) cp_async16(dst, a.xq + (size_t)(row0 + row) * a.K + s * 256 + c * 8);
-            else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
-        }
-        if (tid < NR) {
-            float* dst = sxs + (size_t)(b * NR + tid) * 4;
-            if (tid < nrows) cp_async16(dst, a.sxq + (size_t)(row0 + tid) * G64 + s * 4);
-            else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+    const int lo = (int)((long)ntiles * blockIdx.x / gridDim.x), hi = (int)((long)ntiles * (blockIdx.x + 1) / gridDim.x);
+    const size_t wstep = q4r_w_uint4(a.K), sstep = q4r_s_uint4(a.K);
+    int rt = lo + warp, rs = 0, rslot = 0;                    // the request cursor: tile, slice, ring slot
+    auto request = [&] {
+        if (rt < hi) ring_request(ring + rslot * XR_UNIT, a.q.wr + (size_t)rt * wstep, a.q.sr + (size_t)rt * sstep, rs, lane);
         cp_async_commit();
+        rslot ^= 1;
+        if (++rs == slices) { rs = 0; rt += NW; }
     };
-    SliceRegs cur, n1, n2;                                    // this slice and the next two (weights stream two slices ahead)
-    if (active) { load_slice(cur, wt, stl, 0, lane); if (slices > 1) load_slice(n1, wt, stl, 1, lane); }      // weights: ahead of the programmatic-launch wait
+    static_assert(XR_DEPTH == 2, "two ring slots");
+    request(); request();                                     // weights: ahead of the programmatic-launch wait
     pdl_wait();
     pdl_launch_dependents();
-    stage(0, 0);
-    float tot[RG][4];
-#pragma unroll
-    for (int q = 0; q < RG; ++q) { tot[q][0] = 0.f; tot[q][1] = 0.f; tot[q][2] = 0.f; tot[q][3] = 0.f; }
+    for (int i = tid; i < nrows * (a.K >> 3); i += NW * 32) {
+        const int row = i / (a.K >> 3), c = i - row * (a.K >> 3);
+        cp_async16(xs + (size_t)row * XS + c * 8, a.xq + (size_t)(row0 + row) * a.K + c * 8);
+    }
+    cp_async_commit();
+    for (int i = tid; i < nrows * G64; i += NW * 32) {
+        const int row = i / G64, g = i - row * G64;
+        sxs[g * SXS + row] = __ldcg(a.sxq + (size_t)(row0 + row) * G64 + g);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    const __half* xp = xs + (size_t)r * XS + 16 * t;
+    int slot = 0;
 #pragma unroll 1
-    for (int s = 0; s < slices; ++s) {
-        const int b = s & 1;
-        if (active && s + 2 < slices) load_slice(n2, wt, stl, s + 2, lane);
-        if (s + 1 < slices) { stage(s + 1, b ^ 1); cp_async_wait<1>(); }
-        else cp_async_wait<0>();
-        __syncthreads();
-        if (active) {
+    for (int tile = lo + warp; tile < hi; tile += NW) {
+        float tot[RG][4];
+#pragma unroll
+        for (int q = 0; q < RG; ++q) { tot[q][0] = 0.f; tot[q][1] = 0.f; tot[q][2] = 0.f; tot[q][3] = 0.f; }
+#pragma unroll 1
+        for (int s = 0; s < slices; ++s) {
+            cp_async_wait<XR_DEPTH - 1>();
+            __syncwarp();                                     // every lane's part of the slice is there
             float accS[RG][4], accB[RG][4];
 #pragma unroll
             for (int q = 0; q < RG; ++q)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) { accS[q][i] = 0.f; accB[q][i] = 0.f; }
-            compute_rows<RG>(cur, xs + (size_t)b * NR * RD_XS, RD_XS, sxs + (size_t)b * NR * 4, 4, r, t, accS, accB);
+            compute_rows<RG>(ring + slot * XR_UNIT, xp + s * 256, XS, sxs + s * 4 * SXS + 2 * t, SXS, lane, accS, accB);
             add_slice<RG>(tot, accS, accB);
+            __syncwarp();                                     // every lane has read the slot: it may be filled again
+            request();
+            slot ^= 1;
         }
-        __syncthreads();                       // the buffer may be refilled by the next iteration's stage()
-        cur = n1; n1 = n2;
-    }
-    if (!active) return;
 #pragma unroll
-    for (int q = 0; q < RG; ++q)
+        for (int q = 0; q < RG; ++q)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int xrow = q * 8 + 2 * t + (i & 1), wrow = tile * 16 + r + 8 * (i >> 1);
-            if (xrow < nrows) {
-                const size_t idx = (size_t)(row0 + xrow) * a.ldy + wrow;
-                __half val = f2h(tot[q][i]);
-                if (EPI == EPI_RESID) val = hadd_rn(a.y[idx], val);
-                a.y[idx] = val;
+            for (int i = 0; i < 4; ++i) {
+                const int xrow = q * 8 + 2 * t + (i & 1), wrow = tile * 16 + r + 8 * (i >> 1);
+                if (xrow < nrows) {
+                    const size_t idx = (size_t)(row0 + xrow) * a.ldy + wrow;
+                    __half val = f2h(tot[q][i]);
+                    if (EPI == EPI_RESID) val = hadd_rn(a.y[idx], val);
+                    a.y[idx] = val;
+                }
             }
-        }
+    }
 }
-template <int EPI, int RG>
+// CTAs that share a block of rows
+static int rd_split(int M, int NR, int ntiles) {
+    const int blocks = (M + NR - 1) / NR;
+    int c = sm_count() / blocks;
+    if (c > ntiles) c = ntiles;
+    return c < 1 ? 1 : c;
+}
+template <int EPI, int RG, int NW>
 static void launch_gemv_rows_t(const RowsDenseArgs& a, cudaStream_t st, bool pdl) {
-    const size_t smem = (size_t)2 * 8 * RG * RD_XS * 2 + (size_t)2 * 8 * RG * 4 * 4;
     static bool configured = false;
-    if (!configured) { cudaFuncSetAttribute(k_gemv_rows<EPI, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
-    const dim3 grid((unsigned)(((a.N >> 4) + 7) / 8), (unsigned)((a.M + 8 * RG - 1) / (8 * RG)));
-    profile_launch(EPI == EPI_RESID ? "k_gemv_rows_outproj" : "k_gemv_rows_inproj", st, [&] { return launch_pdl(pdl, k_gemv_rows<EPI, RG>, grid, 256, smem, st, a); });
+    if (!configured) { cudaFuncSetAttribute(k_gemv_rows<EPI, RG, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); configured = true; }
+    const dim3 grid((unsigned)rd_split(a.M, 8 * RG, a.N >> 4), (unsigned)((a.M + 8 * RG - 1) / (8 * RG)));
+    profile_launch(EPI == EPI_RESID ? "k_gemv_rows_outproj" : "k_gemv_rows_inproj", st, [&] {
+        return launch_pdl(pdl, k_gemv_rows<EPI, RG, NW>, grid, NW * 32, rd_smem<RG, NW>(a.K), st, a);
+    });
+}
+template <int EPI>
+static void launch_gemv_rows(const RowsDenseArgs& a, cudaStream_t st, bool pdl) {
+    static int force = getenv("GR") ? atoi(getenv("GR")) : 0;
+    int rg = force ? force : 4;
+    if (rg == 4 && rd_smem<4, 16>(a.K) > (size_t)227 * 1024) rg = 2;
+    if (rg == 4) launch_gemv_rows_t<EPI, 4, 16>(a, st, pdl);
+    else if (rg == 2) launch_gemv_rows_t<EPI, 2, 16>(a, st, pdl);
+    else launch_gemv_rows_t<EPI, 1, 24>(a, st, pdl);
 }
 // dense projection of M > 8 rows: prologue rows, then the tile kernel.  Returns false when the shape is not covered.
 bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl) {
@@ -229,11 +257,7 @@ bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st, bo
     RowsPrepArgs p{a.x, a.ldx, a.nw, a.nw32, a.z, a.ldz, a.eps, a.K, a.xq, a.sxq};
     launch_rows_prep_args(pro, p, a.M, st, pdl);
     RowsDenseArgs d{a.q, a.N, a.K, a.M, a.xq, a.sxq, a.y, a.ldy};
-    // 32 rows per CTA (weights dequantised once per 32 rows) when that still fills the device, else 8
-    const long ctas4 = (long)(((a.N >> 4) + 7) / 8) * ((a.M + 31) / 32);
-    const bool rg4 = ctas4 >= sm_count();
-    if (epi == EPI_RESID) { if (rg4) launch_gemv_rows_t<EPI_RESID, 4>(d, st, pdl); else launch_gemv_rows_t<EPI_RESID, 1>(d, st, pdl); }
-    else { if (rg4) launch_gemv_rows_t<EPI_STORE, 4>(d, st, pdl); else launch_gemv_rows_t<EPI_STORE, 1>(d, st, pdl); }
+    if (epi == EPI_RESID) launch_gemv_rows<EPI_RESID>(d, st, pdl); else launch_gemv_rows<EPI_STORE>(d, st, pdl);
     return true;
 }
 
@@ -250,8 +274,6 @@ bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st, bo
 // straight from L1 instead of staged: eight lines per load, 89 us for gate/up).  Batch of 64 (event times, 4.5 us of
 // them the events'): gate/up 73.6 -> 67.7 us, down 53.4 -> 43.3; 7 rows: 27.0 -> 23.0, 18.9 -> 18.8.
 constexpr int XR_WARPS = 24;
-constexpr int XR_DEPTH = 2;                   // slices in a warp's ring
-constexpr int XR_UNIT = 2048 + 256;           // bytes of a slice of a tile: nibbles, then scales and biases
 constexpr int XR_BLOCKS = 64;                 // most (slot, block) entries of a CTA's run
 constexpr int XR_THREADS = (XR_WARPS + 1) * 32;
 struct XrBlock { int expert; int src[8], dst[8]; };   // expert -1: the shared one; src, dst -1: no row
@@ -356,12 +378,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
         w = q.wr + T * wstep; sc = q.sr + T * sstep;
     };
     auto request = [&](int slot, const uint4* w, const uint4* sc, int s) {      // slice s of a tile into a ring slot: one copy group
-        if (w) {
-            uint4* d = reinterpret_cast<uint4*>(ring + slot * XR_UNIT);
-            const uint4* p = w + s * 128 + lane;
-            cp_async16(d + lane, p); cp_async16(d + lane + 32, p + 32); cp_async16(d + lane + 64, p + 64); cp_async16(d + lane + 96, p + 96);
-            if (lane < 16) cp_async16(d + 128 + lane, sc + s * 16 + lane);
-        }
+        if (w) ring_request(ring + slot * XR_UNIT, w, sc, s, lane);
         cp_async_commit();
     };
     constexpr int NB = XR_DEPTH > S ? XR_DEPTH / S : 1;           // tiles the ring holds at least the start of

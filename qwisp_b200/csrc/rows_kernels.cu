@@ -152,103 +152,200 @@ struct RowsDenseArgs {
     const __half* xq; const float* sxq;  // prepared rows
     __half* y; int ldy;
 };
-// grid (CTAs of a block, blocks of 8*RG rows), NW warps: the CTA holds its block's rows over the whole K in shared memory and
-// its warps walk an equal run of the tiles of 16 weight rows, each warp with its own ring of slices.
-template <int RG, int NW>
-__host__ __device__ constexpr size_t rd_smem(int K) { return (size_t)NW * XR_DEPTH * XR_UNIT + (size_t)8 * RG * (K + 8) * 2 + (size_t)(K >> 6) * (8 * RG + 2) * 4; }
-template <int EPI, int RG, int NW>
-__global__ void __launch_bounds__(NW * 32, 1) k_gemv_rows(RowsDenseArgs a) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int NR = 8 * RG, SXS = NR + 2;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, t = lane & 3;
-    const int slices = a.K >> 8, G64 = a.K >> 6, ntiles = a.N >> 4, XS = a.K + 8;      // 16 bytes of skew: conflict-free loads
-    unsigned char* ring = smem + (size_t)warp * XR_DEPTH * XR_UNIT;
-    __half* xs = reinterpret_cast<__half*>(smem + (size_t)NW * XR_DEPTH * XR_UNIT);    // [NR][K + 8]
-    float* sxs = reinterpret_cast<float*>(xs + (size_t)NR * XS);                       // [K/64][NR + 2]
-    const int row0 = blockIdx.y * NR, nrows = min(NR, a.M - row0);
-    const int lo = (int)((long)ntiles * blockIdx.x / gridDim.x), hi = (int)((long)ntiles * (blockIdx.x + 1) / gridDim.x);
-    const size_t wstep = q4r_w_uint4(a.K), sstep = q4r_s_uint4(a.K);
-    int rt = lo + warp, rs = 0, rslot = 0;                    // the request cursor: tile, slice, ring slot
-    auto request = [&] {
-        if (rt < hi) ring_request(ring + rslot * XR_UNIT, a.q.wr + (size_t)rt * wstep, a.q.sr + (size_t)rt * sstep, rs, lane);
-        cp_async_commit();
-        rslot ^= 1;
-        if (++rs == slices) { rs = 0; rt += NW; }
-    };
-    static_assert(XR_DEPTH == 2, "two ring slots");
-    request(); request();                                     // weights: ahead of the programmatic-launch wait
-    pdl_wait();
-    pdl_launch_dependents();
-    for (int i = tid; i < nrows * (a.K >> 3); i += NW * 32) {
-        const int row = i / (a.K >> 3), c = i - row * (a.K >> 3);
-        cp_async16(xs + (size_t)row * XS + c * 8, a.xq + (size_t)(row0 + row) * a.K + c * 8);
+// Bound by instruction issue, shared-memory reads and MMAs about equally (a slice of 16 weight rows against 32 rows: 485
+// instructions of a warp, 150 cycles of shared-memory reads, 64 MMAs; it takes 235 cycles of a multiprocessor).  The form
+// before had 8 warps a multiprocessor, weights in registers and two CTA barriers a slice.  By events (about 5 us of them
+// the events'), in / out: 512 rows 134 -> 97, 60 -> 51 us; 64 rows 30 -> 23, 20 -> 19; 17 rows 16.6 -> 15.5, 18.7 -> 12.7.
+// Two forms; in both a CTA has one block of rows in shared memory and an equal run of the tiles of 16 weight rows (grid: CTAs
+// of a block, blocks), and every warp its own ring of weight slices, so that no barrier stands in the stream.
+struct RdGeom { int row0, nrows, lo, hi; };                   // the CTA's rows and tiles
+__device__ __forceinline__ RdGeom rd_geom(const RowsDenseArgs& a, int nr) {
+    const int row0 = blockIdx.y * nr, ntiles = a.N >> 4;
+    return {row0, min(nr, a.M - row0), (int)((long)ntiles * blockIdx.x / gridDim.x), (int)((long)ntiles * (blockIdx.x + 1) / gridDim.x)};
+}
+// inputs k0 .. k0 + kc - 1 of the rows into xs [row][kc + 8] (16 bytes of skew: conflict-free loads), their group sums into sxs [group][stride]
+__device__ __forceinline__ void rd_stage(const RowsDenseArgs& a, const RdGeom& g, int k0, int kc, __half* xs, float* sxs, int stride) {
+    const int c8 = kc >> 3, g64 = kc >> 6;
+    for (int i = threadIdx.x; i < g.nrows * c8; i += blockDim.x) {
+        const int row = i / c8, c = i - row * c8;
+        cp_async16(xs + (size_t)row * (kc + 8) + c * 8, a.xq + (size_t)(g.row0 + row) * a.K + k0 + c * 8);
     }
     cp_async_commit();
-    for (int i = tid; i < nrows * G64; i += NW * 32) {
-        const int row = i / G64, g = i - row * G64;
-        sxs[g * SXS + row] = __ldcg(a.sxq + (size_t)(row0 + row) * G64 + g);
+    for (int i = threadIdx.x; i < g.nrows * g64; i += blockDim.x) {
+        const int row = i / g64, c = i - row * g64;
+        sxs[c * stride + row] = __ldcg(a.sxq + (size_t)(g.row0 + row) * (a.K >> 6) + (k0 >> 6) + c);
     }
     cp_async_wait<0>();
     __syncthreads();
+}
+template <int EPI>
+__device__ __forceinline__ void rd_store(const RowsDenseArgs& a, int row, int n, float v) {
+    const size_t idx = (size_t)row * a.ldy + n;
+    __half val = f2h(v);
+    if (EPI == EPI_RESID) val = hadd_rn(a.y[idx], val);
+    a.y[idx] = val;
+}
+// Tile form: a warp takes every NW-th tile of the run over the whole K.  The block's rows are staged in chunks of kc inputs:
+// once when the whole K fits, else again for every round of NW tiles (the totals stay in registers meanwhile).
+template <int RG, int NW>
+__host__ __device__ constexpr size_t rd_smem(int kc) { return (size_t)NW * XR_DEPTH * XR_UNIT + (size_t)8 * RG * (kc + 8) * 2 + (size_t)(kc >> 6) * (8 * RG + 2) * 4; }
+template <int EPI, int RG, int NW>
+__global__ void __launch_bounds__(NW * 32, 1) k_gemv_rows(RowsDenseArgs a, int kc) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int NR = 8 * RG, SXS = NR + 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, t = lane & 3;
+    const int slices = a.K >> 8, cslices = kc >> 8, XS = kc + 8;
+    unsigned char* ring = smem + (size_t)warp * XR_DEPTH * XR_UNIT;
+    __half* xs = reinterpret_cast<__half*>(smem + (size_t)NW * XR_DEPTH * XR_UNIT);
+    float* sxs = reinterpret_cast<float*>(xs + (size_t)NR * XS);
+    const RdGeom geo = rd_geom(a, NR);
+    const size_t wstep = q4r_w_uint4(a.K), sstep = q4r_s_uint4(a.K);
+    int rt = geo.lo + warp, rs = 0, slot = 0;                 // the request cursor: tile, slice; the ring slot read next
+    auto request = [&](int to) {
+        if (rt < geo.hi) ring_request(ring + to * XR_UNIT, a.q.wr + (size_t)rt * wstep, a.q.sr + (size_t)rt * sstep, rs, lane);
+        cp_async_commit();
+        if (++rs == slices) { rs = 0; rt += NW; }
+    };
+    static_assert(XR_DEPTH == 2, "two ring slots");
+    request(0); request(1);                                   // weights: ahead of the programmatic-launch wait
+    pdl_wait();
+    pdl_launch_dependents();
+    if (kc == a.K) rd_stage(a, geo, 0, kc, xs, sxs, SXS);
     const __half* xp = xs + (size_t)r * XS + 16 * t;
-    int slot = 0;
 #pragma unroll 1
-    for (int tile = lo + warp; tile < hi; tile += NW) {
+    for (int t0 = geo.lo; t0 < geo.hi; t0 += NW) {
+        const int tile = t0 + warp;
         float tot[RG][4];
 #pragma unroll
         for (int q = 0; q < RG; ++q) { tot[q][0] = 0.f; tot[q][1] = 0.f; tot[q][2] = 0.f; tot[q][3] = 0.f; }
 #pragma unroll 1
-        for (int s = 0; s < slices; ++s) {
-            cp_async_wait<XR_DEPTH - 1>();
-            __syncwarp();                                     // every lane's part of the slice is there
-            float accS[RG][4], accB[RG][4];
+        for (int c = 0; c < slices; c += cslices) {
+            if (kc != a.K) { __syncthreads(); rd_stage(a, geo, c << 8, kc, xs, sxs, SXS); }
+            if (tile >= geo.hi) continue;
+#pragma unroll 1
+            for (int s = 0; s < cslices; ++s) {
+                cp_async_wait<XR_DEPTH - 1>();
+                __syncwarp();                                 // every lane's part of the slice is there
+                float accS[RG][4], accB[RG][4];
 #pragma unroll
-            for (int q = 0; q < RG; ++q)
+                for (int q = 0; q < RG; ++q)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) { accS[q][i] = 0.f; accB[q][i] = 0.f; }
-            compute_rows<RG>(ring + slot * XR_UNIT, xp + s * 256, XS, sxs + s * 4 * SXS + 2 * t, SXS, lane, accS, accB);
-            add_slice<RG>(tot, accS, accB);
-            __syncwarp();                                     // every lane has read the slot: it may be filled again
-            request();
-            slot ^= 1;
+                    for (int i = 0; i < 4; ++i) { accS[q][i] = 0.f; accB[q][i] = 0.f; }
+                compute_rows<RG>(ring + slot * XR_UNIT, xp + s * 256, XS, sxs + s * 4 * SXS + 2 * t, SXS, lane, accS, accB);
+                add_slice<RG>(tot, accS, accB);
+                __syncwarp();                                 // every lane has read the slot: it may be filled again
+                request(slot);
+                slot ^= 1;
+            }
         }
+        if (tile >= geo.hi) continue;
 #pragma unroll
         for (int q = 0; q < RG; ++q)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int xrow = q * 8 + 2 * t + (i & 1), wrow = tile * 16 + r + 8 * (i >> 1);
-                if (xrow < nrows) {
-                    const size_t idx = (size_t)(row0 + xrow) * a.ldy + wrow;
-                    __half val = f2h(tot[q][i]);
-                    if (EPI == EPI_RESID) val = hadd_rn(a.y[idx], val);
-                    a.y[idx] = val;
-                }
+                const int xrow = q * 8 + 2 * t + (i & 1);
+                if (xrow < geo.nrows) rd_store<EPI>(a, geo.row0 + xrow, tile * 16 + r + 8 * (i >> 1), tot[q][i]);
             }
     }
 }
-// CTAs that share a block of rows
-static int rd_split(int M, int NR, int ntiles) {
-    const int blocks = (M + NR - 1) / NR;
-    int c = sm_count() / blocks;
-    if (c > ntiles) c = ntiles;
-    return c < 1 ? 1 : c;
+// Split form, for runs of few tiles: the warps share out the (tile, slice) pairs of the run; the slice values meet in shared
+// memory and are added in ascending order (as reduce_tiles() does).  With a tile per warp, four tiles of 16 slices were 10 us
+// of waiting for two slices at a time.
+constexpr int RD_SPLIT_WARPS = 16, RD_PART = 8 * 20;          // floats of a pair's values: [column][16 rows + 4], conflict-free stores
+__host__ __device__ constexpr size_t rd_split_smem(int K, int units) { return rd_smem<1, RD_SPLIT_WARPS>(K) + (size_t)units * RD_PART * 4; }
+template <int EPI>
+__global__ void __launch_bounds__(RD_SPLIT_WARPS * 32, 1) k_gemv_rows_split(RowsDenseArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int NW = RD_SPLIT_WARPS, SXS = 8 + 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, t = lane & 3;
+    const int slices = a.K >> 8, XS = a.K + 8;
+    unsigned char* ring = smem + (size_t)warp * XR_DEPTH * XR_UNIT;
+    __half* xs = reinterpret_cast<__half*>(smem + (size_t)NW * XR_DEPTH * XR_UNIT);
+    float* sxs = reinterpret_cast<float*>(xs + (size_t)8 * XS);
+    float* part = sxs + (size_t)(a.K >> 6) * SXS;
+    const RdGeom geo = rd_geom(a, 8);
+    const int units = (geo.hi - geo.lo) * slices;
+    auto request = [&](int u, int to) {
+        if (u < units) {
+            const int tl = u / slices, tile = geo.lo + tl;
+            ring_request(ring + to * XR_UNIT, a.q.wr + (size_t)tile * q4r_w_uint4(a.K), a.q.sr + (size_t)tile * q4r_s_uint4(a.K), u - tl * slices, lane);
+        }
+        cp_async_commit();
+    };
+    request(warp, 0); request(warp + NW, 1);                  // weights: ahead of the programmatic-launch wait
+    pdl_wait();
+    pdl_launch_dependents();
+    rd_stage(a, geo, 0, a.K, xs, sxs, SXS);
+    const __half* xp = xs + (size_t)r * XS + 16 * t;
+    int slot = 0;
+#pragma unroll 1
+    for (int u = warp; u < units; u += NW) {
+        const int s = u % slices;
+        cp_async_wait<XR_DEPTH - 1>();
+        __syncwarp();
+        float accS[1][4] = {{0.f, 0.f, 0.f, 0.f}}, accB[1][4] = {{0.f, 0.f, 0.f, 0.f}};
+        compute_rows<1>(ring + slot * XR_UNIT, xp + s * 256, XS, sxs + s * 4 * SXS + 2 * t, SXS, lane, accS, accB);
+        __syncwarp();
+        request(u + 2 * NW, slot);
+        slot ^= 1;
+        float* p = part + (size_t)u * RD_PART + 2 * t * 20 + r;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[(i & 1) * 20 + 8 * (i >> 1)] = __fadd_rn(accS[0][i], accB[0][i]);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < (geo.hi - geo.lo) * 128; i += NW * 32) {
+        const int tl = i >> 7, col = (i >> 4) & 7, row = i & 15;
+        if (col >= geo.nrows) continue;
+        const float* p = part + (size_t)tl * slices * RD_PART + col * 20 + row;
+        float v = 0.f;
+        for (int s = 0; s < slices; ++s) v = __fadd_rn(v, p[(size_t)s * RD_PART]);
+        rd_store<EPI>(a, geo.row0 + col, (geo.lo + tl) * 16 + row, v);
+    }
+}
+constexpr size_t RD_ROOM = (size_t)227 * 1024;
+// CTAs that share a block of nr rows: all multiprocessors divided by the blocks
+static int rd_ctas(int M, int nr, int ntiles) {
+    const int c = sm_count() / ((M + nr - 1) / nr);
+    return c < 1 ? 1 : (c > ntiles ? ntiles : c);
 }
 template <int EPI, int RG, int NW>
 static void launch_gemv_rows_t(const RowsDenseArgs& a, cudaStream_t st, bool pdl) {
     static bool configured = false;
-    if (!configured) { cudaFuncSetAttribute(k_gemv_rows<EPI, RG, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); configured = true; }
-    const dim3 grid((unsigned)rd_split(a.M, 8 * RG, a.N >> 4), (unsigned)((a.M + 8 * RG - 1) / (8 * RG)));
+    if (!configured) { cudaFuncSetAttribute(k_gemv_rows<EPI, RG, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RD_ROOM); configured = true; }
+    int kc = a.K;                                              // (K: a multiple of 256 up to 4096, so of 512 where halves are needed -- see rd_fits)
+    if (rd_smem<RG, NW>(kc) > RD_ROOM) kc = a.K / 2;
+    const dim3 grid((unsigned)rd_ctas(a.M, 8 * RG, a.N >> 4), (unsigned)((a.M + 8 * RG - 1) / (8 * RG)));
     profile_launch(EPI == EPI_RESID ? "k_gemv_rows_outproj" : "k_gemv_rows_inproj", st, [&] {
-        return launch_pdl(pdl, k_gemv_rows<EPI, RG, NW>, grid, NW * 32, rd_smem<RG, NW>(a.K), st, a);
+        return launch_pdl(pdl, k_gemv_rows<EPI, RG, NW>, grid, NW * 32, rd_smem<RG, NW>(kc), st, a, kc);
     });
 }
 template <int EPI>
 static void launch_gemv_rows(const RowsDenseArgs& a, cudaStream_t st, bool pdl) {
-    static int force = getenv("GR") ? atoi(getenv("GR")) : 0;
-    int rg = force ? force : 4;
-    if (rg == 4 && rd_smem<4, 16>(a.K) > (size_t)227 * 1024) rg = 2;
-    if (rg == 4) launch_gemv_rows_t<EPI, 4, 16>(a, st, pdl);
-    else if (rg == 2) launch_gemv_rows_t<EPI, 2, 16>(a, st, pdl);
+    const int ntiles = a.N >> 4, slices = a.K >> 8;
+    auto tiles_of = [&](int nr) { const int c = rd_ctas(a.M, nr, ntiles); return (ntiles + c - 1) / c; };      // tiles of a CTA
+    // split form: up to 8 tiles a run, a third of the tile form's warps (17 rows: 3 tiles of 16 slices 16.1 -> 12.7 us by events,
+    // 16 tiles of 8 slices 15.5 -> 17.1)
+    const size_t split = rd_split_smem(a.K, tiles_of(8) * slices);
+    if (tiles_of(8) <= 8 && split <= RD_ROOM) {
+        static bool configured = false;
+        if (!configured) { cudaFuncSetAttribute(k_gemv_rows_split<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RD_ROOM); configured = true; }
+        profile_launch(EPI == EPI_RESID ? "k_gemv_rows_outproj" : "k_gemv_rows_inproj", st, [&] {
+            return launch_pdl(pdl, k_gemv_rows_split<EPI>, dim3((unsigned)rd_ctas(a.M, 8, ntiles), (unsigned)((a.M + 7) / 8)), RD_SPLIT_WARPS * 32, split, st, a);
+        });
+        return;
+    }
+    // 8, 16 or 32 rows per CTA: a tile of 8 slices takes 0.41, 0.60 or 1.0 us, the staging 3, 4 or 6 (more rows per block: fewer
+    // expansions of the weights, but fewer CTAs per block and a longer start); waves of CTAs where the blocks are more than the multiprocessors
+    const int nrs[3] = {8, 16, 32}, per_tile[3] = {41, 60, 100}, start[3] = {300, 400, 600};
+    int best = 0; long best_cost = 0;
+    for (int i = 0; i < 3; ++i) {
+        if (i == 2 && rd_smem<4, 16>(a.K) > RD_ROOM && a.K % 512) continue;
+        const long waves = ((a.M + nrs[i] - 1) / nrs[i] + sm_count() - 1) / sm_count();
+        const long cost = waves * ((long)tiles_of(nrs[i]) * slices * per_tile[i] / 8 + start[i]);
+        if (i == 0 || cost <= best_cost) { best = i; best_cost = cost; }
+    }
+    if (best == 2) launch_gemv_rows_t<EPI, 4, 16>(a, st, pdl);
+    else if (best == 1) launch_gemv_rows_t<EPI, 2, 16>(a, st, pdl);
     else launch_gemv_rows_t<EPI, 1, 24>(a, st, pdl);
 }
 // dense projection of M > 8 rows: prologue rows, then the tile kernel.  Returns false when the shape is not covered.

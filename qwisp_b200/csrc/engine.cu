@@ -704,7 +704,7 @@ void enqueue_step(sl_engine* e, int M, int nsegs, HeadMode head, bool want_logit
     if (head == HEAD_NORMED) {
         launch_final_norm(h, e->final_norm, e->cfg.rms_eps, M, e->H, e->normed, st, e->use_pdl);
     } else if (head == HEAD_ARGMAX || head == HEAD_LOGITS) {
-        DenseArgs d{}; d.q = e->r_lm_head; d.N = e->V; d.K = e->H; d.M = M;
+        DenseArgs d{}; d.q = e->r_lm_head; d.N = e->V; d.K = e->H; d.M = M; d.xq = e->use_rows ? e->xq : nullptr; d.sxq = e->sxq;
         d.x = h; d.ldx = e->H; d.nw = e->final_norm; d.eps = e->cfg.rms_eps;
         d.logits = want_logits ? e->logits : nullptr; d.pval = e->pval; d.pidx = e->pidx; d.out_tok = e->out_tok; d.counter = e->counters + 0;
         launch_dense(PRO_RMSNORM, EPI_ARGMAX, d, st, e->use_pdl);

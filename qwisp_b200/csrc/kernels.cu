@@ -374,6 +374,7 @@ static void launch_normgate_rows(int pro, const DenseArgs& a, cudaStream_t st, b
 
 void launch_dense(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl) {
     if (epi == EPI_ARGMAX) {
+        if (pro == PRO_RMSNORM && a.M > ROWS_PER_PASS && launch_head_rows(a, st, pdl)) return;
         if (pro == PRO_RMSNORM) { launch_head_t<PRO_RMSNORM>(a, st, pdl); return; }
         if (pro == PRO_PLAIN) { launch_head_t<PRO_PLAIN>(a, st, pdl); return; }
     }

@@ -232,6 +232,7 @@ int launch_step_persistent(const PStepArgs& a, cudaStream_t st);   // cooperativ
 void launch_dense(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl);
 // many-row forms (more than 8 rows per call); the bool launchers return false when the shape is not covered
 bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl);
+bool launch_head_rows(const DenseArgs& a, cudaStream_t st, bool pdl);      // lm_head + argmax behind the final norm
 void launch_rows_prep_plain(const __half* x, int ldx, int M, int K, __half* xq, float* sxq, cudaStream_t st, bool pdl);
 // prefill mode: the experts of a prompt chunk as grouped GEMMs on the tensor cores (pair lists as built by the router); hbuf in natural order
 bool launch_expert_tc_gateup(const ExpertArgs& a, cudaStream_t st, bool pdl);

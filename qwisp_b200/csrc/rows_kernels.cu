@@ -358,6 +358,137 @@ bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st, bo
     return true;
 }
 
+// ================================================================================ lm_head + argmax
+// The tile form with the argmax of k_head: per tile the largest logit of each row (lower index on a tie) is merged into the
+// warp's table in shared memory, the CTAs' maxima meet in the CTA that finishes last.  k_head reads the whole matrix once per
+// 8 rows (47 us each at 248320 x 2048, the memory's pace); here once per 16, 24 or 32 rows.
+__device__ __forceinline__ bool head_better(float v, int i, float bv, int bi) { return v > bv || (v == bv && i < bi); }
+template <int RG>
+__global__ void __launch_bounds__(512, 1) k_head_rows(RowsDenseArgs a, __half* logits, float* pval, int* pidx, int* out_tok, unsigned* counter) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int NW = 16, NR = 8 * RG, SXS = NR + 2;
+    __shared__ float s_val[NW][NR];
+    __shared__ int s_idx[NW][NR];
+    __shared__ int s_last;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, t = lane & 3;
+    const int slices = a.K >> 8, XS = a.K + 8;
+    unsigned char* ring = smem + (size_t)warp * XR_DEPTH * XR_UNIT;
+    __half* xs = reinterpret_cast<__half*>(smem + (size_t)NW * XR_DEPTH * XR_UNIT);
+    float* sxs = reinterpret_cast<float*>(xs + (size_t)NR * XS);
+    const RdGeom geo = rd_geom(a, NR);
+    const size_t wstep = q4r_w_uint4(a.K), sstep = q4r_s_uint4(a.K);
+    int rt = geo.lo + warp, rs = 0, slot = 0;
+    auto request = [&](int to) {
+        if (rt < geo.hi) ring_request(ring + to * XR_UNIT, a.q.wr + (size_t)rt * wstep, a.q.sr + (size_t)rt * sstep, rs, lane);
+        cp_async_commit();
+        if (++rs == slices) { rs = 0; rt += NW; }
+    };
+    request(0); request(1);                                   // weights: ahead of the programmatic-launch wait
+    if (lane < NR) { s_val[warp][lane] = -INFINITY; s_idx[warp][lane] = 0x7fffffff; }
+    pdl_wait();
+    pdl_launch_dependents();
+    rd_stage(a, geo, 0, a.K, xs, sxs, SXS);
+    const __half* xp = xs + (size_t)r * XS + 16 * t;
+#pragma unroll 1
+    for (int tile = geo.lo + warp; tile < geo.hi; tile += NW) {
+        float tot[RG][4];
+#pragma unroll
+        for (int q = 0; q < RG; ++q) { tot[q][0] = 0.f; tot[q][1] = 0.f; tot[q][2] = 0.f; tot[q][3] = 0.f; }
+#pragma unroll 1
+        for (int s = 0; s < slices; ++s) {
+            cp_async_wait<XR_DEPTH - 1>();
+            __syncwarp();
+            float accS[RG][4], accB[RG][4];
+#pragma unroll
+            for (int q = 0; q < RG; ++q)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) { accS[q][i] = 0.f; accB[q][i] = 0.f; }
+            compute_rows<RG>(ring + slot * XR_UNIT, xp + s * 256, XS, sxs + s * 4 * SXS + 2 * t, SXS, lane, accS, accB);
+            add_slice<RG>(tot, accS, accB);
+            __syncwarp();
+            request(slot);
+            slot ^= 1;
+        }
+#pragma unroll
+        for (int q = 0; q < RG; ++q)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int row = q * 8 + 2 * t + j, n = tile * 16 + r;
+                const __half lo = f2h(tot[q][j]), hi = f2h(tot[q][2 + j]);
+                if (logits && row < geo.nrows) {
+                    logits[(size_t)(geo.row0 + row) * a.N + n] = lo;
+                    logits[(size_t)(geo.row0 + row) * a.N + n + 8] = hi;
+                }
+                float v = h2f(lo); int i = n;
+                if (head_better(h2f(hi), n + 8, v, i)) { v = h2f(hi); i = n + 8; }
+#pragma unroll
+                for (int off = 4; off <= 16; off <<= 1) {
+                    const float ov = __shfl_xor_sync(0xffffffffu, v, off);
+                    const int oi = __shfl_xor_sync(0xffffffffu, i, off);
+                    if (head_better(ov, oi, v, i)) { v = ov; i = oi; }
+                }
+                if (r == 0 && head_better(v, i, s_val[warp][row], s_idx[warp][row])) { s_val[warp][row] = v; s_idx[warp][row] = i; }
+            }
+    }
+    __syncthreads();
+    const int parts = gridDim.x;
+    if ((int)threadIdx.x < geo.nrows) {
+        const int row = threadIdx.x;
+        float bv = -INFINITY; int bi = 0x7fffffff;
+        for (int w = 0; w < NW; ++w) if (head_better(s_val[w][row], s_idx[w][row], bv, bi)) { bv = s_val[w][row]; bi = s_idx[w][row]; }
+        pval[(size_t)(geo.row0 + row) * parts + blockIdx.x] = bv;
+        pidx[(size_t)(geo.row0 + row) * parts + blockIdx.x] = bi;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = (atomicAdd(counter, 1u) == gridDim.x * gridDim.y - 1) ? 1 : 0;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int m = warp; m < a.M; m += NW) {                    // one warp per row over the CTAs' maxima
+        float bv = -INFINITY; int bi = 0x7fffffff;
+        for (int p = lane; p < parts; p += 32) {
+            const float v = __ldcg(pval + (size_t)m * parts + p); const int i = __ldcg(pidx + (size_t)m * parts + p);
+            if (head_better(v, i, bv, bi)) { bv = v; bi = i; }
+        }
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
+            const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
+            if (head_better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+        }
+        if (lane == 0) out_tok[m] = bi;
+    }
+    if (threadIdx.x == 0) *counter = 0u;
+}
+template <int RG>
+static void launch_head_rows_t(const RowsDenseArgs& d, const DenseArgs& a, cudaStream_t st, bool pdl) {
+    static bool configured = false;
+    if (!configured) { cudaFuncSetAttribute(k_head_rows<RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(RD_ROOM - 8192)); configured = true; }
+    const dim3 grid((unsigned)rd_ctas(d.M, 8 * RG, d.N >> 4), (unsigned)((d.M + 8 * RG - 1) / (8 * RG)));
+    profile_launch("k_head", st, [&] { return launch_pdl(pdl, k_head_rows<RG>, grid, 512, rd_smem<RG, 16>(d.K), st, d, a.logits, a.pval, a.pidx, a.out_tok, a.counter); });
+}
+// lm_head of M > 8 rows with the final norm.  Returns false when the shape is not covered.
+bool launch_head_rows(const DenseArgs& a, cudaStream_t st, bool pdl) {
+    if (!a.xq || !a.sxq || a.K % 256 || a.K > 4096 || a.N % 16) return false;
+    // by the pace of a block (tiles x 60, 80 or 100), blocks one after the other
+    const int per_tile[3] = {60, 80, 100};
+    int best = -1; long best_cost = 0;
+    for (int i = 0; i < 3; ++i) {
+        const size_t smem = i == 0 ? rd_smem<2, 16>(a.K) : i == 1 ? rd_smem<3, 16>(a.K) : rd_smem<4, 16>(a.K);
+        const long cost = (long)((a.M + 16 + 8 * i - 1) / (16 + 8 * i)) * per_tile[i];
+        if (smem <= RD_ROOM - 8192 && (best < 0 || cost < best_cost)) { best = i; best_cost = cost; }
+    }
+    if (best < 0) return false;
+    RowsPrepArgs p{a.x, a.ldx, a.nw, nullptr, nullptr, 0, a.eps, a.K, a.xq, a.sxq};
+    launch_rows_prep_args(PRO_RMSNORM, p, a.M, st, pdl);
+    const RowsDenseArgs d{a.q, a.N, a.K, a.M, a.xq, a.sxq, nullptr, 0};
+    if (best == 2) launch_head_rows_t<4>(d, a, st, pdl);
+    else if (best == 1) launch_head_rows_t<3>(d, a, st, pdl);
+    else launch_head_rows_t<2>(d, a, st, pdl);
+    return true;
+}
+
 // ================================================================================ experts
 // Work: (expert slot, block of 8 of its rows) x tiles of 16 weight rows, block-major; slot n_active is the shared expert
 // (all rows).  A CTA per multiprocessor takes an equal, contiguous run of the tiles (one to three blocks at decode sizes)

@@ -661,7 +661,7 @@ void enqueue_mixer(sl_engine* e, const LayerW& L, const __half* rows, const __ha
         g.Hk = c.gdn_k_heads; g.Hv = c.gdn_v_heads; g.eps = c.rms_eps; g.tab = e->tab; g.gdn_index = L.type_index; g.segs = segs_of(e->desc, M); g.y = e->mix;
         g.row_seg = row_seg_of(e->desc, M); g.qk = e->gdn_qk; g.vg = e->gdn_vg; g.err = e->err_flag;
         // segments of many rows: the state-independent part for all rows side by side, then the bare recurrence (same bits)
-        if (e->use_rows && M >= 16) launch_gdn_rows(g, M, nsegs, st, pdl);
+        if (e->use_rows && (M >= 16 || nsegs >= 6)) launch_gdn_rows(g, M, nsegs, st, pdl);
         else launch_gdn_core(g, nsegs, st, pdl);
         o.x = e->mix; o.ldx = e->valDim; o.nw = L.gdn_norm; o.nw32 = L.gdn_norm32; o.z = e->inproj + e->convDim; o.ldz = e->gdn_in;
         launch_dense(L.gdn_norm32 ? PRO_NORMGATE32 : PRO_NORMGATE, resid ? EPI_RESID : EPI_STORE, o, st, pdl);

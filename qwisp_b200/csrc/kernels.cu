@@ -1363,56 +1363,31 @@ void launch_attn_prep(const AttnArgs& a, cudaStream_t st, bool pdl) {
 }
 
 // ---- one-kernel attention: (optional) q/k prep + split-KV decode + merge of the splits ----
-// norm + partial rotation of one 256-wide head held as 8 values per lane; returns the fp16 values
-__device__ __forceinline__ uint4 norm_rope_head(const __half* src, const __half* w, float eps, float theta, int pos, int lane) {
-    uint4 v = reinterpret_cast<const uint4*>(src)[lane];
-    uint4 wv = reinterpret_cast<const uint4*>(w)[lane];
-    const __half* vh = reinterpret_cast<const __half*>(&v);
-    const __half* wh = reinterpret_cast<const __half*>(&wv);
-    float ss = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { float f = h2f(vh[i]); ss = fmaf(f, f, ss); }
-    ss = warp_sum(ss);
-    float inv = __frsqrt_rn(__fadd_rn(__fdiv_rn(ss, 256.0f), eps));
-    float nv[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) nv[i] = h2f(hmul_rn(wh[i], f2h(__fmul_rn(h2f(vh[i]), inv))));
-    float other[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) other[i] = __shfl_xor_sync(0xffffffffu, nv[i], 4);
-    uint4 o; __half* oh = reinterpret_cast<__half*>(&o);
-    const float fpos = (float)pos;
-    const float lnb = logf(theta);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        int d = lane * 8 + i;
-        if (d >= ROPE_D) { oh[i] = f2h(nv[i]); continue; }
-        int ii = (d < 32) ? d : (d - 32);
-        float freq = expf(-2.0f * (float)ii / (float)ROPE_D * lnb);
-        float ang = fpos * freq;
-        float sn, cs; sincosf(ang, &sn, &cs);
-        float x0 = (d < 32) ? nv[i] : other[i], x1 = (d < 32) ? other[i] : nv[i];
-        oh[i] = f2h((d < 32) ? (x0 * cs - x1 * sn) : (x0 * sn + x1 * cs));
-    }
-    return o;
+// grid (runs of splits, KV heads * 2, M), 256 threads, dynamic shared memory AF_SMEM.  A CTA takes four of the kv head's eight
+// query heads and a run of consecutive splits of the row; warp w walks the run's keys w, w + 8, ... (a split is a multiple of
+// 32 keys) and the warps are merged at the end of every split.  Two CTAs fit a multiprocessor.
+// prep != 0 (every row is the only row of its stream in this launch): each CTA norms and rotates its query heads itself,
+// and the CTA whose run holds the row's own position also makes that position's K and V, stores them in the arena and uses
+// them from shared memory.  prep == 0: q and the arena were written by k_attn_prep.  Either way the CTA that finishes last
+// for a (row, four heads) merges the splits, normalises, rounds to fp16 and applies the sigmoid output gate.
+// Bound by latency: a warp has four keys of a 32-key split, and a CTA per split spent 2.4 us on descriptors, pages, two
+// keys in flight and the merge.  So: runs as long as the device stays full, the warp's next eight keys always in flight (a
+// ring in shared memory that every lane fills and reads for itself), and their rows looked up 32 at a time.  By events:
+// 512 rows of one stream 406 -> 278 us, 64 streams 87 -> 48, 17 rows at 1000 keys 64 -> 46.
+__device__ __forceinline__ void af_cp16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-// grid (nsplit, KV heads * 2, M), 256 threads, dynamic shared memory 8*4*256 floats.  A CTA takes four of the kv head's
-// eight query heads, warp w the split's keys w, w + 8, ...: two CTAs fit a multiprocessor (one warp for all eight heads
-// needs 200 registers, so that one CTA's merge had nothing to run beside it).
-// prep != 0 (every row is the only row of its stream in this launch): each CTA norms and rotates its
-// 8 query heads itself, and the CTA whose key range holds the row's own position also makes that
-// position's K and V, stores them in the arena and uses them from shared memory.  prep == 0: q and
-// the arena were written by k_attn_prep.  Either way the CTA that finishes last for a (row, kv head)
-// merges the splits, normalises, rounds to fp16 and applies the sigmoid output gate.
-__global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, unsigned* counters) {
-    extern __shared__ __align__(16) float sm_acc[];           // [8 warps][4 heads][256]
+constexpr int AF_RING = 8;                                    // keys in flight per warp
+constexpr size_t AF_SMEM = (size_t)8 * 4 * ATT_D * 4 + (size_t)8 * AF_RING * ATT_D * 4;
+__global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, int fill, unsigned* counters) {
+    extern __shared__ __align__(16) float sm_acc[];           // [8 warps][4 heads][256], then the rings
     constexpr int HG = 4;                                     // query heads of a CTA
-    __shared__ float sm_m[8][HG], sm_l[8][HG];
+    __shared__ __align__(16) float sm_m[2][8][HG], sm_l[2][8][HG];
     __shared__ __align__(16) __half sq[HG][ATT_D];
     __shared__ __align__(16) __half sk[ATT_D], sv[ATT_D];
     __shared__ int s_last;
     __shared__ float s_cs[32], s_sn[32];
-    const int split = blockIdx.x, kvh = blockIdx.y >> 1, h0 = blockIdx.y * HG, m = blockIdx.z;      // h0: first query head
+    const int kvh = blockIdx.y >> 1, h0 = blockIdx.y * HG, m = blockIdx.z;      // h0: first query head
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Ahead of the programmatic-launch wait: everything that does not depend on this step's in-projection.
     // Stream lengths and page tables were written before the step; with prep != 0 every position below the
@@ -1421,25 +1396,47 @@ __global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, uns
     const int pos_m = row_position(a, m);
     const int N = pos_m + 1;
     int chunk, used, p0, p1;
-    attn_split_range(N, a.nsplit, split, chunk, used, p0, p1);
-    if (split >= used) { pdl_wait(); pdl_launch_dependents(); return; }
-    const bool own = prep && (pos_m >= p0) && (pos_m < p1);
+    attn_split_range(N, a.nsplit, 0, chunk, used, p0, p1);
+    // splits of a CTA: the row's splits over `fill` CTAs, or 16 (a long row must not be one CTA's beside short ones)
+    int runs = max((used + 15) >> 4, min(fill, used));
+    if (runs > (int)gridDim.x) runs = gridDim.x;
+    const int per = (used + runs - 1) / runs;
+    const int sp0 = blockIdx.x * per, sp1 = min(used, sp0 + per);
+    if (sp0 >= used) { pdl_wait(); pdl_launch_dependents(); return; }
+    const int begin = sp0 * chunk, end = min(N, sp1 * chunk);
+    const bool own = prep && pos_m >= begin && pos_m < end;
     const __half* rowp = a.inproj + (size_t)m * a.ld;
-    uint4 kcur = make_uint4(0, 0, 0, 0), vcur = make_uint4(0, 0, 0, 0);
-    const int first = p0 + warp;
-    const bool early_kv = prep && first < p1 && first != pos_m;
-    if (early_kv) {
-        kcur = reinterpret_cast<const uint4*>(kv_ptr(a, slot, first, 0, kvh))[lane];
-        vcur = reinterpret_cast<const uint4*>(kv_ptr(a, slot, first, 1, kvh))[lane];
+    const int first = begin + warp, nk = first < end ? (end - first + 7) >> 3 : 0;
+    const int* pages = a.tab.page_table + (size_t)slot * a.tab.max_pages;
+    const unsigned page_rows = (unsigned)a.n_attn_layers * 2 * a.KV * a.page_size, k_row0 = ((unsigned)a.attn_index * 2 * a.KV + kvh) * a.page_size;
+    const size_t v_off = (size_t)a.KV * a.page_size * ATT_D;
+    uint4* ring = reinterpret_cast<uint4*>(sm_acc + 8 * HG * ATT_D) + (size_t)warp * AF_RING * 64 + lane;      // [key][K | V][32 lanes]
+    unsigned krow = 0;                                        // lane's key of 32: its row of 256 in the arena
+    auto request = [&](int j) {                               // the warp's key j into the ring: one copy group
+        if (j < nk) {
+            if ((j & 31) == 0) {
+                const int pos = first + 8 * (j + lane);
+                if (pos < end) { const int pg = pos / a.page_size; krow = (unsigned)pages[pg] * page_rows + k_row0 + (unsigned)(pos - pg * a.page_size); }
+            }
+            const __half* k = a.kv_pool + (size_t)__shfl_sync(0xffffffffu, krow, j & 31) * ATT_D + lane * 8;
+            if (!own || first + 8 * j != pos_m) {
+                uint4* d = ring + (j % AF_RING) * 64;
+                af_cp16(d, k); af_cp16(d + 32, k + v_off);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (prep) {
+        for (int j = 0; j < AF_RING; ++j) request(j);
+        if (threadIdx.x < 32) rope_table_entry(a.theta, pos_m, threadIdx.x, s_cs[threadIdx.x], s_sn[threadIdx.x]);
     }
-    if (prep && threadIdx.x < 32) rope_table_entry(a.theta, pos_m, threadIdx.x, s_cs[threadIdx.x], s_sn[threadIdx.x]);
     pdl_wait();
     pdl_launch_dependents();
     if (prep) {
         __syncthreads();                                      // the rotation table
         if (warp < HG) {
-        uint4 qo = norm_rope_head_tab(reinterpret_cast<const uint4*>(rowp + (size_t)(h0 + warp) * 2 * ATT_D)[lane], a.q_norm, a.eps, s_cs, s_sn, lane);
-        reinterpret_cast<uint4*>(sq[warp])[lane] = qo;
+            uint4 qo = norm_rope_head_tab(reinterpret_cast<const uint4*>(rowp + (size_t)(h0 + warp) * 2 * ATT_D)[lane], a.q_norm, a.eps, s_cs, s_sn, lane);
+            reinterpret_cast<uint4*>(sq[warp])[lane] = qo;
         }
         if (own && warp == 4) {
             uint4 ko = norm_rope_head_tab(reinterpret_cast<const uint4*>(rowp + a.NH * 2 * ATT_D + kvh * ATT_D)[lane], a.k_norm, a.eps, s_cs, s_sn, lane);
@@ -1451,59 +1448,63 @@ __global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, uns
             reinterpret_cast<uint4*>(sv)[lane] = vo;
             if (!(blockIdx.y & 1)) reinterpret_cast<uint4*>(kv_ptr(a, slot, pos_m, 1, kvh))[lane] = vo;
         }
-    } else if (warp < HG) {
-        reinterpret_cast<uint4*>(sq[warp])[lane] = reinterpret_cast<const uint4*>(a.qrot + ((size_t)m * a.NH + h0 + warp) * ATT_D)[lane];
+    } else {
+        for (int j = 0; j < AF_RING; ++j) request(j);
+        if (warp < HG) reinterpret_cast<uint4*>(sq[warp])[lane] = reinterpret_cast<const uint4*>(a.qrot + ((size_t)m * a.NH + h0 + warp) * ATT_D)[lane];
     }
     __syncthreads();
     const float scale = 0.0625f;                              // 256^-0.5
-    float q[HG][8], acc[HG][8];
+    f32x2 q[HG / 2][8];
 #pragma unroll
-    for (int g = 0; g < HG; ++g) {
-        uint4 qv = reinterpret_cast<const uint4*>(sq[g])[lane];
-        const __half* qh = reinterpret_cast<const __half*>(&qv);
+    for (int p = 0; p < HG / 2; ++p) {
+        const uint4 qa = reinterpret_cast<const uint4*>(sq[2 * p])[lane], qb = reinterpret_cast<const uint4*>(sq[2 * p + 1])[lane];
+        const __half *ah = reinterpret_cast<const __half*>(&qa), *bh = reinterpret_cast<const __half*>(&qb);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) { q[g][i] = scale * h2f(qh[i]); acc[g][i] = 0.f; }
+        for (int i = 0; i < 8; ++i) q[p][i] = pk2(scale * h2f(ah[i]), scale * h2f(bh[i]));
     }
-    float mx = -INFINITY, l = 0.f;                            // of head h0 + lane / 8
-    // keys of this warp: first, first + 8, ...; the next key's K and V are requested before the current one is used
-    auto load_kv = [&](int pos, uint4& kk, uint4& vv) {
-        if (own && pos == pos_m) { kk = reinterpret_cast<const uint4*>(sk)[lane]; vv = reinterpret_cast<const uint4*>(sv)[lane]; }
-        else {
-            kk = reinterpret_cast<const uint4*>(kv_ptr(a, slot, pos, 0, kvh))[lane];
-            vv = reinterpret_cast<const uint4*>(kv_ptr(a, slot, pos, 1, kvh))[lane];
+    int pos = first, j = 0;
+#pragma unroll 1
+    for (int sp = sp0; sp < sp1; ++sp) {
+        const int lim = min(N, (sp + 1) * chunk), pb = (sp - sp0) & 1;
+        f32x2 acc[HG][4];
+#pragma unroll
+        for (int g = 0; g < HG; ++g)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[g][i] = pk2(0.f, 0.f);
+        float mx = -INFINITY, l = 0.f;                        // of head h0 + lane / 8
+#pragma unroll 1
+        for (; pos < lim; pos += 8, ++j) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(AF_RING - 1) : "memory");
+            const uint4* src = ring + (j % AF_RING) * 64;
+            uint4 kk, vv;
+            if (own && pos == pos_m) { kk = reinterpret_cast<const uint4*>(sk)[lane]; vv = reinterpret_cast<const uint4*>(sv)[lane]; }
+            else { kk = src[0]; vv = src[32]; }
+            attn_key_step4(q, kk, vv, mx, l, acc, lane);
+            request(j + AF_RING);                             // into the place just read
         }
-    };
-    if (!early_kv && first < p1) load_kv(first, kcur, vcur);
-    for (int pos = first; pos < p1; pos += 8) {
-        uint4 knext = make_uint4(0, 0, 0, 0), vnext = make_uint4(0, 0, 0, 0);
-        if (pos + 8 < p1) load_kv(pos + 8, knext, vnext);
-        const __half* kh = reinterpret_cast<const __half*>(&kcur);
-        const __half* vh = reinterpret_cast<const __half*>(&vcur);
-        float kf[8], vf[8];
+        // ---- merge the 8 warps: all heads at once through shared memory ----
+        if ((lane & 7) == 0) { sm_m[pb][warp][lane >> 3] = mx; sm_l[pb][warp][lane >> 3] = l; }
+        __syncthreads();                                      // (also: everyone is done with the split before in sm_acc)
+        float4 gm4 = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) { kf[i] = h2f(kh[i]); vf[i] = h2f(vh[i]); }
-        attn_key_step4(q, kf, vf, mx, l, acc, lane);
-        kcur = knext; vcur = vnext;
-    }
-    // ---- merge the 8 warps: all heads at once through shared memory ----
-    if ((lane & 7) == 0) { sm_m[warp][lane >> 3] = mx; sm_l[warp][lane >> 3] = l; }
-    __syncthreads();
+        for (int w = 0; w < 8; ++w) {
+            const float4 v = *reinterpret_cast<const float4*>(sm_m[pb][w]);
+            gm4.x = fmaxf(gm4.x, v.x); gm4.y = fmaxf(gm4.y, v.y); gm4.z = fmaxf(gm4.z, v.z); gm4.w = fmaxf(gm4.w, v.w);
+        }
+        const float4 mine4 = *reinterpret_cast<const float4*>(sm_m[pb][warp]);
+        const float gms[HG] = {gm4.x, gm4.y, gm4.z, gm4.w}, mine[HG] = {mine4.x, mine4.y, mine4.z, mine4.w};
 #pragma unroll
-    for (int g = 0; g < HG; ++g) {
-        float m8[8];
-#pragma unroll
-        for (int w = 0; w < 8; ++w) m8[w] = sm_m[w][g];
-        const float gm = attn_warps_max(m8), mine = sm_m[warp][g];
-        float f = (mine == -INFINITY) ? 0.f : __expf(mine - gm);
-        float4 lo = make_float4(acc[g][0] * f, acc[g][1] * f, acc[g][2] * f, acc[g][3] * f);
-        float4 hi = make_float4(acc[g][4] * f, acc[g][5] * f, acc[g][6] * f, acc[g][7] * f);
-        float4* dst = reinterpret_cast<float4*>(sm_acc + ((size_t)warp * HG + g) * ATT_D + lane * 8);
-        dst[0] = lo; dst[1] = hi;
-    }
-    __syncthreads();
-    {
+        for (int g = 0; g < HG; ++g) {
+            const float f = (mine[g] == -INFINITY) ? 0.f : __expf(mine[g] - gms[g]);
+            const f32x2 f2 = pk2(f, f);
+            float4* dst = reinterpret_cast<float4*>(sm_acc + ((size_t)warp * HG + g) * ATT_D + lane * 8);
+            const float2 a0 = unpk2(mul2(acc[g][0], f2)), a1 = unpk2(mul2(acc[g][1], f2)), a2 = unpk2(mul2(acc[g][2], f2)), a3 = unpk2(mul2(acc[g][3], f2));
+            dst[0] = make_float4(a0.x, a0.y, a1.x, a1.y);
+            dst[1] = make_float4(a2.x, a2.y, a3.x, a3.y);
+        }
+        __syncthreads();
         const int d = threadIdx.x;                            // 256 threads = 256 dims
-        float* po = a.part_o + (((size_t)m * a.NH + h0) * a.nsplit + split) * ATT_D;
+        float* po = a.part_o + (((size_t)m * a.NH + h0) * a.nsplit + sp) * ATT_D;
 #pragma unroll
         for (int g = 0; g < HG; ++g) {
             float o = 0.f;
@@ -1514,21 +1515,21 @@ __global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, uns
         if (threadIdx.x < HG) {
             const int g = threadIdx.x;
             float m8[8], l8[8];
-            for (int w = 0; w < 8; ++w) { m8[w] = sm_m[w][g]; l8[w] = sm_l[w][g]; }
+            for (int w = 0; w < 8; ++w) { m8[w] = sm_m[pb][w][g]; l8[w] = sm_l[pb][w][g]; }
             const float gm = attn_warps_max(m8);
             const float ls = attn_warps_lsum(m8, l8, gm);
-            float* pml = a.part_ml + (((size_t)m * a.NH + h0 + g) * a.nsplit + split) * 2;
+            float* pml = a.part_ml + (((size_t)m * a.NH + h0 + g) * a.nsplit + sp) * 2;
             pml[0] = gm; pml[1] = ls;
         }
     }
-    // ---- the CTA that finishes last for this (row, kv head) merges the splits ----
+    // ---- the CTA that finishes last for this (row, four heads) merges the splits ----
     // (the output gate of this warp's head does not depend on the other CTAs: fetched before the ticket)
     const uint4 gvv = reinterpret_cast<const uint4*>(rowp + (size_t)(h0 + (warp & 3)) * 2 * ATT_D + ATT_D)[lane];
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned ticket = atomicAdd(counters + m * gridDim.y + blockIdx.y, 1u);
-        s_last = (ticket == (unsigned)used - 1) ? 1 : 0;
+        s_last = (ticket == (unsigned)((used + per - 1) / per) - 1) ? 1 : 0;
     }
     __syncthreads();
     if (!s_last) return;
@@ -1546,17 +1547,15 @@ __global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, uns
 }
 void launch_attn_fused(const AttnArgs& a, bool prep, unsigned* counters, cudaStream_t st, bool pdl) {
     static bool configured = false;
-    const size_t smem = (size_t)8 * 4 * ATT_D * sizeof(float);
-    if (!configured) { cudaFuncSetAttribute(k_attn_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(a.max_keys > 0 && a.max_keys < 32 * a.nsplit ? (a.max_keys + 31) / 32 : a.nsplit), (unsigned)a.KV * 2, (unsigned)a.M);
-    cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    set_pdl(cfg, attr, pdl);
-    AttnArgs copy = a; int p = prep ? 1 : 0;
-    ProfScope ps("k_attn_fused", 0.0, st);
-    cudaLaunchKernelEx(&cfg, k_attn_fused, copy, p, counters);
-    COUNT_LAUNCH();
+    if (!configured) { cudaFuncSetAttribute(k_attn_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AF_SMEM); configured = true; }
+    // CTAs of a row: no more than splits can exist, and one wave over all rows, but at least one for 16 splits
+    const int splits = a.max_keys > 0 && a.max_keys < 32 * a.nsplit ? (a.max_keys + 31) / 32 : a.nsplit;
+    int fill = 2 * sm_count() / (a.KV * 2 * a.M);
+    if (fill > splits) fill = splits;
+    if (fill < 1) fill = 1;
+    const int least = (splits + 15) / 16, gx = fill > least ? fill : least;
+    const int p = prep ? 1 : 0;
+    profile_launch("k_attn_fused", st, [&] { return launch_pdl(pdl, k_attn_fused, dim3((unsigned)gx, (unsigned)a.KV * 2, (unsigned)a.M), 256, AF_SMEM, st, a, p, fill, counters); });
 }
 
 

@@ -133,23 +133,38 @@ __device__ __forceinline__ float warp_sum4(float a, float b, float c, float d, i
 }
 // attn_key_step() for four query heads at once: lanes 8i .. 8i+7 keep head i's maximum and normaliser (mx, l) and make its
 // two exponentials, which every lane then fetches for its dims
-__device__ __forceinline__ void attn_key_step4(const float q[4][8], const float kf[8], const float vf[8], float& mx, float& l, float acc[4][8], int lane) {
-    float sc[4];
+// Pairs of f32 values in one 64-bit register: two multiply-adds in one instruction, each with the bits of the scalar one.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk2(float lo, float hi) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ float2 unpk2(f32x2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+// q[p][i]: dim i of heads 2p | 2p + 1 (a dot product is one chain over the dims, so the heads are the pairs there);
+// acc[g][j]: dims 2j | 2j + 1 of head g
+__device__ __forceinline__ void attn_key_step4(const f32x2 q[2][8], uint4 kk, uint4 vv, float& mx, float& l, f32x2 acc[4][4], int lane) {
+    const __half2 *kh = reinterpret_cast<const __half2*>(&kk), *vh = reinterpret_cast<const __half2*>(&vv);
+    f32x2 sc[2] = {pk2(0.f, 0.f), pk2(0.f, 0.f)};
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        sc[g] = 0.f;
+    for (int i = 0; i < 4; ++i) {
+        const float2 k2 = __half22float2(kh[i]);
+        const f32x2 ka = pk2(k2.x, k2.x), kb = pk2(k2.y, k2.y);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) sc[g] = fmaf(q[g][i], kf[i], sc[g]);
+        for (int p = 0; p < 2; ++p) { sc[p] = fma2(q[p][2 * i], ka, sc[p]); sc[p] = fma2(q[p][2 * i + 1], kb, sc[p]); }
     }
-    const float s = warp_sum4(sc[0], sc[1], sc[2], sc[3], lane);
+    const float2 s01 = unpk2(sc[0]), s23 = unpk2(sc[1]);
+    const float s = warp_sum4(s01.x, s01.y, s23.x, s23.y, lane);
     const float nm = fmaxf(mx, s);
     const float factor = __expf(mx - nm), es = __expf(s - nm);
     mx = nm; l = fmaf(l, factor, es);
+    f32x2 v2[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { const float2 v = __half22float2(vh[j]); v2[j] = pk2(v.x, v.y); }
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
         const float fg = __shfl_sync(0xffffffffu, factor, 8 * g), eg = __shfl_sync(0xffffffffu, es, 8 * g);
+        const f32x2 f2 = pk2(fg, fg), e2 = pk2(eg, eg);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[g][i] = fmaf(acc[g][i], fg, eg * vf[i]);
+        for (int j = 0; j < 4; ++j) acc[g][j] = fma2(acc[g][j], f2, mul2(e2, v2[j]));
     }
 }
 // merge of the 8 key-warps of a split for one head: the maximum, and the rescaled normaliser

@@ -579,8 +579,10 @@ int32_t enqueue_moe_ep(sl_engine* e, const LayerW& L, RouterArgs ra, int M, __ha
 }
 
 // next: the layer after L (nullptr after the last one, where the lm_head follows)
+// next_prepared (optional): set where the combine also leaves the next layer's normed rows in xq / sxq
 // defer (optional): where the combine may be left to the next layer's in-projection, it is, and *defer says what it needs
-void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half* rows, int ld, bool apply_norm, int M, __half* resid, __half* plain_out, MoeRow* defer = nullptr) {
+void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half* rows, int ld, bool apply_norm, int M, __half* resid, __half* plain_out, MoeRow* defer = nullptr,
+                 bool* next_prepared = nullptr) {
     cudaStream_t st = e->stream;
     RouterArgs ra{}; ra.h = rows; ra.ldh = ld; ra.norm_w = apply_norm ? L.post_norm : nullptr; ra.eps = e->cfg.rms_eps;
     ra.router = L.router; ra.shared_gate = L.shared_gate; ra.M = M; ra.H = e->H; ra.E = e->E;
@@ -627,7 +629,10 @@ void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half
         if (!prepared) launch_rows_prep_plain(e->p, e->H, M, e->H, e->xq_p, e->sx_p, st, pdl);
         ea.xq = e->xq_p; ea.sxq = e->sx_p; ea.csum = e->csum; ea.tile_counter = nullptr;
         if (launch_expert_rows_gateup(ea, st, pdl) && launch_expert_rows_down(ea, st, pdl)) {
-            launch_moe_combine(e->dbuf, e->dbuf + (size_t)M * e->topk * e->H, e->scores, e->sgl, M, e->H, e->topk, resid, plain_out, st, pdl);
+            const bool prep = next_prepared && next && !e->hybrid && resid && dense_rows_shape(M, (int)next->in_proj.N, e->H);
+            launch_moe_combine(e->dbuf, e->dbuf + (size_t)M * e->topk * e->H, e->scores, e->sgl, M, e->H, e->topk, resid, plain_out, st, pdl,
+                               prep ? next->in_norm : nullptr, e->cfg.rms_eps, prep ? e->xq : nullptr, e->sxq);
+            if (prep) *next_prepared = true;
             return;
         }
         ea.tile_counter = e->tile_counters;
@@ -638,14 +643,14 @@ void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half
 
 // mixer of one layer: input rows are normed inside (norm_w != nullptr) or already normed
 void enqueue_mixer(sl_engine* e, const LayerW& L, const __half* rows, const __half* norm_w, int M, int nsegs,
-                   __half* resid, __half* plain_out, const int* row_pos_override, const MoeRow* pending = nullptr) {
+                   __half* resid, __half* plain_out, const int* row_pos_override, const MoeRow* pending = nullptr, bool prepared = false) {
     cudaStream_t st = e->stream;
     const bool pdl = e->use_pdl;
     const sl_config& c = e->cfg;
     DenseArgs d{}; d.err = e->err_flag; d.norm_scratch = e->normed; d.xq = e->use_rows ? e->xq : nullptr; d.sxq = e->sxq; d.q = L.r_in; d.N = (int)L.in_proj.N; d.K = e->H; d.M = M;
     d.x = rows; d.ldx = e->H; d.nw = norm_w; d.eps = c.rms_eps; d.y = e->inproj; d.ldy = (int)L.in_proj.N;
     if (e->use_prefetch) pf_q4(d.pf, 0, L.r_out);
-    d.tc = e->hybrid;
+    d.tc = e->hybrid; d.prepared = prepared;
     if (pending) d.moe = *pending;                             // rows: the residual before the last block's combine; resid: where it is kept after it
     launch_dense(pending ? PRO_MOERMS : (norm_w ? PRO_RMSNORM : PRO_PLAIN), EPI_STORE, d, st, pdl);
     DenseArgs o{};
@@ -690,6 +695,7 @@ void enqueue_step(sl_engine* e, int M, int nsegs, HeadMode head, bool want_logit
     e->ep_layer_seq = 0;
     launch_embed(e->embed, e->tok_in, M, e->H, e->V, e->h, st);
     __half* h = e->h;                                          // the residual rows
+    bool prepared = false;                                     // the layer's normed rows are in xq / sxq already
     MoeRow moe;                                                // a one-row step's last MoE block, not yet combined (moe.d set)
     for (size_t li = 0; li < e->layers.size(); ++li) {
         const LayerW& L = e->layers[li];
@@ -697,9 +703,9 @@ void enqueue_step(sl_engine* e, int M, int nsegs, HeadMode head, bool want_logit
         const __half* rows = h;
         const MoeRow* pending = moe.d ? &moe : nullptr;
         if (pending) { h = (h == e->h) ? e->h2 : e->h; moe.out = h; }
-        enqueue_mixer(e, L, rows, L.in_norm, M, nsegs, h, nullptr, nullptr, pending);
-        moe = MoeRow{};
-        enqueue_moe(e, L, next, h, e->H, true, M, h, nullptr, next && M == 1 && !e->hybrid && !e->ep_step ? &moe : nullptr);
+        enqueue_mixer(e, L, rows, L.in_norm, M, nsegs, h, nullptr, nullptr, pending, prepared);
+        moe = MoeRow{}; prepared = false;
+        enqueue_moe(e, L, next, h, e->H, true, M, h, nullptr, next && M == 1 && !e->hybrid && !e->ep_step ? &moe : nullptr, &prepared);
     }
     if (head == HEAD_NORMED) {
         launch_final_norm(h, e->final_norm, e->cfg.rms_eps, M, e->H, e->normed, st, e->use_pdl);

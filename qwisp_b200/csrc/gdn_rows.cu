@@ -28,9 +28,7 @@ __global__ void __launch_bounds__(128) k_gdn_prep(GdnArgs a) {
     __shared__ float red_s[R][8];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.y * R, nr = min(R, a.M - m0);
-    pdl_wait();
-    pdl_launch_dependents();
-    const SegDesc seg = a.segs[a.row_seg[m0]];
+    const SegDesc seg = a.segs[a.row_seg[m0]];                // descriptors, history, weights: ahead of the programmatic-launch wait
     const int t0 = m0 - seg.row0;
     const int keyDim = a.Hk * GDN_DK, valDim = a.Hv * GDN_DV, convDim = 2 * keyDim + valDim;
     const int side = a.tab.parity[seg.slot];
@@ -39,13 +37,15 @@ __global__ void __launch_bounds__(128) k_gdn_prep(GdnArgs a) {
     __half* hist_out = a.tab.conv_hist + (size_t)seg.slot * a.tab.hist_stride_stream + (size_t)(side ^ 1) * a.tab.hist_stride_side +
                        (size_t)a.gdn_index * a.tab.hist_stride_layer;
     // taps of rows m0 .. m0 + R - 1: entries t0 .. t0 + R + 2 of [hist(3) | rows of the segment]
+    auto past = [&](int ch, __half x[R + 3]) {
+#pragma unroll
+        for (int j = 0; j < R + 3; ++j) x[j] = j < CONV_K - 1 && t0 + j < CONV_K - 1 ? hist_in[(size_t)(t0 + j) * convDim + ch] : f2h(0.f);
+    };
     auto window = [&](int ch, __half x[R + 3]) {
 #pragma unroll
         for (int j = 0; j < R + 3; ++j) {
             const int idx = t0 + j;
-            x[j] = f2h(0.f);
-            if (idx < CONV_K - 1) x[j] = hist_in[(size_t)idx * convDim + ch];
-            else if (j < nr + 3) x[j] = a.inproj[(size_t)(seg.row0 + idx - (CONV_K - 1)) * a.ld + ch];
+            if (idx >= CONV_K - 1 && j < nr + 3) x[j] = a.inproj[(size_t)(seg.row0 + idx - (CONV_K - 1)) * a.ld + ch];
         }
     };
     auto conv = [&](const __half* x, float4 w) { return gdn_conv_silu(h2f(x[0]), h2f(x[1]), h2f(x[2]), h2f(x[3]), w); };
@@ -61,6 +61,9 @@ __global__ void __launch_bounds__(128) k_gdn_prep(GdnArgs a) {
         const int hk = blockIdx.x, ch_q = hk * GDN_DK + tid, ch_k = keyDim + hk * GDN_DK + tid;
         const float4 wq = *reinterpret_cast<const float4*>(a.conv_w + (size_t)ch_q * 4), wk = *reinterpret_cast<const float4*>(a.conv_w + (size_t)ch_k * 4);
         __half xq[R + 3], xk[R + 3];
+        past(ch_q, xq); past(ch_k, xk);
+        pdl_wait();
+        pdl_launch_dependents();
         window(ch_q, xq); window(ch_k, xk);
         float qc[R], kc[R];
 #pragma unroll
@@ -84,7 +87,11 @@ __global__ void __launch_bounds__(128) k_gdn_prep(GdnArgs a) {
     } else {
         const int hv = blockIdx.x - a.Hk, ch_v = 2 * keyDim + hv * GDN_DV + tid;
         const float4 wv = *reinterpret_cast<const float4*>(a.conv_w + (size_t)ch_v * 4);
+        const float A_log = a.A_log[hv], dt_bias = a.dt_bias[hv];
         __half xv[R + 3];
+        past(ch_v, xv);
+        pdl_wait();
+        pdl_launch_dependents();
         window(ch_v, xv);
         unsigned char* rec = a.vg + ((size_t)(hv * 4 + warp) * a.M + m0) * GS_REC;
 #pragma unroll
@@ -93,7 +100,7 @@ __global__ void __launch_bounds__(128) k_gdn_prep(GdnArgs a) {
         if (lane < nr) {                                      // every warp makes the gates its quarter's records need
             const __half* gp = a.inproj + (size_t)(m0 + lane) * a.ld + convDim + valDim + hv;
             float g, beta;
-            gdn_gate(gp[0], gp[a.Hv], a.A_log[hv], a.dt_bias[hv], g, beta);
+            gdn_gate(gp[0], gp[a.Hv], A_log, dt_bias, g, beta);
             *reinterpret_cast<float4*>(rec + (size_t)lane * GS_REC + 128) = make_float4(g, g, beta, 0.f);
         }
         if (last) leave(ch_v, xv);

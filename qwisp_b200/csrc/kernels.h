@@ -23,6 +23,7 @@ struct DenseArgs {
     __half* y; int ldy;                                          // output rows
     __half* logits;                                              // optional [M][N] (argmax epilogue)
     float* pval; int* pidx; int* out_tok; unsigned* counter;     // argmax partials / result / ticket
+    bool prepared = false;                                       // xq / sxq already hold the prologue's rows (a many-row call)
     PfList pf;                                                   // weights of later kernels to pull into L2
     MoeRow moe;                                                  // PRO_MOERMS: x is the residual row before the last MoE block's combine
 };
@@ -231,6 +232,7 @@ int launch_step_persistent(const PStepArgs& a, cudaStream_t st);   // cooperativ
 
 void launch_dense(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl);
 // many-row forms (more than 8 rows per call); the bool launchers return false when the shape is not covered
+inline bool dense_rows_shape(int M, int N, int K) { return M > 8 && K % 256 == 0 && K <= 4096 && N % 16 == 0; }
 bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl);
 bool launch_head_rows(const DenseArgs& a, cudaStream_t st, bool pdl);      // lm_head + argmax behind the final norm
 void launch_rows_prep_plain(const __half* x, int ldx, int M, int K, __half* xq, float* sxq, cudaStream_t st, bool pdl);
@@ -242,8 +244,9 @@ bool launch_router_rows(const RouterArgs& a, cudaStream_t st, bool pdl);
 bool launch_router_mma(const RouterArgs& a, cudaStream_t st, bool pdl);    // prefill mode, fp16 router: logits on the tensor cores
 bool launch_expert_rows_gateup(const ExpertArgs& a, cudaStream_t st, bool pdl);
 bool launch_expert_rows_down(const ExpertArgs& a, cudaStream_t st, bool pdl);
+// xq / sxq (optional): the rows also normed with nw and prepared for the next layer's in-projection (H a multiple of 256, <= 4096)
 void launch_moe_combine(const __half* dbuf, const __half* shared_rows, const __half* scores, const __half* sgl, int M, int H, int topk,
-                        __half* resid, __half* out, cudaStream_t st, bool pdl);
+                        __half* resid, __half* out, cudaStream_t st, bool pdl, const __half* nw = nullptr, float eps = 0.f, __half* xq = nullptr, float* sxq = nullptr);
 // many-row GEMM on tcgen05 tensor cores with the accumulator in tensor memory (N % 16 == 0, K % 256 == 0); 0 or an error code
 int launch_gemm_tc(const Q4R& q, int N, int K, int M, const __half* x, int ldx, __half* y, int ldy, bool add_to_y, unsigned* err, cudaStream_t st, bool pdl);
 // speculative-sampling rows on fp16 logits [M][V]: categorical draw, draw without the draft token, accept flag

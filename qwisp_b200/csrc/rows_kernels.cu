@@ -350,9 +350,9 @@ static void launch_gemv_rows(const RowsDenseArgs& a, cudaStream_t st, bool pdl) 
 }
 // dense projection of M > 8 rows: prologue rows, then the tile kernel.  Returns false when the shape is not covered.
 bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl) {
-    if (!a.xq || !a.sxq || a.K % 256 || a.K > 4096 || a.N % 16 || (epi != EPI_STORE && epi != EPI_RESID)) return false;
+    if (!a.xq || !a.sxq || !dense_rows_shape(a.M, a.N, a.K) || (epi != EPI_STORE && epi != EPI_RESID)) return false;
     RowsPrepArgs p{a.x, a.ldx, a.nw, a.nw32, a.z, a.ldz, a.eps, a.K, a.xq, a.sxq};
-    launch_rows_prep_args(pro, p, a.M, st, pdl);
+    if (!a.prepared) launch_rows_prep_args(pro, p, a.M, st, pdl);
     RowsDenseArgs d{a.q, a.N, a.K, a.M, a.xq, a.sxq, a.y, a.ldy};
     if (epi == EPI_RESID) launch_gemv_rows<EPI_RESID>(d, st, pdl); else launch_gemv_rows<EPI_STORE>(d, st, pdl);
     return true;
@@ -958,13 +958,15 @@ __global__ void __launch_bounds__(256) k_route_rows(RouterArgs a) {
     }
     const int m = blockIdx.x * 8 + warp;
     if (m < a.M) route_row_warp(a.logits + (size_t)m * a.E, a.E, a.topk, a.inds + m * a.topk, a.scores + m * a.topk, s_route[warp], lane);
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) { const unsigned ticket = atomicAdd(a.counter, 1u); s_last = (ticket == gridDim.x - 1) ? 1 : 0; }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    if (tid == 0) *a.counter = 0u;
+    if (gridDim.x > 1) {
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) { const unsigned ticket = atomicAdd(a.counter, 1u); s_last = (ticket == gridDim.x - 1) ? 1 : 0; }
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        if (tid == 0) *a.counter = 0u;
+    }
     // ---- pairs grouped by expert: counts, then slot numbers and offsets by a block scan (thread = expert)
     s_cnt[tid] = 0; s_cur[tid] = 0;
     __syncthreads();
@@ -1106,9 +1108,14 @@ bool launch_router_rows(const RouterArgs& a, cudaStream_t st, bool pdl) {
 // (swift/Sources/QwispCore/SeedlessFusedVerify.swift:462-484, SeedlessMetalForward.swift:1024-1028)
 // Bound by latency: with one output and 2-byte loads per thread and step the eight steps of a thread were 8 dependent
 // round trips; all 16-byte loads of a thread are now in flight at once.
-__global__ void __launch_bounds__(256) k_moe_combine(const __half* dbuf, const __half* shared_rows, const __half* scores, const __half* sgl,
-                                                     int H, int topk, __half* resid, __half* out) {
+// NORM (grid (M), H / 8 threads): the CTA has the whole residual row, and leaves it normed and prepared for the next layer's
+// in-projection as well (the arithmetic of k_rows_prep<PRO_RMSNORM>; a launch less per layer).
+template <bool NORM>
+__global__ void __launch_bounds__(NORM ? 512 : 256) k_moe_combine(const __half* dbuf, const __half* shared_rows, const __half* scores, const __half* sgl,
+                                                                  int H, int topk, __half* resid, __half* out, const __half* nw, float eps, __half* xq, float* sxq) {
     const int m = blockIdx.x, n = (blockIdx.y * 256 + threadIdx.x) * 8;
+    uint4 wv = make_uint4(0, 0, 0, 0);
+    if (NORM) wv = *reinterpret_cast<const uint4*>(nw + n);
     pdl_wait();
     pdl_launch_dependents();
     if (n >= H) return;
@@ -1136,11 +1143,23 @@ __global__ void __launch_bounds__(256) k_moe_combine(const __half* dbuf, const _
         rh[i] = resid ? hadd_rn(rh[i], res) : res;
     }
     *reinterpret_cast<uint4*>((resid ? resid : out) + (size_t)m * H + n) = rv;
+    if (NORM) {
+        __shared__ float part[16];
+        const int ch = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const float ss = warp_sum(sumsq8(rv));
+        if (lane == 0) part[ch] = ss;
+        __syncthreads();
+        float tot = 0.f;
+        for (int c = 0; c < (H >> 8); ++c) tot += part[c];
+        const float inv = __frsqrt_rn(__fadd_rn(__fdiv_rn(tot, (float)H), eps));
+        rows_store(xq + (size_t)m * H, sxq + (size_t)m * (H >> 6), n, rms_apply8(rv, wv, inv), lane);
+    }
 }
 void launch_moe_combine(const __half* dbuf, const __half* shared_rows, const __half* scores, const __half* sgl, int M, int H, int topk,
-                        __half* resid, __half* out, cudaStream_t st, bool pdl) {
+                        __half* resid, __half* out, cudaStream_t st, bool pdl, const __half* nw, float eps, __half* xq, float* sxq) {
     profile_launch("k_moe_combine", st, [&] {
-        return launch_pdl(pdl, k_moe_combine, dim3((unsigned)M, (unsigned)((H + 2047) / 2048)), 256, 0, st, dbuf, shared_rows, scores, sgl, H, topk, resid, out);
+        if (xq) return launch_pdl(pdl, k_moe_combine<true>, dim3((unsigned)M), (unsigned)H / 8, 0, st, dbuf, shared_rows, scores, sgl, H, topk, resid, out, nw, eps, xq, sxq);
+        return launch_pdl(pdl, k_moe_combine<false>, dim3((unsigned)M, (unsigned)((H + 2047) / 2048)), 256, 0, st, dbuf, shared_rows, scores, sgl, H, topk, resid, out, nw, eps, xq, sxq);
     });
 }
 

@@ -1,3 +1,4 @@
+#include <atomic>
 // engine.cu -- engine / stream objects and the C ABI of libseedless_b200.so.
 //
 // Host-side orchestration of one step (the op order of the reference's fused step,
@@ -160,9 +161,13 @@ int32_t guard(sl_engine* e) {
     return SL_OK;
 }
 
+// (a device once found stays: asking the driver again cost each single-operator call about a microsecond)
 bool device_ok() {
+    static std::atomic<bool> found{false};
+    if (found.load(std::memory_order_relaxed)) return true;
     int n = 0;
     if (cudaGetDeviceCount(&n) != cudaSuccess || n <= 0) { cudaGetLastError(); return false; }
+    found.store(true, std::memory_order_relaxed);
     return true;
 }
 

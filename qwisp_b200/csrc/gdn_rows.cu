@@ -272,6 +272,9 @@ static void launch_scan_t(const GdnArgs& a, int nsegs, cudaStream_t st) {
 void launch_gdn_rows(const GdnArgs& in, int M, int nsegs, cudaStream_t st, bool pdl) {
     GdnArgs a = in; a.M = M;
     profile_launch("k_gdn_prep", st, [&] {
+        // (8 rows per CTA once that fills the device four times over; of fewer rows, 2)
+        if (nsegs == 1 && (long)(a.Hk + a.Hv) * ((M + 7) / 8) < 4l * sm_count())
+            return launch_pdl(pdl, k_gdn_prep<2>, dim3((unsigned)(a.Hk + a.Hv), (unsigned)((M + 1) / 2)), 128, 0, st, a);
         if (nsegs == 1) return launch_pdl(pdl, k_gdn_prep<8>, dim3((unsigned)(a.Hk + a.Hv), (unsigned)((M + 7) / 8)), 128, 0, st, a);
         return launch_pdl(pdl, k_gdn_prep<1>, dim3((unsigned)(a.Hk + a.Hv), (unsigned)M), 128, 0, st, a);
     });

@@ -1464,7 +1464,7 @@ int32_t sl_op_qmm4_device(const void* x_dev, const void* wr_dev, const void* sr_
     if (M <= 0 || N <= 0 || K <= 0 || N % 16 || !k_ok(K)) return SL_ERR_INVALID;
     if (!device_ok()) return SL_ERR_NO_DEVICE;
     DenseArgs a{}; a.q.wr = (const uint4*)wr_dev; a.q.sr = (const uint4*)sr_dev; a.q.tiles = N / 16; a.q.K = K; a.N = N; a.K = K; a.M = M;
-    a.x = (const __half*)x_dev; a.ldx = K; a.y = (__half*)y_dev; a.ldy = N;
+    a.x = (const __half*)x_dev; a.ldx = K; a.y = (__half*)y_dev; a.ldy = N; a.direct = true;
     launch_dense(PRO_PLAIN, EPI_STORE, a, (cudaStream_t)cuda_stream, false);
     return cudaGetLastError() == cudaSuccess ? SL_OK : SL_ERR_CUDA;
 }

@@ -13,6 +13,7 @@ struct DenseArgs {
     __half* norm_scratch = nullptr;      // [M][K] scratch for the tensor-core path (normed rows); nullptr keeps the GEMV path
     bool tc = false;                     // prefill mode: dense projections on the tcgen05 GEMM (set per call by the caller)
     __half* xq = nullptr; float* sxq = nullptr;   // [M][K] / [M][K/64] scratch of the many-row kernels (calls with more than 8 rows); nullptr: pass kernels
+    bool direct = false;                 // a many-row product of plain rows may run without that scratch
     Q4R q;                                                       // repacked weights (tiles of 16 rows)
     int N, K, M;                                                 // N outputs (= 16 * tiles)
     const __half* x; int ldx;                                    // activations (plain) / residual stream (rmsnorm) / y (normgate)

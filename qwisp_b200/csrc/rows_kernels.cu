@@ -151,6 +151,7 @@ struct RowsDenseArgs {
     Q4R q; int N, K, M;
     const __half* xq; const float* sxq;  // prepared rows
     __half* y; int ldy;
+    const __half* x; int ldx;            // or plain rows, which every CTA prepares for itself (x != nullptr)
 };
 // Bound by instruction issue, shared-memory reads and MMAs about equally (a slice of 16 weight rows against 32 rows: 485
 // instructions of a warp, 150 cycles of shared-memory reads, 64 MMAs; it takes 235 cycles of a multiprocessor).  The form
@@ -166,6 +167,28 @@ __device__ __forceinline__ RdGeom rd_geom(const RowsDenseArgs& a, int nr) {
 // inputs k0 .. k0 + kc - 1 of the rows into xs [row][kc + 8] (16 bytes of skew: conflict-free loads), their group sums into sxs [group][stride]
 __device__ __forceinline__ void rd_stage(const RowsDenseArgs& a, const RdGeom& g, int k0, int kc, __half* xs, float* sxs, int stride) {
     const int c8 = kc >> 3, g64 = kc >> 6;
+    if (a.x) {                                                // the arithmetic of rows_store(), two units of 256 inputs in flight per warp
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, chunks = kc >> 8, units = g.nrows * chunks;
+        for (int u0 = warp; u0 < units; u0 += 2 * nw) {
+            uint4 v[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int u = u0 + i * nw, row = u / chunks, ch = u - row * chunks;
+                if (u < units) v[i] = __ldcg(reinterpret_cast<const uint4*>(a.x + (size_t)(g.row0 + row) * a.ldx + k0 + ch * 256 + lane * 8));
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int u = u0 + i * nw, row = u / chunks, ch = u - row * chunks;
+                if (u >= units) break;
+                float s;                                      // (of lanes 0, 8, 16, 24: one group each)
+                rows_store(xs + (size_t)row * (kc + 8) + ch * 256 + lane * 8, &s, 0, v[i], lane);
+                if ((lane & 7) == 0) sxs[(ch * 4 + (lane >> 3)) * stride + row] = s;
+            }
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        return;
+    }
     for (int i = threadIdx.x; i < g.nrows * c8; i += blockDim.x) {
         const int row = i / c8, c = i - row * c8;
         cp_async16(xs + (size_t)row * (kc + 8) + c * 8, a.xq + (size_t)(g.row0 + row) * a.K + k0 + c * 8);
@@ -350,10 +373,13 @@ static void launch_gemv_rows(const RowsDenseArgs& a, cudaStream_t st, bool pdl) 
 }
 // dense projection of M > 8 rows: prologue rows, then the tile kernel.  Returns false when the shape is not covered.
 bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl) {
-    if (!a.xq || !a.sxq || !dense_rows_shape(a.M, a.N, a.K) || (epi != EPI_STORE && epi != EPI_RESID)) return false;
+    // plain rows need no prologue kernel; of more than 32 the preparation in every CTA costs more than the launch
+    const bool plain = pro == PRO_PLAIN && !a.prepared && (a.direct || a.M <= 32);
+    if (!(a.xq && a.sxq) && !(plain && a.direct)) return false;
+    if (!dense_rows_shape(a.M, a.N, a.K) || (epi != EPI_STORE && epi != EPI_RESID)) return false;
     RowsPrepArgs p{a.x, a.ldx, a.nw, a.nw32, a.z, a.ldz, a.eps, a.K, a.xq, a.sxq};
-    if (!a.prepared) launch_rows_prep_args(pro, p, a.M, st, pdl);
-    RowsDenseArgs d{a.q, a.N, a.K, a.M, a.xq, a.sxq, a.y, a.ldy};
+    if (!a.prepared && !plain) launch_rows_prep_args(pro, p, a.M, st, pdl);
+    RowsDenseArgs d{a.q, a.N, a.K, a.M, a.xq, a.sxq, a.y, a.ldy, plain ? a.x : nullptr, a.ldx};
     if (epi == EPI_RESID) launch_gemv_rows<EPI_RESID>(d, st, pdl); else launch_gemv_rows<EPI_STORE>(d, st, pdl);
     return true;
 }
@@ -482,7 +508,7 @@ bool launch_head_rows(const DenseArgs& a, cudaStream_t st, bool pdl) {
     if (best < 0) return false;
     RowsPrepArgs p{a.x, a.ldx, a.nw, nullptr, nullptr, 0, a.eps, a.K, a.xq, a.sxq};
     launch_rows_prep_args(PRO_RMSNORM, p, a.M, st, pdl);
-    const RowsDenseArgs d{a.q, a.N, a.K, a.M, a.xq, a.sxq, nullptr, 0};
+    const RowsDenseArgs d{a.q, a.N, a.K, a.M, a.xq, a.sxq, nullptr, 0, nullptr, 0};
     if (best == 2) launch_head_rows_t<4>(d, a, st, pdl);
     else if (best == 1) launch_head_rows_t<3>(d, a, st, pdl);
     else launch_head_rows_t<2>(d, a, st, pdl);

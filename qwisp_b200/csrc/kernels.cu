@@ -403,7 +403,12 @@ void launch_dense(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pd
     }
 gemv_path:
     if (a.M > ROWS_PER_PASS && launch_dense_rows(pro, epi, a, st, pdl)) return;
-    const GemvPlan pl = gemv_plan(a.K, epi == EPI_SWIGLU ? a.N / 8 : a.N / 16, 1, sm_count());
+    GemvPlan pl = gemv_plan(a.K, epi == EPI_SWIGLU ? a.N / 8 : a.N / 16, 1, sm_count());
+    // (6 to 8 rows of 4096 inputs leave no shared memory for three units of weights per warp)
+    const int slices = a.K >> 8, pass_rows = a.M < ROWS_PER_PASS ? a.M : ROWS_PER_PASS;
+    while (pl.upw > 1 && GemvSmem::wstage_bytes(16 * pl.upw) + GemvSmem::bytes(pass_rows, a.K, 16 * pl.upw, pl.tpc) > (size_t)200 * 1024 && 16 * (pl.upw - 1) % slices == 0) {
+        --pl.upw; pl.tpc = 16 * pl.upw / slices;
+    }
 #define SL_CASE(P, E)                                                                                       \
     if (pro == P && epi == E) {                                                                             \
         if (pl.upw == 1) launch_gemv_t<P, E, 16, 1>(a, pl, st, pdl);                                        \

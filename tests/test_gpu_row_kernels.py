@@ -1,0 +1,137 @@
+"""Edges of the kernels that a call's shape selects: remainders of row blocks and tiles, runs of attention splits, chunks of the
+state scan, step graphs of many shapes, page edges of the state blob.  References: the same rows one at a time, the
+pass kernels (SL_FLAG_PASS_KERNELS, same bits by contract), and the CPU oracle."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import MINI, TINY, f16_report, gpu_engine
+from test_gpu_engine import prompt
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def engines():
+    import qwisp_b200 as Q
+    args = dict(max_rows=512, kv_pages=512)
+    a, b = gpu_engine(MINI, **args), gpu_engine(MINI, flags=Q._lib.SL_FLAG_PASS_KERNELS, **args)
+    yield a, b
+    a.close(); b.close()
+
+
+def same(x, y):
+    return np.array_equal(np.asarray(x).view(np.uint16), np.asarray(y).view(np.uint16))
+
+
+# passes of 8, the split form, blocks of 8 / 16 / 32 rows, halves of K, a single tile, rows that fill no block
+@pytest.mark.parametrize("M,K,N", [(7, 4096, 8192), (9, 256, 16), (16, 2048, 2064), (17, 512, 1040), (24, 4096, 48), (33, 4096, 2048),
+                                   (64, 2048, 12352), (65, 1024, 4096), (200, 4096, 256), (1200, 256, 32)])
+def test_qmm4_row_blocks(M, K, N):
+    import torch
+    import qwisp_b200 as Q
+    from oracle import oracle as O
+    L = Q.lib()
+    packed, scales, biases = O.synth_q4(3, f"rows.w.{N}.{K}", N, K)
+    x = O.synth_f16(3, f"rows.x.{M}.{K}", M * K, 0.0, 1.0).reshape(M, K)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a).view(np.uint8).reshape(-1)).cuda()
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    dw, ds, db, dx = dev(packed), dev(scales), dev(biases), dev(x)
+    wr = torch.empty((N // 16) * (K // 128) * 1024, dtype=torch.uint8, device="cuda")
+    sr = torch.empty((N // 16) * (K // 128) * 128, dtype=torch.uint8, device="cuda")
+    assert L.sl_op_repack_q4_device(ptr(dw), ptr(ds), ptr(db), K, N, ptr(wr), ptr(sr), None) == 0
+    y = torch.zeros(M * N, dtype=torch.float16, device="cuda")
+    one = torch.zeros(M * N, dtype=torch.float16, device="cuda")
+    assert L.sl_op_qmm4_device(ptr(dx), ptr(wr), ptr(sr), M, K, N, ptr(y), None) == 0
+    for m in range(M):
+        assert L.sl_op_qmm4_device(C.c_void_p(dx.data_ptr() + m * K * 2), ptr(wr), ptr(sr), 1, K, N, C.c_void_p(one.data_ptr() + m * N * 2), None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(y.view(torch.int16), one.view(torch.int16))
+    if K % 512:
+        return                                        # (the oracle walks blocks of 512 inputs)
+    few = [0, M // 2, M - 1]
+    assert f16_report(y.cpu().numpy().reshape(M, N)[few], O.qmm4(np.ascontiguousarray(x[few]), packed, scales, biases))["max_abs"] <= 2e-2
+
+
+# rows of one stream behind nothing, behind one 32-key split and behind more splits than a CTA's run
+@pytest.mark.parametrize("base", [0, 33, 1100])
+@pytest.mark.parametrize("M", [2, 8, 16, 24, 25, 32, 33, 64, 131])
+def test_rows_of_one_stream(engines, base, M):
+    V = MINI["vocab"]
+    toks = prompt(V, base + M + 1, f"rowk.{base}.{M}")
+    out = []
+    for e in engines:
+        s = e.stream(base + M + 8)
+        for i in range(0, base, 300):
+            s.forward(toks[i:min(i + 300, base)], want_hidden=False)
+        out.append((s.step_logits(toks[base:base + M]), s.step_argmax(toks[base + M:]), s.state_save()))
+        assert not e.gpu_fault()
+        s.close()
+    (la, ta, ba), (lb, tb, bb) = out
+    assert same(la, lb) and np.array_equal(ta, tb) and np.array_equal(ba, bb)
+
+
+# streams of very different lengths in one step: the one-row form of the state update, the two-kernel form, one wave of attention and more
+@pytest.mark.parametrize("B", [2, 5, 6, 9, 17, 23])
+def test_batches_of_ragged_streams(engines, B):
+    V = MINI["vocab"]
+    a = engines[0]
+    lens = [1 + (i * 37) % 90 + (700 if i == 1 else 0) for i in range(B)]
+    solo, lane, cur = [], [], []
+    for i, n in enumerate(lens):
+        p = prompt(V, n, f"ragged.{i}")
+        for group in (solo, lane):
+            s = a.stream(n + 8)
+            for j in range(0, n, 300):
+                t = s.step_argmax(p[j:j + 300])
+            group.append(s)
+        cur.append(int(t[-1]))
+    cur_lane = list(cur)
+    for _ in range(2):
+        cur = [int(s.step_argmax([t])[0]) for s, t in zip(solo, cur)]
+        cur_lane = [int(t) for t in a.batch_step_argmax(lane, cur_lane)]
+        assert cur == cur_lane
+    for x, y in zip(solo, lane):
+        assert np.array_equal(x.state_save(), y.state_save())
+        x.close(); y.close()
+
+
+# token tiles and weight-row groups of the tensor-core product
+@pytest.mark.parametrize("M,K,N", [(1, 512, 16), (31, 512, 128), (33, 512, 144), (65, 1024, 2064), (129, 4096, 272), (1000, 512, 144)])
+def test_tensor_core_tiles(M, K, N):
+    from test_gpu_ops import test_tensor_core_gemm_matches_gemv_and_oracle as check
+    check(M, K, N)
+
+
+# more shapes of strict calls than the graph cache holds, some of them again
+def test_step_graphs_of_many_shapes():
+    import qwisp_b200 as Q
+    V = TINY["vocab"]
+    a, b = gpu_engine(TINY), gpu_engine(TINY, flags=Q._lib.SL_FLAG_NO_GRAPH)
+    try:
+        toks = prompt(V, 64, "graphs")
+        for rows in list(range(2, 65)) + [64, 3, 2]:
+            got = []
+            for e in (a, b):
+                s = e.stream(160)
+                got.append((s.step_argmax(toks[:rows]), s.step_argmax(toks[:2]), s.step_logits(toks[:rows])))
+                s.close()
+            assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1]) and same(got[0][2], got[1][2]), rows
+        assert not a.gpu_fault()
+    finally:
+        a.close(); b.close()
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 64, 250])
+def test_state_blob_at_page_edges(engines, n):
+    V = MINI["vocab"]
+    a, b = engines[0], engines[1]
+    s = a.stream(n + 8)
+    s.step_argmax(prompt(V, n, f"page.{n}"))
+    blob = s.state_save()
+    t = b.stream(n + 40)                              # other arena, other pages
+    assert t.state_restore(blob) and np.array_equal(t.state_save(), blob)
+    assert np.array_equal(s.step_argmax([7, 11]), t.step_argmax([7, 11]))
+    assert np.array_equal(s.state_save(), t.state_save())
+    s.close(); t.close()

@@ -402,7 +402,10 @@ void launch_dense(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pd
         return;
     }
 gemv_path:
-    if (a.M > ROWS_PER_PASS && launch_dense_rows(pro, epi, a, st, pdl)) return;
+    // The many-row kernel takes more than 8 rows, and a stand-alone product of few rows that is more than one wave of k_gemv
+    // (16 warps of at most three units): 1 row of 2048 x 16384 9.3 -> 6.8 us, 8 rows 11.9 -> 7.8, of 4096 x 16384 24.1 -> 13.1.
+    const bool waves = a.direct && (long)(a.N >> 4) * (a.K >> 8) > 48l * sm_count();
+    if ((a.M > ROWS_PER_PASS || waves) && launch_dense_rows(pro, epi, a, st, pdl)) return;
     GemvPlan pl = gemv_plan(a.K, epi == EPI_SWIGLU ? a.N / 8 : a.N / 16, 1, sm_count());
     // (6 to 8 rows of 4096 inputs leave no shared memory for three units of weights per warp)
     const int slices = a.K >> 8, pass_rows = a.M < ROWS_PER_PASS ? a.M : ROWS_PER_PASS;

@@ -26,7 +26,7 @@ def same(x, y):
 
 
 # passes of 8, the split form, blocks of 8 / 16 / 32 rows, halves of K, a single tile, rows that fill no block
-@pytest.mark.parametrize("M,K,N", [(7, 4096, 8192), (9, 256, 16), (16, 2048, 2064), (17, 512, 1040), (24, 4096, 48), (33, 4096, 2048),
+@pytest.mark.parametrize("M,K,N", [(7, 4096, 6144), (7, 4096, 8192), (3, 2048, 16384), (9, 256, 16), (16, 2048, 2064), (17, 512, 1040), (24, 4096, 48), (33, 4096, 2048),
                                    (64, 2048, 12352), (65, 1024, 4096), (200, 4096, 256), (1200, 256, 32)])
 def test_qmm4_row_blocks(M, K, N):
     import torch

@@ -76,7 +76,7 @@ struct sl_engine {
     int *desc = nullptr;            // a call's tokens and row / segment descriptors, one block (see row_seg_of); tok_in = its start
     unsigned* counters = nullptr; unsigned* tile_counters = nullptr; unsigned* att_counters = nullptr; unsigned* err_flag = nullptr; unsigned* err_host = nullptr; float* adj_buf = nullptr; int* samp_buf = nullptr; unsigned* slot_sync = nullptr; unsigned* router_groups = nullptr;
     bool use_route_in_experts = true;   // with the fused kernel: routing done by its CTAs (SL_FLAG_ROUTE_IN_ROUTER: by the router's last CTA)
-    bool use_rows = true;           // calls with more than 8 rows use the many-row kernels (SL_FLAG_PASS_KERNELS turns it off)
+    bool use_rows = true;           // calls with more than one row use the many-row kernels (SL_FLAG_PASS_KERNELS turns it off)
     bool use_fused_experts = true;  // batch-1 decode: gate/up + down in one launch (SL_FLAG_SPLIT_EXPERTS turns it off)
     // expert-parallel decode (experts [ep_e0, ep_e1) are this rank's; see sl_ep_init)
     int ep_rank = 0, ep_world = 1, ep_rows = 0, ep_e0 = 0, ep_e1 = 0;
@@ -670,8 +670,8 @@ void enqueue_mixer(sl_engine* e, const LayerW& L, const __half* rows, const __ha
         GdnArgs g{}; g.inproj = e->inproj; g.ld = e->gdn_in; g.conv_w = L.conv_w; g.A_log = L.A_log; g.dt_bias = L.dt_bias;
         g.Hk = c.gdn_k_heads; g.Hv = c.gdn_v_heads; g.eps = c.rms_eps; g.tab = e->tab; g.gdn_index = L.type_index; g.segs = segs_of(e->desc, M); g.y = e->mix;
         g.row_seg = row_seg_of(e->desc, M); g.qk = e->gdn_qk; g.vg = e->gdn_vg; g.err = e->err_flag;
-        // segments of many rows: the state-independent part for all rows side by side, then the bare recurrence (same bits)
-        if (e->use_rows && (M >= 16 || nsegs >= 6)) launch_gdn_rows(g, M, nsegs, st, pdl);
+        // more than one row: the state-independent part for all rows side by side, then the bare recurrence (same bits)
+        if (e->use_rows && M > 1) launch_gdn_rows(g, M, nsegs, st, pdl);
         else launch_gdn_core(g, nsegs, st, pdl);
         o.x = e->mix; o.ldx = e->valDim; o.nw = L.gdn_norm; o.nw32 = L.gdn_norm32; o.z = e->inproj + e->convDim; o.ldz = e->gdn_in;
         launch_dense(L.gdn_norm32 ? PRO_NORMGATE32 : PRO_NORMGATE, resid ? EPI_RESID : EPI_STORE, o, st, pdl);

@@ -402,10 +402,13 @@ void launch_dense(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pd
         return;
     }
 gemv_path:
-    // The many-row kernel takes more than 8 rows, and a stand-alone product of few rows that is more than one wave of k_gemv
-    // (16 warps of at most three units): 1 row of 2048 x 16384 9.3 -> 6.8 us, 8 rows 11.9 -> 7.8, of 4096 x 16384 24.1 -> 13.1.
-    const bool waves = a.direct && (long)(a.N >> 4) * (a.K >> 8) > 48l * sm_count();
-    if ((a.M > ROWS_PER_PASS || waves) && launch_dense_rows(pro, epi, a, st, pdl)) return;
+    // A step's many-row kernels take two rows and more: the gated norm of a row costs every CTA of k_gemv what it costs one CTA
+    // of the prologue kernel (out-projection of 7 rows 12 -> 6 us; steps of 2, 5 and 8 rows 2.00 -> 1.97, 2.76 -> 2.43,
+    // 3.47 -> 2.86 ms with the state update in two kernels).  A stand-alone product of plain rows has no prologue: more than 8
+    // rows, or more than one wave of k_gemv (16 warps of at most three units): 1 row of 2048 x 16384 9.3 -> 6.8 us, 8 rows
+    // 11.9 -> 7.8, of 4096 x 16384 24.1 -> 13.1.
+    const bool rows = !a.direct || a.M > ROWS_PER_PASS || (long)(a.N >> 4) * (a.K >> 8) > 48l * sm_count();
+    if (rows && launch_dense_rows(pro, epi, a, st, pdl)) return;
     GemvPlan pl = gemv_plan(a.K, epi == EPI_SWIGLU ? a.N / 8 : a.N / 16, 1, sm_count());
     // (6 to 8 rows of 4096 inputs leave no shared memory for three units of weights per warp)
     const int slices = a.K >> 8, pass_rows = a.M < ROWS_PER_PASS ? a.M : ROWS_PER_PASS;

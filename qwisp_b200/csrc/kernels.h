@@ -12,7 +12,7 @@ struct DenseArgs {
     unsigned* err = nullptr;             // set to 1 if a bounded wait on a bulk copy gave up
     __half* norm_scratch = nullptr;      // [M][K] scratch for the tensor-core path (normed rows); nullptr keeps the GEMV path
     bool tc = false;                     // prefill mode: dense projections on the tcgen05 GEMM (set per call by the caller)
-    __half* xq = nullptr; float* sxq = nullptr;   // [M][K] / [M][K/64] scratch of the many-row kernels (calls with more than 8 rows); nullptr: pass kernels
+    __half* xq = nullptr; float* sxq = nullptr;   // [M][K] / [M][K/64] scratch of the many-row kernels (calls with more than one row); nullptr: pass kernels
     bool direct = false;                 // a many-row product of plain rows may run without that scratch
     Q4R q;                                                       // repacked weights (tiles of 16 rows)
     int N, K, M;                                                 // N outputs (= 16 * tiles)
@@ -232,8 +232,8 @@ bool ps_plan(PsGeom& g, int n_sm);           // fills the derived fields; false 
 int launch_step_persistent(const PStepArgs& a, cudaStream_t st);   // cooperative launch; returns a cudaError_t
 
 void launch_dense(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl);
-// many-row forms (more than 8 rows per call); the bool launchers return false when the shape is not covered
-inline bool dense_rows_shape(int M, int N, int K) { return M > 8 && K % 256 == 0 && K <= 4096 && N % 16 == 0; }
+// many-row forms (more than one row per call); the bool launchers return false when the shape is not covered
+inline bool dense_rows_shape(int M, int N, int K) { return M > 1 && K % 256 == 0 && K <= 4096 && N % 16 == 0; }
 bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl);
 bool launch_head_rows(const DenseArgs& a, cudaStream_t st, bool pdl);      // lm_head + argmax behind the final norm
 void launch_rows_prep_plain(const __half* x, int ldx, int M, int K, __half* xq, float* sxq, cudaStream_t st, bool pdl);

@@ -371,12 +371,12 @@ static void launch_gemv_rows(const RowsDenseArgs& a, cudaStream_t st, bool pdl) 
     else if (best == 1) launch_gemv_rows_t<EPI, 2, 16>(a, st, pdl);
     else launch_gemv_rows_t<EPI, 1, 24>(a, st, pdl);
 }
-// dense projection of M > 8 rows (a.direct: of any): prologue rows, then the tile kernel.  Returns false when the shape is not covered.
+// dense projection of M > 1 rows (a.direct: of any number): prologue rows, then the tile kernel.  Returns false when the shape is not covered.
 bool launch_dense_rows(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pdl) {
     // plain rows need no prologue kernel; of more than 32 the preparation in every CTA costs more than the launch
     const bool plain = pro == PRO_PLAIN && !a.prepared && (a.direct || a.M <= 32);
     if (!(a.xq && a.sxq) && !(plain && a.direct)) return false;
-    if (!dense_rows_shape(a.direct ? 9 : a.M, a.N, a.K) || (epi != EPI_STORE && epi != EPI_RESID)) return false;
+    if (!dense_rows_shape(a.direct ? 2 : a.M, a.N, a.K) || (epi != EPI_STORE && epi != EPI_RESID)) return false;
     RowsPrepArgs p{a.x, a.ldx, a.nw, a.nw32, a.z, a.ldz, a.eps, a.K, a.xq, a.sxq};
     if (!a.prepared && !plain) launch_rows_prep_args(pro, p, a.M, st, pdl);
     RowsDenseArgs d{a.q, a.N, a.K, a.M, a.xq, a.sxq, a.y, a.ldy, plain ? a.x : nullptr, a.ldx};

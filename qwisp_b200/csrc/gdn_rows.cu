@@ -1,5 +1,5 @@
-// gdn_rows.cu -- the gated delta net for calls whose segments have many rows (prompt chunks, long verify calls) or that
-// have many segments (batched decode), in two kernels:
+// gdn_rows.cu -- the gated delta net of calls with more than one row (prompt chunks, verify rows, batched decode), in two
+// kernels:
 //   k_gdn_prep   everything that does not depend on the state, for all rows side by side: conv + SiLU of every channel, the
 //                q/k norms and scales, decay and beta, the conv history the call leaves.
 //   k_gdn_scan   the recurrence alone, the rows of a segment in sequence.
@@ -22,7 +22,7 @@ __device__ __forceinline__ int gs_paired(int dk) { const int leaf = dk >> 2, e =
 // grid (Hk + Hv, ceil(M / R)), 128 threads: CTAs [0, Hk) own a key head's q and k channels, CTAs [Hk, Hk + Hv) a value
 // head's v channels and gates, for R rows.  R = 8 (one segment): the four conv taps of consecutive rows overlap, so a
 // thread loads 11 values per channel for its 8 rows, all of them before it uses the first: 43 us for 967 rows, 62 with one
-// row per CTA (46k CTAs).  R = 1: rows of several segments.
+// row per CTA (46k CTAs).  R = 2: of fewer rows than fill the device that way.  R = 1: rows of several segments.
 template <int R>
 __global__ void __launch_bounds__(128) k_gdn_prep(GdnArgs a) {
     __shared__ float red_s[R][8];

@@ -382,7 +382,7 @@ void launch_dense(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pd
     // tensor-core GEMM, with the RMSNorm done by a row kernel first.  Every row's result there is
     // independent of how many rows share the call, so a prompt split into chunks in any way gives the
     // same bits; the gated norm of the GDN out-projection runs as a row kernel too.  Every call outside
-    // prefill mode uses the GEMV family, which walks the rows in passes of 8.
+    // prefill mode uses the GEMV family: one row, passes of 8, or the many-row kernels.
     if (a.tc && a.N % 16 == 0 && a.K % 256 == 0 && (epi == EPI_STORE || epi == EPI_RESID) &&
         (pro == PRO_PLAIN || a.norm_scratch)) {
         const __half* x = a.x; int ldx = a.ldx;

@@ -1,7 +1,7 @@
-// rows_kernels.cu -- the many-row forms of the 4-bit group-64 GEMV family: calls with more than 8 activation rows
-// (batched decode, long verify rows, strict-mode prompt chunks).
+// rows_kernels.cu -- the many-row forms of the 4-bit group-64 GEMV family: calls with more than one activation row
+// (batched decode, verify rows, strict-mode prompt chunks).
 //
-// The one-to-eight-row kernels (kernels.cu) walk the rows in passes of 8 and pay one grid wave, one weight fetch and
+// The pass kernels (kernels.cu) walk the rows in passes of 8 and pay one grid wave, one weight fetch and
 // one dequantisation per pass.  Here the weights of a tile are fetched and dequantised ONCE per 8*RG rows and a row's
 // arithmetic is kept exactly as in the pass kernels, so every output is bit-identical to what the same row gives
 // alone (the batch-invariance rule of the reference, swift/Sources/QwispCore/SeedlessMetalForward.swift:160-185):
@@ -11,9 +11,9 @@
 //
 //   k_rows_prep      the prologue (plain / RMSNorm / gated RMSNorm) of every row, written once per call: activations in the
 //                    paired order the dequantiser produces (0,4,1,5,2,6,3,7 inside every 8) + the per-group sums.
-//   k_gemv_rows      dense projection: a CTA of 8 warps = 8 tiles x (8*RG rows); the rows' slice of 256 inputs is staged in
-//                    shared memory (cp.async, two buffers) and shared by the warps; each warp streams its tile's slices
-//                    from global memory two slices ahead.
+//   k_gemv_rows      dense projection: a CTA holds a block of 8, 16 or 32 rows over the whole K, its warps stream tiles of 16
+//                    weight rows through rings of their own (k_gemv_rows_split: short runs, shared out by slices).
+//   k_head_rows      lm_head + argmax in the same form.
 //   k_expert_rows    routed + shared experts grouped by expert: every warp walks tiles of its CTA's run on its own.
 //   k_moe_combine    weighted sum of a row's top-k expert rows in ascending k + shared expert + residual.
 #include "kernels.h"

@@ -445,7 +445,8 @@ __global__ void __launch_bounds__(512, 1) k_head_rows(RowsDenseArgs a, __half* l
                     logits[(size_t)(geo.row0 + row) * a.N + n] = lo;
                     logits[(size_t)(geo.row0 + row) * a.N + n + 8] = hi;
                 }
-                float v = h2f(lo); int i = n;
+                float v = -INFINITY; int i = 0x7fffffff;      // (a NaN is never better: it must not stand for the lane's other logit)
+                if (head_better(h2f(lo), n, v, i)) { v = h2f(lo); i = n; }
                 if (head_better(h2f(hi), n + 8, v, i)) { v = h2f(hi); i = n + 8; }
 #pragma unroll
                 for (int off = 4; off <= 16; off <<= 1) {

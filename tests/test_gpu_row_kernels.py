@@ -135,3 +135,25 @@ def test_state_blob_at_page_edges(engines, n):
     assert np.array_equal(s.step_argmax([7, 11]), t.step_argmax([7, 11]))
     assert np.array_equal(s.state_save(), t.state_save())
     s.close(); t.close()
+
+
+# one vocabulary row gives NaN: it is passed over, and hides no other logit of its 16-row tile (9 rows and more: the many-row head)
+@pytest.mark.parametrize("rows", [8, 9, 16, 17, 33])
+def test_head_passes_over_nan_logits(tiny_oracle, rows):
+    import qwisp_b200 as Q
+    V, H = TINY["vocab"], TINY["hidden"]
+    tensors = {n: tiny_oracle.tensor_bytes(n).copy() for n in tiny_oracle.tensor_names()}
+    cfg = Q.config(**TINY, max_rows=64, max_streams=2, kv_page_size=32, kv_pages=8)
+    toks = prompt(V, rows, "nan")
+    clean = Q.Engine.from_tensors(cfg, tensors)
+    want = clean.stream(64).step_argmax(toks)
+    clean.close()
+    bad = {int(t) // 16 * 16 for t in want} - {int(t) for t in want}
+    assert bad
+    biases = tensors["lm_head.b"].view(np.float16).reshape(V, H // 64).copy()
+    biases[sorted(bad)] = np.nan
+    tensors["lm_head.b"] = biases
+    eng = Q.Engine.from_tensors(cfg, tensors)
+    got = eng.stream(64).step_argmax(toks)
+    eng.close()
+    assert np.array_equal(got, want)

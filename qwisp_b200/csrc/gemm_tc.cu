@@ -141,8 +141,7 @@ __device__ __forceinline__ void tc_group_A(const TcQuad& q, uint4 wv, uint32_t s
 // ================================================================================ the two kinds of work
 // Items are numbered (rows block, 128 weight rows), weight rows fastest; a CTA walks a contiguous run of them, so most
 // steps stay inside a block.  A work type gives the weights of a tile of an item (moved along by a cursor), the place of a
-// block's activation rows (halves from base(), 32 bits: at most 17k rows of 4096), and the epilogue.
-constexpr uint32_t TC_NO_ROW = 0xffffffffu;
+// block's activation rows (halves from base(); Place: wide enough for the rows that the kind of work can have), and the epilogue.
 struct TcTile { const uint4 *w, *s; int blk, rt; };   // fragment-major nibbles and scales of a tile (nullptr: none) of weight-row group rt
 
 struct GemmTcArgs {
@@ -157,6 +156,8 @@ template <int NT>
 struct DenseWork {
     using Args = GemmTcArgs;
     static constexpr bool STRIDED = true;                                   // rows of a block lie stride() halves apart
+    using Place = size_t;                                                   // (a product of the caller's own size: any M)
+    static constexpr Place NO_ROW = ~(Place)0;
     struct Shared {};
     const Args& a;
     int NRT;                                                                // weight-row groups
@@ -172,7 +173,7 @@ struct DenseWork {
     }
     __device__ const __half* base() const { return a.x; }
     __device__ uint32_t stride() const { return (uint32_t)a.ldx; }
-    __device__ uint32_t row(int blk, int n) const { return blk * NT + n < a.M ? (uint32_t)(blk * NT + n) * (uint32_t)a.ldx : TC_NO_ROW; }
+    __device__ Place row(int blk, int n) const { return blk * NT + n < a.M ? (Place)(blk * NT + n) * (Place)a.ldx : NO_ROW; }
     struct Epi {};
     // quarter: accumulator lanes 32 * quarter ..; taddr: the item's columns in TMEM; release() once they have been read
     template <class Release>
@@ -207,6 +208,8 @@ template <bool DOWN, int NT>
 struct ExpertWork {
     using Args = ExpertArgs;
     static constexpr bool STRIDED = false;
+    using Place = uint32_t;                                                 // (an engine has at most 1024 rows: 17k pair rows of 4096)
+    static constexpr Place NO_ROW = ~(Place)0;
     struct Shared { SlotTable tab; int dst[2][NT]; };
     const Args& a;
     Shared& sh;
@@ -241,10 +244,10 @@ struct ExpertWork {
     }
     __device__ const __half* base() const { return DOWN ? a.hbuf : a.p; }
     __device__ uint32_t stride() const { return 0; }
-    __device__ uint32_t row(int blk, int n) const {
+    __device__ Place row(int blk, int n) const {
         const int p = pair_of(blk, n);
-        if (p < 0) return TC_NO_ROW;
-        return (uint32_t)(DOWN ? p : (p >= npair ? a.shared_row0 + p - npair : p / a.topk)) * (uint32_t)K;
+        if (p < 0) return NO_ROW;
+        return (Place)(DOWN ? p : (p >= npair ? a.shared_row0 + p - npair : p / a.topk)) * (Place)K;
     }
     struct Epi { int blk = -1, buf = 0, count = 0; };                       // the block whose rows are listed in sh.dst[buf]
     template <class Release>
@@ -408,7 +411,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         const int n0 = ((lt >> 6) << 3) + (lt & 7), chunk = (lt >> 3) & 7;  // rows n0 + 16 h, the same chunk of both groups
         const uint32_t off0 = smem_u32(smem) + tc_off(n0, chunk);
         const __half* base = work.base() + chunk * 8;
-        uint32_t src[W::STRIDED ? 1 : NP];                                  // row places (strided: of the first row)
+        typename W::Place src[W::STRIDED ? 1 : NP];                         // row places (strided: of the first row)
         int st = 0; uint32_t ph = 1;
         int blk = blk0, rt = rt0, held = -1, have = 0;                      // held: the block whose row places are in src; have: its rows (strided)
         for (int k = 0; k < hi - lo && ok; ++k) {
@@ -416,7 +419,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
                 held = blk;
                 if (W::STRIDED) {
                     src[0] = work.row(blk, n0); have = 0;
-                    for (int h = 0; h < NP; ++h) have += work.row(blk, n0 + 16 * h) != TC_NO_ROW;
+                    for (int h = 0; h < NP; ++h) have += work.row(blk, n0 + 16 * h) != W::NO_ROW;
                 } else {
 #pragma unroll
                     for (int h = 0; h < NP; ++h) src[W::STRIDED ? 0 : h] = work.row(blk, n0 + 16 * h);
@@ -439,8 +442,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
                 } else {
 #pragma unroll
                     for (int h = 0; h < NP; ++h) {
-                        const uint32_t o = src[W::STRIDED ? 0 : h];
-                        if (o != TC_NO_ROW) copy(h, base + o + s * 128);
+                        const typename W::Place o = src[W::STRIDED ? 0 : h];
+                        if (o != W::NO_ROW) copy(h, base + o + s * 128);
                     }
                 }
                 // the barrier counts this thread in when its copies have landed: nobody waits for them here

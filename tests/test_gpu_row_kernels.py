@@ -157,3 +157,28 @@ def test_head_passes_over_nan_logits(tiny_oracle, rows):
     got = eng.stream(64).step_argmax(toks)
     eng.close()
     assert np.array_equal(got, want)
+
+
+# rows whose places pass 2^32 halves (8.6 GB of activations): each row gives what it gives alone
+def test_tensor_core_product_of_very_many_rows():
+    import torch
+    import qwisp_b200 as Q
+    from oracle import oracle as O
+    L = Q.lib()
+    K, N, M = 4096, 16, (1 << 20) + 200
+    packed, scales, biases = O.synth_q4(3, "tall.w", N, K)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a).view(np.uint8).reshape(-1)).cuda()
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    dw, ds, db = dev(packed), dev(scales), dev(biases)
+    wr = torch.empty((N // 16) * (K // 128) * 1024, dtype=torch.uint8, device="cuda")
+    sr = torch.empty((N // 16) * (K // 128) * 128, dtype=torch.uint8, device="cuda")
+    assert L.sl_op_repack_q4_device(ptr(dw), ptr(ds), ptr(db), K, N, ptr(wr), ptr(sr), None) == 0
+    x = torch.zeros((M, K), dtype=torch.float16, device="cuda")
+    few = 300                                         # the rows on both sides of the boundary
+    x[M - few:] = torch.randn((few, K), generator=torch.Generator(device="cuda").manual_seed(5), device="cuda").half()
+    y = torch.empty((M, N), dtype=torch.float16, device="cuda")
+    want = torch.empty((few, N), dtype=torch.float16, device="cuda")
+    assert L.sl_op_qmm4_tc_device(ptr(x), ptr(wr), ptr(sr), M, K, N, ptr(y), None) == 0
+    assert L.sl_op_qmm4_tc_device(ptr(x[M - few:]), ptr(wr), ptr(sr), few, K, N, ptr(want), None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(y[M - few:].view(torch.int16), want.view(torch.int16)) and not y[:M - few].any()

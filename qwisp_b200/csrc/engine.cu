@@ -110,7 +110,7 @@ struct sl_engine {
     PStepArgs ps{};
     uint32_t* ps_timeline = nullptr;
     StateIoRing sio;                // slots of state save / restore
-    bool poisoned = false, inject = false;
+    bool poisoned = false, inject = false, stall = false;
     std::string fault;
 };
 
@@ -600,6 +600,7 @@ void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half
     ExpertArgs ea{}; ea.gu = L.r_gu; ea.down = L.r_down; ea.sh_gu = L.r_sh_gu; ea.sh_down = L.r_sh_down;
     ea.lists = e->lists; ea.p = e->p; ea.hbuf = e->hbuf; ea.dbuf = e->dbuf; ea.M = M; ea.H = e->H; ea.I = e->I; ea.topk = e->topk;
     ea.scores = e->scores; ea.sgl = e->sgl; ea.resid = resid; ea.out = plain_out; ea.tile_counter = e->tile_counters; ea.err = e->err_flag;
+    ea.stall = e->stall;
     if (e->use_prefetch) { if (next) pf_q4(ea.pf, 0, next->r_in); else pf_q4(ea.pf, 0, e->r_lm_head, (size_t)24 << 20); }
     int nslots = M * e->topk < e->E ? M * e->topk : e->E;
     ea.slot_sync = e->slot_sync;
@@ -1064,6 +1065,11 @@ const char* sl_last_fault(sl_engine* e) {
 int32_t sl_debug_wait_timeout(sl_engine* e) {
     int32_t rc = guard(e); if (rc) return rc;
     launch_wait_probe(e->err_flag, e->stream);
+    return SL_OK;
+}
+int32_t sl_debug_expert_timeout(sl_engine* e) {
+    int32_t rc = guard(e); if (rc) return rc;
+    e->stall = true;
     return SL_OK;
 }
 int32_t sl_inject_fault(sl_engine* e, int32_t on) { if (!e) return SL_ERR_INVALID; e->inject = on != 0; return SL_OK; }

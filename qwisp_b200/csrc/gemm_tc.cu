@@ -82,17 +82,21 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_arrive(uint64_t* b) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory"); }
 
-// Bounded wait of a role.  The first that runs out (seconds) raises the CTA's abort word; every later wait of the CTA then
-// gives up at once, so the roles leave their loops one after another.
+// Bounded wait of a role.  The first that runs out (a poll takes up to 4 us, so some 17 s) raises the CTA's abort word; every
+// later wait of the CTA then gives up after 256 polls.  The outcome is a lane's own, but what follows a wait needs whole warps:
+// a role goes on to the end of its item whatever its waits said (its results are discarded then) and leaves by tc_agree().
+// Warps need not agree: none waits for another but here and at the end of the kernel.
+template <int LIMIT>
 __device__ __forceinline__ bool tc_wait(uint64_t* b, uint32_t parity, volatile int* abort_word) {
     if (mbar_try_wait(b, parity)) return true;
-    for (int i = 0; i < (1 << 22); ++i) {
+    for (int i = 0; i < LIMIT; ++i) {
         if (mbar_try_wait(b, parity)) return true;
         if ((i & 255) == 255 && *abort_word) return false;
     }
     *abort_word = 1;
     return false;
 }
+__device__ __forceinline__ bool tc_agree(bool ok) { return __all_sync(0xffffffffu, ok); }
 
 // ---- one K group (64 inputs) of a 16-row tile: fragment register -> A operand
 // Lane 4r + t holds inputs 16t .. 16t + 15 of rows A_r and B_r = r + 8 (two words each); the MMA wants inputs 16c .. 16c + 15
@@ -175,6 +179,7 @@ struct DenseWork {
     __device__ uint32_t stride() const { return (uint32_t)a.ldx; }
     __device__ Place row(int blk, int n) const { return blk * NT + n < a.M ? (Place)(blk * NT + n) * (Place)a.ldx : NO_ROW; }
     struct Epi {};
+    __device__ void begin(Epi&, int, int, int) const {}
     // quarter: accumulator lanes 32 * quarter ..; taddr: the item's columns in TMEM; release() once they have been read
     template <class Release>
     __device__ void epilogue(Epi&, int blk, int rt, int quarter, int lane, uint32_t taddr, Release release) const {
@@ -210,7 +215,7 @@ struct ExpertWork {
     static constexpr bool STRIDED = false;
     using Place = uint32_t;                                                 // (an engine has at most 1024 rows: 17k pair rows of 4096)
     static constexpr Place NO_ROW = ~(Place)0;
-    struct Shared { SlotTable tab; int dst[2][NT]; };
+    struct Shared { SlotTable tab; int dst[TC_EPI][NT]; };                  // dst: a list of each epilogue warp
     const Args& a;
     Shared& sh;
     int n_active, K, ntiles, NRT, npair, nshared;
@@ -249,18 +254,23 @@ struct ExpertWork {
         if (p < 0) return NO_ROW;
         return (Place)(DOWN ? p : (p >= npair ? a.shared_row0 + p - npair : p / a.topk)) * (Place)K;
     }
-    struct Epi { int blk = -1, buf = 0, count = 0; };                       // the block whose rows are listed in sh.dst[buf]
+    struct Epi { int blk = -1, count = 0; };                                // the block whose rows are listed in sh.dst
+    // The rows of a block, listed before its accumulators are waited for.  Each warp makes the list for itself, so that the four
+    // have nothing to meet for (behind the wait it cost a prompt 1.2 %).
+    __device__ void begin(Epi& e, int blk, int quarter, int lane) const {
+        if (blk == e.blk) return;
+        e.blk = blk;
+        __syncwarp();
+#pragma unroll
+        for (int n = 0; n < NT; n += 32) sh.dst[quarter][n + lane] = pair_of(blk, n + lane);
+        const int j = slot_of(sh.tab, n_active, blk);
+        e.count = min(NT, (j == n_active ? nshared : sh.tab.cnt[j]) - (blk - sh.tab.base[j]) * NT);
+        __syncwarp();
+    }
     template <class Release>
-    __device__ void epilogue(Epi& e, int blk, int rt, int quarter, int lane, uint32_t taddr, Release release) const {
+    __device__ void epilogue(Epi& e, int, int rt, int quarter, int lane, uint32_t taddr, Release release) const {
         const int i = quarter * 32 + lane;
-        if (blk != e.blk) {
-            e.blk = blk; e.buf ^= 1;
-            for (int n = i; n < NT; n += TC_EPI * 32) sh.dst[e.buf][n] = pair_of(blk, n);
-            const int j = slot_of(sh.tab, n_active, blk);
-            e.count = min(NT, (j == n_active ? nshared : sh.tab.cnt[j]) - (blk - sh.tab.base[j]) * NT);
-            asm volatile("bar.sync 1, 128;" ::: "memory");                  // the epilogue warps: the list is there
-        }
-        const int* dsts = sh.dst[e.buf];
+        const int* dsts = sh.dst[quarter];
         const int i16 = i & 15, etile = rt * 8 + (i >> 4);
         const bool up = i16 >= 8, have = etile < ntiles;
         __half* out = DOWN ? a.dbuf + (size_t)rt * TC_ROWS + i : a.hbuf + etile * 8 + (i16 & 7);
@@ -293,11 +303,12 @@ struct ExpertWork {
 // ================================================================================ the kernel
 // ST: stages (even); U: stages' fragments a dequant warp has in flight (K / 256 is a multiple of it)
 // TMEM columns: [2][NT] accumulators, [ST][64] A operands
-template <class W, int NT, int ST, int U>
+// STALL: a test's form, in which no row is ever loaded, so that every wait runs out, and soon
+template <class W, int NT, int ST, int U, bool STALL>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];             // ST stages x [2 groups][NT rows x 128 B]
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // tiles start on 1024-byte boundaries
-    constexpr int TILE = NT * 128, STAGE = 2 * TILE;
+    constexpr int TILE = NT * 128, STAGE = 2 * TILE, LIMIT = STALL ? 1 << 10 : 1 << 22;
     static_assert(2 * NT + ST * 64 <= 512 && ST % 2 == 0, "tensor memory");
     __shared__ __align__(8) uint64_t s_full[ST], s_empty[ST], s_acc_full[2], s_acc_empty[2];
     __shared__ uint32_t s_tmem;
@@ -332,12 +343,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         const uint32_t ta0 = tmem + 2 * NT;
         int st = 0; uint32_t ph = 0;
         for (int k = 0; k < hi - lo && ok; ++k) {
-            if (k >= 2) ok = tc_wait(&s_acc_empty[k & 1], (uint32_t)(((k >> 1) - 1) & 1), &s_abort);
+            if (k >= 2) ok = tc_wait<LIMIT>(&s_acc_empty[k & 1], (uint32_t)(((k >> 1) - 1) & 1), &s_abort) && ok;
             tc_fence_after();
             const uint32_t acc = tmem + (uint32_t)((k & 1) * NT);
 #pragma unroll 1
             for (int s = 0; s < KS; ++s) {
-                if (!tc_wait(&s_full[st], ph, &s_abort)) { ok = false; break; }
+                ok = tc_wait<LIMIT>(&s_full[st], ph, &s_abort) && ok;
                 tc_fence_after();
                 tc_fence_proxy();                                           // the rows other threads' asynchronous copies wrote are operand data now
                 const uint64_t db = db0 + (uint32_t)(st * (STAGE >> 4));    // (the address field counts 16 bytes: a K step of 16 halves is 2)
@@ -352,6 +363,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
                 __syncwarp();
                 if (++st == ST) { st = 0; ph ^= 1u; }
             }
+            ok = tc_agree(ok);
         }
     } else if (warp >= TC_DQ0 && warp < TC_DQ0 + TC_DQ) {
         // ------------------------------------------------------------ dequant: tile tl of every item, stages par, par + 2, ...
@@ -383,10 +395,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
             const bool valid = work.has_tile(rt, tl);
             if (++rt == NRT) rt = 0;
 #pragma unroll 1
-            for (int s = 0; s < KS >> 1 && ok; s += U) {
+            for (int s = 0; s < KS >> 1; s += U) {
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    ok = tc_wait(&s_empty[st], ph, &s_abort) && ok;
+                    ok = tc_wait<LIMIT>(&s_empty[st], ph, &s_abort) && ok;
                     if (valid) {                                            // (of a tile the matrix does not have the outputs are not stored)
                         tc_fence_after();
                         tc_group_A(quad, w0[u], sv[u].x, sv[u].y, ta + st * 64);
@@ -400,6 +412,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
                     st += 2; if (st >= ST) { st -= ST; ph ^= 1u; }
                 }
             }
+            ok = tc_agree(ok);
         }
     } else if (warp < TC_EPI0 || warp >= TC_DQ0) {
         // ------------------------------------------------------------ load: the activation rows of every stage
@@ -414,7 +427,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         typename W::Place src[W::STRIDED ? 1 : NP];                         // row places (strided: of the first row)
         int st = 0; uint32_t ph = 1;
         int blk = blk0, rt = rt0, held = -1, have = 0;                      // held: the block whose row places are in src; have: its rows (strided)
-        for (int k = 0; k < hi - lo && ok; ++k) {
+        for (int k = 0; k < hi - lo && ok && !STALL; ++k) {
             if (blk != held) {
                 held = blk;
                 if (W::STRIDED) {
@@ -427,8 +440,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
             }
             if (++rt == NRT) { rt = 0; ++blk; }
 #pragma unroll 1
-            for (int s = 0; s < KS && ok; ++s) {
-                ok = tc_wait(&s_empty[st], ph, &s_abort) && ok;
+            for (int s = 0; s < KS; ++s) {
+                ok = tc_wait<LIMIT>(&s_empty[st], ph, &s_abort) && ok;
                 const uint32_t B = off0 + (uint32_t)st * STAGE;
                 auto copy = [&](int h, const __half* p) {
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(B + 2048u * h), "l"(p) : "memory");
@@ -450,6 +463,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
                 asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&s_full[st])) : "memory");
                 if (++st == ST) { st = 0; ph ^= 1u; }
             }
+            ok = tc_agree(ok);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
@@ -459,7 +473,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         const int quarter = warp - TC_EPI0;
         int blk = blk0, rt = rt0;
         for (int k = 0; k < hi - lo && ok; ++k) {
-            ok = tc_wait(&s_acc_full[k & 1], (uint32_t)((k >> 1) & 1), &s_abort);
+            work.begin(epi, blk, quarter, lane);
+            ok = tc_agree(tc_wait<LIMIT>(&s_acc_full[k & 1], (uint32_t)((k >> 1) & 1), &s_abort));
             tc_fence_after();
             if (ok) work.epilogue(epi, blk, rt, quarter, lane, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((k & 1) * NT), [&] {
                 tc_fence_before();
@@ -478,16 +493,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512u) : "memory");
 }
-template <class W, int NT, int ST, int U>
+template <class W, int NT, int ST, int U, bool STALL = false>
 static int launch_tc_t(const typename W::Args& a, int grid, cudaStream_t st, bool pdl) {
     constexpr size_t smem = (size_t)ST * NT * 256 + 1024;
     static bool configured = false;
     if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(k_tc<W, NT, ST, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t err = cudaFuncSetAttribute(k_tc<W, NT, ST, U, STALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (err != cudaSuccess) return (int)err;
         configured = true;
     }
-    return launch_pdl(pdl, k_tc<W, NT, ST, U>, dim3((unsigned)grid), TC_THREADS, smem, st, a);
+    return launch_pdl(pdl, k_tc<W, NT, ST, U, STALL>, dim3((unsigned)grid), TC_THREADS, smem, st, a);
 }
 template <int NT, int ST>
 static int launch_gemm_tc_t(const GemmTcArgs& a, cudaStream_t st, bool pdl) {
@@ -520,6 +535,8 @@ static bool launch_expert_tc_t(const ExpertArgs& a, cudaStream_t st, bool pdl) {
     if (K % 256 || a.ep_pairs_per_rank > 0) return false;              // (expert-parallel calls keep the row kernels)
     int rc = 0;
     profile_launch(DOWN ? "k_expert_umma_down" : "k_expert_umma_gateup", st, [&] {
+        if constexpr (!DOWN)
+            if (a.stall) return rc = launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, 1, true>(a, sm_count(), st, pdl);
         rc = K % 512 == 0 ? launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, 2>(a, sm_count(), st, pdl) : launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, 1>(a, sm_count(), st, pdl);
         return rc;
     });

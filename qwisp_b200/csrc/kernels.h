@@ -103,7 +103,7 @@ struct ExpertArgs {
     // many-row kernels: the normed rows in paired order + their group sums (gate/up input), and the chunk sums of the
     // SwiGLU rows ([(M*topk + M)][I/8], written by gate/up, read by down; hbuf is then in paired order too)
     const __half* xq = nullptr; const float* sxq = nullptr; float* csum = nullptr;
-    bool stall = false;                  // test hook: the prefill-mode gate/up kernel in the form whose waits run out
+    bool stall = false;                  // test hook: the gate/up kernel in the form whose waits run out
 };
 
 struct GdnArgs {

@@ -85,15 +85,20 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
 }
 // Wait of the expert kernel's ring, bounded in TIME (~50 ms): the first wait of a CTA that runs out raises the CTA's
 // abort word, and every later wait of that CTA gives up at once, so a stall costs one timeout per CTA, not one per block.
+// For whole warps: the lanes agree on the outcome, because what follows needs all of them.
 constexpr long long XR_TIMEOUT = 100000000ll;                 // cycles
-__device__ __forceinline__ bool xr_wait(uint64_t* bar, uint32_t parity, volatile int* abort_word) {
+__device__ __forceinline__ bool xr_wait_lane(uint64_t* bar, uint32_t parity, volatile int* abort_word, long long timeout) {
     if (mbar_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
     for (;;) {
         for (int i = 0; i < 64; ++i) if (mbar_try_wait(bar, parity)) return true;
         if (*abort_word) return false;
-        if (clock64() - t0 > XR_TIMEOUT) { *abort_word = 1; return false; }
+        if (clock64() - t0 > timeout) { *abort_word = 1; return false; }
     }
+}
+template <bool STALL>
+__device__ __forceinline__ bool xr_wait(uint64_t* bar, uint32_t parity, volatile int* abort_word) {
+    return __all_sync(0xffffffffu, xr_wait_lane(bar, parity, abort_word, STALL ? XR_TIMEOUT / 32 : XR_TIMEOUT));
 }
 
 constexpr int XR_DEPTH = 2;                   // slices in a warp's ring
@@ -546,8 +551,8 @@ __device__ __forceinline__ XrStage xr_carve(unsigned char* base, int K) {
     s.craw = reinterpret_cast<float*>(base);
     return s;
 }
-// S: slices of K
-template <bool DOWN, int S>
+// S: slices of K.  STALL: a test's form, in which no row is ever fetched, so that every consumer's wait runs out, and soon
+template <bool DOWN, int S, bool STALL>
 __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int lg_tiles, int nstages) {
     extern __shared__ __align__(16) unsigned char smem[];        // weight rings, then nstages stages
     __shared__ __align__(8) uint64_t s_full[8], s_empty[8], s_raw[8];
@@ -588,10 +593,10 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
     if (warp == XR_WARPS) {
         // ------------------------------------------------------------ producer: the rows of the run's blocks, stage after stage
         if (DOWN) pdl_wait();                                  // the gate/up kernel's rows
-        for (int k = 0; k < nb; ++k) {
+        for (int k = 0; k < nb && !STALL; ++k) {
             const int stg = k % nstages, use = k / nstages;
             const XrStage St = xr_carve(stages + (size_t)stg * stage_bytes, K);
-            if (use > 0 && !xr_wait(&s_empty[stg], (uint32_t)((use - 1) & 1), &s_abort)) { fail_code |= 16u; break; }
+            if (use > 0 && !xr_wait<STALL>(&s_empty[stg], (uint32_t)((use - 1) & 1), &s_abort)) { fail_code |= 16u; break; }
             if (lane < 8) {
                 uint64_t* bar = DOWN ? &s_raw[stg] : &s_full[stg];
                 const int src = s_blk[k].src[lane];
@@ -606,7 +611,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
             }
             if (DOWN) {
                 // group sums from the chunk sums: eight of them combined in the butterfly order of rows_store()
-                if (!xr_wait(&s_raw[stg], (uint32_t)(use & 1), &s_abort)) { fail_code |= 32u; break; }
+                if (!xr_wait<STALL>(&s_raw[stg], (uint32_t)(use & 1), &s_abort)) { fail_code |= 32u; break; }
                 for (int i = lane; i < 8 * G64; i += 32) {
                     const int row = i / G64, g = i - row * G64;
                     const float* c = St.craw + (size_t)row * (K / 8) + g * 8;
@@ -653,7 +658,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
             if (lane == 0) for (int u = cur; u < bi; ++u) mbar_arrive(&s_empty[u % nstages]);
             cur = bi; here = false;
         }
-        if (!here && !xr_wait(&s_full[bi % nstages], (uint32_t)((bi / nstages) & 1), &s_abort)) { fail_code |= 64u; break; }
+        if (!here && !xr_wait<STALL>(&s_full[bi % nstages], (uint32_t)((bi / nstages) & 1), &s_abort)) { fail_code |= 64u; break; }
         here = true;
         const XrStage St = xr_carve(stages + (size_t)(bi % nstages) * stage_bytes, K);
         const __half* xp = St.xs + (size_t)r * XS + 16 * t;
@@ -738,7 +743,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
             st_release_sys(a.ep_sig.flags[tid] + 8 + a.ep_sig.rank, ep_seq(a.ep_sig.ctr, a.ep_sig.layer, 1));
     }
 }
-template <bool DOWN, int S>
+template <bool DOWN, int S, bool STALL = false>
 static bool launch_expert_rows_t(const ExpertArgs& a, cudaStream_t st, bool pdl) {
     const int ntiles = DOWN ? a.H / 16 : a.I / 8, grid = sm_count();
     int lg = 0; while ((1 << lg) < ntiles) ++lg;
@@ -749,8 +754,8 @@ static bool launch_expert_rows_t(const ExpertArgs& a, cudaStream_t st, bool pdl)
     if ((1 << lg) != ntiles || blocks / grid + 2 > XR_BLOCKS || nstages < 1) return false;
     const size_t smem = ring + sb * nstages;
     static bool configured = false;
-    if (!configured) { cudaFuncSetAttribute(k_expert_rows<DOWN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
-    profile_launch(DOWN ? "k_expert_rows_down" : "k_expert_rows_gateup", st, [&] { return launch_pdl(pdl, k_expert_rows<DOWN, S>, dim3((unsigned)grid), XR_THREADS, smem, st, a, lg, nstages); });
+    if (!configured) { cudaFuncSetAttribute(k_expert_rows<DOWN, S, STALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
+    profile_launch(DOWN ? "k_expert_rows_down" : "k_expert_rows_gateup", st, [&] { return launch_pdl(pdl, k_expert_rows<DOWN, S, STALL>, dim3((unsigned)grid), XR_THREADS, smem, st, a, lg, nstages); });
     return true;
 }
 template <bool DOWN>
@@ -758,7 +763,7 @@ static bool launch_expert_rows_d(const ExpertArgs& a, cudaStream_t st, bool pdl)
     if (!a.csum || (!DOWN && (!a.xq || !a.sxq))) return false;
     switch (DOWN ? a.I : a.H) {
         case 256: return launch_expert_rows_t<DOWN, 1>(a, st, pdl);
-        case 512: return launch_expert_rows_t<DOWN, 2>(a, st, pdl);
+        case 512: return !DOWN && a.stall ? launch_expert_rows_t<DOWN, 2, !DOWN>(a, st, pdl) : launch_expert_rows_t<DOWN, 2>(a, st, pdl);
         case 1024: return launch_expert_rows_t<DOWN, 4>(a, st, pdl);
         case 2048: return launch_expert_rows_t<DOWN, 8>(a, st, pdl);
         case 4096: return launch_expert_rows_t<DOWN, 16>(a, st, pdl);

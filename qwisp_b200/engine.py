@@ -106,7 +106,7 @@ class Engine:
         self._check(lib().sl_debug_wait_timeout(self._h), "sl_debug_wait_timeout")
 
     def debug_expert_timeout(self):
-        """Test hook: the waits of the next prefill-mode call's expert kernel run out (nothing faults); that call fails."""
+        """Test hook: the waits of the next call's expert kernels run out (nothing faults); that call fails."""
         self._check(lib().sl_debug_expert_timeout(self._h), "sl_debug_expert_timeout")
 
     def set_cuda_stream(self, cuda_stream_handle):

@@ -338,20 +338,21 @@ def test_device_wait_timeout_poisons_engine():
         e.close()
 
 
-def test_prefill_wait_timeout_poisons_engine():
-    """The same for the kernel whose warps wait for one another (prefill-mode experts): rows that never arrive make every role
-    give up its own bounded wait and leave, none waits for one that has left, and the call reports it."""
+@pytest.mark.parametrize("call", ["forward_hybrid", "forward"])
+def test_expert_wait_timeout_poisons_engine(call):
+    """The same for the kernels whose warps wait for one another (experts in prefill mode and of many rows): rows that never arrive
+    make every warp give up its own bounded wait and leave, none waits for one that has left, and the call reports it."""
     import time
     import qwisp_b200 as Q
     e = gpu_engine(TINY, max_streams=2)
     try:
         s = e.stream(80)
         toks = prompt(TINY["vocab"], 40, "stall")
-        assert s.forward_hybrid(toks).shape == (40, TINY["hidden"]) and e.gpu_fault() is None
+        assert getattr(s, call)(toks).shape == (40, TINY["hidden"]) and e.gpu_fault() is None
         e.debug_expert_timeout()
         t0 = time.perf_counter()
         with pytest.raises(Q.SeedlessError) as ei:
-            s.forward_hybrid(toks)
+            getattr(s, call)(toks[1:])
         assert ei.value.code == -3 and time.perf_counter() - t0 < 5.0
         assert "bounded wait" in e.gpu_fault()
     finally:

@@ -204,7 +204,9 @@ int32_t sl_full_restore(sl_stream* s, const sl_fullsnap* snap);
 int32_t sl_fullsnap_free(sl_fullsnap* snap);
 /* persistentStateData / restorePersistentState (SeedlessFusedVerify.swift:4077-4154): the
  * self-describing "QWS1" blob; restorable into a stream of a different max_seq_len.
- * sl_state_restore returns SL_ERR_FORMAT on any mismatch; the stream must then be reset. */
+ * sl_state_restore returns SL_ERR_FORMAT on any mismatch; the stream must then be reset.  The first save or restore
+ * of an engine allocates 32 MB of page-locked and 32 MB of device memory; without room for them it returns SL_ERR_CAPACITY, with
+ * stream and engine as they were. */
 int32_t sl_state_size(sl_stream* s, uint64_t* nbytes);
 int32_t sl_state_save(sl_stream* s, void* buf, uint64_t nbytes);
 int32_t sl_state_restore(sl_stream* s, const void* buf, uint64_t nbytes);

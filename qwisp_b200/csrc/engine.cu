@@ -1407,12 +1407,19 @@ static StateIoArgs state_io_args(sl_stream* s, int len) {
     a.state = cur_state(s); a.hist = cur_hist(s); a.kv_pool = e->kv_pool; a.pages = e->tab.page_table + (size_t)s->slot * e->tab.max_pages;
     return a;
 }
+// No room for the slots: the call is refused and nothing has changed.  Any other failure is the device's.
+static int32_t state_io_ready(sl_engine* e, const char* what) {
+    const cudaError_t err = (cudaError_t)e->sio.init();
+    if (err == cudaSuccess) return SL_OK;
+    return err == cudaErrorMemoryAllocation ? SL_ERR_CAPACITY : poison(e, what, err);
+}
 int32_t sl_state_save(sl_stream* s, void* buf, uint64_t nbytes) {
     if (!s || !buf) return SL_ERR_INVALID;
     sl_engine* e = s->e;
     int32_t rc = guard(e); if (rc) return rc;
     uint64_t need; sl_state_size(s, &need);
     if (nbytes < need) return SL_ERR_CAPACITY;
+    if ((rc = state_io_ready(e, "sl_state_save"))) return rc;
     const int err = state_io(e->sio, state_io_args(s, s->kv_len), true, (uint8_t*)buf, need, e->stream);
     if (err) return poison(e, "sl_state_save", (cudaError_t)err);
     return sync_check(e);
@@ -1445,6 +1452,7 @@ int32_t sl_state_restore(sl_stream* s, const void* buf, uint64_t nbytes) {
     }
     if (off != nbytes) return SL_ERR_FORMAT;
     if (len < 0) len = 0;
+    if ((rc = state_io_ready(e, "sl_state_restore"))) return rc;
     if ((rc = ensure_pages(s, len))) return rc;
     // pass 2: copy
     const int err = state_io(e->sio, state_io_args(s, len), false, const_cast<uint8_t*>(b), nbytes, e->stream);

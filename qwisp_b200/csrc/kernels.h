@@ -310,13 +310,13 @@ struct StateIoArgs {
     float* state; __half* hist;             // current side of the stream, GDN layers in order
     __half* kv_pool; const int* pages;      // the stream's page table row (device)
 };
-struct StateIoRing {                        // page-locked slots and their device counterparts, made at the first use
+struct StateIoRing {                        // page-locked slots and their device counterparts (32 MB each), made at the first use
     uint8_t *pinned = nullptr, *dev = nullptr;
     cudaEvent_t done[16] = {};
-    int init();
+    int init();                             // 0 or a cudaError_t; after a failure nothing is held, and it may be tried again
     void destroy();
 };
-// copies the whole blob out of (save) or into the stream's caches; when it returns, a save is complete in `host` and a
+// (the ring initialised) copies the whole blob out of (save) or into the stream's caches; when it returns, a save is complete in `host` and a
 // restore has read all of `host` (its device work may still be in flight on st).  0 or a cudaError_t.
 int state_io(StateIoRing& ring, const StateIoArgs& a, bool save, uint8_t* host, size_t bytes, cudaStream_t st);
 void launch_set_pages(int* dst, const int* pages, int n, cudaStream_t st);     // dst[i] = pages[i]; pages (host) is read before the call returns

@@ -67,7 +67,7 @@ int StateIoRing::init() {
     cudaError_t e = cudaMallocHost(&pinned, bytes);
     if (e == cudaSuccess) e = cudaMalloc(&dev, bytes);
     for (int i = 0; i < 2 * SIO_THREADS && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming);
-    if (e != cudaSuccess) destroy();
+    if (e != cudaSuccess) { destroy(); cudaGetLastError(); }
     return (int)e;
 }
 void StateIoRing::destroy() {
@@ -109,9 +109,8 @@ static cudaError_t sio_worker(StateIoRing& ring, const StateIoArgs& a, bool save
     return e;
 }
 int state_io(StateIoRing& ring, const StateIoArgs& a, bool save, uint8_t* host, size_t bytes, cudaStream_t st) {
-    cudaError_t e = (cudaError_t)ring.init();
     int device = 0;
-    if (e == cudaSuccess) e = cudaGetDevice(&device);
+    cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return (int)e;
     // a thread per four ranges (8 MB): starting one costs about what copying a megabyte does
     int T = (int)(bytes / (4 * SIO_SLOT));

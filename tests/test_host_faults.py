@@ -1,0 +1,88 @@
+"""Host-side failures and host-side rules of the library, without a GPU: each test runs a child process in which a stand-in for the
+CUDA runtime (fake_cudart.cpp) is preloaded.  It gives memory, runs no kernels, and fails the calls it is told to fail."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT, TINY
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+PRELUDE = f"""
+import ctypes as C, sys
+sys.path.insert(0, {ROOT!r})
+import numpy as np
+import qwisp_b200 as Q
+F = C.CDLL(None)
+F.fake_count.restype = C.c_long
+F.fake_unpacked.restype = C.c_long
+F.fake_fail_alloc.argtypes = [C.c_size_t]
+F.fake_fail_threads.argtypes = F.fake_fail_launches.argtypes = [C.c_long]
+count = lambda what: F.fake_count(what.encode())
+GEOM = {TINY!r}
+
+def engine(**kw):
+    args = dict(max_rows=128, max_streams=80, kv_page_size=32, kv_pages=1024)
+    args.update(kw)
+    return Q.Engine.synthetic(Q.config(**GEOM, **args), seed=1)
+
+def refused(code, fn, *a):
+    try:
+        fn(*a)
+    except Q.SeedlessError as e:
+        assert e.code == code, e
+    else:
+        raise AssertionError("the call went through")
+
+def filled(eng, n):
+    s = eng.stream(n + 8)
+    for i in range(0, n, 128):
+        s.forward(list(range(min(128, n - i))), want_hidden=False)
+    assert s.length == n
+    return s
+
+def blob_of(n):          # a valid blob of n positions, its data words numbered
+    gdn = [np.array([2, 3 * 4096, 16 * 128 * 128], dtype=np.uint32), np.zeros(3 * 4096 // 2 + 16 * 128 * 128, dtype=np.uint32)]
+    att = [np.array([1, 1, 256, n], dtype=np.uint32), np.zeros(2 * n * 128, dtype=np.uint32)]
+    w = np.concatenate([np.array([0x31535751, 1, 4], dtype=np.uint32)] + gdn + att + gdn + att)
+    zero = w == 0
+    w[zero] = np.arange(w.size, dtype=np.uint32)[zero]
+    return w
+"""
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "fake_cudart.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I/usr/local/cuda/include", os.path.join(HERE, "fake_cudart.cpp"),
+                    "-o", so, "-ldl", "-lpthread"], check=True, timeout=120)
+
+    def run(script):
+        out = subprocess.run([sys.executable, "-c", PRELUDE + script], env=dict(os.environ, LD_PRELOAD=so), capture_output=True, text=True, timeout=120)
+        assert out.returncode == 0, out.stdout[-2000:] + out.stderr[-3000:]
+    return run
+
+
+def test_state_io_without_room_is_refused_and_the_engine_goes_on(fake):
+    """The slots of state save and restore cannot be allocated: the call is refused, the stream is as it was, a later call works."""
+    fake("""
+e = engine()
+s = filled(e, 40)
+F.fake_fail_alloc(32 << 20)
+refused(-5, s.state_save)
+assert e.gpu_fault() is None and s.length == 40
+assert len(s.step_argmax([1, 2])) == 2 and s.length == 42
+F.fake_fail_alloc(0)
+blob = s.state_save()
+e2 = engine()
+t = e2.stream(64)
+F.fake_fail_alloc(32 << 20)
+good = blob_of(42).view(np.uint8)
+assert good.size == blob.size
+refused(-5, t.state_restore, good)
+assert e2.gpu_fault() is None and t.length == 0
+F.fake_fail_alloc(0)
+assert t.state_restore(good) and t.length == 42
+""")

@@ -233,6 +233,31 @@ def test_state_blob_cross_arena_and_oracle_interop(tiny_engine, tiny_oracle):
         s.close()
 
 
+def test_state_blob_on_a_per_thread_stream(tiny_engine):
+    """A host that works on cudaStreamPerThread (handle 2): save and restore are ordered with the steps before and after them,
+    also where no call has waited for those, and a blob long enough for several copying threads is complete."""
+    n, k = 9000, 6
+    e = gpu_engine(TINY, max_rows=512, max_streams=3, kv_pages=900)
+    try:
+        e.set_cuda_stream(2)
+        toks = prompt(TINY["vocab"], n, "perthread")
+        a = e.stream(n + 64)
+        for i in range(0, n, 512):
+            a.forward(toks[i:i + 512], want_hidden=False)
+        first = int(a.step_argmax([3])[0])
+        a.chained_enqueue(first, k)                                         # (nothing waits for these steps)
+        blob = a.state_save()
+        assert len(blob) > (16 << 20)
+        last = int(a.chained_collect(k)[-1])
+        assert np.array_equal(a.state_save(), blob)
+        b = e.stream(n + 64)
+        assert b.state_restore(blob)
+        assert np.array_equal(b.chained_step_argmax(last, k), a.chained_step_argmax(last, k))
+        assert np.array_equal(a.state_save(), b.state_save())
+    finally:
+        e.close()
+
+
 def test_lane_batch_equals_solo(tiny_engine):
     """lane_batch_argmax_bitexact: B=3 lanes with different histories == each lane solo, 4 steps."""
     V = TINY["vocab"]

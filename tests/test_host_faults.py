@@ -86,3 +86,35 @@ assert e2.gpu_fault() is None and t.length == 0
 F.fake_fail_alloc(0)
 assert t.state_restore(good) and t.length == 42
 """)
+
+
+@pytest.mark.parametrize("n", [1, 1000, 3000, 4088, 16000])
+def test_state_io_moves_every_word_and_only_the_calling_thread_calls_cuda(fake, n):
+    """A blob of one range, some, and more than there are slots: each word is saved and restored once, and no helper thread makes a
+    CUDA call (a host's per-thread stream would be another stream there)."""
+    fake(f"n = {n}" + """
+e = engine(kv_pages=520)
+s = filled(e, n)
+blob = s.state_save().view(np.uint32)
+assert np.array_equal(blob, np.arange(blob.size, dtype=np.uint32))     # (the stand-in packs each word's number)
+t = engine(kv_pages=520).stream(n + 8)
+want = blob_of(n)
+assert want.size == blob.size and t.state_restore(want.view(np.uint8)) and t.length == n
+got = np.zeros_like(want)
+assert F.fake_unpacked(got.ctypes.data_as(C.c_void_p), C.c_long(want.size)) == want.size
+assert np.array_equal(got, want)
+assert count("other_thread") == 0
+""")
+
+
+def test_state_io_reports_a_failed_launch(fake):
+    """A pack kernel that cannot be launched is an error of the call, from whichever range on."""
+    fake("""
+e = engine(kv_pages=520)
+s = filled(e, 16000)
+F.fake_fail_launches(9)
+refused(-3, s.state_save)
+assert e.gpu_fault() is not None
+F.fake_fail_launches(-1)
+refused(-4, s.step_argmax, [1])
+""")

@@ -88,7 +88,7 @@ struct SioCopies {
     uint8_t* const host;
     uint8_t* const slots;
     const size_t bytes;
-    const int most;                                           // threads
+    int most;                                                 // threads
     std::mutex m;
     std::condition_variable work, copied;
     size_t posted = 0, taken = 0, done[SIO_SLOTS] = {};       // done: ranges copied by way of a slot
@@ -124,7 +124,9 @@ struct SioCopies {
         }
     }
     void post() {                                             // range `posted`
-        if (started < most) { pool[started] = std::thread([this] { run(); }); ++started; }
+        if (started < most) {                                 // (no thread to be had: the ones there are, or the caller, do the work)
+            try { pool[started] = std::thread([this] { run(); }); ++started; } catch (...) { most = started; }
+        }
         std::unique_lock<std::mutex> l(m);
         ++posted;
         if (started) work.notify_one(); else take(l);

@@ -118,3 +118,24 @@ assert e.gpu_fault() is not None
 F.fake_fail_launches(-1)
 refused(-4, s.step_argmax, [1])
 """)
+
+
+@pytest.mark.parametrize("threads", [0, 1, 3])
+def test_state_io_without_threads_to_be_had(fake, threads):
+    """Thread starts fail from some point on: the threads there are, or the caller alone, do the work."""
+    fake(f"threads = {threads}" + """
+n = 16000
+e = engine(kv_pages=520)
+s = filled(e, n)
+t = engine(kv_pages=520).stream(n + 8)
+before = count("threads")
+F.fake_fail_threads(threads)
+blob = s.state_save().view(np.uint32)
+assert np.array_equal(blob, np.arange(blob.size, dtype=np.uint32)) and count("threads") == before + threads
+F.fake_fail_threads(threads)
+want = blob_of(n)
+assert t.state_restore(want.view(np.uint8))
+got = np.zeros_like(want)
+assert F.fake_unpacked(got.ctypes.data_as(C.c_void_p), C.c_long(want.size)) == want.size and np.array_equal(got, want)
+F.fake_fail_threads(-1)
+""")

@@ -139,3 +139,16 @@ got = np.zeros_like(want)
 assert F.fake_unpacked(got.ctypes.data_as(C.c_void_p), C.c_long(want.size)) == want.size and np.array_equal(got, want)
 F.fake_fail_threads(-1)
 """)
+
+
+def test_batched_steps_of_any_size_replay_a_graph(fake):
+    """Batches of more than 64 streams are captured at their second step and replayed from then on, like smaller ones."""
+    fake("""
+e = engine()
+streams = [e.stream(32) for _ in range(80)]
+for b in (64, 65, 80):
+    for k in range(4):
+        made, ran = count("graphs_made"), count("graph_launches")
+        e.batch_step_argmax(streams[:b], [1] * b)
+        assert (count("graphs_made") - made, count("graph_launches") - ran) == [(0, 0), (1, 1), (0, 1), (0, 1)][k], (b, k)
+""")

@@ -26,7 +26,7 @@ namespace {
 constexpr int NSPLIT = 64;          // KV splits of the decode attention
 
 struct Tensor { void* ptr; size_t bytes; };
-struct StepGraph { cudaGraphExec_t exec = nullptr; int kernels = 0, eager_runs = 0; uint64_t used = 0; };   // kernels: inside the graph, so that replays are counted
+struct StepGraph { cudaGraphExec_t exec = nullptr; int kernels = 0, eager_runs = 0; };   // kernels: inside the graph, so that replays are counted
 
 struct LayerW {
     bool is_attn = false;
@@ -98,7 +98,6 @@ struct sl_engine {
     std::vector<int> free_pages;
     std::vector<int> free_slots;
     std::map<uint64_t, StepGraph> graphs;      // by shape, see enqueue_call
-    uint64_t graph_clock = 0;
     bool use_graph = true;
     bool use_prefetch = false;      // L2 prefetch of the weights later kernels read (SL_FLAG_L2_PREFETCH); slower now that
                                     // every kernel starts its own weight copies ahead of the launch wait
@@ -762,12 +761,12 @@ int32_t upload_descs(sl_engine* e, const std::vector<SegDesc>& segs, const int32
 // first runs eagerly, so that one-time set-up is outside the capture): a step is hundreds of launches, and a replay spends
 // neither the host's time on them nor the gaps between them.  The shape is (rows, segments, head); descriptors live where the
 // rows alone decide.  Of the full-size model a replay saves 0.19 ms whatever the rows (8 streams 3.16 -> 2.98 ms, 64 8.03 ->
-// 7.84, 208 15.60 -> 15.42; 64 rows of one stream 5.96 -> 5.78), a capture costs 2 to 4 ms.  So every batch size has its graph,
-// the same sizes coming again and again; calls of one stream have one up to 64 rows, the lengths of verify and sampling calls,
-// and none above, the lengths of prompts, which seldom come often enough to pay for one.
-// At most GRAPH_CAP graphs are kept, the least recently used one goes.
+// 7.84, 208 15.60 -> 15.42; 64 rows of one stream 5.96 -> 5.78), a capture costs 2 to 4 ms, and a graph holds 1.4 MB of device
+// and 3.1 MB of host memory.  So every batch size has its graph, the same sizes coming again and again; calls of one stream
+// have one up to 64 rows, the lengths of verify and sampling calls, and none above, the lengths of prompts, which seldom come
+// often enough to pay for one.  That is at most three heads times 64 rows beside the batch sizes, so none is ever dropped (with
+// room for 64 in all, a host that went round 65 shapes paid for a capture on every call).
 constexpr int GRAPH_MAX_ROWS = 64;
-constexpr size_t GRAPH_CAP = 64;
 int32_t enqueue_call(sl_engine* e, int rows, int nsegs, HeadMode head, bool want_logits) {
     // a single stream's decode step: one launch of the step kernel does the whole token
     if (rows == 1 && head == HEAD_ARGMAX && !want_logits && !e->hybrid && !e->ep_step && e->ps_ok && e->use_persistent) {
@@ -780,16 +779,8 @@ int32_t enqueue_call(sl_engine* e, int rows, int nsegs, HeadMode head, bool want
     if (!e->use_graph || e->hybrid || (rows > GRAPH_MAX_ROWS && nsegs != rows)) { enqueue_step(e, rows, nsegs, head, want_logits); return e->poisoned ? SL_ERR_CUDA : SL_OK; }
     const uint64_t key = (uint64_t)rows | (uint64_t)nsegs << 16 | (uint64_t)head << 32 | (uint64_t)want_logits << 40 | (uint64_t)e->ep_step << 41;
     StepGraph& g = e->graphs[key];
-    g.used = ++e->graph_clock;
     if (!g.exec) {
         if (g.eager_runs++ == 0) { enqueue_step(e, rows, nsegs, head, want_logits); return e->poisoned ? SL_ERR_CUDA : SL_OK; }
-        if (e->graphs.size() > GRAPH_CAP) {
-            auto old = e->graphs.end();
-            for (auto it = e->graphs.begin(); it != e->graphs.end(); ++it) if (it->first != key && (old == e->graphs.end() || it->second.used < old->second.used)) old = it;
-            CU(e, cudaStreamSynchronize(e->stream));               // it may still be running
-            if (old->second.exec) cudaGraphExecDestroy(old->second.exec);
-            e->graphs.erase(old);
-        }
         cudaGraph_t graph = nullptr;
         CU(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
         const int64_t before = kernel_launch_count();

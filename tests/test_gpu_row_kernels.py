@@ -104,7 +104,7 @@ def test_tensor_core_tiles(M, K, N):
     check(M, K, N)
 
 
-# more shapes of strict calls than the graph cache holds, some of them again
+# strict calls of every length that has a step graph, with two heads, some of them again
 def test_step_graphs_of_many_shapes():
     import qwisp_b200 as Q
     V = TINY["vocab"]

@@ -152,3 +152,23 @@ for b in (64, 65, 80):
         e.batch_step_argmax(streams[:b], [1] * b)
         assert (count("graphs_made") - made, count("graph_launches") - ran) == [(0, 0), (1, 1), (0, 1), (0, 1)][k], (b, k)
 """)
+
+
+def test_step_graphs_are_made_once_per_shape(fake):
+    """Every verify, sampling and forward length of one stream and many batch sizes, round and round: a capture each, no graph dropped."""
+    fake("""
+e = engine(kv_pages=2000)
+s = e.stream(30000)
+streams = [e.stream(200) for _ in range(40)]
+for turn in range(3):
+    made, ran = count("graphs_made"), count("graph_launches")
+    for rows in range(2, 65):
+        s.step_argmax([1] * rows)
+        s.step_logits([1] * rows)
+        s.forward([1] * rows)
+    for b in range(2, 41):
+        e.batch_step_argmax(streams[:b], [1] * b)
+    shapes = 3 * 63 + 39
+    assert (count("graphs_made") - made, count("graph_launches") - ran) == [(0, 0), (shapes, shapes), (0, shapes)][turn], turn
+assert count("graphs_dropped") == 0
+""")

@@ -776,7 +776,8 @@ int32_t enqueue_call(sl_engine* e, int rows, int nsegs, HeadMode head, bool want
     }
     // (expert-parallel steps contain no collective -- the exchange is this library's own kernels over peer memory --
     // so they are captured like any other step)
-    if (!e->use_graph || e->hybrid || (rows > GRAPH_MAX_ROWS && nsegs != rows)) { enqueue_step(e, rows, nsegs, head, want_logits); return e->poisoned ? SL_ERR_CUDA : SL_OK; }
+    // (the legacy default stream, which a host may have handed over, cannot be captured)
+    if (!e->use_graph || e->stream == cudaStreamLegacy || e->hybrid || (rows > GRAPH_MAX_ROWS && nsegs != rows)) { enqueue_step(e, rows, nsegs, head, want_logits); return e->poisoned ? SL_ERR_CUDA : SL_OK; }
     const uint64_t key = (uint64_t)rows | (uint64_t)nsegs << 16 | (uint64_t)head << 32 | (uint64_t)want_logits << 40 | (uint64_t)e->ep_step << 41;
     StepGraph& g = e->graphs[key];
     if (!g.exec) {

@@ -233,6 +233,21 @@ def test_state_blob_cross_arena_and_oracle_interop(tiny_engine, tiny_oracle):
         s.close()
 
 
+def test_calls_on_the_legacy_stream(tiny_engine):
+    """A host on cudaStreamLegacy (handle 1), which cannot be captured: repeated calls of one shape give what they give elsewhere."""
+    e = gpu_engine(TINY, max_streams=2)
+    try:
+        e.set_cuda_stream(1)
+        a, b = e.stream(64), tiny_engine.stream(64)
+        for i in range(4):
+            toks = prompt(TINY["vocab"], 5, f"legacy.{i}")
+            assert np.array_equal(a.step_argmax(toks), b.step_argmax(toks))
+            assert np.array_equal(a.step_argmax(toks[:1]), b.step_argmax(toks[:1]))
+        assert np.array_equal(a.state_save(), b.state_save()) and e.gpu_fault() is None
+    finally:
+        e.close()
+
+
 def test_state_blob_on_a_per_thread_stream(tiny_engine):
     """A host that works on cudaStreamPerThread (handle 2): save and restore are ordered with the steps before and after them,
     also where no call has waited for those, and a blob long enough for several copying threads is complete."""

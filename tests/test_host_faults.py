@@ -172,3 +172,19 @@ for turn in range(3):
     assert (count("graphs_made") - made, count("graph_launches") - ran) == [(0, 0), (shapes, shapes), (0, shapes)][turn], turn
 assert count("graphs_dropped") == 0
 """)
+
+
+def test_calls_on_the_legacy_stream_run_eagerly(fake):
+    """A host that handed over cudaStreamLegacy (handle 1), which cannot be captured: calls of every kind go on without graphs."""
+    fake("""
+e = engine()
+e.set_cuda_stream(1)
+s = e.stream(200)
+streams = [e.stream(32) for _ in range(3)]
+for _ in range(3):
+    s.forward([1, 2, 3])
+    s.step_argmax([1, 2])
+    s.step_argmax([1])
+    e.batch_step_argmax(streams, [1, 2, 3])
+assert count("captures") == 0 and e.gpu_fault() is None
+""")

@@ -26,7 +26,7 @@ namespace {
 constexpr int NSPLIT = 64;          // KV splits of the decode attention
 
 struct Tensor { void* ptr; size_t bytes; };
-struct StepGraph { cudaGraphExec_t exec = nullptr; int kernels = 0, eager_runs = 0; };   // kernels: inside the graph, so that replays are counted
+struct StepGraph { cudaGraphExec_t exec = nullptr; int kernels = 0, eager_runs = 0; bool no_room = false; };   // kernels: inside the graph, so that replays are counted
 
 struct LayerW {
     bool is_attn = false;
@@ -776,12 +776,13 @@ int32_t enqueue_call(sl_engine* e, int rows, int nsegs, HeadMode head, bool want
     }
     // (expert-parallel steps contain no collective -- the exchange is this library's own kernels over peer memory --
     // so they are captured like any other step)
+    auto eager = [&]() -> int32_t { enqueue_step(e, rows, nsegs, head, want_logits); return e->poisoned ? SL_ERR_CUDA : SL_OK; };
     // (the legacy default stream, which a host may have handed over, cannot be captured)
-    if (!e->use_graph || e->stream == cudaStreamLegacy || e->hybrid || (rows > GRAPH_MAX_ROWS && nsegs != rows)) { enqueue_step(e, rows, nsegs, head, want_logits); return e->poisoned ? SL_ERR_CUDA : SL_OK; }
+    if (!e->use_graph || e->stream == cudaStreamLegacy || e->hybrid || (rows > GRAPH_MAX_ROWS && nsegs != rows)) return eager();
     const uint64_t key = (uint64_t)rows | (uint64_t)nsegs << 16 | (uint64_t)head << 32 | (uint64_t)want_logits << 40 | (uint64_t)e->ep_step << 41;
     StepGraph& g = e->graphs[key];
     if (!g.exec) {
-        if (g.eager_runs++ == 0) { enqueue_step(e, rows, nsegs, head, want_logits); return e->poisoned ? SL_ERR_CUDA : SL_OK; }
+        if (g.no_room || g.eager_runs++ == 0) return eager();
         cudaGraph_t graph = nullptr;
         CU(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
         const int64_t before = kernel_launch_count();
@@ -789,8 +790,11 @@ int32_t enqueue_call(sl_engine* e, int rows, int nsegs, HeadMode head, bool want
         g.kernels = (int)(kernel_launch_count() - before);
         count_launches(-(int64_t)g.kernels);                       // the capture itself launched nothing
         CU(e, cudaStreamEndCapture(e->stream, &graph));
-        CU(e, cudaGraphInstantiate(&g.exec, graph, 0));
+        const cudaError_t made = cudaGraphInstantiate(&g.exec, graph, 0);
         cudaGraphDestroy(graph);
+        if (made != cudaSuccess) g.exec = nullptr;
+        if (made == cudaErrorMemoryAllocation) { cudaGetLastError(); g.no_room = true; return eager(); }      // a call needs no graph
+        CU(e, made);
     }
     CU(e, cudaGraphLaunch(g.exec, e->stream));
     count_launches(g.kernels);

@@ -25,6 +25,7 @@ thread_local cudaError_t last = cudaSuccess;              // as the runtime keep
 struct Config { dim3 grid, block; size_t smem; void* stream; };
 thread_local Config config;
 size_t fail_bytes = 0;
+bool fail_graphs = false;
 std::atomic<long> threads_left{-1}, launches_left{-1};
 bool capturing = false;
 
@@ -62,6 +63,7 @@ long fake_count(const char* what) { std::lock_guard<std::mutex> l(mu); return co
 void fake_fail_alloc(size_t bytes) { fail_bytes = bytes; }                    // allocations of exactly this size fail (0: none)
 void fake_fail_threads(long after) { threads_left = after; }                  // thread starts fail after that many (-1: none)
 void fake_fail_launches(long after) { launches_left = after; }                // kernel launches fail after that many (-1: none)
+void fake_fail_graphs(int on) { fail_graphs = on != 0; }                      // no memory for graphs
 long fake_unpacked(uint32_t* out, long n) {                                   // words that arrived, in order; -1 if one is missing
     std::lock_guard<std::mutex> l(mu);
     if ((long)unpacked.size() != n) return -1;
@@ -133,7 +135,7 @@ cudaError_t cudaStreamBeginCapture(cudaStream_t s, cudaStreamCaptureMode) {
     return cudaSuccess;
 }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) { capturing = false; *g = reinterpret_cast<cudaGraph_t>(new char); return cudaSuccess; }
-cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t, unsigned long long) { note("graphs_made"); *x = reinterpret_cast<cudaGraphExec_t>(new char); return cudaSuccess; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t, unsigned long long) { if (fail_graphs) return ret(cudaErrorMemoryAllocation); note("graphs_made"); *x = reinterpret_cast<cudaGraphExec_t>(new char); return cudaSuccess; }
 cudaError_t cudaGraphDestroy(cudaGraph_t g) { delete reinterpret_cast<char*>(g); return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t x) { note("graphs_dropped"); delete reinterpret_cast<char*>(x); return cudaSuccess; }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { note("graph_launches"); return cudaSuccess; }

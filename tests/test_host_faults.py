@@ -188,3 +188,20 @@ for _ in range(3):
     e.batch_step_argmax(streams, [1, 2, 3])
 assert count("captures") == 0 and e.gpu_fault() is None
 """)
+
+
+def test_no_room_for_a_graph_is_no_failure(fake):
+    """A graph that cannot be made for lack of memory: the call, and later ones of its shape, are launched eagerly."""
+    fake("""
+e = engine()
+s = e.stream(200)
+F.fake_fail_graphs(1)
+for _ in range(4):
+    assert len(s.step_argmax([1, 2, 3])) == 3
+assert count("graphs_made") == 0 and count("graph_launches") == 0 and e.gpu_fault() is None
+assert count("captures") == 1                                  # (tried once)
+F.fake_fail_graphs(0)
+for _ in range(3):
+    s.step_argmax([1, 2])
+assert count("graphs_made") == 1 and count("graph_launches") == 2
+""")

@@ -7,7 +7,8 @@
 // histogram of fixed-point softmax weights over the scaled gap (gmax - L)/T.
 //
 // exp and log are evaluated by the small deterministic routines below (IEEE add / multiply /
-// divide only, no fused contraction), so the CPU restatement used by the tests reproduces every
+// divide only, no fused contraction; ln 2 split in two as by Cody and Waite, then the Taylor series of exp and the
+// series of 2 atanh(f / (2 + f)) for log), so the CPU restatement used by the tests reproduces every
 // draw and every accept flag bit for bit; their ~1e-7 relative error is irrelevant for sampling.
 #include "kernels.h"
 
@@ -169,7 +170,10 @@ __global__ void __launch_bounds__(SAMP_T) k_sample_rows(const __half* logits, co
 }
 void launch_sample_rows(const __half* logits, const float* adj, const int* draft, int* samp_full, int* samp_resid, int* accept, int M, int V,
                         float invT, float top_p, uint32_t seed_lo, uint32_t seed_hi, uint32_t base_pos, cudaStream_t st) {
-    k_sample_rows<<<M, SAMP_T, 0, st>>>(logits, adj, draft, samp_full, samp_resid, accept, invT, V, seed_lo, seed_hi, base_pos, top_p);
+    profile_launch("k_sample_rows", st, [&] {
+        k_sample_rows<<<M, SAMP_T, 0, st>>>(logits, adj, draft, samp_full, samp_resid, accept, invT, V, seed_lo, seed_hi, base_pos, top_p);
+        return 0;
+    });
 }
 
 }  // namespace sl

@@ -205,3 +205,21 @@ for _ in range(3):
     s.step_argmax([1, 2])
 assert count("graphs_made") == 1 and count("graph_launches") == 2
 """)
+
+
+def test_every_launch_is_counted(fake):
+    """sl_engine_launch_count counts each kernel that a call launches: steps, sampling, prefill, state save and restore, rollback."""
+    fake("""
+e = engine()
+e.use_graphs(False)
+s, t = e.stream(200), e.stream(200)
+blob = blob_of(40).view(np.uint8)
+snap = s.snapshot()
+calls = [lambda: s.step_argmax([1]), lambda: s.rollback(snap), lambda: s.step_sample_rows([1, 2], None, 1.0, 0.9, 1, 2, 0), lambda: s.forward_hybrid([1] * 40),
+         lambda: s.forward([1] * 40), lambda: s.step_argmax([1, 2]), lambda: e.batch_step_argmax([s, t], [1, 2]), lambda: s.state_save(),
+         lambda: t.state_restore(blob), lambda: Q.ops.lm_head(e, np.zeros((3, 512), np.float16))]
+for i, call in enumerate(calls):
+    ran, counted = count("launches"), e.launch_count()
+    call()
+    assert count("launches") - ran == e.launch_count() - counted > 0, (i, count("launches") - ran, e.launch_count() - counted)
+""")

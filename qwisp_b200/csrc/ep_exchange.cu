@@ -4,9 +4,10 @@
 // normed rows and routing choices of ALL ranks (dispatch), and afterwards gets back, for each of its own (row, k)
 // pairs, the one expert output that some rank computed (combine).  Both are tiny (a few hundred KB per layer) and
 // latency-bound, so they are done with plain peer stores from this library's own kernels instead of collectives:
-//   dispatch  the router kernel's last CTA (k_moe_router, RouterArgs::epd) stores the rank's M normed rows and
-//             M*top_k indices straight into every peer's gather buffers, then (after a system fence) a sequence
-//             number into that peer's flag word for this rank;
+//   dispatch  the norm kernel ahead of the router (k_final_norm_ep) stores the rank's M normed rows straight into every
+//             peer's gather buffer, the routing kernel (k_route_rows, RouterArgs::epd) each row's top_k indices; its last
+//             CTA then (after a system fence) stores a sequence number into each peer's flag word for this rank.  With one
+//             row per rank the last CTA of k_moe_router does all of it;
 //   wait      k_ep_lists: one CTA waits for all ranks' flags, then groups the pairs that chose a local expert;
 //   combine   the down-projection kernel stores each pair's output row directly into the pair OWNER's buffer
 //             (ExpertArgs::peer_dbuf); its last CTA raises this rank's flag at every peer, and k_ep_combine waits

@@ -85,7 +85,7 @@ def test_rows_equal_sequential(tiny_engine, plan):
 
 
 def test_many_row_kernels_equal_pass_kernels():
-    """Calls with more than 8 rows run the many-row kernels (weights dequantised once per block of rows, experts
+    """Calls with more than one row run the many-row kernels (weights dequantised once per block of rows, experts
     without CTA-wide barriers); SL_FLAG_PASS_KERNELS walks the same rows in passes of 8 with the one-to-eight-row
     kernels.  Both must give the same bits: logits of a 37-row call, the state it leaves, and 12 lanes batched."""
     import qwisp_b200 as Q

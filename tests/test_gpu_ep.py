@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("rows_per_rank", [4, 12])
 def test_expert_parallel_tokens_match_single_gpu(rows_per_rank):
-    """4 rows per rank: the one-to-eight-row kernels on the gathered rows; 12: the many-row router and expert kernels."""
+    """4 rows per rank: the pass kernels for the experts of the 8 gathered rows; 12: the many-row expert kernels.  (The router and the
+    rank's own projections and mixers are the many-row forms in both.)"""
     import torch
     if torch.cuda.device_count() < 2:
         pytest.skip("needs 2 GPUs")

@@ -433,7 +433,7 @@ class LaneBatchSlots:
             lcp = max(s.max_common_prefix(prompt) for s in stores)
             plan = admit_plan(len(prompt), len(hit[0]) if hit else 0, lcp, self.min_shared)
             if plan.restore_len > 0:
-                if self._streams[slot].state_restore(hit[1]):
+                if self._restored(slot, hit[1]):
                     self._resume[slot] = plan.restore_len        # restored tokens are not charged to the budget
                     self.restored_tokens += plan.restore_len
                     self.restore_hits += 1
@@ -442,6 +442,24 @@ class LaneBatchSlots:
                     self._streams[slot] = self.engine.stream(seq_budget or self.default_seq_budget)
                     plan.restore_len = 0
         self._plan[slot] = plan
+
+    # The stores only save prefill: a blob that the engine has no room to move is one that is not there.
+    def _restored(self, slot, blob):
+        try:
+            return self._streams[slot].state_restore(blob)
+        except SeedlessError as e:
+            if e.code != _lib.SL_ERR_CAPACITY:
+                raise
+            return False
+
+    def _saved(self, store, tokens, stream):
+        try:
+            store.save(tokens, stream.state_save())
+            return 1
+        except SeedlessError as e:
+            if e.code != _lib.SL_ERR_CAPACITY:
+                raise
+            return 0
 
     def admit_step(self, prompt, slot, token_budget, seq_budget=0):
         """-> ("prefilling", consumed) | ("done", first_token, consumed) | ("failed",)"""
@@ -474,12 +492,11 @@ class LaneBatchSlots:
                 self.prefilled_tokens += n
                 first = False
                 if plan.capture_at is not None and pos == plan.capture_at and self.shared_store is not None:
-                    self.shared_store.save(prompt[:pos], st.state_save())
-                    self.captures += 1
+                    self.captures += self._saved(self.shared_store, prompt[:pos], st)
                 if last:
                     self._resume[slot] = pos
                     if plan.save_at_end and self.prefix_store is not None and self.prefix_store.budget > 0:
-                        self.prefix_store.save(prompt, st.state_save())
+                        self._saved(self.prefix_store, prompt, st)
                     return ("done", tok, consumed)
             self._resume[slot] = pos
             return ("prefilling", consumed)

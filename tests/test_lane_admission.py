@@ -3,6 +3,7 @@ cut into calls, what is captured, restored and charged.  No GPU: the engine belo
 outputs from the token history, so a restored stream and a cold one can be compared exactly."""
 import numpy as np
 
+from qwisp_b200 import SeedlessError
 from qwisp_b200.engine import LaneBatchSlots
 from qwisp_b200.prefix import PrefixRAMStore
 from qwisp_b200.scheduler import ContinuousScheduler, Request
@@ -100,6 +101,42 @@ def test_capture_at_the_exact_boundary_then_restore_and_charge_only_the_tail():
     want = cs.admit_step(prompts[2], 0, 1 << 20, 512)
     assert want[1] == r2[1] and eng.streams[2].history == cold.streams[0].history
     assert slots.step([None, None, r2[1]])[2] == cs.step([want[1]])[0]
+
+
+def test_a_blob_there_is_no_room_to_move_fails_no_request():
+    """The engine refuses to save, or to restore, for lack of room: requests are served as if the store had nothing; any other
+    failure still fails the request."""
+    class Refusing(FakeStream):
+        code = -5
+
+        def state_save(self):
+            raise SeedlessError(self.code, "sl_state_save")
+
+        def state_restore(self, blob):
+            raise SeedlessError(self.code, "sl_state_restore")
+
+    class RefusingEngine(FakeEngine):
+        def stream(self, max_seq_len):
+            self.streams.append(Refusing(self, max_seq_len))
+            return self.streams[-1]
+
+    common, prompts = _prompts()
+    want = []
+    for p in prompts:
+        want.append(LaneBatchSlots(FakeEngine(), 1, chunk=64, default_seq_budget=512, hybrid=True).admit_step(p, 0, 1 << 20, 512)[1])
+    stores = PrefixRAMStore(1 << 20), PrefixRAMStore(1 << 20)
+    refusing = LaneBatchSlots(RefusingEngine(), 3, chunk=64, default_seq_budget=512, prefix_store=stores[0], shared_store=stores[1], hybrid=True, min_shared=32)
+    assert refusing.admit_step(prompts[0], 0, 1 << 20, 512)[:2] == ("done", want[0])
+    assert stores[0].entries == [] and stores[1].entries == []
+    # another engine fills the stores; the restore is refused, the request starts cold
+    filling = LaneBatchSlots(FakeEngine(), 2, chunk=64, default_seq_budget=512, prefix_store=stores[0], shared_store=stores[1], hybrid=True, min_shared=32)
+    for i in (0, 1):
+        filling.admit_step(prompts[i], i, 1 << 20, 512)
+    assert filling.captures == 1
+    r = refusing.admit_step(prompts[2], 1, 1 << 20, 512)
+    assert r == ("done", want[2], len(prompts[2])) and refusing.restore_hits == 0 and refusing.captures == 0
+    Refusing.code = -3
+    assert refusing.admit_step(prompts[2], 2, 1 << 20, 512) == ("failed",)
 
 
 def test_budget_resumes_mid_prompt_and_always_makes_one_chunk_of_progress():

@@ -131,11 +131,11 @@ int32_t sl_inject_fault(sl_engine* e, int32_t on);
  * reports through the engine's error word.  Nothing faults or hangs.  The next call that synchronises
  * returns SL_ERR_CUDA and poisons the engine, as it does when a real kernel's wait gives up. */
 int32_t sl_debug_wait_timeout(sl_engine* e);
-/* Test hook for the waits inside the expert kernels whose warps wait for one another: the next call in prefill mode, or (hidden
- * size 512) of more than one row, runs its gate/up products in a form whose loading warps bring no rows, so that the other warps'
- * bounded waits (a few milliseconds in that form) run out.  Nothing faults or hangs; the call returns SL_ERR_CUDA and poisons
- * the engine. */
-int32_t sl_debug_expert_timeout(sl_engine* e);
+/* Test hook for the waits inside the kernels that wait for their own copies or whose warps wait for one another (the state update
+ * and the experts of prefill mode and, with hidden size 512, of more than one row): the next such call of one stream runs them in a
+ * form that brings no rows, so that the bounded waits (a few milliseconds in that form) run out.  Nothing faults or hangs; the call
+ * returns SL_ERR_CUDA and poisons the engine. */
+int32_t sl_debug_rows_timeout(sl_engine* e);
 /* Kernels this library has launched so far (bench bookkeeping). */
 int64_t sl_engine_launch_count(sl_engine* e);
 /* Replay decode steps as CUDA graphs (default on) or launch every kernel eagerly. */

@@ -70,7 +70,7 @@ SYMBOLS = {
     "sl_forward_hybrid": (_I32, [_VP, _VP, _I32, _VP]),
     "sl_hybrid_chunk": (_I32, [_VP]),
     "sl_debug_wait_timeout": (_I32, [_VP]),
-    "sl_debug_expert_timeout": (_I32, [_VP]),
+    "sl_debug_rows_timeout": (_I32, [_VP]),
     "sl_engine_use_persistent": (_I32, [_VP, _I32]),
     "sl_debug_step_timeline": (_I32, [_VP, _I32, _VP, _U64]),
     "sl_step_argmax": (_I32, [_VP, _VP, _I32, _VP]),

@@ -669,7 +669,7 @@ void enqueue_mixer(sl_engine* e, const LayerW& L, const __half* rows, const __ha
     if (!L.is_attn) {
         GdnArgs g{}; g.inproj = e->inproj; g.ld = e->gdn_in; g.conv_w = L.conv_w; g.A_log = L.A_log; g.dt_bias = L.dt_bias;
         g.Hk = c.gdn_k_heads; g.Hv = c.gdn_v_heads; g.eps = c.rms_eps; g.tab = e->tab; g.gdn_index = L.type_index; g.segs = segs_of(e->desc, M); g.y = e->mix;
-        g.row_seg = row_seg_of(e->desc, M); g.qk = e->gdn_qk; g.vg = e->gdn_vg; g.err = e->err_flag;
+        g.row_seg = row_seg_of(e->desc, M); g.qk = e->gdn_qk; g.vg = e->gdn_vg; g.err = e->err_flag; g.stall = e->stall;
         // more than one row: the state-independent part for all rows side by side, then the bare recurrence (same bits)
         if (e->use_rows && M > 1) launch_gdn_rows(g, M, nsegs, st, pdl);
         else launch_gdn_core(g, nsegs, st, pdl);
@@ -1067,7 +1067,7 @@ int32_t sl_debug_wait_timeout(sl_engine* e) {
     launch_wait_probe(e->err_flag, e->stream);
     return SL_OK;
 }
-int32_t sl_debug_expert_timeout(sl_engine* e) {
+int32_t sl_debug_rows_timeout(sl_engine* e) {
     int32_t rc = guard(e); if (rc) return rc;
     e->stall = true;
     return SL_OK;

@@ -123,7 +123,8 @@ __device__ __forceinline__ void lds2(const void* p, f32x2& a, f32x2& b) { asm vo
 // segments from 60 to 48).  The readout's sum is off the chain, see below.
 // 32 state rows per CTA (8 per warp), 128 CTAs per stream: one warp per SM sub-partition, which is what the 4096 rows of
 // a stream give.  grid (4, Hv, nsegs), 128 threads; k / q / v / gates of CH rows at a time by bulk copies, two buffers.
-template <int CH>
+// STALL: a test's form, in which no operands are ever fetched, so that the wait for them runs out, and soon
+template <int CH, bool STALL>
 __global__ void __launch_bounds__(128) k_gdn_scan(GdnArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];    // [2][CH][1024] k | q, then [2][CH][144] v | gates
     __shared__ __align__(8) uint64_t bar[2];
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(128) k_gdn_scan(GdnArgs a) {
     float* S_out = a.tab.gdn_state + base + (size_t)(side ^ 1) * a.tab.state_stride_side;
     const int nchunks = (seg.nrows + CH - 1) / CH;
     auto fetch = [&](int c) {
+        if (STALL) return;
         const int b = c & 1, t0 = c * CH, n = min(CH, seg.nrows - t0);
         mbar_expect_tx(&bar[b], (uint32_t)n * (1024 + GS_REC));
         bulk_g2s(smem + (size_t)b * CH * 1024, a.qk + ((size_t)hk * a.M + seg.row0 + t0) * 256, (uint32_t)n * 1024, &bar[b]);
@@ -214,7 +216,7 @@ __global__ void __launch_bounds__(128) k_gdn_scan(GdnArgs a) {
     __syncthreads();                                          // the barriers are initialised
     for (int c = 0; c < nchunks; ++c) {
         const int b = c & 1, t0 = c * CH, n = min(CH, seg.nrows - t0);
-        ok = mbar_wait_bounded(&bar[b], (uint32_t)((c >> 1) & 1)) && ok;
+        ok = ok && mbar_wait_bounded(&bar[b], (uint32_t)((c >> 1) & 1), STALL ? 1 << 10 : 1 << 22);      // (one that ran out is not followed by others)
         const unsigned char* kq = smem + (size_t)b * CH * 1024;
         const unsigned char* vg = smem + (size_t)2 * CH * 1024 + (size_t)b * CH * GS_REC;
         f32x2 k[8];
@@ -256,18 +258,22 @@ __global__ void __launch_bounds__(128) k_gdn_scan(GdnArgs a) {
             *reinterpret_cast<float4*>(S_out + w * GDN_DK + (j + 8 * i) * 4) = lo;
             *reinterpret_cast<float4*>(S_out + w * GDN_DK + (j + 8 * i + 16) * 4) = hi;
         }
-    if (!ok && a.err && lane == 0) atomicOr(a.err, 1u);
+    if (!ok) {                                 // copies of this CTA may still be landing: outlast them
+        if (a.err && lane == 0) atomicOr(a.err, 1u);
+        const long long c0 = clock64();
+        while (clock64() - c0 < 200000ll) { }
+    }
 }
 
 size_t gdn_qk_floats(int Hk, int rows) { return (size_t)Hk * rows * 256; }
 size_t gdn_vg_bytes(int Hv, int rows) { return (size_t)Hv * 4 * rows * GS_REC; }
 
-template <int CH>
+template <int CH, bool STALL = false>
 static void launch_scan_t(const GdnArgs& a, int nsegs, cudaStream_t st) {
     const size_t smem = (size_t)2 * CH * (1024 + GS_REC) + 256;     // (the last token reads one record of gates past its own)
     static bool configured = false;
-    if (!configured) { cudaFuncSetAttribute(k_gdn_scan<CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
-    profile_launch("k_gdn_scan", st, [&] { k_gdn_scan<CH><<<dim3(4, (unsigned)a.Hv, (unsigned)nsegs), 128, smem, st>>>(a); return 0; });
+    if (!configured) { cudaFuncSetAttribute(k_gdn_scan<CH, STALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
+    profile_launch("k_gdn_scan", st, [&] { k_gdn_scan<CH, STALL><<<dim3(4, (unsigned)a.Hv, (unsigned)nsegs), 128, smem, st>>>(a); return 0; });
 }
 void launch_gdn_rows(const GdnArgs& in, int M, int nsegs, cudaStream_t st, bool pdl) {
     GdnArgs a = in; a.M = M;
@@ -282,6 +288,7 @@ void launch_gdn_rows(const GdnArgs& in, int M, int nsegs, cudaStream_t st, bool 
     // several to one, and 17 rows took 7 us longer)
     // one row per segment (batched decode): the state's traffic is the time, small buffers leave room for more CTAs per SM
     if (M == nsegs) launch_scan_t<1>(a, nsegs, st);
+    else if (a.stall) launch_scan_t<32, true>(a, nsegs, st);
     else launch_scan_t<32>(a, nsegs, st);
 }
 

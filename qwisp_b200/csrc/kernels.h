@@ -119,6 +119,7 @@ struct GdnArgs {
     unsigned char* vg = nullptr;         // gdn_vg_bytes(): conv + SiLU of v, (decay, beta)
     int M = 0;                           // rows of the call (filled by the launcher)
     unsigned* err = nullptr;
+    bool stall = false;                  // test hook: the scan in the form whose wait runs out
 };
 
 struct AttnArgs {

@@ -105,9 +105,9 @@ class Engine:
         """Test hook: enqueue a kernel whose bounded wait runs out (nothing faults); the next call fails."""
         self._check(lib().sl_debug_wait_timeout(self._h), "sl_debug_wait_timeout")
 
-    def debug_expert_timeout(self):
-        """Test hook: the waits of the next call's expert kernels run out (nothing faults); that call fails."""
-        self._check(lib().sl_debug_expert_timeout(self._h), "sl_debug_expert_timeout")
+    def debug_rows_timeout(self):
+        """Test hook: the waits of the next many-row call's kernels run out (nothing faults); that call fails."""
+        self._check(lib().sl_debug_rows_timeout(self._h), "sl_debug_rows_timeout")
 
     def set_cuda_stream(self, cuda_stream_handle):
         self._check(lib().sl_engine_set_cuda_stream(self._h, C.c_void_p(cuda_stream_handle)), "sl_engine_set_cuda_stream")

@@ -379,17 +379,18 @@ def test_device_wait_timeout_poisons_engine():
 
 
 @pytest.mark.parametrize("call", ["forward_hybrid", "forward"])
-def test_expert_wait_timeout_poisons_engine(call):
-    """The same for the kernels whose warps wait for one another (experts in prefill mode and of many rows): rows that never arrive
-    make every warp give up its own bounded wait and leave, none waits for one that has left, and the call reports it."""
+def test_rows_wait_timeout_poisons_engine(call):
+    """The same for the kernels that wait for their own copies (the state scan, over several chunks) or whose warps wait for one another
+    (experts in prefill mode and of many rows): rows that never arrive make every warp give up its own bounded wait and leave,
+    none waits for one that has left, and the call reports it."""
     import time
     import qwisp_b200 as Q
-    e = gpu_engine(TINY, max_streams=2)
+    e = gpu_engine(TINY, max_streams=2, max_rows=256)
     try:
-        s = e.stream(80)
-        toks = prompt(TINY["vocab"], 40, "stall")
-        assert getattr(s, call)(toks).shape == (40, TINY["hidden"]) and e.gpu_fault() is None
-        e.debug_expert_timeout()
+        s = e.stream(400)
+        toks = prompt(TINY["vocab"], 200, "stall")
+        assert getattr(s, call)(toks).shape == (200, TINY["hidden"]) and e.gpu_fault() is None
+        e.debug_rows_timeout()
         t0 = time.perf_counter()
         with pytest.raises(Q.SeedlessError) as ei:
             getattr(s, call)(toks[1:])

@@ -17,9 +17,9 @@
 //             "empty" barrier.  It is warp 0: the other warps keep the issue slots busy;
 //   load       4 warps: the NT x 128 activations of the stage, 16-byte asynchronous copies that count themselves in at
 //             the stage's "full" barrier;
-//   dequant   16 warps: a warp owns one 16-row tile of the item and every second stage; its fragments are loaded two of
-//             its stages ahead (across items), turned into MMA order by two shuffles per word pair, expanded to fp16 (scale
-//             and bias by one fp16x2 multiply-add per pair) and stored to the A operand in TMEM;
+//   dequant   16 warps: a warp owns 32 weight rows of the item (a lane a row: a lane of tensor memory is a row) and every
+//             fourth stage; its words are loaded two of its stages ahead (across items), expanded to fp16 (scale and bias by
+//             one fp16x2 multiply-add per pair) and stored to the A operand in TMEM as they are;
 //   epilogue   4 warps: read the finished accumulator while the next item accumulates in the other half of its TMEM.
 // The first form (256 threads that all loaded, expanded, synchronised and waited in turn, one pair of groups ahead)
 // spent 2.5 us on a pair of groups whose MMAs take 0.3: every pair paid the latency of its weights and of its rows.
@@ -67,9 +67,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t r[16]) {
                  : "r"(taddr) : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-// 16 lanes x 32 columns.  Registers 4c .. 4c+3 of lane 4r + t: (row r, columns 8c + 2t, + 1), (row r + 8, the same columns)
-__device__ __forceinline__ void tmem_st16x256(uint32_t taddr, const uint32_t v[16]) {
-    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+// 32 lanes (rows) x 16 columns
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t v[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
                  :: "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
                     "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
 }
@@ -99,53 +99,31 @@ __device__ __forceinline__ bool tc_wait(uint64_t* b, uint32_t parity, volatile i
 }
 __device__ __forceinline__ bool tc_agree(bool ok) { return __all_sync(0xffffffffu, ok); }
 
-// ---- one K group (64 inputs) of a 16-row tile: fragment register -> A operand
-// Lane 4r + t holds inputs 16t .. 16t + 15 of rows A_r and B_r = r + 8 (two words each); the MMA wants inputs 16c .. 16c + 15
-// in column block c, of which this lane stores 4t .. 4t + 3.  So the four lanes of a quad transpose a 4 x 4 matrix of
-// 16-bit items (4 nibbles): a shuffle with lane ^ 2 and one with lane ^ 1 per row.
-struct TcQuad { bool hi; bool odd; uint32_t own, send; };                   // what a lane needs to know for it
-__device__ __forceinline__ TcQuad tc_quad(int t) {
-    // after the first exchange lanes 0, 1 hold (blocks t, t + 2) in (keep, got), lanes 2, 3 (blocks t, t - 2); the byte selectors
-    // pick this lane's halves (even lanes the low ones, odd lanes the high ones) resp. its neighbour's, lower block first
-    TcQuad q; q.hi = t >= 2; q.odd = (t & 1) != 0;
-    const uint32_t lo = q.hi ? 0x1054u : 0x5410u, up = q.hi ? 0x3276u : 0x7632u;
-    q.own = q.odd ? up : lo; q.send = q.odd ? lo : up;
-    return q;
-}
-// words of one row -> e: items of blocks 0 | 2, o: items of blocks 1 | 3
-__device__ __forceinline__ void tc_transpose(const TcQuad& q, uint32_t x, uint32_t y, uint32_t& e, uint32_t& o) {
-    const uint32_t keep = q.hi ? y : x, got = __shfl_xor_sync(0xffffffffu, q.hi ? x : y, 2);
-    const uint32_t own = __byte_perm(keep, got, q.own), nb = __shfl_xor_sync(0xffffffffu, __byte_perm(keep, got, q.send), 1);
-    e = q.odd ? nb : own; o = q.odd ? own : nb;
-}
-// two items -> the halves of block `c` (low item) and c + 2 (high item), scaled
-__device__ __forceinline__ void tc_expand(uint32_t w, __half2 sc, __half2 bi, uint32_t* c0, uint32_t* c2) {
-    uint32_t d[4], v[4];
-    dequant8(w, d);                                                          // (n0 of the low item, n0 of the high one), (n1, n1), ...
+// ---- one K group (64 inputs) of a row of a tile: packed words -> A operand.  A lane of tensor memory is a weight row, and the
+// weights arrive by rows (gemv.cuh), so a lane expands what it has loaded and stores it as it is: 32 columns of two halves.
+// Bound by the issue of these instructions: 13 per word of 8 weights.
+__device__ __forceinline__ void tc_expand(uint32_t w, __half2 sc, __half2 bi, uint32_t* c) {
+    uint32_t d[4];
+    dequant8(w, d);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const __half2 h = __hfma2(*reinterpret_cast<const __half2*>(&d[j]), sc, bi);
-        v[j] = *reinterpret_cast<const uint32_t*>(&h);
+        c[j == 1 ? 2 : j == 2 ? 1 : j] = *reinterpret_cast<const uint32_t*>(&h);
     }
-    c0[0] = __byte_perm(v[0], v[1], 0x5410); c0[1] = __byte_perm(v[2], v[3], 0x5410);
-    c2[0] = __byte_perm(v[0], v[1], 0x7632); c2[1] = __byte_perm(v[2], v[3], 0x7632);
 }
-// s2: (scale, bias) of rows A_r and B_r; taddr: the tile's lanes, the group's first column
-__device__ __forceinline__ void tc_group_A(const TcQuad& q, uint4 wv, uint32_t sa, uint32_t sb, uint32_t taddr) {
-    const __half2 hA = *reinterpret_cast<const __half2*>(&sa), hB = *reinterpret_cast<const __half2*>(&sb);
-    uint32_t v[16], e, o;
-    tc_transpose(q, wv.x, wv.y, e, o);
-    tc_expand(e, __half2half2(__low2half(hA)), __half2half2(__high2half(hA)), v, v + 8);
-    tc_expand(o, __half2half2(__low2half(hA)), __half2half2(__high2half(hA)), v + 4, v + 12);
-    tc_transpose(q, wv.z, wv.w, e, o);
-    tc_expand(e, __half2half2(__low2half(hB)), __half2half2(__high2half(hB)), v + 2, v + 10);
-    tc_expand(o, __half2half2(__low2half(hB)), __half2half2(__high2half(hB)), v + 6, v + 14);
-    tmem_st16x256(taddr, v);
+// w: the words of the group; sb: its (scale, bias); taddr: the warp's lanes, the group's first column
+__device__ __forceinline__ void tc_group_A(const uint2 w[4], uint32_t sb, uint32_t taddr) {
+    const __half2 h = *reinterpret_cast<const __half2*>(&sb), sc = __half2half2(__low2half(h)), bi = __half2half2(__high2half(h));
+    uint32_t v[16];
+    tc_expand(w[0].x, sc, bi, v); tc_expand(w[0].y, sc, bi, v + 4); tc_expand(w[1].x, sc, bi, v + 8); tc_expand(w[1].y, sc, bi, v + 12);
+    tmem_st16(taddr, v);
+    tc_expand(w[2].x, sc, bi, v); tc_expand(w[2].y, sc, bi, v + 4); tc_expand(w[3].x, sc, bi, v + 8); tc_expand(w[3].y, sc, bi, v + 12);
+    tmem_st16(taddr + 16, v);
 }
 
 // ================================================================================ the two kinds of work
-// Items are numbered (rows block, 128 weight rows), weight rows fastest; a CTA walks a contiguous run of them, so most
-// steps stay inside a block.  A work type gives the weights of a tile of an item (moved along by a cursor), the place of a
+// Items are (rows block, 128 weight rows), weight rows fastest; a CTA walks a contiguous run of them, so most steps stay
+// inside a block.  A work type gives the weights of a tile of an item (moved along by a cursor), the place of a
 // block's activation rows (halves from base(); Place: wide enough for the rows that the kind of work can have), and the epilogue.
 struct TcTile { const uint4 *w, *s; int blk, rt; };   // fragment-major nibbles and scales of a tile (nullptr: none) of weight-row group rt
 
@@ -168,6 +146,9 @@ struct DenseWork {
     int NRT;                                                                // weight-row groups
     __device__ DenseWork(const Args& args, Shared&) : a(args), NRT((args.N + TC_ROWS - 1) / TC_ROWS) {}
     __device__ int items() const { return NRT * ((a.M + NT - 1) / NT); }
+    struct Walk { int blk, rt; };                                           // a role's place in its CTA's run
+    __device__ Walk walk(int item) const { return {item / NRT, item % NRT}; }
+    __device__ void next(Walk& w) const { if (++w.rt == NRT) { w.rt = 0; ++w.blk; } }
     __device__ int inputs() const { return a.K; }
     __device__ unsigned* err() const { return a.err; }
     __device__ bool has_tile(int rt, int tl) const { return rt * 8 + tl < a.N >> 4; }
@@ -231,6 +212,9 @@ struct ExpertWork {
         __syncthreads();
     }
     __device__ int items() const { return sh.tab.base[n_active + 1] * NRT; }
+    struct Walk { int blk, rt; };
+    __device__ Walk walk(int item) const { return {item / NRT, item % NRT}; }
+    __device__ void next(Walk& w) const { if (++w.rt == NRT) { w.rt = 0; ++w.blk; } }
     __device__ int inputs() const { return K; }
     __device__ unsigned* err() const { return a.err; }
     __device__ bool has_tile(int rt, int tl) const { return rt * 8 + tl < ntiles; }
@@ -302,7 +286,7 @@ struct ExpertWork {
 };
 
 // ================================================================================ the kernel
-// ST: stages (even); U: stages' fragments a dequant warp has in flight (K / 256 is a multiple of it)
+// ST: stages (even, at least 4); U: stages whose weights a dequant warp has in flight
 // TMEM columns: [2][NT] accumulators, [ST][64] A operands
 // STALL: a test's form, in which no row is ever loaded, so that every wait runs out, and soon
 template <class W, int NT, int ST, int U, bool STALL>
@@ -310,7 +294,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];             // ST stages x [2 groups][NT rows x 128 B]
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // tiles start on 1024-byte boundaries
     constexpr int TILE = NT * 128, STAGE = 2 * TILE, LIMIT = STALL ? 1 << 10 : 1 << 22;
-    static_assert(2 * NT + ST * 64 <= 512 && ST % 2 == 0, "tensor memory");
+    static_assert(2 * NT + ST * 64 <= 512 && ST >= 4 && ST % 2 == 0, "tensor memory");
     __shared__ __align__(8) uint64_t s_full[ST], s_empty[ST], s_acc_full[2], s_acc_empty[2];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
@@ -318,7 +302,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // (the shuffle tells the compiler that it is uniform)
     if (tid == 0) {
         s_abort = 0;
-        for (int i = 0; i < ST; ++i) { mbar_init(&s_full[i], TC_DQ / 2 + TC_LD * 32); mbar_init(&s_empty[i], 1); }
+        for (int i = 0; i < ST; ++i) { mbar_init(&s_full[i], TC_DQ / 4 + TC_LD * 32); mbar_init(&s_empty[i], 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(&s_acc_full[i], 1); mbar_init(&s_acc_empty[i], TC_EPI); }
         mbar_fence_init();
     }
@@ -332,9 +316,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     tc_fence_after();
     pdl_launch_dependents();
     const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
-    const int items = work.items(), KS = work.inputs() >> 7, NRT = work.NRT;              // KS: stages per item (even)
+    const int items = work.items(), KS = work.inputs() >> 7;              // KS: stages per item (even)
     const int lo = (int)((long)items * blockIdx.x / gridDim.x), hi = (int)((long)items * (blockIdx.x + 1) / gridDim.x);
-    const int blk0 = lo / NRT, rt0 = lo - blk0 * NRT;
     bool ok = true;
     if (warp == 0) {
         // ------------------------------------------------------------ mma
@@ -367,50 +350,60 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
             ok = tc_agree(ok);
         }
     } else if (warp >= TC_DQ0 && warp < TC_DQ0 + TC_DQ) {
-        // ------------------------------------------------------------ dequant: tile tl of every item, stages par, par + 2, ...
-        // (a warp reaches the TMEM lanes 32 * (warp % 4) ..: two tiles)
-        const int d = warp - TC_DQ0, par = d >> 3, half = (d >> 2) & 1, tl = (d & 3) * 2 + half, r = lane >> 2;
-        const TcQuad quad = tc_quad(lane & 3);
-        const uint32_t ta = tmem + 2 * NT + ((uint32_t)((d & 3) * 32 + half * 16) << 16);
-        uint4 w0[U], w1[U], sv[U];
-        int f_left = hi - lo, f_s = 0;                                      // the fetch cursor (f_s counts this warp's stages of an item)
-        TcTile ft = f_left > 0 ? work.tile(blk0, rt0, tl) : TcTile{nullptr, nullptr, 0, 0};
-        auto fetch = [&](uint4& a0, uint4& a1, uint4& sc) {
-            if (ft.w) {
-                const uint4* p = ft.w + f_s * 128 + par * 64 + lane;
-                a0 = ldg_nc_u4(p); a1 = ldg_nc_u4(p + 32);
-                sc = ldg_nc_u4(ft.s + f_s * 16 + par * 8 + r);
-            }
-            if (++f_s == KS >> 1) {
-                f_s = 0;
-                if (--f_left <= 0) ft.w = nullptr;
-                else if (ft.rt + 1 == NRT) ft = work.tile(ft.blk + 1, 0, tl);
-                else if (ft.w && work.has_tile(ft.rt + 1, tl)) { ft.w += KS * 512; ft.s += KS * 64; ++ft.rt; }      // eight tiles on
-                else { ft.w = nullptr; ++ft.rt; }
+        // ------------------------------------------------------------ dequant: 32 rows of the item (two tiles), every fourth stage
+        // (a warp reaches the TMEM lanes 32 * (warp % 4) ..).  Stages are counted through the run: an item of two stages leaves
+        // two of the four warps of a quarter without one.
+        const int d = warp - TC_DQ0, quarter = d & 3, tl = quarter * 2 + (lane >> 4), row = lane & 15;
+        const uint32_t ta = tmem + 2 * NT + ((uint32_t)(quarter * 32) << 16);
+        uint2 wv[U][8]; uint32_t sv[U][2];                                  // [stage in flight][group, two words], (scale, bias)
+        int f_k = 0, f_s = d >> 2;                                          // the fetch cursor: item of the run, stage of it
+        typename W::Walk fw = work.walk(lo);
+        TcTile ft = hi > lo ? work.tile(fw.blk, fw.rt, tl) : TcTile{nullptr, nullptr, 0, 0};
+        auto seek = [&] {                                                   // past the end of an item: on to the one that has stage f_s
+            while (f_s >= KS) {
+                f_s -= KS;
+                if (++f_k >= hi - lo) { ft.w = nullptr; f_s = 0; return; }
+                work.next(fw);
+                if (ft.w && fw.blk == ft.blk && fw.rt == ft.rt + 1 && work.has_tile(fw.rt, tl)) { ft.w += KS * 512; ft.s += KS * 64; ++ft.rt; }      // eight tiles on
+                else ft = work.tile(fw.blk, fw.rt, tl);
             }
         };
+        seek();
+        auto fetch = [&](uint2 w[8], uint32_t sc[2]) {
+            if (ft.w) {
+                const uint2* p = reinterpret_cast<const uint2*>(ft.w + f_s * 64 + (row & 7) * 4) + (row >> 3);
 #pragma unroll
-        for (int u = 0; u < U; ++u) fetch(w0[u], w1[u], sv[u]);
-        int st = par, rt = rt0; uint32_t ph = 1;                            // parity of the stage's "empty" (a fresh barrier passes at 1)
-        for (int k = 0; k < hi - lo && ok; ++k) {
-            const bool valid = work.has_tile(rt, tl);
-            if (++rt == NRT) rt = 0;
-#pragma unroll 1
-            for (int s = 0; s < KS >> 1; s += U) {
+                for (int i = 0; i < 8; ++i) w[i] = __ldg(p + (i >> 2) * 64 + (i & 3) * 2);
+                const uint32_t* q = reinterpret_cast<const uint32_t*>(ft.s + f_s * 8 + (row & 7)) + (row >> 3);
+                sc[0] = __ldg(q); sc[1] = __ldg(q + 2);
+            }
+            if (f_k < hi - lo) { f_s += 4; seek(); }
+        };
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
+        for (int u = 0; u < U; ++u) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) wv[u][i] = make_uint2(0, 0);        // (rows the matrix does not have)
+            sv[u][0] = 0; sv[u][1] = 0;
+            fetch(wv[u], sv[u]);
+        }
+        const int total = (hi - lo) * KS;                                   // stages of the run
+        int n = d >> 2, st = n;
+        uint32_t ph = 1;                                                    // parity of the stage's "empty" (a fresh barrier passes at 1)
+        while (n < total && ok) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (n < total) {
                     ok = tc_wait<LIMIT>(&s_empty[st], ph, &s_abort) && ok;
-                    if (valid) {                                            // (of a tile the matrix does not have the outputs are not stored)
-                        tc_fence_after();
-                        tc_group_A(quad, w0[u], sv[u].x, sv[u].y, ta + st * 64);
-                        tc_group_A(quad, w1[u], sv[u].z, sv[u].w, ta + st * 64 + 32);
-                    }
-                    fetch(w0[u], w1[u], sv[u]);
+                    tc_fence_after();                                       // (rows the matrix does not have are expanded too: their outputs are not stored)
+                    tc_group_A(wv[u], sv[u][0], ta + st * 64);
+                    tc_group_A(wv[u] + 4, sv[u][1], ta + st * 64 + 32);
+                    fetch(wv[u], sv[u]);
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) tc_arrive(&s_full[st]);
-                    st += 2; if (st >= ST) { st -= ST; ph ^= 1u; }
+                    n += 4;
+                    st += 4; if (st >= ST) { st -= ST; ph ^= 1u; }
                 }
             }
             ok = tc_agree(ok);
@@ -427,8 +420,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         const __half* base = work.base() + chunk * 8;
         typename W::Place src[W::STRIDED ? 1 : NP];                         // row places (strided: of the first row)
         int st = 0; uint32_t ph = 1;
-        int blk = blk0, rt = rt0, held = -1, have = 0;                      // held: the block whose row places are in src; have: its rows (strided)
+        typename W::Walk at = work.walk(lo);
+        int held = -1, have = 0;                                            // held: the block whose row places are in src; have: its rows (strided)
         for (int k = 0; k < hi - lo && ok && !STALL; ++k) {
+            const int blk = at.blk;
             if (blk != held) {
                 held = blk;
                 if (W::STRIDED) {
@@ -439,7 +434,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
                     for (int h = 0; h < NP; ++h) src[W::STRIDED ? 0 : h] = work.row(blk, n0 + 16 * h);
                 }
             }
-            if (++rt == NRT) { rt = 0; ++blk; }
+            work.next(at);
 #pragma unroll 1
             for (int s = 0; s < KS; ++s) {
                 ok = tc_wait<LIMIT>(&s_empty[st], ph, &s_abort) && ok;
@@ -472,17 +467,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         pdl_wait();                                                         // (residual rows, and rows that the kernel before may still read)
         typename W::Epi epi;
         const int quarter = warp - TC_EPI0;
-        int blk = blk0, rt = rt0;
+        typename W::Walk at = work.walk(lo);
         for (int k = 0; k < hi - lo && ok; ++k) {
-            work.begin(epi, blk, quarter, lane);
+            work.begin(epi, at.blk, quarter, lane);
             ok = tc_agree(tc_wait<LIMIT>(&s_acc_full[k & 1], (uint32_t)((k >> 1) & 1), &s_abort));
             tc_fence_after();
-            if (ok) work.epilogue(epi, blk, rt, quarter, lane, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((k & 1) * NT), [&] {
+            if (ok) work.epilogue(epi, at.blk, at.rt, quarter, lane, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((k & 1) * NT), [&] {
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) tc_arrive(&s_acc_empty[k & 1]);
             });
-            if (++rt == NRT) { rt = 0; ++blk; }
+            work.next(at);
         }
     }
     if (!ok) {                                 // MMAs of this CTA may still be running: outlast them before TMEM is given back
@@ -494,6 +489,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512u) : "memory");
 }
+constexpr int TC_U = 2;
 template <class W, int NT, int ST, int U, bool STALL = false>
 static int launch_tc_t(const typename W::Args& a, int grid, cudaStream_t st, bool pdl) {
     constexpr size_t smem = (size_t)ST * NT * 256 + 1024;
@@ -508,8 +504,7 @@ static int launch_tc_t(const typename W::Args& a, int grid, cudaStream_t st, boo
 template <int NT, int ST>
 static int launch_gemm_tc_t(const GemmTcArgs& a, cudaStream_t st, bool pdl) {
     const int items = ((a.N + TC_ROWS - 1) / TC_ROWS) * ((a.M + NT - 1) / NT), grid = items < sm_count() ? items : sm_count();
-    if (a.K % 512 == 0) return launch_tc_t<DenseWork<NT>, NT, ST, 2>(a, grid, st, pdl);
-    return launch_tc_t<DenseWork<NT>, NT, ST, 1>(a, grid, st, pdl);
+    return launch_tc_t<DenseWork<NT>, NT, ST, TC_U>(a, grid, st, pdl);
 }
 int launch_gemm_tc(const Q4R& q, int N, int K, int M, const __half* x, int ldx, __half* y, int ldy, bool add_to_y, unsigned* err, cudaStream_t st, bool pdl) {
     if (N % 16 || K % 256) return -1;
@@ -537,9 +532,8 @@ static bool launch_expert_tc_t(const ExpertArgs& a, cudaStream_t st, bool pdl) {
     int rc = 0;
     profile_launch(DOWN ? "k_expert_umma_down" : "k_expert_umma_gateup", st, [&] {
         if constexpr (!DOWN)
-            if (a.stall) return rc = launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, 1, true>(a, sm_count(), st, pdl);
-        rc = K % 512 == 0 ? launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, 2>(a, sm_count(), st, pdl) : launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, 1>(a, sm_count(), st, pdl);
-        return rc;
+            if (a.stall) return rc = launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, TC_U, true>(a, sm_count(), st, pdl);
+        return rc = launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, TC_U>(a, sm_count(), st, pdl);
     });
     return rc == 0;
 }

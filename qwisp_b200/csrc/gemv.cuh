@@ -7,15 +7,17 @@
 // B200 formulation.  HBM-bound; the work per weight nibble on the SM must stay small, and it is
 // the integer/logic pipe (half rate) that saturates first:
 //   * nibbles become exact fp16 integers in registers with one logic op per PAIR of weights:
-//     (w & 0x000F000F) | 0x64006400 is the fp16x2 {1024+q0, 1024+q4}, (w & 0x00F000F0) | 0x64006400
-//     is {1024+16*q1, 1024+16*q5}; the same two masks on w >> 8 give q2,q6 and q3,q7.  One fp16x2
+//     (w & 0x000F000F) | 0x64006400 is the fp16x2 {1024+q0, 1024+q1} of a repacked word, (w & 0x00F000F0) |
+//     0x64006400 is {1024+16*q4, 1024+16*q5}; the same two masks on w >> 8 give q2,q3 and q6,q7.  One fp16x2
 //     subtract (or multiply-add with 1/16, -64) per register removes offset and factor exactly;
 //     that runs on the FMA pipe, which has room.  (An fp8 e4m3 operand path was timed first and is slower.)
 //   * mma.sync m16n8k16 f16 x f16 -> f32: 16 weight rows x 16 inputs per instruction, the eight
 //     columns are eight activation rows, so one pass serves up to 8 rows.  Products are exact
 //     (4-bit integer x fp16), accumulation is f32;
-//   * the pairing (q_i, q_{i+4}) is matched by storing each 8 activations in shared memory in the
-//     order 0,4,1,5,2,6,3,7, so one 128-bit shared load is the B operand of two instructions;
+//   * every 8 activations are stored in shared memory in the order 0,1,4,5,2,3,6,7 (the middle words of a 128-bit store
+//     exchanged), so one 128-bit shared load is the B operand of two instructions: the first takes inputs 0, 1, 4, 5, the
+//     second 2, 3, 6, 7.  (Which inputs meet in an instruction decides the bits of the sum, their order inside it does not:
+//     the tensor cores add a step's 16 products as one sum, on mma.sync and on tcgen05 alike.)
 //   * per group of 64 inputs: acc += scale * C + bias * sum(x): two FMAs per group and output
 //     instead of per element (the algebra the reference uses, SeedlessMetalForward.swift:249-258);
 //   * a warp owns 16 weight rows x 256 inputs (one "slice" = 4 groups); weights are read in the
@@ -36,7 +38,7 @@ enum { EPI_STORE = 0, EPI_RESID = 1, EPI_SWIGLU = 2, EPI_ARGMAX = 3 };
 constexpr int ROWS_PER_PASS = 8;     // activation rows per MMA pass (the 8 columns of m16n8k16)
 
 struct XStage {
-    __half* xs;          // [rows][stride] fp16, every 8 consecutive inputs stored as 0,4,1,5,2,6,3,7
+    __half* xs;          // [rows][stride] fp16, every 8 consecutive inputs stored as 0,1,4,5,2,3,6,7
     float* sxs;          // [K/64][8] per-group sums of x (bias term)
     float* part;         // [8][16] scratch for the rmsnorm prologue
     int stride;          // K + 8 (halves) between rows: 16 bytes of skew keeps the B loads conflict-free
@@ -53,23 +55,18 @@ __device__ __forceinline__ float sum8_f32(uint4 v) {
     return h2f(a) + h2f(b);
 }
 // lane holds 8 consecutive activations of pass-row `col` starting at k0 (multiple of 8): write
-// them in the paired order and accumulate the group sum (8 consecutive lanes cover one group of 64)
+// them in that order and accumulate the group sum (8 consecutive lanes cover one group of 64)
 __device__ __forceinline__ void store_staged(const XStage& st, int col, int k0, uint4 v, int lane) {
     float s = sum8_f32(v);
     s += __shfl_xor_sync(0xffffffffu, s, 4);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     if ((lane & 7) == 0) st.sxs[(k0 >> 6) * 8 + col] = s;
-    uint4 o;
-    o.x = __byte_perm(v.x, v.z, 0x5410);       // (x0, x4)
-    o.y = __byte_perm(v.x, v.z, 0x7632);       // (x1, x5)
-    o.z = __byte_perm(v.y, v.w, 0x5410);       // (x2, x6)
-    o.w = __byte_perm(v.y, v.w, 0x7632);       // (x3, x7)
-    *reinterpret_cast<uint4*>(st.xs + (size_t)col * st.stride + k0) = o;
+    *reinterpret_cast<uint4*>(st.xs + (size_t)col * st.stride + k0) = make_uint4(v.x, v.z, v.y, v.w);
 }
 
-// The same for the many-row kernels, whose prepared rows live in global memory ([M][K] paired order, [M][K/64] sums):
-// lane holds the 8 prologue'd activations (row, k0 .. k0+7): paired-order store + group sum (8 lanes = one group),
+// The same for the many-row kernels, whose prepared rows live in global memory ([M][K] in the same order, [M][K/64] sums):
+// lane holds the 8 prologue'd activations (row, k0 .. k0+7): store + group sum (8 lanes = one group),
 // the arithmetic of store_staged()
 __device__ __forceinline__ void rows_store(__half* xq_row, float* sx_row, int k0, uint4 v, int lane) {
     float s = sum8_f32(v);
@@ -77,12 +74,7 @@ __device__ __forceinline__ void rows_store(__half* xq_row, float* sx_row, int k0
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     if ((lane & 7) == 0) sx_row[k0 >> 6] = s;
-    uint4 o;
-    o.x = __byte_perm(v.x, v.z, 0x5410);
-    o.y = __byte_perm(v.x, v.z, 0x7632);
-    o.z = __byte_perm(v.y, v.w, 0x5410);
-    o.w = __byte_perm(v.y, v.w, 0x7632);
-    *reinterpret_cast<uint4*>(xq_row + k0) = o;
+    *reinterpret_cast<uint4*>(xq_row + k0) = make_uint4(v.x, v.z, v.y, v.w);
 }
 // ---- prologues: stage `mr` (<= ROWS_PER_PASS) activation rows of width K ----
 // A warp owns 256-wide chunks (unit u = row * chunks + chunk, units u = warp, warp + nw, ...).
@@ -290,11 +282,13 @@ __device__ __forceinline__ void prefetch_ranges(const PfList& pf, int cta, int n
 // A tile is 16 weight rows: A_0..A_7 and B_0..B_7 (for a dense matrix rows 16T..16T+7 and 16T+8..16T+15;
 // for the fused gate/up projection 8 gate rows and the 8 up rows of the same outputs).  K = 64*G
 // groups, taken in pairs (GP = G/2).  For tile T and group pair gp:
-//   Wr: uint4 [T][gp][2 groups][32 lanes]   lane (r = lane/4, t = lane%4), group g = 2gp+gi:
-//         { A_r word 8g+2t, A_r word 8g+2t+1, B_r word 8g+2t, B_r word 8g+2t+1 }   (word = 8 nibbles of the MLX layout)
-//   Sr: uint4 [T][gp][8 rows r]             fp16 { sA(g0), bA(g0), sB(g0), bB(g0), sA(g1), bA(g1), sB(g1), bB(g1) }
-// so a warp's loads are 512 contiguous bytes of nibbles per group and 128 bytes of scales per pair,
-// each lane exactly the 16 inputs x 2 rows its tensor-core fragments need.  Same 0.5625 B/weight.
+//   Wr: uint4 [T][gp][2 groups][32 lanes]     lane (r = lane/4, t = lane%4), group g = 2gp+gi:
+//         { A_r word 8g+2t, A_r word 8g+2t+1, B_r word 8g+2t, B_r word 8g+2t+1 }.  A word holds 8 inputs x0..x7: x0, x4, x2, x6 in
+//         its low half, x1, x5, x3, x7 in its high half (lowest nibble first), so that one mask gives a pair of neighbours
+//   Sr: uint4 [T][gp][8 rows r]               fp16 { sA(g0), bA(g0), sB(g0), bB(g0), sA(g1), bA(g1), sB(g1), bB(g1) }
+// Two readers share it.  The mma.sync kernels take a lane's 16 bytes as they are: the 16 inputs x 2 rows that its fragments
+// need.  The tcgen05 kernels want a lane per row, because a lane of tensor memory is a row: it takes its 8 bytes of four
+// pieces, and the first level cache serves the other halves of their sectors.  Same 0.5625 B/weight.
 struct Q4R { const uint4* wr = nullptr; const uint4* sr = nullptr; int tiles = 0; int K = 0; };
 
 __host__ __device__ inline size_t q4r_w_uint4(int K) { return (size_t)(K / 128) * 64; }   // per tile
@@ -334,7 +328,7 @@ __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
     asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
-// one word (8 nibbles q0..q7) -> fp16x2 registers {q0,q4}, {q1,q5}, {q2,q6}, {q3,q7}, exact
+// one repacked word (inputs x0..x7) -> fp16x2 registers {q0,q1}, {q4,q5}, {q2,q3}, {q6,q7}, exact
 __device__ __forceinline__ void dequant8(uint32_t w, uint32_t d[4]) {
     const uint32_t w8 = w >> 8;
     const uint32_t mlo = 0x000F000Fu, mhi = 0x00F000F0u, magic = 0x64006400u;

@@ -476,7 +476,7 @@ void launch_embed(const __half* embed, const int* tokens, int M, int H, int voca
 }
 
 // block-wide rmsnorm of one row of width H (multiple of 256, <= 4096) with 256 threads
-// xq_row / sx_row (optional): the normed row also in the prepared form of the many-row kernels (paired order + group sums)
+// xq_row / sx_row (optional): the normed row also in the prepared form of the many-row kernels (products' order + group sums)
 __device__ __forceinline__ void block_rmsnorm_row(const __half* src, const __half* w, float eps, int H, __half* dst, float* sm8,
                                                   bool pre = false, uint4 pv = make_uint4(0, 0, 0, 0), uint4 pw = make_uint4(0, 0, 0, 0),
                                                   __half* xq_row = nullptr, float* sx_row = nullptr) {

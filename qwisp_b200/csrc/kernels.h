@@ -100,8 +100,8 @@ struct ExpertArgs {
     int ep_pairs_per_rank = 0;
     EpSignal ep_sig;                     // down kernel: its last CTA raises the combine flags
     PfList pf;                           // static prefetch (gate/up kernel: next layer's in-projection)
-    // many-row kernels: the normed rows in paired order + their group sums (gate/up input), and the chunk sums of the
-    // SwiGLU rows ([(M*topk + M)][I/8], written by gate/up, read by down; hbuf is then in paired order too)
+    // many-row kernels: the normed rows in the products' order (gemv.cuh) + their group sums (gate/up input), and the chunk sums of the
+    // SwiGLU rows ([(M*topk + M)][I/8], written by gate/up, read by down; hbuf is then in that order too)
     const __half* xq = nullptr; const float* sxq = nullptr; float* csum = nullptr;
     bool stall = false;                  // test hook: the gate/up kernel in the form whose waits run out
 };

@@ -9,8 +9,8 @@
 //   - scale * sum and bias * (sum of the group's activations) accumulated over the 4 groups of a 256-input slice;
 //   - slice values added in ascending order starting from 0.
 //
-//   k_rows_prep      the prologue (plain / RMSNorm / gated RMSNorm) of every row, written once per call: activations in the
-//                    paired order the dequantiser produces (0,4,1,5,2,6,3,7 inside every 8) + the per-group sums.
+//   k_rows_prep      the prologue (plain / RMSNorm / gated RMSNorm) of every row, written once per call: the
+//                    activations in the products' order (0,1,4,5,2,3,6,7 inside every 8) + the per-group sums.
 //   k_gemv_rows      dense projection: a CTA holds a block of 8, 16 or 32 rows over the whole K, its warps stream tiles of 16
 //                    weight rows through rings of their own (k_gemv_rows_split: short runs, shared out by slices).
 //   k_head_rows      lm_head + argmax in the same form.
@@ -29,7 +29,7 @@ struct RowsPrepArgs {
     const __half* nw; const float* nw32; // norm weight
     const __half* z; int ldz;            // gate input of the gated norm
     float eps; int K;
-    __half* xq; float* sxq;              // out: [M][K] paired order, [M][K/64]
+    __half* xq; float* sxq;              // out: [M][K] in the products' order, [M][K/64]
 };
 // grid (M), K/256 warps: warp = one 256-input chunk of the row (the unit of stage_finish())
 template <int PRO>
@@ -111,7 +111,7 @@ __device__ __forceinline__ void ring_request(unsigned char* slot, const uint4* w
     if (lane < 16) cp_async16(d + 128 + lane, sc + s * 16 + lane);
 }
 // One slice (4 groups of 64 inputs) of a 16-row tile, in a ring slot, against 8*RG staged rows.
-// xp: the slice's activations of this lane's row of group 0 (row r, paired order, + 16 t), rows xstride halves apart; sxp: the
+// xp: the slice's activations of this lane's row of group 0 (row r, + 16 t), rows xstride halves apart; sxp: the
 // group sums [group][row] of the slice, at column 2t, groups sxstride floats apart.  acc[q]: (row A, col 2t), (A, 2t+1),
 // (B, 2t), (B, 2t+1) of row group q.  The order of operations per column is that of compute_slice_x().
 template <int RG>
@@ -702,7 +702,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
             }
         } else {
             // SwiGLU of (gate row r, up row r) per column; the 8 outputs of a column (lanes with the same t) form one
-            // 8-chunk of the down projection's input: stored in the paired order with its chunk sum
+            // 8-chunk of the down projection's input: stored in the products' order with its chunk sum
 #pragma unroll
             for (int jc = 0; jc < 2; ++jc) {
                 const __half hv = swiglu_h(f2h(tot[0][jc]), f2h(tot[0][2 + jc]));
@@ -713,8 +713,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
                 const int dst = b.dst[2 * t + jc];
                 if (r == 0 && dst >= 0) {
                     const uint4 nat = make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
-                    const uint4 prd = make_uint4(v[0] | (v[4] << 16), v[1] | (v[5] << 16), v[2] | (v[6] << 16), v[3] | (v[7] << 16));
-                    *reinterpret_cast<uint4*>(a.hbuf + (size_t)dst * a.I + tile * 8) = prd;
+                    *reinterpret_cast<uint4*>(a.hbuf + (size_t)dst * a.I + tile * 8) = make_uint4(nat.x, nat.z, nat.y, nat.w);
                     a.csum[(size_t)dst * (a.I / 8) + tile] = sum8_f32(nat);
                 }
             }

@@ -48,7 +48,7 @@ constexpr int PS_RED_UNITS = 64;
 constexpr int PS_OFF_RING = 0;
 constexpr int PS_OFF_FULL = PS_OFF_RING + PS_NS * PS_SLOT;
 constexpr int PS_OFF_EMPTY = PS_OFF_FULL + PS_NS * 8;
-constexpr int PS_OFF_XS = PS_OFF_EMPTY + PS_NS * 8;            // activation stage (paired order) + group sums; 12 KB
+constexpr int PS_OFF_XS = PS_OFF_EMPTY + PS_NS * 8;            // activation stage + group sums; 12 KB
 constexpr int PS_XS_BYTES = 12288;
 constexpr int PS_OFF_PPLAIN = PS_OFF_XS + PS_XS_BYTES;         // normed post-attention row, plain order (router dots); 8 KB with the next
 constexpr int PS_OFF_HMID = PS_OFF_PPLAIN + 4096 * 2 / 2;      // residual stream after the mixer (combine)

@@ -125,6 +125,16 @@ void launch_quantize_q4(const __half* w, int64_t N, int64_t K, uint32_t* packed,
     k_quantize_q4<<<grid_for(ng, 128), 128, 0, st>>>(w, ng, packed, s, b);
 }
 // ---- MLX affine layout -> fragment-major layout (see gemv.cuh) ----
+// nibbles 0, 4, 2, 6 of a word into its low half, 1, 5, 3, 7 into its high half
+__device__ __forceinline__ uint32_t neighbours(uint32_t w) {
+    uint32_t o = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int at = 4 * (i == 1 ? 2 : i == 2 ? 1 : i);                   // inputs 2i and 2i + 1
+        o |= ((w >> (8 * i)) & 0xFu) << at | ((w >> (8 * i + 4)) & 0xFu) << (at + 16);
+    }
+    return o;
+}
 __global__ void k_repack_q4(const uint32_t* wA, const __half* sA, const __half* bA, const uint32_t* wB, const __half* sB, const __half* bB,
                             int pair, int64_t tiles, int K, uint4* wr, uint4* sr) {
     const int GP = K / 128, K8 = K / 8, KG = K / 64;
@@ -138,7 +148,7 @@ __global__ void k_repack_q4(const uint32_t* wA, const __half* sA, const __half* 
             int word = 8 * (2 * gp + gi) + 2 * t;
             int64_t rowA = pair ? 8 * T + r : 16 * T + r, rowB = pair ? 8 * T + r : 16 * T + 8 + r;
             const uint32_t* srcB = pair ? wB : wA;
-            wr[i] = make_uint4(wA[rowA * K8 + word], wA[rowA * K8 + word + 1], srcB[rowB * K8 + word], srcB[rowB * K8 + word + 1]);
+            wr[i] = make_uint4(neighbours(wA[rowA * K8 + word]), neighbours(wA[rowA * K8 + word + 1]), neighbours(srcB[rowB * K8 + word]), neighbours(srcB[rowB * K8 + word + 1]));
         } else {
             int64_t j = i - total_w;
             int64_t T = j / (GP * 8); int rem = (int)(j - T * (GP * 8));

@@ -200,7 +200,7 @@ struct ExpertWork {
     struct Shared { SlotTable tab; int dst[TC_EPI][NT]; };                  // dst: a list of each epilogue warp
     const Args& a;
     Shared& sh;
-    int n_active, K, ntiles, NRT, npair, nshared;
+    int n_active, K, ntiles, NRT, npair, nshared, S, T;
     __device__ ExpertWork(const Args& args, Shared& s) : a(args), sh(s) {
         K = DOWN ? a.I : a.H;
         ntiles = DOWN ? a.H / 16 : a.I / 8;                                 // tiles of 16 weight rows per expert
@@ -210,11 +210,29 @@ struct ExpertWork {
         pdl_wait();                                                         // (the lists)
         n_active = slot_table(sh.tab, a.lists, NT, nshared);
         __syncthreads();
+        T = items(); S = T - sh.tab.base[n_active] * NRT;
     }
     __device__ int items() const { return sh.tab.base[n_active + 1] * NRT; }
-    struct Walk { int blk, rt; };
-    __device__ Walk walk(int item) const { return {item / NRT, item % NRT}; }
-    __device__ void next(Walk& w) const { if (++w.rt == NRT) { w.rt = 0; ++w.blk; } }
+    // The shared expert's items are dealt out evenly among the others (item t is one of the S of T where t * S mod T wraps):
+    // its blocks are full, a routed expert's hold few rows, and an item's epilogue is as long as its rows.  At the end of the
+    // numbering they made ten of 148 CTAs finish a third later than the rest.
+    struct Walk { int blk, rt, acc, rb, rr, sb, sr; bool sh; };
+    __device__ void place(Walk& w) const { w.sh = w.acc + S >= T; w.blk = w.sh ? w.sb : w.rb; w.rt = w.sh ? w.sr : w.rr; }
+    __device__ Walk walk(int item) const {
+        const int s = (int)((long)item * S / T), b = sh.tab.base[n_active];
+        Walk w;
+        w.acc = (int)((long)item * S - (long)s * T);
+        w.rb = (item - s) / NRT; w.rr = (item - s) - w.rb * NRT;
+        w.sb = s / NRT; w.sr = s - w.sb * NRT; w.sb += b;
+        place(w);
+        return w;
+    }
+    __device__ void next(Walk& w) const {
+        if (w.sh) { if (++w.sr == NRT) { w.sr = 0; ++w.sb; } }
+        else if (++w.rr == NRT) { w.rr = 0; ++w.rb; }
+        w.acc += S - (w.sh ? T : 0);
+        place(w);
+    }
     __device__ int inputs() const { return K; }
     __device__ unsigned* err() const { return a.err; }
     __device__ bool has_tile(int rt, int tl) const { return rt * 8 + tl < ntiles; }
@@ -331,8 +349,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
             tc_fence_after();
             const uint32_t acc = tmem + (uint32_t)((k & 1) * NT);
 #pragma unroll 1
-            for (int s = 0; s < KS; ++s) {
+            for (int s = 0; s < KS; s += 2) {                               // (KS and ST are even)
                 ok = tc_wait<LIMIT>(&s_full[st], ph, &s_abort) && ok;
+                ok = tc_wait<LIMIT>(&s_full[st + 1], ph, &s_abort) && ok;
                 tc_fence_after();
                 tc_fence_proxy();                                           // the rows other threads' asynchronous copies wrote are operand data now
                 const uint64_t db = db0 + (uint32_t)(st * (STAGE >> 4));    // (the address field counts 16 bytes: a K step of 16 halves is 2)
@@ -342,10 +361,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
 #pragma unroll
                     for (int j = 1; j < 8; ++j) umma_f16_ts(acc, ta + j * 8, db + (j >> 2) * (TILE >> 4) + (j & 3) * 2, idesc, 1u);
                     umma_commit(&s_empty[st]);
-                    if (s == KS - 1) umma_commit(&s_acc_full[k & 1]);
+#pragma unroll
+                    for (int j = 8; j < 16; ++j) umma_f16_ts(acc, ta + j * 8, db + (j >> 2) * (TILE >> 4) + (j & 3) * 2, idesc, 1u);
+                    umma_commit(&s_empty[st + 1]);
+                    if (s == KS - 2) umma_commit(&s_acc_full[k & 1]);
                 }
                 __syncwarp();
-                if (++st == ST) { st = 0; ph ^= 1u; }
+                st += 2; if (st == ST) { st = 0; ph ^= 1u; }
             }
             ok = tc_agree(ok);
         }

@@ -34,18 +34,25 @@ __device__ __forceinline__ float half_warp_sum(float v) {
 __device__ __forceinline__ float h2f(__half h) { return __half2float(h); }
 __device__ __forceinline__ __half f2h(float f) { return __float2half_rn(f); }
 
-// correctly rounded fp16 arithmetic done through one f32 operation (f32 carries >= 2*11+2 bits)
-__device__ __forceinline__ __half hadd_rn(__half a, __half b) { return f2h(__fadd_rn(h2f(a), h2f(b))); }
-__device__ __forceinline__ __half hsub_rn(__half a, __half b) { return f2h(__fsub_rn(h2f(a), h2f(b))); }
-__device__ __forceinline__ __half hmul_rn(__half a, __half b) { return f2h(__fmul_rn(h2f(a), h2f(b))); }
-__device__ __forceinline__ __half hdiv_rn(__half a, __half b) { return f2h(__fdiv_rn(h2f(a), h2f(b))); }
+// correctly rounded fp16 arithmetic, never fused
+__device__ __forceinline__ __half hadd_rn(__half a, __half b) { return __hadd_rn(a, b); }
+__device__ __forceinline__ __half hsub_rn(__half a, __half b) { return __hsub_rn(a, b); }
+__device__ __forceinline__ __half hmul_rn(__half a, __half b) { return __hmul_rn(a, b); }
+__device__ __forceinline__ __half hdiv_rn(__half a, __half b) { return f2h(__fdiv_rn(h2f(a), h2f(b))); }     // (f32 carries >= 2*11+2 bits: rounding twice is rounding once)
+// 1 / a.  The last bit of the hardware's approximate reciprocal never reaches the fp16 result: equal to hdiv_rn(1, a) for every
+// half (all 65536 compared).  Without the branch of the exact form eight of them overlap.
+__device__ __forceinline__ __half hrcp_rn(__half a) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(h2f(a)));
+    return f2h(r);
+}
 
 // "stable sigmoid" in fp16 arithmetic: y = 1/(1+exp(|x|)); x<0 ? y : 1-y
 // (swift/Sources/QwispCore/SeedlessMetalForward.swift:986-988)
 __device__ __forceinline__ __half sigmoid_h(__half x) {
     const __half one = f2h(1.0f);
     __half ex = f2h(expf(fabsf(h2f(x))));
-    __half y = hdiv_rn(one, hadd_rn(one, ex));
+    __half y = hrcp_rn(hadd_rn(one, ex));
     return (h2f(x) < 0.0f) ? y : hsub_rn(one, y);
 }
 // same in f32 (SeedlessMetalForward.swift:1599-1602)

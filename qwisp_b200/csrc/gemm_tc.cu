@@ -276,17 +276,20 @@ struct ExpertWork {
         const int* dsts = sh.dst[quarter];
         const int i16 = i & 15, etile = rt * 8 + (i >> 4);
         const bool up = i16 >= 8, have = etile < ntiles;
-        __half* out = DOWN ? a.dbuf + (size_t)rt * TC_ROWS + i : a.hbuf + etile * 8 + (i16 & 7);
+        __half* out = DOWN ? a.dbuf + (size_t)rt * TC_ROWS + (i & ~1) : a.hbuf + etile * 8 + (i16 & 7);
 #pragma unroll 1
         for (int c0 = 0; c0 < e.count; c0 += 16) {
             uint32_t d[16];
             tmem_ld16(taddr + (uint32_t)c0, d);
             if (c0 + 16 >= e.count) release();
             if (DOWN) {
+                // two columns at a time: an even lane stores its row and the next of the first, an odd lane of the second
 #pragma unroll
-                for (int n = 0; n < 16; ++n) {
-                    const int dst = dsts[c0 + n];
-                    if (dst >= 0 && have) out[(size_t)dst * a.H] = f2h(__uint_as_float(d[n]));
+                for (int n = 0; n < 16; n += 2) {
+                    const __half2 h = __floats2half2_rn(__uint_as_float(d[n]), __uint_as_float(d[n + 1]));
+                    const uint32_t mine = *reinterpret_cast<const uint32_t*>(&h), other = __shfl_xor_sync(0xffffffffu, mine, 1);
+                    const int dst = dsts[c0 + n + (lane & 1)];
+                    if (dst >= 0 && have) *reinterpret_cast<uint32_t*>(out + (size_t)dst * a.H) = __byte_perm(mine, other, (lane & 1) ? 0x3276 : 0x5410);
                 }
             } else {
                 // two columns at a time: the gate lane finishes the first, the up lane the second; each sends what the other lacks

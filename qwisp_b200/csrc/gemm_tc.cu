@@ -197,7 +197,7 @@ struct ExpertWork {
     static constexpr bool STRIDED = false;
     using Place = uint32_t;                                                 // (an engine has at most 1024 rows: 17k pair rows of 4096)
     static constexpr Place NO_ROW = ~(Place)0;
-    struct Shared { SlotTable tab; int dst[TC_EPI][NT]; };                  // dst: a list of each epilogue warp
+    struct Shared { SlotTable tab; int dst[TC_EPI][(NT + 31) / 32 * 32]; };                  // dst: a list of each epilogue warp
     const Args& a;
     Shared& sh;
     int n_active, K, ntiles, NRT, npair, nshared, S, T;
@@ -308,14 +308,14 @@ struct ExpertWork {
 
 // ================================================================================ the kernel
 // ST: stages (even, at least 4); U: stages whose weights a dequant warp has in flight
-// TMEM columns: [2][NT] accumulators, [ST][64] A operands
+// TMEM columns: [2][ACC] accumulators, [ST][64] A operands
 // STALL: a test's form, in which no row is ever loaded, so that every wait runs out, and soon
 template <class W, int NT, int ST, int U, bool STALL>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];             // ST stages x [2 groups][NT rows x 128 B]
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // tiles start on 1024-byte boundaries
-    constexpr int TILE = NT * 128, STAGE = 2 * TILE, LIMIT = STALL ? 1 << 10 : 1 << 22;
-    static_assert(2 * NT + ST * 64 <= 512 && ST >= 4 && ST % 2 == 0, "tensor memory");
+    constexpr int TILE = NT * 128, STAGE = 2 * TILE, ACC = NT == 48 ? 64 : NT, LIMIT = STALL ? 1 << 10 : 1 << 22;
+    static_assert(2 * ACC + ST * 64 <= 512 && ST >= 4 && ST % 2 == 0, "tensor memory");
     __shared__ __align__(8) uint64_t s_full[ST], s_empty[ST], s_acc_full[2], s_acc_empty[2];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
@@ -345,12 +345,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         // The whole warp walks the stages, so that addresses and descriptors stay in uniform registers; one elected lane issues.
         const uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(TC_ROWS >> 4) << 24);   // f32 accumulate, f16 x f16, K-major B
         const uint64_t db0 = umma_desc_sw128(smem);
-        const uint32_t ta0 = tmem + 2 * NT;
+        const uint32_t ta0 = tmem + 2 * ACC;
         int st = 0; uint32_t ph = 0;
         for (int k = 0; k < hi - lo && ok; ++k) {
             if (k >= 2) ok = tc_wait<LIMIT>(&s_acc_empty[k & 1], (uint32_t)(((k >> 1) - 1) & 1), &s_abort) && ok;
             tc_fence_after();
-            const uint32_t acc = tmem + (uint32_t)((k & 1) * NT);
+            const uint32_t acc = tmem + (uint32_t)((k & 1) * ACC);
 #pragma unroll 1
             for (int s = 0; s < KS; s += 2) {                               // (KS and ST are even)
                 ok = tc_wait<LIMIT>(&s_full[st], ph, &s_abort) && ok;
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         // (a warp reaches the TMEM lanes 32 * (warp % 4) ..).  Stages are counted through the run: an item of two stages leaves
         // two of the four warps of a quarter without one.
         const int d = warp - TC_DQ0, quarter = d & 3, tl = quarter * 2 + (lane >> 4), row = lane & 15;
-        const uint32_t ta = tmem + 2 * NT + ((uint32_t)(quarter * 32) << 16);
+        const uint32_t ta = tmem + 2 * ACC + ((uint32_t)(quarter * 32) << 16);
         uint2 wv[U][8]; uint32_t sv[U][2];                                  // [stage in flight][group, two words], (scale, bias)
         int f_k = 0, f_s = d >> 2;                                          // the fetch cursor: item of the run, stage of it
         typename W::Walk fw = work.walk(lo);
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
             work.begin(epi, at.blk, quarter, lane);
             ok = tc_agree(tc_wait<LIMIT>(&s_acc_full[k & 1], (uint32_t)((k >> 1) & 1), &s_abort));
             tc_fence_after();
-            if (ok) work.epilogue(epi, at.blk, at.rt, quarter, lane, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((k & 1) * NT), [&] {
+            if (ok) work.epilogue(epi, at.blk, at.rt, quarter, lane, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((k & 1) * ACC), [&] {
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) tc_arrive(&s_acc_empty[k & 1]);
@@ -549,16 +549,24 @@ int launch_gemm_tc(const Q4R& q, int N, int K, int M, const __half* x, int ldx, 
     return launch_gemm_tc_t<32, 6>(a, st, pdl);
 }
 
-constexpr int XT_NT = 64;            // rows of an expert's block: a 1024-token chunk gives an expert about 32
+// Rows of an expert's block.  Each row beyond the block's is another expansion of the expert's weights, and each column of the
+// tile without a row costs its share of the loads and MMAs: the narrowest tile that most experts' rows fit into once.  Prompt
+// calls of the 40-layer, 256-expert geometry in ms with 32 / 48 / 64 rows a block: 129 rows (4 an expert) 8.31 / 8.52 / 8.80;
+// 512 (16) 14.2 / 14.3 / 14.7; 640 (20) 16.73 / 16.76 / 17.20; 768 (24) 18.6 / 18.4 / 18.9; 1024 (32) 23.0 / 22.2 / 22.5.
+template <bool DOWN, int NT>
+static int launch_expert_tc_n(const ExpertArgs& a, cudaStream_t st, bool pdl) {
+    if constexpr (!DOWN)
+        if (a.stall) return launch_tc_t<ExpertWork<DOWN, NT>, NT, 6, TC_U, true>(a, sm_count(), st, pdl);
+    return launch_tc_t<ExpertWork<DOWN, NT>, NT, 6, TC_U>(a, sm_count(), st, pdl);
+}
 template <bool DOWN>
 static bool launch_expert_tc_t(const ExpertArgs& a, cudaStream_t st, bool pdl) {
     const int K = DOWN ? a.I : a.H;
     if (K % 256 || a.ep_pairs_per_rank > 0) return false;              // (expert-parallel calls keep the row kernels)
     int rc = 0;
+    const int mean = a.M * a.topk / a.E, nt = mean <= 20 ? 32 : mean <= 34 ? 48 : 64;
     profile_launch(DOWN ? "k_expert_umma_down" : "k_expert_umma_gateup", st, [&] {
-        if constexpr (!DOWN)
-            if (a.stall) return rc = launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, TC_U, true>(a, sm_count(), st, pdl);
-        return rc = launch_tc_t<ExpertWork<DOWN, XT_NT>, XT_NT, 6, TC_U>(a, sm_count(), st, pdl);
+        return rc = nt == 32 ? launch_expert_tc_n<DOWN, 32>(a, st, pdl) : nt == 48 ? launch_expert_tc_n<DOWN, 48>(a, st, pdl) : launch_expert_tc_n<DOWN, 64>(a, st, pdl);
     });
     return rc == 0;
 }

@@ -104,6 +104,18 @@ def test_tensor_core_tiles(M, K, N):
     check(M, K, N)
 
 
+# expert blocks of 32, 48 and 64 rows (means of 20, 21, 34, 35 rows an expert and others) in prefill mode: the same rows in one call
+@pytest.mark.parametrize("cuts", [[41, 42], [69, 70], [1, 61, 130], [300, 42]])
+def test_prefill_expert_blocks(engines, cuts):
+    e = engines[0]
+    toks = prompt(MINI["vocab"], sum(cuts), "blocks")
+    a, b = e.stream(400), e.stream(400)
+    whole = a.forward_hybrid(toks)
+    parts = np.concatenate([b.forward_hybrid(toks[sum(cuts[:i]):sum(cuts[:i + 1])]) for i in range(len(cuts))])
+    assert same(whole, parts) and np.array_equal(a.state_save(), b.state_save())
+    a.close(); b.close()
+
+
 # strict calls of every length that has a step graph, with two heads, some of them again
 def test_step_graphs_of_many_shapes():
     import qwisp_b200 as Q

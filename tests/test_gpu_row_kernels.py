@@ -116,6 +116,26 @@ def test_prefill_expert_blocks(engines, cuts):
     a.close(); b.close()
 
 
+# vocabularies of less than a strand, of a remainder in the last CTA, of many rounds, and of more logits than shared memory holds
+@pytest.mark.parametrize("vocab", [16, 1040, 20496, 431104])
+def test_sampler_vocabularies(vocab):
+    import qwisp_b200 as Q
+    from oracle import oracle as O
+    e = gpu_engine(dict(TINY, vocab=vocab, n_layers=2), max_streams=1, max_rows=4)
+    try:
+        logits = O.synth_f16(7, "vocab.logits", 3 * vocab, 0.0, 2.5).reshape(3, vocab)
+        adj = O.synth_f16(7, "vocab.adj", vocab, 0.0, 0.5).astype(np.float32)
+        logits[1, :] = logits[1, 0]                               # a tie of all
+        logits[2, vocab - 3] = np.float16(-np.inf)
+        draft = np.array([int(np.argmax(logits[0].astype(np.float32))), vocab - 1, -1], dtype=np.int32)
+        for inv_t, top_p, a in ((0.0, 1.0, None), (1.0 / 0.7, 1.0, adj), (1.0, 0.9, None), (1.0 / 0.7, 0.95, adj)):
+            got = Q.ops.sample_rows(e, logits, draft, inv_t, top_p, 5, 6, 40, logit_adj=a)
+            ref = O.sample_rows(logits, draft, inv_t, top_p, 5, 6, 40, logit_adj=a)
+            assert all(np.array_equal(g, r) for g, r in zip(got, ref)), (inv_t, top_p, got, ref)
+    finally:
+        e.close()
+
+
 # strict calls of every length that has a step graph, with two heads, some of them again
 def test_step_graphs_of_many_shapes():
     import qwisp_b200 as Q

@@ -57,7 +57,7 @@ __device__ __forceinline__ __half sigmoid_h(__half x) {
 }
 // same in f32 (SeedlessMetalForward.swift:1599-1602)
 __device__ __forceinline__ float sigmoid_f(float x) {
-    float y = __fdiv_rn(1.0f, 1.0f + expf(fabsf(x)));
+    float y = __frcp_rn(1.0f + expf(fabsf(x)));
     return (x < 0.0f) ? y : (1.0f - y);
 }
 // SwiGLU in fp16: (g*sigmoid(g))*u (SeedlessMetalForward.swift:982-990)

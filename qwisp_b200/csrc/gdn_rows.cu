@@ -19,13 +19,29 @@ namespace sl {
 constexpr int GS_REC = 144;
 __device__ __forceinline__ int gs_paired(int dk) { const int leaf = dk >> 2, e = dk & 3; return (e >> 1) * 64 + (leaf & 15) * 4 + (e & 1) * 2 + (leaf >> 4); }
 
+// The warp's sums of N values at once (N a power of two): the butterfly of warp_sum() on each, the same additions, but a lane
+// keeps only half of the values at every level -- N + 5 - log2 N shuffles instead of 5 N.  Lane l gets value l / (32 / N).
+template <int N>
+__device__ __forceinline__ float warp_sums(float v[N], int lane) {
+    int off = 16;
+#pragma unroll
+    for (int n = N / 2; n >= 1; n /= 2, off /= 2) {
+        const bool up = (lane & off) != 0;
+#pragma unroll
+        for (int i = 0; i < n; ++i) v[i] = __fadd_rn(up ? v[i + n] : v[i], __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + n], off));
+    }
+    for (; off >= 1; off /= 2) v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], off));
+    return v[0];
+}
 // grid (Hk + Hv, ceil(M / R)), 128 threads: CTAs [0, Hk) own a key head's q and k channels, CTAs [Hk, Hk + Hv) a value
 // head's v channels and gates, for R rows.  R = 8 (one segment): the four conv taps of consecutive rows overlap, so a
-// thread loads 11 values per channel for its 8 rows, all of them before it uses the first: 43 us for 967 rows, 62 with one
-// row per CTA (46k CTAs).  R = 2: of fewer rows than fill the device that way.  R = 1: rows of several segments.
+// thread loads 11 values per channel for its 8 rows, all of them before it uses the first.  R = 2: of fewer rows than fill the
+// device that way.  R = 1: rows of several segments.
+// Bound by instruction issue (72 % of the slots at 967 rows, memory at a quarter): with a butterfly per value and the two inverse
+// norms of a row formed by all 128 threads it took 41 us for 967 rows by events, with neither 27 (129 rows 13.2 -> 10.7).
 template <int R>
 __global__ void __launch_bounds__(128) k_gdn_prep(GdnArgs a) {
-    __shared__ float red_s[R][8];
+    __shared__ float red_s[2 * R][4], inv_s[2 * R];           // [2 r]: q of row r, [2 r + 1]: k
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.y * R, nr = min(R, a.M - m0);
     const SegDesc seg = a.segs[a.row_seg[m0]];                // descriptors, history, weights: ahead of the programmatic-launch wait
@@ -41,11 +57,15 @@ __global__ void __launch_bounds__(128) k_gdn_prep(GdnArgs a) {
 #pragma unroll
         for (int j = 0; j < R + 3; ++j) x[j] = j < CONV_K - 1 && t0 + j < CONV_K - 1 ? hist_in[(size_t)(t0 + j) * convDim + ch] : f2h(0.f);
     };
+    const bool inner = t0 >= CONV_K - 1 && nr == R;           // every entry is a row of the call
     auto window = [&](int ch, __half x[R + 3]) {
+        const __half* p = a.inproj + ((long)m0 - (CONV_K - 1)) * a.ld + ch;
+        if (inner) {
 #pragma unroll
-        for (int j = 0; j < R + 3; ++j) {
-            const int idx = t0 + j;
-            if (idx >= CONV_K - 1 && j < nr + 3) x[j] = a.inproj[(size_t)(seg.row0 + idx - (CONV_K - 1)) * a.ld + ch];
+            for (int j = 0; j < R + 3; ++j, p += a.ld) x[j] = *p;
+        } else {
+#pragma unroll
+            for (int j = 0; j < R + 3; ++j, p += a.ld) if (t0 + j >= CONV_K - 1 && j < nr + 3) x[j] = *p;
         }
     };
     auto conv = [&](const __half* x, float4 w) { return gdn_conv_silu(h2f(x[0]), h2f(x[1]), h2f(x[2]), h2f(x[3]), w); };
@@ -65,23 +85,23 @@ __global__ void __launch_bounds__(128) k_gdn_prep(GdnArgs a) {
         pdl_wait();
         pdl_launch_dependents();
         window(ch_q, xq); window(ch_k, xk);
-        float qc[R], kc[R];
+        float qc[R], kc[R], sq[2 * R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             qc[r] = conv(xq + r, wq); kc[r] = conv(xk + r, wk);
-            const float sq = warp_sum(qc[r] * qc[r]), sk = warp_sum(kc[r] * kc[r]);
-            if (lane == 0) { red_s[r][warp] = sq; red_s[r][4 + warp] = sk; }
+            sq[2 * r] = qc[r] * qc[r]; sq[2 * r + 1] = kc[r] * kc[r];
         }
+        const float sum = warp_sums<2 * R>(sq, lane);
+        if (lane % (16 / R) == 0) red_s[lane / (16 / R)][warp] = sum;
         __syncthreads();
-        const int at = gs_paired(tid);
+        if (tid < 2 * R) inv_s[tid] = gdn_head_inv(red_s[tid][0], red_s[tid][1], red_s[tid][2], red_s[tid][3], a.eps);
+        __syncthreads();
+        float* rec = a.qk + ((size_t)hk * a.M + m0) * 256 + gs_paired(tid);
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
+        for (int r = 0; r < R; ++r, rec += 256) {
             if (r >= nr) break;
-            const float iq = gdn_head_inv(red_s[r][0], red_s[r][1], red_s[r][2], red_s[r][3], a.eps);
-            const float ik = gdn_head_inv(red_s[r][4], red_s[r][5], red_s[r][6], red_s[r][7], a.eps);
-            float* rec = a.qk + ((size_t)hk * a.M + m0 + r) * 256;
-            rec[at] = gdn_scale_k(kc[r], ik);
-            rec[128 + at] = gdn_scale_q(qc[r], iq);
+            rec[0] = gdn_scale_k(kc[r], inv_s[2 * r + 1]);
+            rec[128] = gdn_scale_q(qc[r], inv_s[2 * r]);
         }
         if (last) { leave(ch_q, xq); leave(ch_k, xk); }
     } else {

@@ -30,7 +30,7 @@ __device__ __forceinline__ void gdn_gate(__half bh, __half ah, float A_log_h, fl
 }
 // inverse rms of a 128-wide head from the four 32-lane partial sums of squares (added left to right)
 __device__ __forceinline__ float gdn_head_inv(float r0, float r1, float r2, float r3, float eps) {
-    return __frsqrt_rn(__fadd_rn(__fdiv_rn(r0 + r1 + r2 + r3, 128.0f), eps));
+    return __frsqrt_rn(__fadd_rn(__fmul_rn(r0 + r1 + r2 + r3, 1.0f / 128.0f), eps));      // (a power of two: the quotient, exactly)
 }
 // q <- fp16(1/128) * fp16(q * inv), k <- fp16(128^-0.5) * fp16(k * inv), as f32 values of the fp16 results
 __device__ __forceinline__ float gdn_scale_q(float qc, float iq) {

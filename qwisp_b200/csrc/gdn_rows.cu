@@ -141,6 +141,8 @@ __device__ __forceinline__ void lds2(const void* p, f32x2& a, f32x2& b) { asm vo
 // has one level less, but every operand read from shared memory then serves one row instead of two and the shared-memory
 // pipe sets the time (0.225 us a token; this form 0.20: a 967-row chunk went from 319 to 197 us, a batch of 64 one-row
 // segments from 60 to 48).  The readout's sum is off the chain, see below.
+// The loop's code is a limit of its own: eight tokens a turn 196 us for 967 rows, four 187, two 189, three 183 (in chunks of 32 rows;
+// 48 rows 179); scalar multiply-adds 188 to 206, the operands' loads moved about no change.
 // 32 state rows per CTA (8 per warp), 128 CTAs per stream: one warp per SM sub-partition, which is what the 4096 rows of
 // a stream give.  grid (4, Hv, nsegs), 128 threads; k / q / v / gates of CH rows at a time by bulk copies, two buffers.
 // STALL: a test's form, in which no operands are ever fetched, so that the wait for them runs out, and soon
@@ -246,10 +248,10 @@ __global__ void __launch_bounds__(128) k_gdn_scan(GdnArgs a) {
         int r = 0;
 #pragma unroll 1
         while (r < n) {
-            if (CH >= 8 && behind == 2 && r + 8 <= n) {       // eight tokens at a time: constant offsets, one branch
+            if (CH >= 3 && behind == 2 && r + 3 <= n) {       // three tokens at a time: constant offsets, one branch
 #pragma unroll
-                for (int u = 0; u < 8; ++u) token(kq + u * 1024, vg + u * GS_REC, k, g2, beta, true);
-                r += 8; kq += 8 * 1024; vg += 8 * GS_REC;
+                for (int u = 0; u < 3; ++u) token(kq + u * 1024, vg + u * GS_REC, k, g2, beta, true);
+                r += 3; kq += 3 * 1024; vg += 3 * GS_REC;
             } else {
                 token(kq, vg, k, g2, beta, behind == 2);
                 behind += behind < 2; ++r; kq += 1024; vg += GS_REC;
@@ -288,6 +290,7 @@ __global__ void __launch_bounds__(128) k_gdn_scan(GdnArgs a) {
 size_t gdn_qk_floats(int Hk, int rows) { return (size_t)Hk * rows * 256; }
 size_t gdn_vg_bytes(int Hv, int rows) { return (size_t)Hv * 4 * rows * GS_REC; }
 
+constexpr int GS_CH = 48;             // rows a chunk: a multiple of the three tokens of a turn
 template <int CH, bool STALL = false>
 static void launch_scan_t(const GdnArgs& a, int nsegs, cudaStream_t st) {
     const size_t smem = (size_t)2 * CH * (1024 + GS_REC) + 256;     // (the last token reads one record of gates past its own)
@@ -308,8 +311,8 @@ void launch_gdn_rows(const GdnArgs& in, int M, int nsegs, cudaStream_t st, bool 
     // several to one, and 17 rows took 7 us longer)
     // one row per segment (batched decode): the state's traffic is the time, small buffers leave room for more CTAs per SM
     if (M == nsegs) launch_scan_t<1>(a, nsegs, st);
-    else if (a.stall) launch_scan_t<32, true>(a, nsegs, st);
-    else launch_scan_t<32>(a, nsegs, st);
+    else if (a.stall) launch_scan_t<GS_CH, true>(a, nsegs, st);
+    else launch_scan_t<GS_CH>(a, nsegs, st);
 }
 
 }  // namespace sl

@@ -72,6 +72,20 @@ def test_rows_of_one_stream(engines, base, M):
     assert same(la, lb) and np.array_equal(ta, tb) and np.array_equal(ba, bb)
 
 
+# chunks of the state scan: a chunk less or more one row, remainders of its turns, behind a history
+@pytest.mark.parametrize("M", [3, 5, 47, 48, 49, 50, 97, 145])
+def test_state_scan_chunks(engines, M):
+    V = MINI["vocab"]
+    toks = prompt(V, 5 + M, f"scan.{M}")
+    out = []
+    for e in engines:
+        s = e.stream(M + 8)
+        s.forward(toks[:5], want_hidden=False)
+        out.append((s.forward(toks[5:]), s.state_save()))
+        s.close()
+    assert same(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
 # streams of very different lengths in one step: the one-row form of the state update, the two-kernel form, one wave of attention and more
 @pytest.mark.parametrize("B", [2, 5, 6, 9, 17, 23])
 def test_batches_of_ragged_streams(engines, B):

@@ -27,11 +27,11 @@ __device__ __forceinline__ void ap_cp16(void* dst, const void* src) {
 __device__ __forceinline__ void ap_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void ap_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void ldsm_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(smem_u32(p)));
+__device__ __forceinline__ void ldsm_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, uint32_t p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(p));
 }
-__device__ __forceinline__ void ldsm_x4_t(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(smem_u32(p)));
+__device__ __forceinline__ void ldsm_x4_t(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, uint32_t p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(p));
 }
 __device__ __forceinline__ void ap_mma(float c[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
@@ -44,13 +44,16 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// grid (ceil(M / 64), NH), 128 threads; dynamic shared memory: Q 32 KB + 2 x (K 16 KB + V 16 KB)
-__global__ void __launch_bounds__(128) k_attn_prefill(AttnArgs a) {
+// grid (ceil(M / 64) * NH), 128 threads; dynamic shared memory: Q 32 KB + 2 x (K 16 KB + V 16 KB).
+// `wave`: CTAs that get a multiprocessor for themselves at first; they take the longest blocks, the longest first, and those that
+// join them the shortest, the shortest first (with the rows in order, calls of a 2900-token prompt took 166 us by events, so 149).
+__global__ void __launch_bounds__(128) k_attn_prefill(AttnArgs a, int wave) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __half* Qs = reinterpret_cast<__half*>(smem_raw);                       // [64][256]
     __half* KVs = Qs + AP_BM * ATT_D;                                        // [2][K: 32 x 256 | V: 32 x 256]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * AP_BM, h = blockIdx.y, kvh = h / ATT_G;
+    const int nblk = (int)gridDim.x, order = (int)blockIdx.x < wave ? (int)blockIdx.x : nblk - 1 - ((int)blockIdx.x - wave);   // by length, descending
+    const int m0 = (nblk / a.NH - 1 - order / a.NH) * AP_BM, h = order % a.NH, kvh = h / ATT_G;
     const SegDesc seg = a.segs[0];
     const int slot = seg.slot;
     const int pos0 = a.tab.kv_len[slot];                                     // position of the call's first row
@@ -100,12 +103,20 @@ __global__ void __launch_bounds__(128) k_attn_prefill(AttnArgs a) {
     const int prow[2] = {pos0 + m0 + warp * 16 + (lane >> 2), pos0 + m0 + warp * 16 + (lane >> 2) + 8};   // positions of the two rows
     const int pwarp_last = pos0 + m0 + warp * 16 + 15;
     const float scale = 0.0625f;                                             // 256^-0.5
+    // ldmatrix addresses: this lane's row of a block of rows, pieces 8 j + 2 b + (0 or 1) at 128 j + a swizzled offset of b alone
+    const int l7 = lane & 7, b3 = (lane >> 3) & 1, b4 = lane >> 4;
+    uint32_t qa[4], ka[4], va[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        qa[b] = smem_u32(Qs) + (warp * 16 + l7 + b3 * 8) * (ATT_D * 2) + (((2 * b + b4) ^ l7) << 4);
+        ka[b] = smem_u32(KVs) + (b4 * 8 + l7) * (ATT_D * 2) + (((2 * b + b3) ^ l7) << 4);
+        va[b] = smem_u32(KVs) + (AP_BN + b3 * 8 + l7) * (ATT_D * 2) + (((2 * b + b4) ^ l7) << 4);
+    }
     for (int tile = 0; tile < ntiles; ++tile) {
         const int buf = tile & 1;
         if (tile + 1 < ntiles) { load_tile(tile + 1, buf ^ 1); ap_wait<1>(); } else ap_wait<0>();
         __syncthreads();
-        __half* Ks = KVs + (size_t)buf * 2 * AP_BN * ATT_D;
-        __half* Vs = Ks + AP_BN * ATT_D;
+        const uint32_t at = (uint32_t)buf * (2 * AP_BN * ATT_D * 2);
         if (tile * AP_BN <= pwarp_last) {                                    // else: every key of the tile lies behind all 16 rows
             // ---- S = Q K^T: 4 key groups of 8
             float s[4][4];
@@ -114,12 +125,11 @@ __global__ void __launch_bounds__(128) k_attn_prefill(AttnArgs a) {
 #pragma unroll
             for (int ks = 0; ks < 16; ++ks) {
                 uint32_t a0, a1, a2, a3;
-                ldsm_x4(a0, a1, a2, a3, ap_at(Qs, warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, ks * 2 + (lane >> 4)));
+                ldsm_x4(a0, a1, a2, a3, qa[ks & 3] + (ks >> 2) * 128);
 #pragma unroll
                 for (int np = 0; np < 2; ++np) {
                     uint32_t b0, b1, b2, b3;
-                    const int mi = lane >> 3;
-                    ldsm_x4(b0, b1, b2, b3, ap_at(Ks, (np * 2 + (mi >> 1)) * 8 + (lane & 7), ks * 2 + (mi & 1)));
+                    ldsm_x4(b0, b1, b2, b3, ka[ks & 3] + at + (ks >> 2) * 128 + np * 16 * (ATT_D * 2));
                     ap_mma(s[np * 2], a0, a1, a2, a3, b0, b1);
                     ap_mma(s[np * 2 + 1], a0, a1, a2, a3, b2, b3);
                 }
@@ -171,8 +181,7 @@ __global__ void __launch_bounds__(128) k_attn_prefill(AttnArgs a) {
 #pragma unroll
                 for (int dp = 0; dp < 16; ++dp) {                            // pairs of dim tiles
                     uint32_t b0, b1, b2, b3;
-                    const int mi = lane >> 3;
-                    ldsm_x4_t(b0, b1, b2, b3, ap_at(Vs, kk * 16 + (mi & 1) * 8 + (lane & 7), dp * 2 + (mi >> 1)));
+                    ldsm_x4_t(b0, b1, b2, b3, va[dp & 3] + at + (dp >> 2) * 128 + kk * 16 * (ATT_D * 2));
                     ap_mma(o[dp * 2], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b0, b1);
                     ap_mma(o[dp * 2 + 1], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b2, b3);
                 }
@@ -210,8 +219,8 @@ bool launch_attn_prefill(const AttnArgs& a, int nsegs, cudaStream_t st, bool pdl
     const size_t smem = (size_t)(AP_BM * ATT_D + 2 * 2 * AP_BN * ATT_D) * sizeof(__half);
     static bool configured = false;
     if (!configured) { cudaFuncSetAttribute(k_attn_prefill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
-    const dim3 grid((unsigned)((a.M + AP_BM - 1) / AP_BM), (unsigned)a.NH);
-    profile_launch("k_attn_prefill", st, [&] { return launch_pdl(pdl, k_attn_prefill, grid, 128, smem, st, a); });
+    const int ctas = (a.M + AP_BM - 1) / AP_BM * a.NH, wave = ctas < sm_count() ? ctas : sm_count();
+    profile_launch("k_attn_prefill", st, [&] { return launch_pdl(pdl, k_attn_prefill, dim3((unsigned)ctas), 128, smem, st, a, wave); });
     return true;
 }
 

@@ -527,7 +527,7 @@ bool enqueue_router(sl_engine* e, const RouterArgs& ra, int M, bool pdl, __half*
     cudaStream_t st = e->stream;
     // From 2 rows on: the one-kernel router ends in one CTA that routes and groups everything (33 us at 4 rows, 9 at one).
     // (prefill mode takes it for ANY row count: which kernels run must not depend on how a prompt is cut into calls)
-    if ((M > 1 || e->hybrid) && e->use_rows && !ra.no_route && e->E <= 256 && ra.norm_w && ra.ldh == e->H) {
+    if ((M > 1 || (e->hybrid && !ra.no_route)) && e->use_rows && e->E <= 256 && ra.norm_w && ra.ldh == e->H) {
         const bool ep = ra.epd.sig.world > 0;
         if (ep) launch_final_norm_ep(ra.h, ra.norm_w, ra.eps, M, e->H, ra.p, ra.epd, st);     // the rows leave for the peers here
         else launch_final_norm(ra.h, ra.norm_w, ra.eps, M, e->H, ra.p, st, pdl, xq, sxq);
@@ -617,6 +617,11 @@ void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half
     const bool tc_experts = e->hybrid && e->E <= 256 && e->use_rows;      // prefill mode: for any row count (chunk-split invariance)
     const bool rows_experts = !tc_experts && M > 1 && e->E <= 256 && e->use_rows;
     const bool pdl = e->use_pdl;
+    // a call of few rows: the router stops at the logits and the CTAs of the expert kernels route the rows themselves
+    if (rows_experts) {
+        ea.xq = e->xq_p; ea.sxq = e->sx_p; ea.csum = e->csum;
+        if (e->use_route_in_experts && expert_rows_route(ea)) ra.no_route = ea.route_here = 1;
+    }
     const bool prepared = enqueue_router(e, ra, M, pdl, rows_experts ? e->xq_p : nullptr, e->sx_p);
     if (fused && launch_expert_fused(ea, st, pdl)) return;                      // one launch for gate/up + down
     if (tc_experts) {

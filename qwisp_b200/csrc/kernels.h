@@ -57,7 +57,7 @@ struct RouterArgs {
     int topk; int* inds; __half* scores; // [M][topk] routing result (written by the last CTA)
     MoeLists lists; unsigned* counter;
     unsigned* group_counter;             // [ceil(M/8)] tickets of the row groups, zero between launches
-    int no_route = 0;                    // 1: stop after the logits; the consumer (fused expert kernel) routes from them itself
+    int no_route = 0;                    // 1: stop after the logits; the consumer (the expert kernel) routes from them itself
     EpDispatch epd;                      // expert-parallel: the last CTA sends the rows and indices to every rank instead of building lists
     int ep_rows_sent = 0;                // expert-parallel, many-row router: the norm kernel has sent the rows already; only the indices remain
     PfList pf;                           // static prefetch (every CTA)
@@ -82,9 +82,9 @@ struct ExpertArgs {
     __half* hbuf;                        // [(M*topk + M)][I]
     __half* dbuf;                        // [(M*topk + M)][H]
     int M, H, I, topk;
-    const __half* rlogits = nullptr;     // fused kernel, route_here: router logits [E] of the row; every CTA routes from them itself
-    int E = 0; int route_here = 0;       //   (deterministic, so all CTAs agree) instead of waiting for a routing tail in the router kernel
-    int* inds_out = nullptr; __half* scores_out = nullptr;   //   CTA (0,0) publishes the result
+    const __half* rlogits = nullptr;     // route_here: router logits [M][E]; every CTA routes from them itself (deterministic, so all CTAs
+    int E = 0; int route_here = 0;       //   agree) instead of waiting for a routing kernel or a routing tail in the router kernel
+    int* inds_out = nullptr; __half* scores_out = nullptr;   //   the result, published by one CTA (fused kernel) or one CTA per row
     int lg_slices2 = 0;                  // fused kernel: log2(I/256) of the down phase
     unsigned* slot_sync = nullptr;       // fused kernel: [2][top_k + 1] counters, zero between launches
     int nstages = 1;                     // weight stages per CTA (2: a CTA walks several expert slots, filled by the launcher)
@@ -245,6 +245,7 @@ bool launch_expert_tc_down(const ExpertArgs& a, cudaStream_t st, bool pdl);
 // router for many rows: a.h holds rows that are already normed; logits kernel + routing / pair lists kernel
 bool launch_router_rows(const RouterArgs& a, cudaStream_t st, bool pdl);
 bool launch_router_mma(const RouterArgs& a, cudaStream_t st, bool pdl);    // prefill mode, fp16 router: logits on the tensor cores
+bool expert_rows_route(const ExpertArgs& a);     // may the expert kernels of this call route for themselves (route_here)?
 bool launch_expert_rows_gateup(const ExpertArgs& a, cudaStream_t st, bool pdl);
 bool launch_expert_rows_down(const ExpertArgs& a, cudaStream_t st, bool pdl);
 // xq / sxq (optional): the rows also normed with nw and prepared for the next layer's in-projection (H a multiple of 256, <= 4096)

@@ -551,6 +551,46 @@ __device__ __forceinline__ XrStage xr_carve(unsigned char* base, int K) {
     s.craw = reinterpret_cast<float*>(base);
     return s;
 }
+// The routing of a call of at most XR_ROUTE rows, done by every CTA from the logits (a warp per row) in place of a kernel that routes and
+// leaves lists: the choices, the slots in the order of their experts and the pairs of each slot in the order of their rows (all CTAs
+// must agree on which pairs are a block).  All threads; rows, first: 256 words each; the caller synchronises before it reads t and pairs.
+// Returns n_active.
+constexpr int XR_ROUTE = 24;
+__device__ __forceinline__ int slot_route(SlotTable& t, unsigned* rows, int* first, int* pairs, const ExpertArgs& a, int rows_per_block, int nshared) {
+    const int tid = threadIdx.x, m = tid >> 5, lane = tid & 31;
+    if (tid < 256) rows[tid] = 0u;
+    int id = 0;
+    if (m < a.M) id = route_select(route_load<false>(a.rlogits + (size_t)m * a.E, a.E, lane), a.E, a.topk, lane);
+    const bool mine = m < a.M && lane < a.topk;
+    __syncthreads();
+    if (mine) atomicOr(&rows[id], 1u << m);
+    __syncthreads();
+    // pairs (at most 24 x 32), slots and blocks (at most 256) of the experts so far, ten bits each
+    unsigned c = 0, own = 0, inc = 0;
+    if (tid < 256) {
+        c = (unsigned)__popc(rows[tid]);                        // (the choices are slots below E: top_k is at most E)
+        own = c | (c > 0 ? 1u << 10 : 0u) | ((c + rows_per_block - 1) / rows_per_block) << 20;
+        inc = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) { const unsigned o = __shfl_up_sync(0xffffffffu, inc, d); if (lane >= d) inc += o; }
+        if (lane == 31) t.ws[m] = (int)inc;
+    }
+    __syncthreads();
+    unsigned all = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) { const unsigned o = (unsigned)t.ws[w]; all += o; if (w < m) inc += o; }
+    const int n_active = (int)(all >> 10 & 1023u), blocks = (int)(all >> 20);
+    if (tid < 256 && c > 0) {
+        const unsigned before = inc - own;
+        const int slot = (int)(before >> 10 & 1023u), off = (int)(before & 1023u);
+        t.cnt[slot] = (int)c; t.expert[slot] = tid; t.off[slot] = off; t.base[slot + 1] = (int)(inc >> 20);
+        first[tid] = off;
+    }
+    if (tid == 0) { t.base[0] = 0; t.base[n_active + 1] = blocks + (nshared + rows_per_block - 1) / rows_per_block; }
+    __syncthreads();
+    if (mine) pairs[first[id] + __popc(rows[id] & ((1u << m) - 1u))] = m * a.topk + lane;
+    return n_active;
+}
 // S: slices of K.  STALL: a test's form, in which no row is ever fetched, so that every consumer's wait runs out, and soon
 template <bool DOWN, int S, bool STALL>
 __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int lg_tiles, int nstages) {
@@ -558,7 +598,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
     __shared__ __align__(8) uint64_t s_full[8], s_empty[8], s_raw[8];
     __shared__ SlotTable s_tab;
     __shared__ XrBlock s_blk[XR_BLOCKS];
-    __shared__ int s_sig, s_abort;
+    __shared__ int s_sig, s_abort, s_pairs[XR_ROUTE * 32];
     constexpr int K = S << 8, G64 = K >> 6, SXS = G64 + 4, XS = K + 8;
     constexpr size_t stage_bytes = xr_stage_bytes<DOWN>(K);
     unsigned char* stages = smem + (size_t)XR_WARPS * XR_DEPTH * XR_UNIT;
@@ -570,9 +610,12 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
         for (int i = 0; i < nstages; ++i) { mbar_init(&s_full[i], DOWN ? 1 : 8); mbar_init(&s_empty[i], XR_WARPS); mbar_init(&s_raw[i], 8); }
         mbar_fence_init();
     }
-    if (!DOWN) pdl_wait();                                      // the lists (down: they were there before gate/up started)
+    if (!DOWN) pdl_wait();                                      // the lists, or the logits (down: they were there before gate/up started)
     pdl_launch_dependents();
-    const int n_active = slot_table(s_tab, a.lists, 8, nshared);
+    unsigned* scratch = reinterpret_cast<unsigned*>(s_blk);     // (filled below)
+    static_assert(sizeof(s_blk) >= 512 * sizeof(int), "counters of slot_route()");
+    const int n_active = a.route_here ? slot_route(s_tab, scratch, reinterpret_cast<int*>(scratch + 256), s_pairs, a, 8, nshared) : slot_table(s_tab, a.lists, 8, nshared);
+    const int* pairs = a.route_here ? s_pairs : a.lists.pairs;
     __syncthreads();
     const long total = (long)s_tab.base[n_active + 1] << lg_tiles;
     const int lo = (int)(total * blockIdx.x / gridDim.x), hi = (int)(total * (blockIdx.x + 1) / gridDim.x);
@@ -583,7 +626,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
         const bool have = ridx < (shared ? nshared : s_tab.cnt[j]);
         int dst = -1, src = -1;
         if (have && shared) { dst = npair + ridx; src = DOWN ? dst : a.shared_row0 + ridx; }
-        else if (have) { dst = a.lists.pairs[s_tab.off[j] + ridx]; src = DOWN ? dst : dst / a.topk; }
+        else if (have) { dst = pairs[s_tab.off[j] + ridx]; src = DOWN ? dst : dst / a.topk; }
         XrBlock& b = s_blk[i >> 3];
         b.src[i & 7] = src; b.dst[i & 7] = dst;
         if ((i & 7) == 0) b.expert = shared ? -1 : s_tab.expert[j];
@@ -622,6 +665,14 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&s_full[stg]);
+            }
+        }
+        // the choices and gates of row m, for the combine, from CTA m (nobody waits for them here)
+        if (!DOWN && a.route_here) {
+            __shared__ float s_gate[256];
+            for (int m = blockIdx.x; m < a.M; m += gridDim.x) {
+                __syncwarp();
+                route_row_warp(a.rlogits + (size_t)m * a.E, a.E, a.topk, a.inds_out + m * a.topk, a.scores_out + m * a.topk, s_gate, lane);
             }
         }
     } else {
@@ -742,16 +793,28 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
             st_release_sys(a.ep_sig.flags[tid] + 8 + a.ep_sig.rank, ep_seq(a.ep_sig.ctr, a.ep_sig.layer, 1));
     }
 }
+// the tiles (their binary logarithm) and the stages of a launch; false: shape not covered
+template <bool DOWN>
+static bool expert_rows_shape(const ExpertArgs& a, int& lg, int& nstages) {
+    const int ntiles = DOWN ? a.H / 16 : a.I / 8, K = DOWN ? a.I : a.H;
+    if (!a.csum || (!DOWN && (!a.xq || !a.sxq)) || (K != 256 && K != 512 && K != 1024 && K != 2048 && K != 4096)) return false;
+    lg = 0; while ((1 << lg) < ntiles) ++lg;
+    const long pairs = (long)a.M * a.topk, blocks = pairs / 8 + (pairs < 256 ? pairs : 256) + a.M / 8 + 1;    // at most one partial block per expert
+    nstages = (int)(((size_t)216 * 1024 - (size_t)XR_WARPS * XR_DEPTH * XR_UNIT) / xr_stage_bytes<DOWN>(K));
+    if (nstages > 8) nstages = 8;
+    return (1 << lg) == ntiles && blocks / sm_count() + 2 <= XR_BLOCKS && nstages >= 1;
+}
+// A warp per row: more rows would be routed in turns by every CTA, and a kernel of its own is done sooner.
+bool expert_rows_route(const ExpertArgs& a) {
+    int lg, nstages;
+    return a.M <= XR_ROUTE && a.E <= 256 && a.topk <= 32 && a.ep_pairs_per_rank == 0 && expert_rows_shape<false>(a, lg, nstages) && expert_rows_shape<true>(a, lg, nstages);
+}
 template <bool DOWN, int S, bool STALL = false>
 static bool launch_expert_rows_t(const ExpertArgs& a, cudaStream_t st, bool pdl) {
-    const int ntiles = DOWN ? a.H / 16 : a.I / 8, grid = sm_count();
-    int lg = 0; while ((1 << lg) < ntiles) ++lg;
-    const long pairs = (long)a.M * a.topk, blocks = pairs / 8 + (pairs < 256 ? pairs : 256) + a.M / 8 + 1;    // at most one partial block per expert
-    const size_t ring = (size_t)XR_WARPS * XR_DEPTH * XR_UNIT, sb = xr_stage_bytes<DOWN>(S << 8);
-    int nstages = (int)(((size_t)216 * 1024 - ring) / sb);
-    if (nstages > 8) nstages = 8;
-    if ((1 << lg) != ntiles || blocks / grid + 2 > XR_BLOCKS || nstages < 1) return false;
-    const size_t smem = ring + sb * nstages;
+    const int grid = sm_count();
+    int lg, nstages;
+    if (!expert_rows_shape<DOWN>(a, lg, nstages)) return false;
+    const size_t smem = (size_t)XR_WARPS * XR_DEPTH * XR_UNIT + xr_stage_bytes<DOWN>(S << 8) * nstages;
     static bool configured = false;
     if (!configured) { cudaFuncSetAttribute(k_expert_rows<DOWN, S, STALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
     profile_launch(DOWN ? "k_expert_rows_down" : "k_expert_rows_gateup", st, [&] { return launch_pdl(pdl, k_expert_rows<DOWN, S, STALL>, dim3((unsigned)grid), XR_THREADS, smem, st, a, lg, nstages); });
@@ -759,7 +822,6 @@ static bool launch_expert_rows_t(const ExpertArgs& a, cudaStream_t st, bool pdl)
 }
 template <bool DOWN>
 static bool launch_expert_rows_d(const ExpertArgs& a, cudaStream_t st, bool pdl) {
-    if (!a.csum || (!DOWN && (!a.xq || !a.sxq))) return false;
     switch (DOWN ? a.I : a.H) {
         case 256: return launch_expert_rows_t<DOWN, 1>(a, st, pdl);
         case 512: return !DOWN && a.stall ? launch_expert_rows_t<DOWN, 2, !DOWN>(a, st, pdl) : launch_expert_rows_t<DOWN, 2>(a, st, pdl);
@@ -1107,6 +1169,12 @@ bool launch_router_mma(const RouterArgs& a, cudaStream_t st, bool pdl) {
     return true;
 }
 
+// (nothing to launch where the expert kernels route for themselves)
+static void launch_route_rows(const RouterArgs& a, cudaStream_t st, bool pdl) {
+    if (a.no_route) return;
+    const unsigned grid = (unsigned)(a.epd.sig.world > 0 ? a.M : (a.M + 7) / 8);
+    profile_launch("k_route_rows", st, [&] { return launch_pdl(pdl, k_route_rows, dim3(grid), 256, 0, st, a); });
+}
 // rows already normed in a.h (ldh); E <= 256.  Returns false when the shape is not covered.
 bool launch_router_rows(const RouterArgs& a, cudaStream_t st, bool pdl) {
     if (a.E > 256 || a.H % 256 || a.H > 4096 || a.norm_w) return false;
@@ -1128,8 +1196,7 @@ bool launch_router_rows(const RouterArgs& a, cudaStream_t st, bool pdl) {
     else profile_launch("k_router_rows", st, [&] {
         return launch_pdl(pdl, q8 ? k_router_rows<true> : k_router_rows<false>, grid, 256, smem, st, a);
     });
-    const int route_grid = a.epd.sig.world > 0 ? a.M : ngroups;
-    profile_launch("k_route_rows", st, [&] { return launch_pdl(pdl, k_route_rows, dim3((unsigned)route_grid), 256, 0, st, a); });
+    launch_route_rows(a, st, pdl);
     return true;
 }
 

@@ -72,6 +72,22 @@ def test_rows_of_one_stream(engines, base, M):
     assert same(la, lb) and np.array_equal(ta, tb) and np.array_equal(ba, bb)
 
 
+# rows that the expert kernels route for themselves (up to 24) and one more; experts of one block and of several
+@pytest.mark.parametrize("M", [2, 8, 9, 23, 24, 25])
+def test_rows_routed_by_the_expert_kernels(engines, M):
+    import qwisp_b200 as Q
+    toks = prompt(MINI["vocab"], 3 + M, f"route.{M}")
+    x = np.random.default_rng(M).standard_normal((M, MINI["hidden"])).astype(np.float16)
+    out = []
+    for e in engines:
+        s = e.stream(M + 8)
+        s.forward(toks[:3], want_hidden=False)
+        out.append((s.forward(toks[3:]), s.state_save()) + tuple(Q.ops.moe_block(e, 0, x)))
+        s.close()
+    (ha, ba, oa, ia, sa), (hb, bb, ob, ib, sb) = out
+    assert same(ha, hb) and np.array_equal(ba, bb) and same(oa, ob) and np.array_equal(ia, ib) and same(sa, sb)
+
+
 # chunks of the state scan: a chunk less or more one row, remainders of its turns, behind a history
 @pytest.mark.parametrize("M", [3, 5, 47, 48, 49, 50, 97, 145])
 def test_state_scan_chunks(engines, M):

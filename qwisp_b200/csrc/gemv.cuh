@@ -355,6 +355,17 @@ __device__ __forceinline__ void load_xregs(XRegs& xr, const XStage& st, int slic
         xr.sx[g] = *reinterpret_cast<const float2*>(st.sxs + (slice * 4 + g) * 8 + 2 * t);
     }
 }
+// scale and bias parts of a group.  ONE: a single row, so that only column 0 is looked at and the odd columns need no arithmetic
+// (16 of about 300 instructions of a slice)
+template <bool ONE>
+__device__ __forceinline__ void scale_group(const float c[4], float2 fa, float2 fb, float2 sx, float accS[4], float accB[4]) {
+    accS[0] = fmaf(fa.x, c[0], accS[0]); accS[2] = fmaf(fb.x, c[2], accS[2]);
+    accB[0] = fmaf(fa.y, sx.x, accB[0]); accB[2] = fmaf(fb.y, sx.x, accB[2]);
+    if (!ONE) {
+        accS[1] = fmaf(fa.x, c[1], accS[1]); accS[3] = fmaf(fb.x, c[3], accS[3]);
+        accB[1] = fmaf(fa.y, sx.y, accB[1]); accB[3] = fmaf(fb.y, sx.y, accB[3]);
+    }
+}
 // The slice's weights expanded ahead of the activations: fp16 integers as MMA operands; scales and biases as loaded
 struct SliceA { uint32_t a[4][16]; uint4 sc[2]; };
 __device__ __forceinline__ void expand_slice(SliceA& e, const uint4* w_unit, const uint4* s_unit, int lane) {
@@ -365,7 +376,8 @@ __device__ __forceinline__ void expand_slice(SliceA& e, const uint4* w_unit, con
     }
     e.sc[0] = s_unit[lane >> 2]; e.sc[1] = s_unit[8 + (lane >> 2)];
 }
-// what remains of compute_slice() then (same operations)
+// what remains of compute_slice() then (same operations; ONE as there)
+template <bool ONE>
 __device__ __forceinline__ void compute_expanded(const SliceA& e, const XStage& st, int slice, int n, int t, int mr, float accS[4], float accB[4]) {
     const __half* xp = st.xs + (size_t)n * st.stride + slice * 256 + 16 * t;
 #pragma unroll
@@ -382,14 +394,12 @@ __device__ __forceinline__ void compute_expanded(const SliceA& e, const XStage& 
         const uint4 sv = e.sc[g >> 1];
         const uint32_t sa_ba = (g & 1) ? sv.z : sv.x, sb_bb = (g & 1) ? sv.w : sv.y;
         const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&sa_ba)), fb = __half22float2(*reinterpret_cast<const __half2*>(&sb_bb));
-        accS[0] = fmaf(fa.x, c[0], accS[0]); accS[1] = fmaf(fa.x, c[1], accS[1]);
-        accS[2] = fmaf(fb.x, c[2], accS[2]); accS[3] = fmaf(fb.x, c[3], accS[3]);
-        accB[0] = fmaf(fa.y, sx2.x, accB[0]); accB[1] = fmaf(fa.y, sx2.y, accB[1]);
-        accB[2] = fmaf(fb.y, sx2.x, accB[2]); accB[3] = fmaf(fb.y, sx2.y, accB[3]);
+        scale_group<ONE>(c, fa, fb, sx2, accS, accB);
     }
 }
 // One slice (4 groups) of a 16-row tile.
 // accS/accB [4]: (row A, col 2t), (row A, col 2t+1), (row B, col 2t), (row B, col 2t+1).
+template <bool ONE = false>
 __device__ __forceinline__ void compute_slice_x(const SliceRegs& r, const XRegs& xr, float accS[4], float accB[4]) {
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
@@ -408,17 +418,15 @@ __device__ __forceinline__ void compute_slice_x(const SliceRegs& r, const XRegs&
         const uint32_t sa_ba = (g & 1) ? sv.z : sv.x, sb_bb = (g & 1) ? sv.w : sv.y;
         float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&sa_ba));    // (scale A, bias A)
         float2 fb = __half22float2(*reinterpret_cast<const __half2*>(&sb_bb));    // (scale B, bias B)
-        accS[0] = fmaf(fa.x, c[0], accS[0]); accS[1] = fmaf(fa.x, c[1], accS[1]);
-        accS[2] = fmaf(fb.x, c[2], accS[2]); accS[3] = fmaf(fb.x, c[3], accS[3]);
-        accB[0] = fmaf(fa.y, sx2.x, accB[0]); accB[1] = fmaf(fa.y, sx2.y, accB[1]);
-        accB[2] = fmaf(fb.y, sx2.x, accB[2]); accB[3] = fmaf(fb.y, sx2.y, accB[3]);
+        scale_group<ONE>(c, fa, fb, sx2, accS, accB);
     }
 }
+template <bool ONE>
 __device__ __forceinline__ void compute_slice(const SliceRegs& r, const XStage& st, int slice, int n, int t, int mr,
                                               float accS[4], float accB[4]) {
     XRegs xr;
     load_xregs(xr, st, slice, n, t, mr);
-    compute_slice_x(r, xr, accS, accB);
+    compute_slice_x<ONE>(r, xr, accS, accB);
 }
 // scale part + bias part of the slice
 __device__ __forceinline__ void finish_acc4(const float accS[4], const float accB[4], int t, float v[4]) {

@@ -85,8 +85,8 @@ static void set_pdl(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, bool pdl
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
 }
-// NW warps per CTA, UPW units per warp; the CTA's NW*UPW units arrive in rounds of 16.
-template <int PRO, int EPI, int NW, int UPW>
+// NW warps per CTA, UPW units per warp; the CTA's NW*UPW units arrive in rounds of 16.  ONE: a single row.
+template <int PRO, int EPI, int NW, int UPW, bool ONE>
 __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) k_gemv(DenseArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) k_gemv(DenseArgs a) 
             SliceRegs rg;
             load_slice_smem(rg, ws.w + (size_t)u * 128, ws.s + (size_t)u * 16, lane);
             float accS[4] = {0.f, 0.f, 0.f, 0.f}, accB[4] = {0.f, 0.f, 0.f, 0.f}, v[4];
-            compute_slice_x(rg, xr, accS, accB);
+            compute_slice_x<ONE>(rg, xr, accS, accB);
             finish_acc4(accS, accB, t, v);
             store_partial(red, u, lane, v);
         }
@@ -164,11 +164,11 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) k_gemv(DenseArgs a) 
         }
     }
 }
-template <int PRO, int EPI, int NW, int UPW>
-static void launch_gemv_t(const DenseArgs& a, const GemvPlan& pl, cudaStream_t st, bool pdl) {
+template <int PRO, int EPI, int NW, int UPW, bool ONE>
+static void launch_gemv_o(const DenseArgs& a, const GemvPlan& pl, cudaStream_t st, bool pdl) {
     size_t smem = GemvSmem::wstage_bytes(NW * UPW) + GemvSmem::bytes(a.M < ROWS_PER_PASS ? a.M : ROWS_PER_PASS, a.K, NW * UPW, pl.tpc);
     static bool configured = false;
-    if (!configured) { cudaFuncSetAttribute(k_gemv<PRO, EPI, NW, UPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); configured = true; }
+    if (!configured) { cudaFuncSetAttribute(k_gemv<PRO, EPI, NW, UPW, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); configured = true; }
     int ntiles = EPI == EPI_SWIGLU ? a.N / 8 : a.N / 16;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((ntiles + pl.tpc - 1) / pl.tpc), (unsigned)((a.M + ROWS_PER_PASS - 1) / ROWS_PER_PASS));
@@ -178,12 +178,17 @@ static void launch_gemv_t(const DenseArgs& a, const GemvPlan& pl, cudaStream_t s
     DenseArgs copy = a; copy.lg_slices = pl.lg_slices;
     // profiling tag by role: the in-projection form stores its rows, the out-projection form adds the residual
     ProfScope ps(EPI == EPI_RESID ? "k_gemv_outproj" : "k_gemv_inproj", (double)a.N * a.K * 0.5625 + (double)a.M * (a.K + a.N) * 2, st);
-    cudaLaunchKernelEx(&cfg, k_gemv<PRO, EPI, NW, UPW>, copy);
+    cudaLaunchKernelEx(&cfg, k_gemv<PRO, EPI, NW, UPW, ONE>, copy);
     COUNT_LAUNCH();
+}
+template <int PRO, int EPI, int NW, int UPW>
+static void launch_gemv_t(const DenseArgs& a, const GemvPlan& pl, cudaStream_t st, bool pdl) {
+    if (a.M == 1) launch_gemv_o<PRO, EPI, NW, UPW, true>(a, pl, st, pdl); else launch_gemv_o<PRO, EPI, NW, UPW, false>(a, pl, st, pdl);
 }
 
 __device__ __forceinline__ bool better(float v, int i, float bv, int bi) { return v > bv || (v == bv && i < bi); }
-template <int PRO>
+// ONE: a single row
+template <int PRO, bool ONE>
 __global__ void __launch_bounds__(256) k_head(DenseArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -214,7 +219,7 @@ __global__ void __launch_bounds__(256) k_head(DenseArgs a) {
             if (ns == slices) { ns = 0; ntile = tile + stride; }
             if (ntile < ntiles) load(nxt, ntile, ns);
             float accS[4] = {0.f, 0.f, 0.f, 0.f}, accB[4] = {0.f, 0.f, 0.f, 0.f};
-            compute_slice(cur, st, sidx, r, t, mr, accS, accB);
+            compute_slice<ONE>(cur, st, sidx, r, t, mr, accS, accB);
             float v[4];
             finish_acc4(accS, accB, t, v);
 #pragma unroll
@@ -284,16 +289,16 @@ __global__ void __launch_bounds__(256) k_head(DenseArgs a) {
     if (threadIdx.x == 0) *a.counter = 0u;
 }
 
-template <int PRO>
-static void launch_head_t(const DenseArgs& a, cudaStream_t st, bool pdl) {
+template <int PRO, bool ONE>
+static void launch_head_o(const DenseArgs& a, cudaStream_t st, bool pdl) {
     size_t smem = GemvSmem::bytes(a.M < ROWS_PER_PASS ? a.M : ROWS_PER_PASS, a.K, 1, 1);
     static bool configured = false;
-    if (!configured) { cudaFuncSetAttribute(k_head<PRO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024); configured = true; }
+    if (!configured) { cudaFuncSetAttribute(k_head<PRO, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024); configured = true; }
     int ntiles = a.N / 16;
     // one wave of persistent CTAs: as many as are resident at once with this kernel's registers and shared memory
     static int per_sm = 0;
     if (per_sm == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_head<PRO>, 256, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_head<PRO, ONE>, 256, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
         if (per_sm > 3) per_sm = 3;
     }
     int gx = (ntiles + 7) / 8; if (gx > sm_count() * per_sm) gx = sm_count() * per_sm;
@@ -304,8 +309,12 @@ static void launch_head_t(const DenseArgs& a, cudaStream_t st, bool pdl) {
     set_pdl(cfg, attr, pdl);
     DenseArgs copy = a;
     ProfScope ps("k_head", (double)a.N * a.K * 0.5625 + (double)a.M * a.K * 2, st);
-    cudaLaunchKernelEx(&cfg, k_head<PRO>, copy);
+    cudaLaunchKernelEx(&cfg, k_head<PRO, ONE>, copy);
     COUNT_LAUNCH();
+}
+template <int PRO>
+static void launch_head_t(const DenseArgs& a, cudaStream_t st, bool pdl) {
+    if (a.M == 1) launch_head_o<PRO, true>(a, st, pdl); else launch_head_o<PRO, false>(a, st, pdl);
 }
 
 // ---- lm_head + greedy argmax with its scratch in a fixed module-scope array (no allocation) ----
@@ -331,7 +340,7 @@ int launch_head_static(const DenseArgs& in, cudaStream_t st) {
         unsigned char* ptr = nullptr;
         err = cudaGetSymbolAddress((void**)&ptr, g_head_static_scratch);
         if (err != cudaSuccess) return (int)err;
-        err = cudaFuncSetAttribute(k_head<PRO_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+        err = cudaFuncSetAttribute(k_head<PRO_PLAIN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
         if (err != cudaSuccess) return (int)err;
         base[dev] = ptr;
     }
@@ -344,7 +353,7 @@ int launch_head_static(const DenseArgs& in, cudaStream_t st) {
     err = cudaMemsetAsync(a.counter, 0, sizeof(unsigned), st);
     if (err != cudaSuccess) return (int)err;
     const size_t smem = GemvSmem::bytes(a.M < ROWS_PER_PASS ? a.M : ROWS_PER_PASS, a.K, 1, 1);
-    k_head<PRO_PLAIN><<<dim3((unsigned)gx, (unsigned)((a.M + ROWS_PER_PASS - 1) / ROWS_PER_PASS)), 256, smem, st>>>(a);
+    k_head<PRO_PLAIN, false><<<dim3((unsigned)gx, (unsigned)((a.M + ROWS_PER_PASS - 1) / ROWS_PER_PASS)), 256, smem, st>>>(a);
     return (int)cudaGetLastError();
 }
 
@@ -1039,7 +1048,7 @@ __global__ void __launch_bounds__(512, 1) k_expert_fused(ExpertArgs a) {
                 SliceRegs rg;
                 load_slice_smem(rg, ws1.w + (size_t)u * 128, ws1.s + (size_t)u * 16, lane);
                 float accS[4] = {0.f, 0.f, 0.f, 0.f}, accB[4] = {0.f, 0.f, 0.f, 0.f}, v[4];
-                compute_slice_x(rg, xr, accS, accB);
+                compute_slice_x<true>(rg, xr, accS, accB);
                 finish_acc4(accS, accB, t, v);
                 store_partial(red, u, lane, v);
             }
@@ -1089,7 +1098,7 @@ __global__ void __launch_bounds__(512, 1) k_expert_fused(ExpertArgs a) {
         if (UD == 1) {
             if (warp < nvu2) {
                 float accS[4] = {0.f, 0.f, 0.f, 0.f}, accB[4] = {0.f, 0.f, 0.f, 0.f}, v[4];
-                compute_expanded(ex, st, warp & (sl2 - 1), r, t, 1, accS, accB);
+                compute_expanded<true>(ex, st, warp & (sl2 - 1), r, t, 1, accS, accB);
                 finish_acc4(accS, accB, t, v);
                 store_partial(red, warp, lane, v);
             }
@@ -1104,7 +1113,7 @@ __global__ void __launch_bounds__(512, 1) k_expert_fused(ExpertArgs a) {
                 SliceRegs rg;
                 load_slice_smem(rg, ws2.w + (size_t)u * 128, ws2.s + (size_t)u * 16, lane);
                 float accS[4] = {0.f, 0.f, 0.f, 0.f}, accB[4] = {0.f, 0.f, 0.f, 0.f}, v[4];
-                compute_slice_x(rg, xr, accS, accB);
+                compute_slice_x<true>(rg, xr, accS, accB);
                 finish_acc4(accS, accB, t, v);
                 store_partial(red, u, lane, v);
             }

@@ -1543,8 +1543,10 @@ __global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, int
         }
     }
     // ---- the CTA that finishes last for this (row, four heads) merges the splits ----
-    // (the output gate of this warp's head does not depend on the other CTAs: fetched before the ticket)
-    const uint4 gvv = reinterpret_cast<const uint4*>(rowp + (size_t)(h0 + (warp & 3)) * 2 * ATT_D + ATT_D)[lane];
+    // (two warps a head, sixteen splits in flight: at 8192 keys, 52 splits, one warp with eight was seven round trips to L2.  The output
+    // gate of this warp's half head does not depend on the other CTAs: fetched before the ticket)
+    const int h = h0 + (warp >> 1), d0 = (warp & 1) * 128 + lane * 4;
+    const uint2 gvv = *reinterpret_cast<const uint2*>(rowp + (size_t)h * 2 * ATT_D + ATT_D + d0);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1554,15 +1556,13 @@ __global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, int
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    if (warp < HG) {
-        const int h = h0 + warp;
-        const float* po = a.part_o + ((size_t)m * a.NH + h) * a.nsplit * ATT_D;
-        const float* pml = a.part_ml + ((size_t)m * a.NH + h) * a.nsplit * 2;
-        const uint4 outv = attn_merge_splits(used, lane, gvv,
-            [&](int sp, float4& x0, float4& x1) { const float4* src = reinterpret_cast<const float4*>(po + (size_t)sp * ATT_D + lane * 8); x0 = __ldcg(src); x1 = __ldcg(src + 1); },
-            [&](int sp) { return __ldcg(reinterpret_cast<const float2*>(pml) + sp); });
-        reinterpret_cast<uint4*>(a.gated + ((size_t)m * a.NH + h) * ATT_D)[lane] = outv;
-    }
+    const float* po = a.part_o + ((size_t)m * a.NH + h) * a.nsplit * ATT_D + d0;
+    const float* pml = a.part_ml + ((size_t)m * a.NH + h) * a.nsplit * 2;
+    uint2 outv;
+    attn_merge_splits<4, 16>(used, lane, reinterpret_cast<const __half*>(&gvv), reinterpret_cast<__half*>(&outv),
+        [&](int sp, float4* x) { x[0] = __ldcg(reinterpret_cast<const float4*>(po + (size_t)sp * ATT_D)); },
+        [&](int sp) { return __ldcg(reinterpret_cast<const float2*>(pml) + sp); });
+    *reinterpret_cast<uint2*>(a.gated + ((size_t)m * a.NH + h) * ATT_D + d0) = outv;
     if (threadIdx.x == 0) counters[m * gridDim.y + blockIdx.y] = 0u;
 }
 void launch_attn_fused(const AttnArgs& a, bool prep, unsigned* counters, cudaStream_t st, bool pdl) {

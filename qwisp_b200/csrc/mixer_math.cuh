@@ -179,11 +179,11 @@ __device__ __forceinline__ float attn_warps_lsum(const float m8[8], const float 
     for (int w = 0; w < 8; ++w) ls += (m8[w] == -INFINITY) ? 0.f : l8[w] * __expf(m8[w] - gm);
     return ls;
 }
-// Merge of the splits of one (row, head) by one warp: part_o [used][256] f32, part_ml [used][2] f32 (both read
-// with the loader ld_f / ld_f2 the caller provides), output gate values gvv (8 halves of this lane) ->
-// 8 gated fp16 outputs of this lane.  used <= 64.
-template <typename LoadF4, typename LoadF2>
-__device__ __forceinline__ uint4 attn_merge_splits(int used, int lane, uint4 gvv, LoadF4 ld_o, LoadF2 ld_ml) {
+// Merge of the splits of one (row, head): part_o [used][256] f32, part_ml [used][2] f32 (both read with the loaders the caller
+// provides) and the lane's output gates (gv: its D halves) -> its D gated fp16 outputs.  By whole warps, every lane D dims of the head
+// (D = 8: one warp does a head, 4: two); ld_o(split, D / 4 quads).  INF: splits' partials in flight at a time.  used <= 64.
+template <int D, int INF, typename LoadO, typename LoadF2>
+__device__ __forceinline__ void attn_merge_splits(int used, int lane, const __half* gv, __half* out, LoadO ld_o, LoadF2 ld_ml) {
     float msv[2], lsv[2], fv[2];                          // two splits per lane
     float gm = -INFINITY;
 #pragma unroll
@@ -198,29 +198,28 @@ __device__ __forceinline__ uint4 attn_merge_splits(int used, int lane, uint4 gvv
 #pragma unroll
     for (int j = 0; j < 2; ++j) { fv[j] = (msv[j] == -INFINITY) ? 0.f : __expf(msv[j] - gm); tot += lsv[j] * fv[j]; }
     tot = warp_sum(tot);
-    float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int s0 = 0; s0 < used; s0 += 8) {                // eight splits' partials in flight at a time, added in ascending order
-        float4 x0[8], x1[8];
+    float o[D];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) if (s0 + i < used) ld_o(s0 + i, x0[i], x1[i]);
+    for (int i = 0; i < D; ++i) o[i] = 0.f;
+    for (int s0 = 0; s0 < used; s0 += INF) {              // added in ascending order
+        float4 x[INF][D / 4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < INF; ++i) if (s0 + i < used) ld_o(s0 + i, x[i]);
+#pragma unroll
+        for (int i = 0; i < INF; ++i) {
             const int sp = s0 + i;
             const float f = __shfl_sync(0xffffffffu, (sp < 32) ? fv[0] : fv[1], sp & 31);
             if (sp < used) {
-                o[0] = fmaf(x0[i].x, f, o[0]); o[1] = fmaf(x0[i].y, f, o[1]); o[2] = fmaf(x0[i].z, f, o[2]); o[3] = fmaf(x0[i].w, f, o[3]);
-                o[4] = fmaf(x1[i].x, f, o[4]); o[5] = fmaf(x1[i].y, f, o[5]); o[6] = fmaf(x1[i].z, f, o[6]); o[7] = fmaf(x1[i].w, f, o[7]);
+#pragma unroll
+                for (int q = 0; q < D / 4; ++q) {
+                    o[4 * q] = fmaf(x[i][q].x, f, o[4 * q]); o[4 * q + 1] = fmaf(x[i][q].y, f, o[4 * q + 1]);
+                    o[4 * q + 2] = fmaf(x[i][q].z, f, o[4 * q + 2]); o[4 * q + 3] = fmaf(x[i][q].w, f, o[4 * q + 3]);
+                }
             }
         }
     }
-    const __half* gh = reinterpret_cast<const __half*>(&gvv);
-    uint4 outv; __half* oh = reinterpret_cast<__half*>(&outv);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        __half out = f2h(tot == 0.f ? o[i] : o[i] / tot);
-        oh[i] = hmul_rn(out, sigmoid_h(gh[i]));
-    }
-    return outv;
+    for (int i = 0; i < D; ++i) out[i] = hmul_rn(f2h(tot == 0.f ? o[i] : o[i] / tot), sigmoid_h(gv[i]));
 }
 
 }  // namespace sl

@@ -776,14 +776,15 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_step_persistent(PStepArgs a) 
                 if (warp == 0) {
                     const uint4 gvv = ll_load8(XI, hd * 2 * ATT_D + ATT_D + lane * 8, seq, w);
                     const uint4* src = XP + (size_t)hd * a.nsplit * 129;
-                    const uint4 outv = attn_merge_splits(used, lane, gvv,
-                        [&](int sp, float4& x0, float4& x1) {
+                    uint4 outv;
+                    attn_merge_splits<8, 8>(used, lane, reinterpret_cast<const __half*>(&gvv), reinterpret_cast<__half*>(&outv),
+                        [&](int sp, float4* x) {
                             uint32_t d[8];
                             const uint4* l0 = src + (size_t)sp * 129 + lane * 4;
                             const uint4* const ln[4] = {l0, l0 + 1, l0 + 2, l0 + 3};
                             ll_load_n<4>(ln, seq, d, w);
-                            x0 = make_float4(__uint_as_float(d[0]), __uint_as_float(d[1]), __uint_as_float(d[2]), __uint_as_float(d[3]));
-                            x1 = make_float4(__uint_as_float(d[4]), __uint_as_float(d[5]), __uint_as_float(d[6]), __uint_as_float(d[7])); },
+                            x[0] = make_float4(__uint_as_float(d[0]), __uint_as_float(d[1]), __uint_as_float(d[2]), __uint_as_float(d[3]));
+                            x[1] = make_float4(__uint_as_float(d[4]), __uint_as_float(d[5]), __uint_as_float(d[6]), __uint_as_float(d[7])); },
                         [&](int sp) { uint32_t d0, d1; ll_load(src + (size_t)sp * 129 + 128, seq, d0, d1, w); return make_float2(__uint_as_float(d0), __uint_as_float(d1)); });
                     uint4* dst = Xw + a.x_off_mix + ((hd * ATT_D + lane * 8) >> 2);
                     ll_store_rep(dst, rp, outv.x, outv.y, seq);

@@ -1324,61 +1324,38 @@ void launch_gdn_core(const GdnArgs& a, int nsegs, cudaStream_t st, bool pdl) {
 // (prep: SeedlessFusedVerify.swift:1183-1360; attention: SeedlessMetalForward.swift:4922-4989;
 //  output gate: SeedlessMetalForward.swift:1012-1022)
 // ============================================================================================
-// grid (NH + 2*KV, M), 32 threads: one warp per (row, head); lane owns dims 8*lane..8*lane+7
-__global__ void __launch_bounds__(32) k_attn_prep(AttnArgs a) {
-    const int m = blockIdx.y, hidx = blockIdx.x, lane = threadIdx.x;
+// grid (M, parts of a row's heads), a warp per head (NH query, KV key, KV value heads), at most AP_WARPS of them; lane owns dims
+// 8*lane..8*lane+7.  Bound by latency (descriptors, angles, row: 3 us a CTA): as many CTAs as fit a multiprocessor.  967 rows by
+// events: 26.9 us with one warp per CTA, each with its own angles, 25.8 with a whole row per CTA (one CTA at a time), now 14.7.
+constexpr int AP_WARPS = 10;
+__global__ void __launch_bounds__(AP_WARPS * 32, 5) k_attn_prep(AttnArgs a) {
+    __shared__ float s_cs[32], s_sn[32];
+    const int m = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slot = a.segs[a.row_seg[m]].slot;
     const int pos = row_position(a, m);
+    if (warp == 0) rope_table_entry(a.theta, pos, lane, s_cs[lane], s_sn[lane]);      // ahead of the programmatic-launch wait
     pdl_wait();
     pdl_launch_dependents();
+    __syncthreads();
     const __half* rowp = a.inproj + (size_t)m * a.ld;
+    const int hidx = blockIdx.y * (blockDim.x >> 5) + warp;
+    if (hidx >= a.NH + 2 * a.KV) return;
     if (hidx >= a.NH + a.KV) {                               // V copy
-        int kvh = hidx - a.NH - a.KV;
+        const int kvh = hidx - a.NH - a.KV;
         const __half* src = rowp + a.NH * 2 * ATT_D + a.KV * ATT_D + kvh * ATT_D;
-        __half* dst = kv_ptr(a, slot, pos, 1, kvh);
-        reinterpret_cast<uint4*>(dst)[lane] = reinterpret_cast<const uint4*>(src)[lane];
+        reinterpret_cast<uint4*>(kv_ptr(a, slot, pos, 1, kvh))[lane] = reinterpret_cast<const uint4*>(src)[lane];
         return;
     }
     const bool isq = hidx < a.NH;
     const __half* src = isq ? (rowp + (size_t)hidx * 2 * ATT_D) : (rowp + a.NH * 2 * ATT_D + (hidx - a.NH) * ATT_D);
-    const __half* w = isq ? a.q_norm : a.k_norm;
-    uint4 v = reinterpret_cast<const uint4*>(src)[lane];
-    uint4 wv = reinterpret_cast<const uint4*>(w)[lane];
-    const __half* vh = reinterpret_cast<const __half*>(&v);
-    const __half* wh = reinterpret_cast<const __half*>(&wv);
-    float ss = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { float f = h2f(vh[i]); ss = fmaf(f, f, ss); }
-    ss = warp_sum(ss);
-    float inv = __frsqrt_rn(__fadd_rn(__fdiv_rn(ss, 256.0f), a.eps));
-    float nv[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) nv[i] = h2f(hmul_rn(wh[i], f2h(__fmul_rn(h2f(vh[i]), inv))));
-    // rotate dims [0,64): pairs (d, d+32); lanes 0..3 hold d<32, lanes 4..7 hold d+32
-    float other[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) other[i] = __shfl_xor_sync(0xffffffffu, nv[i], 4);
-    uint4 o; __half* oh = reinterpret_cast<__half*>(&o);
-    const float fpos = (float)pos;
-    const float lnb = logf(a.theta);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        int d = lane * 8 + i;
-        if (d >= ROPE_D) { oh[i] = f2h(nv[i]); continue; }
-        int ii = (d < 32) ? d : (d - 32);
-        float freq = expf(-2.0f * (float)ii / (float)ROPE_D * lnb);
-        float ang = fpos * freq;
-        float sn, cs; sincosf(ang, &sn, &cs);
-        float x0 = (d < 32) ? nv[i] : other[i], x1 = (d < 32) ? other[i] : nv[i];
-        oh[i] = f2h((d < 32) ? (x0 * cs - x1 * sn) : (x0 * sn + x1 * cs));
-    }
+    const uint4 o = norm_rope_head_tab(reinterpret_cast<const uint4*>(src)[lane], isq ? a.q_norm : a.k_norm, a.eps, s_cs, s_sn, lane);
     if (isq) reinterpret_cast<uint4*>(a.qrot + ((size_t)m * a.NH + hidx) * ATT_D)[lane] = o;
     else reinterpret_cast<uint4*>(kv_ptr(a, slot, pos, 0, hidx - a.NH))[lane] = o;
 }
 void launch_attn_prep(const AttnArgs& a, cudaStream_t st, bool pdl) {
-    dim3 grid(a.NH + 2 * a.KV, a.M);
+    const int heads = a.NH + 2 * a.KV, parts = (heads + AP_WARPS - 1) / AP_WARPS;
     ProfScope ps("k_attn_prep", 0.0, st);
-    launch_pdl(pdl, k_attn_prep, grid, 32, 0, st, a);
+    launch_pdl(pdl, k_attn_prep, dim3((unsigned)a.M, (unsigned)parts), (unsigned)((heads + parts - 1) / parts) * 32u, 0, st, a);
     COUNT_LAUNCH();
 }
 

@@ -340,7 +340,10 @@ int32_t build_runtime(sl_engine* e) {
     if ((rc = dalloc(e, &e->lists.slot_expert, (size_t)256))) return rc;
     if ((rc = dalloc(e, &e->lists.slot_off, (size_t)256))) return rc;
     if ((rc = dalloc(e, &e->lists.slot_cnt, (size_t)256))) return rc;
-    if ((rc = dalloc(e, &e->lists.pairs, (size_t)R * e->topk))) return rc;
+    e->lists.cap = R;                                          // (a row's choices are distinct)
+    if ((rc = dalloc(e, &e->lists.pairs, (size_t)R * (e->E > e->topk ? e->E : e->topk)))) return rc;
+    if ((rc = dalloc(e, &e->lists.counts, (size_t)256))) return rc;
+    CU(e, cudaMemset(e->lists.counts, 0, 256 * sizeof(int)));
     if ((rc = dalloc(e, &e->tile_counters, (size_t)(H / 16)))) return rc;
     CU(e, cudaMemset(e->tile_counters, 0, (size_t)(H / 16) * sizeof(unsigned)));
     CU(e, cudaMemset(e->counters, 0, 8 * sizeof(unsigned)));

@@ -631,7 +631,11 @@ void enqueue_moe(sl_engine* e, const LayerW& L, const LayerW* next, const __half
         // prefill mode: grouped GEMMs on the tensor cores, then the combine kernel
         ea.tile_counter = nullptr;
         if (launch_expert_tc_gateup(ea, st, pdl) && launch_expert_tc_down(ea, st, pdl)) {
-            launch_moe_combine(e->dbuf, e->dbuf + (size_t)M * e->topk * e->H, e->scores, e->sgl, M, e->H, e->topk, resid, plain_out, st, pdl);
+            // (rows of up to 2048: k_final_norm adds the squares of wider ones in another order)
+            const bool prep = next_prepared && next && resid && e->H % 256 == 0 && e->H <= 2048 && next->in_proj.N % 16 == 0;
+            launch_moe_combine(e->dbuf, e->dbuf + (size_t)M * e->topk * e->H, e->scores, e->sgl, M, e->H, e->topk, resid, plain_out, st, pdl,
+                               prep ? next->in_norm : nullptr, e->cfg.rms_eps, prep ? e->normed : nullptr, nullptr);
+            if (prep) *next_prepared = true;
             return;
         }
         ea.tile_counter = e->tile_counters;

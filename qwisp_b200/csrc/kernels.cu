@@ -397,7 +397,7 @@ void launch_dense(int pro, int epi, const DenseArgs& a, cudaStream_t st, bool pd
         const __half* x = a.x; int ldx = a.ldx;
         if (pro == PRO_RMSNORM) {
             if (a.ldx != a.K) goto gemv_path;                  // the row kernel reads dense rows
-            launch_final_norm(a.x, a.nw, a.eps, a.M, a.K, a.norm_scratch, st, pdl);
+            if (!a.prepared) launch_final_norm(a.x, a.nw, a.eps, a.M, a.K, a.norm_scratch, st, pdl);
             x = a.norm_scratch; ldx = a.K;
         } else if (pro_is_normgate(pro)) {
             launch_normgate_rows(pro, a, st, pdl);

@@ -24,7 +24,7 @@ struct DenseArgs {
     __half* y; int ldy;                                          // output rows
     __half* logits;                                              // optional [M][N] (argmax epilogue)
     float* pval; int* pidx; int* out_tok; unsigned* counter;     // argmax partials / result / ticket
-    bool prepared = false;                                       // xq / sxq already hold the prologue's rows (a many-row call)
+    bool prepared = false;                                       // xq / sxq (prefill mode: norm_scratch) already hold the prologue's rows (a many-row call)
     PfList pf;                                                   // weights of later kernels to pull into L2
     MoeRow moe;                                                  // PRO_MOERMS: x is the residual row before the last MoE block's combine
 };
@@ -39,7 +39,9 @@ struct MoeLists {
     int* slot_expert;    // [E]
     int* slot_off;       // [E]
     int* slot_cnt;       // [E]
-    int* pairs;          // [M*top_k] pair ids (row*top_k + k) grouped by expert slot
+    int* pairs;          // pair ids (row*top_k + k) grouped by expert slot, from slot_off on
+    int* counts;         // [E] pairs of each expert so far, zero between launches (k_route_rows)
+    int cap;             // its room for an expert's pairs: pair ids of expert e from pairs[e * cap] on
 };
 
 struct RouterArgs {
@@ -248,7 +250,8 @@ bool launch_router_mma(const RouterArgs& a, cudaStream_t st, bool pdl);    // pr
 bool expert_rows_route(const ExpertArgs& a);     // may the expert kernels of this call route for themselves (route_here)?
 bool launch_expert_rows_gateup(const ExpertArgs& a, cudaStream_t st, bool pdl);
 bool launch_expert_rows_down(const ExpertArgs& a, cudaStream_t st, bool pdl);
-// xq / sxq (optional): the rows also normed with nw and prepared for the next layer's in-projection (H a multiple of 256, <= 4096)
+// xq / sxq (optional): the rows also normed with nw and prepared for the next layer's in-projection (H a multiple of 256, <= 4096);
+// xq alone: normed as plain rows
 void launch_moe_combine(const __half* dbuf, const __half* shared_rows, const __half* scores, const __half* sgl, int M, int H, int topk,
                         __half* resid, __half* out, cudaStream_t st, bool pdl, const __half* nw = nullptr, float eps = 0.f, __half* xq = nullptr, float* sxq = nullptr);
 // many-row GEMM on tcgen05 tensor cores with the accumulator in tensor memory (N % 16 == 0, K % 256 == 0); 0 or an error code

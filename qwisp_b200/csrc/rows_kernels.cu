@@ -1196,8 +1196,8 @@ bool launch_router_rows(const RouterArgs& a, cudaStream_t st, bool pdl) {
 // (swift/Sources/QwispCore/SeedlessFusedVerify.swift:462-484, SeedlessMetalForward.swift:1024-1028)
 // Bound by latency: with one output and 2-byte loads per thread and step the eight steps of a thread were 8 dependent
 // round trips; all 16-byte loads of a thread are now in flight at once.
-// NORM (grid (M), H / 8 threads): the CTA has the whole residual row, and leaves it normed and prepared for the next layer's
-// in-projection as well (the arithmetic of k_rows_prep<PRO_RMSNORM>; a launch less per layer).
+// NORM (grid (M), H / 8 threads): the CTA has the whole residual row, and leaves it normed for the next layer's in-projection as
+// well, prepared (the arithmetic of k_rows_prep<PRO_RMSNORM>) or, without sxq, as plain rows; a launch less per layer.
 template <bool NORM>
 __global__ void __launch_bounds__(NORM ? 512 : 256) k_moe_combine(const __half* dbuf, const __half* shared_rows, const __half* scores, const __half* sgl,
                                                                   int H, int topk, __half* resid, __half* out, const __half* nw, float eps, __half* xq, float* sxq) {
@@ -1240,7 +1240,9 @@ __global__ void __launch_bounds__(NORM ? 512 : 256) k_moe_combine(const __half* 
         float tot = 0.f;
         for (int c = 0; c < (H >> 8); ++c) tot += part[c];
         const float inv = __frsqrt_rn(__fadd_rn(__fdiv_rn(tot, (float)H), eps));
-        rows_store(xq + (size_t)m * H, sxq + (size_t)m * (H >> 6), n, rms_apply8(rv, wv, inv), lane);
+        const uint4 o = rms_apply8(rv, wv, inv);
+        if (sxq) rows_store(xq + (size_t)m * H, sxq + (size_t)m * (H >> 6), n, o, lane);
+        else *reinterpret_cast<uint4*>(xq + (size_t)m * H + n) = o;
     }
 }
 void launch_moe_combine(const __half* dbuf, const __half* shared_rows, const __half* scores, const __half* sgl, int M, int H, int topk,

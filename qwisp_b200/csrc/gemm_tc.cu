@@ -122,9 +122,10 @@ __device__ __forceinline__ void tc_group_A(const uint2 w[4], uint32_t sb, uint32
 }
 
 // ================================================================================ the two kinds of work
-// Items are (rows block, 128 weight rows), weight rows fastest; a CTA walks a contiguous run of them, so most steps stay
-// inside a block.  A work type gives the weights of a tile of an item (moved along by a cursor), the place of a
-// block's activation rows (halves from base(); Place: wide enough for the rows that the kind of work can have), and the epilogue.
+// Items are (rows block, 128 weight rows), weight rows fastest.  A work type says which items a CTA has, the weights of a tile of an
+// item (moved along by a cursor), the place of a block's activation rows (halves from base(); Place: wide enough for the rows that
+// the kind of work can have), and the epilogue.
+struct TcRun { int blk, rt, count; };                      // a role's place in its CTA's items, and how many the CTA has
 struct TcTile { const uint4 *w, *s; int blk, rt; };   // fragment-major nibbles and scales of a tile (nullptr: none) of weight-row group rt
 
 struct GemmTcArgs {
@@ -146,9 +147,9 @@ struct DenseWork {
     int NRT;                                                                // weight-row groups
     __device__ DenseWork(const Args& args, Shared&) : a(args), NRT((args.N + TC_ROWS - 1) / TC_ROWS) {}
     __device__ int items() const { return NRT * ((a.M + NT - 1) / NT); }
-    struct Walk { int blk, rt; };                                           // a role's place in its CTA's run
-    __device__ Walk walk(int item) const { return {item / NRT, item % NRT}; }
-    __device__ void next(Walk& w) const { if (++w.rt == NRT) { w.rt = 0; ++w.blk; } }
+    // CTA b of n: a contiguous run, so that most steps stay inside a block
+    __device__ TcRun run(int b, int n) const { const int lo = (int)((long)items() * b / n), hi = (int)((long)items() * (b + 1) / n); return {lo / NRT, lo % NRT, hi - lo}; }
+    __device__ void next(TcRun& w) const { if (++w.rt == NRT) { w.rt = 0; ++w.blk; } }
     __device__ int inputs() const { return a.K; }
     __device__ unsigned* err() const { return a.err; }
     __device__ bool has_tile(int rt, int tl) const { return rt * 8 + tl < a.N >> 4; }
@@ -197,10 +198,11 @@ struct ExpertWork {
     static constexpr bool STRIDED = false;
     using Place = uint32_t;                                                 // (an engine has at most 1024 rows: 17k pair rows of 4096)
     static constexpr Place NO_ROW = ~(Place)0;
-    struct Shared { SlotTable tab; int dst[TC_EPI][(NT + 31) / 32 * 32]; };                  // dst: a list of each epilogue warp
+    static constexpr int MAX_BLK = 1024;
+    struct Shared { SlotTable tab; short slot[MAX_BLK]; int dst[TC_EPI][(NT + 31) / 32 * 32]; };      // slot: of a block; dst: a list of each epilogue warp
     const Args& a;
     Shared& sh;
-    int n_active, K, ntiles, NRT, npair, nshared, S, T;
+    int n_active, K, ntiles, NRT, npair, nshared, step_b, step_r;
     __device__ ExpertWork(const Args& args, Shared& s) : a(args), sh(s) {
         K = DOWN ? a.I : a.H;
         ntiles = DOWN ? a.H / 16 : a.I / 8;                                 // tiles of 16 weight rows per expert
@@ -210,35 +212,28 @@ struct ExpertWork {
         pdl_wait();                                                         // (the lists)
         n_active = slot_table(sh.tab, a.lists, NT, nshared);
         __syncthreads();
-        T = items(); S = T - sh.tab.base[n_active] * NRT;
+        for (int b = threadIdx.x; b < min(sh.tab.base[n_active + 1], MAX_BLK); b += TC_THREADS) sh.slot[b] = (short)slot_of(sh.tab, n_active, b);
+        __syncthreads();
+        step_b = (int)gridDim.x / NRT; step_r = (int)gridDim.x % NRT;
     }
     __device__ int items() const { return sh.tab.base[n_active + 1] * NRT; }
-    // The shared expert's items are dealt out evenly among the others (item t is one of the S of T where t * S mod T wraps):
-    // its blocks are full, a routed expert's hold few rows, and an item's epilogue is as long as its rows.  At the end of the
-    // numbering they made ten of 148 CTAs finish a third later than the rest.
-    struct Walk { int blk, rt, acc, rb, rr, sb, sr; bool sh; };
-    __device__ void place(Walk& w) const { w.sh = w.acc + S >= T; w.blk = w.sh ? w.sb : w.rb; w.rt = w.sh ? w.sr : w.rr; }
-    __device__ Walk walk(int item) const {
-        const int s = (int)((long)item * S / T), b = sh.tab.base[n_active];
-        Walk w;
-        w.acc = (int)((long)item * S - (long)s * T);
-        w.rb = (item - s) / NRT; w.rr = (item - s) - w.rb * NRT;
-        w.sb = s / NRT; w.sr = s - w.sb * NRT; w.sb += b;
-        place(w);
-        return w;
+    // CTA b of n: every n-th item.  An item's loads and epilogue are as long as its rows, and a routed expert's blocks hold few rows or
+    // many, the shared expert's are full: dealt out like this every CTA has some of each.  In contiguous runs with the shared expert's
+    // items dealt out among them, a prompt of 2900 tokens took 62.5 ms, now 59.5, one of 129 7.95 and 7.73 ms; 256 experts
+    // routed evenly (gate/up, down): 129 rows 79.3, 48.5 -> 76.6, 47.3 us, 1024 rows 103.8, 73.8 -> 101.3, 69.9.
+    // A new block with every item asks for its slot and its rows' places each time: the slots in a table, the places an item ahead.
+    __device__ TcRun run(int b, int n) const { return {b / NRT, b % NRT, b < items() ? (items() - b + n - 1) / n : 0}; }
+    __device__ void next(TcRun& w) const {
+        w.blk += step_b; w.rt += step_r;
+        if (w.rt >= NRT) { w.rt -= NRT; ++w.blk; }
     }
-    __device__ void next(Walk& w) const {
-        if (w.sh) { if (++w.sr == NRT) { w.sr = 0; ++w.sb; } }
-        else if (++w.rr == NRT) { w.rr = 0; ++w.rb; }
-        w.acc += S - (w.sh ? T : 0);
-        place(w);
-    }
+    __device__ int slot(int blk) const { return blk < MAX_BLK ? sh.slot[blk] : slot_of(sh.tab, n_active, blk); }
     __device__ int inputs() const { return K; }
     __device__ unsigned* err() const { return a.err; }
     __device__ bool has_tile(int rt, int tl) const { return rt * 8 + tl < ntiles; }
     __device__ TcTile tile(int blk, int rt, int tl) const {
         if (!has_tile(rt, tl)) return {nullptr, nullptr, blk, rt};
-        const int j = slot_of(sh.tab, n_active, blk);
+        const int j = slot(blk);
         const bool shared = (j == n_active);
         const Q4R& q = DOWN ? (shared ? a.sh_down : a.down) : (shared ? a.sh_gu : a.gu);
         const size_t T = (size_t)(shared ? 0 : sh.tab.expert[j]) * ntiles + rt * 8 + tl;
@@ -246,14 +241,13 @@ struct ExpertWork {
     }
     // row n of a block: its pair id (shared expert: npair + row), or -1
     __device__ int pair_of(int blk, int n) const {
-        const int j = slot_of(sh.tab, n_active, blk), i = (blk - sh.tab.base[j]) * NT + n;
+        const int j = slot(blk), i = (blk - sh.tab.base[j]) * NT + n;
         if (j == n_active) return i < nshared ? npair + i : -1;
         return i < sh.tab.cnt[j] ? a.lists.pairs[sh.tab.off[j] + i] : -1;
     }
     __device__ const __half* base() const { return DOWN ? a.hbuf : a.p; }
     __device__ uint32_t stride() const { return 0; }
-    __device__ Place row(int blk, int n) const {
-        const int p = pair_of(blk, n);
+    __device__ Place place(int p) const {                                   // of a pair
         if (p < 0) return NO_ROW;
         return (Place)(DOWN ? p : (p >= npair ? a.shared_row0 + p - npair : p / a.topk)) * (Place)K;
     }
@@ -266,7 +260,7 @@ struct ExpertWork {
         __syncwarp();
 #pragma unroll
         for (int n = 0; n < NT; n += 32) sh.dst[quarter][n + lane] = pair_of(blk, n + lane);
-        const int j = slot_of(sh.tab, n_active, blk);
+        const int j = slot(blk);
         e.count = min(NT, (j == n_active ? nshared : sh.tab.cnt[j]) - (blk - sh.tab.base[j]) * NT);
         __syncwarp();
     }
@@ -337,8 +331,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     tc_fence_after();
     pdl_launch_dependents();
     const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
-    const int items = work.items(), KS = work.inputs() >> 7;              // KS: stages per item (even)
-    const int lo = (int)((long)items * blockIdx.x / gridDim.x), hi = (int)((long)items * (blockIdx.x + 1) / gridDim.x);
+    const int KS = work.inputs() >> 7;                                      // stages per item (even)
+    const TcRun run = work.run(blockIdx.x, gridDim.x);
     bool ok = true;
     if (warp == 0) {
         // ------------------------------------------------------------ mma
@@ -347,7 +341,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         const uint64_t db0 = umma_desc_sw128(smem);
         const uint32_t ta0 = tmem + 2 * ACC;
         int st = 0; uint32_t ph = 0;
-        for (int k = 0; k < hi - lo && ok; ++k) {
+        for (int k = 0; k < run.count && ok; ++k) {
             if (k >= 2) ok = tc_wait<LIMIT>(&s_acc_empty[k & 1], (uint32_t)(((k >> 1) - 1) & 1), &s_abort) && ok;
             tc_fence_after();
             const uint32_t acc = tmem + (uint32_t)((k & 1) * ACC);
@@ -382,12 +376,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         const uint32_t ta = tmem + 2 * ACC + ((uint32_t)(quarter * 32) << 16);
         uint2 wv[U][8]; uint32_t sv[U][2];                                  // [stage in flight][group, two words], (scale, bias)
         int f_k = 0, f_s = d >> 2;                                          // the fetch cursor: item of the run, stage of it
-        typename W::Walk fw = work.walk(lo);
-        TcTile ft = hi > lo ? work.tile(fw.blk, fw.rt, tl) : TcTile{nullptr, nullptr, 0, 0};
+        TcRun fw = run;
+        TcTile ft = run.count > 0 ? work.tile(fw.blk, fw.rt, tl) : TcTile{nullptr, nullptr, 0, 0};
         auto seek = [&] {                                                   // past the end of an item: on to the one that has stage f_s
             while (f_s >= KS) {
                 f_s -= KS;
-                if (++f_k >= hi - lo) { ft.w = nullptr; f_s = 0; return; }
+                if (++f_k >= run.count) { ft.w = nullptr; f_s = 0; return; }
                 work.next(fw);
                 if (ft.w && fw.blk == ft.blk && fw.rt == ft.rt + 1 && work.has_tile(fw.rt, tl)) { ft.w += KS * 512; ft.s += KS * 64; ++ft.rt; }      // eight tiles on
                 else ft = work.tile(fw.blk, fw.rt, tl);
@@ -402,7 +396,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
                 const uint32_t* q = reinterpret_cast<const uint32_t*>(ft.s + f_s * 8 + (row & 7)) + (row >> 3);
                 sc[0] = __ldg(q); sc[1] = __ldg(q + 2);
             }
-            if (f_k < hi - lo) { f_s += 4; seek(); }
+            if (f_k < run.count) { f_s += 4; seek(); }
         };
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -411,7 +405,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
             sv[u][0] = 0; sv[u][1] = 0;
             fetch(wv[u], sv[u]);
         }
-        const int total = (hi - lo) * KS;                                   // stages of the run
+        const int total = run.count * KS;                                     // stages of the run
         int n = d >> 2, st = n;
         uint32_t ph = 1;                                                    // parity of the stage's "empty" (a fresh barrier passes at 1)
         while (n < total && ok) {
@@ -445,21 +439,26 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         const __half* base = work.base() + chunk * 8;
         typename W::Place src[W::STRIDED ? 1 : NP];                         // row places (strided: of the first row)
         int st = 0; uint32_t ph = 1;
-        typename W::Walk at = work.walk(lo);
+        TcRun at = run;
         int held = -1, have = 0;                                            // held: the block whose row places are in src; have: its rows (strided)
-        for (int k = 0; k < hi - lo && ok && !STALL; ++k) {
+        int next[W::STRIDED ? 1 : NP];                                      // the next item's pairs, looked up an item ahead
+        if constexpr (!W::STRIDED) { for (int h = 0; h < NP; ++h) next[h] = run.count > 0 ? work.pair_of(at.blk, n0 + 16 * h) : -1; }
+        for (int k = 0; k < run.count && ok && !STALL; ++k) {
             const int blk = at.blk;
-            if (blk != held) {
-                held = blk;
-                if (W::STRIDED) {
+            work.next(at);
+            if constexpr (W::STRIDED) {
+                if (blk != held) {
+                    held = blk;
                     src[0] = work.row(blk, n0); have = 0;
                     for (int h = 0; h < NP; ++h) have += work.row(blk, n0 + 16 * h) != W::NO_ROW;
-                } else {
+                }
+            } else {
 #pragma unroll
-                    for (int h = 0; h < NP; ++h) src[W::STRIDED ? 0 : h] = work.row(blk, n0 + 16 * h);
+                for (int h = 0; h < NP; ++h) {
+                    src[h] = work.place(next[h]);
+                    if (k + 1 < run.count && at.blk != blk) next[h] = work.pair_of(at.blk, n0 + 16 * h);
                 }
             }
-            work.next(at);
 #pragma unroll 1
             for (int s = 0; s < KS; ++s) {
                 ok = tc_wait<LIMIT>(&s_empty[st], ph, &s_abort) && ok;
@@ -492,8 +491,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         pdl_wait();                                                         // (residual rows, and rows that the kernel before may still read)
         typename W::Epi epi;
         const int quarter = warp - TC_EPI0;
-        typename W::Walk at = work.walk(lo);
-        for (int k = 0; k < hi - lo && ok; ++k) {
+        TcRun at = run;
+        for (int k = 0; k < run.count && ok; ++k) {
             work.begin(epi, at.blk, quarter, lane);
             ok = tc_agree(tc_wait<LIMIT>(&s_acc_full[k & 1], (uint32_t)((k >> 1) & 1), &s_abort));
             tc_fence_after();

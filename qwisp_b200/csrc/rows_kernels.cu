@@ -522,9 +522,9 @@ bool launch_head_rows(const DenseArgs& a, cudaStream_t st, bool pdl) {
 }
 
 // ================================================================================ experts
-// Work: (expert slot, block of 8 of its rows) x tiles of 16 weight rows, block-major; slot n_active is the shared expert
+// Work: (expert slot, block of 8 or 16 of its rows) x tiles of 16 weight rows, block-major; slot n_active is the shared expert
 // (all rows).  A CTA per multiprocessor takes an equal, contiguous run of the tiles (one to three blocks at decode sizes)
-// and its 24 consumer warps walk that run, a tile over the whole K each.  A producer warp gathers the rows of the next block
+// and its 24 (16) consumer warps walk that run, a tile over the whole K each.  A producer warp gathers the rows of the next block
 // into a ring of shared-memory stages with bulk copies (mbarrier full / empty): no CTA-wide barrier between experts, which
 // is what bounded the pass kernels when every expert has one or two rows.
 // Bound: instruction issue first (the 4-bit expansion is about 150 of the 260 instructions that a slice of 16 x 256 weights
@@ -532,24 +532,60 @@ bool launch_head_rows(const DenseArgs& a, cudaStream_t st, bool pdl) {
 // the issue slots empty), whole runs instead of items of 16 tiles (seven rounds for the work of 6.2), and a slice's weights
 // by 16-byte asynchronous copies two slices ahead (110 KB per SM in flight; bulk copies of 2 KB arrive later; rows
 // straight from L1 instead of staged: eight lines per load, 89 us for gate/up).  Batch of 64 (event times, 4.5 us of
-// them the events'): gate/up 73.6 -> 67.7 us, down 53.4 -> 43.3; 7 rows: 27.0 -> 23.0, 18.9 -> 18.8.
-constexpr int XR_WARPS = 24;
-constexpr int XR_BLOCKS = 64;                 // most (slot, block) entries of a CTA's run
-constexpr int XR_THREADS = (XR_WARPS + 1) * 32;
-struct XrBlock { int expert; int src[8], dst[8]; };   // expert -1: the shared one; src, dst -1: no row
-struct XrStage {                              // the rows of a block in shared memory
-    __half* xs;                               // [8][K + 8]
-    float* sxs;                               // [8][K/64 + 4]
-    float* craw;                              // down: [8][K/8] chunk sums as written by the gate/up kernel
+// them the events'): gate/up 73.6 -> 64 us, down 53.4 -> 43.
+// Blocks of 16 rows share the expansion (512 rows: 152 + 94 -> 129 + 80 us); the second half of a block of at most 8 rows is not computed.
+__host__ __device__ constexpr int xr_blocks(int RG) { return 64 / RG; }        // most (slot, block) entries of a CTA's run
+__host__ __device__ constexpr int xr_warps(int RG) { return RG == 1 ? 24 : 16; }       // consumer warps
+template <int NR>
+struct XrBlock { int expert, count; int src[NR], dst[NR]; };   // expert -1: the shared one; count: rows; src, dst -1: no row
+struct XrStage {                              // the NR rows of a block in shared memory
+    __half* xs;                               // [NR][K + 8]
+    float* sxs;                               // [NR][K/64 + 4]
+    float* craw;                              // down: [NR][K/8] chunk sums as written by the gate/up kernel
 };
 template <bool DOWN>
-__host__ __device__ constexpr size_t xr_stage_bytes(int K) { return (size_t)8 * (K + 8) * 2 + (size_t)8 * (K / 64 + 4) * 4 + (DOWN ? (size_t)8 * (K / 8) * 4 : 0); }
+__host__ __device__ constexpr size_t xr_stage_bytes(int K, int NR) { return (size_t)NR * (K + 8) * 2 + (size_t)NR * (K / 64 + 4) * 4 + (DOWN ? (size_t)NR * (K / 8) * 4 : 0); }
+template <int NR>
 __device__ __forceinline__ XrStage xr_carve(unsigned char* base, int K) {
     XrStage s;
-    s.xs = reinterpret_cast<__half*>(base); base += (size_t)8 * (K + 8) * 2;
-    s.sxs = reinterpret_cast<float*>(base); base += (size_t)8 * (K / 64 + 4) * 4;
+    s.xs = reinterpret_cast<__half*>(base); base += (size_t)NR * (K + 8) * 2;
+    s.sxs = reinterpret_cast<float*>(base); base += (size_t)NR * (K / 64 + 4) * 4;
     s.craw = reinterpret_cast<float*>(base);
     return s;
+}
+// One slice of a tile, in a ring slot, against RG x 8 rows of a stage (xp: this lane's row of the first eight, sx: the slice's group
+// sums of column 2t, of column 2t + 1 SXS floats on).  The order of operations per column is that of compute_slice_x().
+template <int RG, int XS, int SXS>
+__device__ __forceinline__ void xr_slice(const unsigned char* slot, const __half* xp, const float* sx, int lane, float (*tot)[4]) {
+    const uint4* w = reinterpret_cast<const uint4*>(slot);
+    float4 sa[RG], sb[RG];
+    float accS[RG][4], accB[RG][4];
+#pragma unroll
+    for (int q = 0; q < RG; ++q) {
+        sa[q] = *reinterpret_cast<const float4*>(sx + q * 8 * SXS); sb[q] = *reinterpret_cast<const float4*>(sx + (q * 8 + 1) * SXS);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) accS[q][i] = accB[q][i] = 0.f;
+    }
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        const uint4 wv = w[g * 32 + lane];
+        uint32_t a0[4], b0[4], a1[4], b1[4];
+        dequant8(wv.x, a0); dequant8(wv.z, b0); dequant8(wv.y, a1); dequant8(wv.w, b1);
+        const uint2 sv = *reinterpret_cast<const uint2*>(slot + 2048 + (g >> 1) * 128 + (lane >> 2) * 16 + (g & 1) * 8);
+        const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&sv.x)), fb = __half22float2(*reinterpret_cast<const __half2*>(&sv.y));
+#pragma unroll
+        for (int q = 0; q < RG; ++q) {
+            const uint4 X0 = *reinterpret_cast<const uint4*>(xp + q * 8 * XS + 64 * g), X1 = *reinterpret_cast<const uint4*>(xp + q * 8 * XS + 64 * g + 8);
+            float c[4];
+            mma_f16_z(c, a0[0], b0[0], a0[1], b0[1], X0.x, X0.y);
+            mma_f16(c, a0[2], b0[2], a0[3], b0[3], X0.z, X0.w);
+            mma_f16(c, a1[0], b1[0], a1[1], b1[1], X1.x, X1.y);
+            mma_f16(c, a1[2], b1[2], a1[3], b1[3], X1.z, X1.w);
+            const float sx0 = g == 0 ? sa[q].x : g == 1 ? sa[q].y : g == 2 ? sa[q].z : sa[q].w, sx1 = g == 0 ? sb[q].x : g == 1 ? sb[q].y : g == 2 ? sb[q].z : sb[q].w;
+            scale_group<false>(c, fa, fb, make_float2(sx0, sx1), accS[q], accB[q]);
+        }
+    }
+    add_slice<RG>(tot, accS, accB);
 }
 // The routing of a call of at most XR_ROUTE rows, done by every CTA from the logits (a warp per row) in place of a kernel that routes and
 // leaves lists: the choices, the slots in the order of their experts and the pairs of each slot in the order of their rows (all CTAs
@@ -591,45 +627,47 @@ __device__ __forceinline__ int slot_route(SlotTable& t, unsigned* rows, int* fir
     if (mine) pairs[first[id] + __popc(rows[id] & ((1u << m) - 1u))] = m * a.topk + lane;
     return n_active;
 }
-// S: slices of K.  STALL: a test's form, in which no row is ever fetched, so that every consumer's wait runs out, and soon
-template <bool DOWN, int S, bool STALL>
-__global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int lg_tiles, int nstages) {
+// S: slices of K.  RG: blocks of 8 or 16 rows.  STALL: a test's form, in which no row is ever fetched, so that every consumer's wait runs out, and soon
+template <bool DOWN, int S, int RG, bool STALL>
+__global__ void __launch_bounds__((xr_warps(RG) + 1) * 32, 1) k_expert_rows(ExpertArgs a, int lg_tiles, int nstages) {
     extern __shared__ __align__(16) unsigned char smem[];        // weight rings, then nstages stages
     __shared__ __align__(8) uint64_t s_full[8], s_empty[8], s_raw[8];
     __shared__ SlotTable s_tab;
-    __shared__ XrBlock s_blk[XR_BLOCKS];
+    constexpr int XR_WARPS = xr_warps(RG), XR_THREADS = (XR_WARPS + 1) * 32, NR = 8 * RG;
+    __shared__ XrBlock<NR> s_blk[xr_blocks(RG)];
     __shared__ int s_sig, s_abort, s_pairs[XR_ROUTE * 32];
     constexpr int K = S << 8, G64 = K >> 6, SXS = G64 + 4, XS = K + 8;
-    constexpr size_t stage_bytes = xr_stage_bytes<DOWN>(K);
+    constexpr size_t stage_bytes = xr_stage_bytes<DOWN>(K, NR);
     unsigned char* stages = smem + (size_t)XR_WARPS * XR_DEPTH * XR_UNIT;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, t = lane & 3;
     const int ntiles = 1 << lg_tiles, npair = a.M * a.topk;
     const int nshared = a.M_shared >= 0 ? a.M_shared : a.M;
     if (tid == 0) {
         s_abort = 0;
-        for (int i = 0; i < nstages; ++i) { mbar_init(&s_full[i], DOWN ? 1 : 8); mbar_init(&s_empty[i], XR_WARPS); mbar_init(&s_raw[i], 8); }
+        for (int i = 0; i < nstages; ++i) { mbar_init(&s_full[i], DOWN ? 1 : NR); mbar_init(&s_empty[i], XR_WARPS); mbar_init(&s_raw[i], NR); }
         mbar_fence_init();
     }
     if (!DOWN) pdl_wait();                                      // the lists, or the logits (down: they were there before gate/up started)
     pdl_launch_dependents();
     unsigned* scratch = reinterpret_cast<unsigned*>(s_blk);     // (filled below)
     static_assert(sizeof(s_blk) >= 512 * sizeof(int), "counters of slot_route()");
-    const int n_active = a.route_here ? slot_route(s_tab, scratch, reinterpret_cast<int*>(scratch + 256), s_pairs, a, 8, nshared) : slot_table(s_tab, a.lists, 8, nshared);
-    const int* pairs = a.route_here ? s_pairs : a.lists.pairs;
+    const int n_active = RG == 1 && a.route_here ? slot_route(s_tab, scratch, reinterpret_cast<int*>(scratch + 256), s_pairs, a, NR, nshared) : slot_table(s_tab, a.lists, NR, nshared);
+    const int* pairs = RG == 1 && a.route_here ? s_pairs : a.lists.pairs;
     __syncthreads();
     const long total = (long)s_tab.base[n_active + 1] << lg_tiles;
     const int lo = (int)(total * blockIdx.x / gridDim.x), hi = (int)(total * (blockIdx.x + 1) / gridDim.x);
     const int b0 = lo >> lg_tiles, nb = hi > lo ? ((hi - 1) >> lg_tiles) - b0 + 1 : 0;
-    for (int i = tid; i < nb * 8; i += XR_THREADS) {           // the rows of the run's blocks
-        const int sb = b0 + (i >> 3), j = slot_of(s_tab, n_active, sb), first = (sb - s_tab.base[j]) * 8, ridx = first + (i & 7);
+    for (int i = tid; i < nb * NR; i += XR_THREADS) {           // the rows of the run's blocks
+        const int sb = b0 + i / NR, n = i % NR, j = slot_of(s_tab, n_active, sb), first = (sb - s_tab.base[j]) * NR, ridx = first + n;
         const bool shared = (j == n_active);
-        const bool have = ridx < (shared ? nshared : s_tab.cnt[j]);
+        const int cnt = shared ? nshared : s_tab.cnt[j];
+        const bool have = ridx < cnt;
         int dst = -1, src = -1;
         if (have && shared) { dst = npair + ridx; src = DOWN ? dst : a.shared_row0 + ridx; }
         else if (have) { dst = pairs[s_tab.off[j] + ridx]; src = DOWN ? dst : dst / a.topk; }
-        XrBlock& b = s_blk[i >> 3];
-        b.src[i & 7] = src; b.dst[i & 7] = dst;
-        if ((i & 7) == 0) b.expert = shared ? -1 : s_tab.expert[j];
+        XrBlock<NR>& b = s_blk[i / NR];
+        b.src[n] = src; b.dst[n] = dst;
+        if (n == 0) { b.count = cnt - first; b.expert = shared ? -1 : s_tab.expert[j]; }
     }
     __syncthreads();
     unsigned fail_code = 0;          // which wait ran out: 16 producer/empty, 32 producer/chunk sums, 64 consumer/full
@@ -638,9 +676,9 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
         if (DOWN) pdl_wait();                                  // the gate/up kernel's rows
         for (int k = 0; k < nb && !STALL; ++k) {
             const int stg = k % nstages, use = k / nstages;
-            const XrStage St = xr_carve(stages + (size_t)stg * stage_bytes, K);
+            const XrStage St = xr_carve<NR>(stages + (size_t)stg * stage_bytes, K);
             if (use > 0 && !xr_wait<STALL>(&s_empty[stg], (uint32_t)((use - 1) & 1), &s_abort)) { fail_code |= 16u; break; }
-            if (lane < 8) {
+            if (lane < NR) {
                 uint64_t* bar = DOWN ? &s_raw[stg] : &s_full[stg];
                 const int src = s_blk[k].src[lane];
                 if (src >= 0) {
@@ -655,7 +693,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
             if (DOWN) {
                 // group sums from the chunk sums: eight of them combined in the butterfly order of rows_store()
                 if (!xr_wait<STALL>(&s_raw[stg], (uint32_t)(use & 1), &s_abort)) { fail_code |= 32u; break; }
-                for (int i = lane; i < 8 * G64; i += 32) {
+                for (int i = lane; i < NR * G64; i += 32) {
                     const int row = i / G64, g = i - row * G64;
                     const float* c = St.craw + (size_t)row * (K / 8) + g * 8;
                     const float4 lo4 = *reinterpret_cast<const float4*>(c), hi4 = *reinterpret_cast<const float4*>(c + 4);
@@ -668,7 +706,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
             }
         }
         // the choices and gates of row m, for the combine, from CTA m (nobody waits for them here)
-        if (!DOWN && a.route_here) {
+        if (RG == 1 && !DOWN && a.route_here) {
             __shared__ float s_gate[256];
             for (int m = blockIdx.x; m < a.M; m += gridDim.x) {
                 __syncwarp();
@@ -703,7 +741,7 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
     for (int i = lo + warp; i < hi; i += XR_WARPS) {
         tile_of(i + NB * XR_WARPS, wn, cn);
         const int bi = (i >> lg_tiles) - b0, tile = i & (ntiles - 1);
-        const XrBlock& b = s_blk[bi];
+        const XrBlock<NR>& b = s_blk[bi];
         if (bi != cur) {                                          // done with the stages of the blocks before
             __syncwarp();
             if (lane == 0) for (int u = cur; u < bi; ++u) mbar_arrive(&s_empty[u % nstages]);
@@ -711,28 +749,38 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
         }
         if (!here && !xr_wait<STALL>(&s_full[bi % nstages], (uint32_t)((bi / nstages) & 1), &s_abort)) { fail_code |= 64u; break; }
         here = true;
-        const XrStage St = xr_carve(stages + (size_t)(bi % nstages) * stage_bytes, K);
+        const XrStage St = xr_carve<NR>(stages + (size_t)(bi % nstages) * stage_bytes, K);
         const __half* xp = St.xs + (size_t)r * XS + 16 * t;
         const float *sx0 = St.sxs + 2 * t * SXS, *sx1 = sx0 + SXS;
-        float tot[1][4] = {{0.f, 0.f, 0.f, 0.f}};
+        float tot[RG][4];
+#pragma unroll
+        for (int i = 0; i < RG * 4; ++i) tot[i >> 2][i & 3] = 0.f;
+        const bool full = RG == 1 || b.count > 8;                 // (16 rows: of a block's last eight there may be none)
 #pragma unroll
         for (int s = 0; s < S; ++s) {
             const int slot = S >= XR_DEPTH ? s % XR_DEPTH : odd;
-            XRegs xr;
-            const float4 sa = *reinterpret_cast<const float4*>(sx0 + s * 4), sb = *reinterpret_cast<const float4*>(sx1 + s * 4);
-            xr.sx[0] = make_float2(sa.x, sb.x); xr.sx[1] = make_float2(sa.y, sb.y); xr.sx[2] = make_float2(sa.z, sb.z); xr.sx[3] = make_float2(sa.w, sb.w);
+            if constexpr (RG == 1) {
+                XRegs xr;
+                const float4 sa = *reinterpret_cast<const float4*>(sx0 + s * 4), sb = *reinterpret_cast<const float4*>(sx1 + s * 4);
+                xr.sx[0] = make_float2(sa.x, sb.x); xr.sx[1] = make_float2(sa.y, sb.y); xr.sx[2] = make_float2(sa.z, sb.z); xr.sx[3] = make_float2(sa.w, sb.w);
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                xr.x[2 * g] = *reinterpret_cast<const uint4*>(xp + s * 256 + 64 * g);
-                xr.x[2 * g + 1] = *reinterpret_cast<const uint4*>(xp + s * 256 + 64 * g + 8);
+                for (int g = 0; g < 4; ++g) {
+                    xr.x[2 * g] = *reinterpret_cast<const uint4*>(xp + s * 256 + 64 * g);
+                    xr.x[2 * g + 1] = *reinterpret_cast<const uint4*>(xp + s * 256 + 64 * g + 8);
+                }
+                cp_async_wait<XR_DEPTH - 1>();
+                __syncwarp();                                         // every lane's part of the slice is there
+                SliceRegs rg;
+                load_slice_smem(rg, reinterpret_cast<const uint4*>(ring + slot * XR_UNIT), reinterpret_cast<const uint4*>(ring + slot * XR_UNIT + 2048), lane);
+                float accS[1][4] = {{0.f, 0.f, 0.f, 0.f}}, accB[1][4] = {{0.f, 0.f, 0.f, 0.f}};
+                compute_slice_x(rg, xr, accS[0], accB[0]);
+                add_slice<1>(tot, accS, accB);
+            } else {
+                cp_async_wait<XR_DEPTH - 1>();
+                __syncwarp();
+                if (full) xr_slice<RG, XS, SXS>(ring + slot * XR_UNIT, xp + s * 256, sx0 + s * 4, lane, tot);
+                else xr_slice<1, XS, SXS>(ring + slot * XR_UNIT, xp + s * 256, sx0 + s * 4, lane, tot);
             }
-            cp_async_wait<XR_DEPTH - 1>();
-            __syncwarp();                                         // every lane's part of the slice is there
-            SliceRegs rg;
-            load_slice_smem(rg, reinterpret_cast<const uint4*>(ring + slot * XR_UNIT), reinterpret_cast<const uint4*>(ring + slot * XR_UNIT + 2048), lane);
-            float accS[1][4] = {{0.f, 0.f, 0.f, 0.f}}, accB[1][4] = {{0.f, 0.f, 0.f, 0.f}};
-            compute_slice_x(rg, xr, accS[0], accB[0]);
-            add_slice<1>(tot, accS, accB);
             __syncwarp();                                         // every lane has read the slot: it may be filled again
             if (S > XR_DEPTH && s + XR_DEPTH < S) request(slot, w0, c0, s + XR_DEPTH);
             else request(slot, wn, cn, S > XR_DEPTH ? s + XR_DEPTH - S : s);
@@ -740,28 +788,30 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
         w0 = wn; c0 = cn; odd ^= 1;
         if (DOWN) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int dst = b.dst[2 * t + (u & 1)];
+            for (int u = 0; u < 4 * RG; ++u) {
+                const int dst = b.dst[(u >> 2) * 8 + 2 * t + (u & 1)];
                 if (dst >= 0) {
                     __half* rowp = a.dbuf + (size_t)dst * a.H;
                     if (a.ep_pairs_per_rank > 0 && dst < npair) {       // routed pair in expert-parallel mode: the owner's buffer
                         const int own = dst / a.ep_pairs_per_rank;
                         rowp = a.peer_dbuf[own] + (size_t)(dst - own * a.ep_pairs_per_rank) * a.H;
                     }
-                    rowp[tile * 16 + r + 8 * (u >> 1)] = f2h(tot[0][u]);
+                    rowp[tile * 16 + r + 8 * (u >> 1 & 1)] = f2h(tot[u >> 2][u & 3]);
                 }
             }
         } else {
             // SwiGLU of (gate row r, up row r) per column; the 8 outputs of a column (lanes with the same t) form one
             // 8-chunk of the down projection's input: stored in the products' order with its chunk sum
 #pragma unroll
-            for (int jc = 0; jc < 2; ++jc) {
-                const __half hv = swiglu_h(f2h(tot[0][jc]), f2h(tot[0][2 + jc]));
+            for (int j = 0; j < 2 * RG; ++j) {
+                const int q = j >> 1, jc = j & 1;
+                if (q > 0 && !full) break;
+                const __half hv = swiglu_h(f2h(tot[q][jc]), f2h(tot[q][2 + jc]));
                 const unsigned hb = __half_as_ushort(hv);
                 unsigned v[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) v[u] = __shfl_sync(0xffffffffu, hb, u * 4 + t);
-                const int dst = b.dst[2 * t + jc];
+                const int dst = b.dst[q * 8 + 2 * t + jc];
                 if (r == 0 && dst >= 0) {
                     const uint4 nat = make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
                     *reinterpret_cast<uint4*>(a.hbuf + (size_t)dst * a.I + tile * 8) = make_uint4(nat.x, nat.z, nat.y, nat.w);
@@ -793,41 +843,49 @@ __global__ void __launch_bounds__(XR_THREADS, 1) k_expert_rows(ExpertArgs a, int
             st_release_sys(a.ep_sig.flags[tid] + 8 + a.ep_sig.rank, ep_seq(a.ep_sig.ctr, a.ep_sig.layer, 1));
     }
 }
-// the tiles (their binary logarithm) and the stages of a launch; false: shape not covered
+// the tiles (their binary logarithm) and the stages of a launch with blocks of 8 RG rows; false: shape not covered
 template <bool DOWN>
-static bool expert_rows_shape(const ExpertArgs& a, int& lg, int& nstages) {
-    const int ntiles = DOWN ? a.H / 16 : a.I / 8, K = DOWN ? a.I : a.H;
+static bool expert_rows_shape(const ExpertArgs& a, int RG, int& lg, int& nstages) {
+    const int ntiles = DOWN ? a.H / 16 : a.I / 8, K = DOWN ? a.I : a.H, NR = 8 * RG;
     if (!a.csum || (!DOWN && (!a.xq || !a.sxq)) || (K != 256 && K != 512 && K != 1024 && K != 2048 && K != 4096)) return false;
     lg = 0; while ((1 << lg) < ntiles) ++lg;
-    const long pairs = (long)a.M * a.topk, blocks = pairs / 8 + (pairs < 256 ? pairs : 256) + a.M / 8 + 1;    // at most one partial block per expert
-    nstages = (int)(((size_t)216 * 1024 - (size_t)XR_WARPS * XR_DEPTH * XR_UNIT) / xr_stage_bytes<DOWN>(K));
+    const long pairs = (long)a.M * a.topk, blocks = pairs / NR + (pairs < 256 ? pairs : 256) + a.M / NR + 1;    // at most one partial block per expert
+    nstages = (int)(((size_t)216 * 1024 - (size_t)xr_warps(RG) * XR_DEPTH * XR_UNIT) / xr_stage_bytes<DOWN>(K, NR));
     if (nstages > 8) nstages = 8;
-    return (1 << lg) == ntiles && blocks / sm_count() + 2 <= XR_BLOCKS && nstages >= 1;
+    return (1 << lg) == ntiles && blocks / sm_count() + 2 <= xr_blocks(RG) && nstages >= RG;
 }
 // A warp per row: more rows would be routed in turns by every CTA, and a kernel of its own is done sooner.
 bool expert_rows_route(const ExpertArgs& a) {
     int lg, nstages;
-    return a.M <= XR_ROUTE && a.E <= 256 && a.topk <= 32 && a.ep_pairs_per_rank == 0 && expert_rows_shape<false>(a, lg, nstages) && expert_rows_shape<true>(a, lg, nstages);
+    return a.M <= XR_ROUTE && a.E <= 256 && a.topk <= 32 && a.ep_pairs_per_rank == 0 && expert_rows_shape<false>(a, 1, lg, nstages) && expert_rows_shape<true>(a, 1, lg, nstages);
 }
-template <bool DOWN, int S, bool STALL = false>
+template <bool DOWN, int S, int RG, bool STALL = false>
 static bool launch_expert_rows_t(const ExpertArgs& a, cudaStream_t st, bool pdl) {
     const int grid = sm_count();
     int lg, nstages;
-    if (!expert_rows_shape<DOWN>(a, lg, nstages)) return false;
-    const size_t smem = (size_t)XR_WARPS * XR_DEPTH * XR_UNIT + xr_stage_bytes<DOWN>(S << 8) * nstages;
+    if (!expert_rows_shape<DOWN>(a, RG, lg, nstages)) return false;
+    const size_t smem = (size_t)xr_warps(RG) * XR_DEPTH * XR_UNIT + xr_stage_bytes<DOWN>(S << 8, 8 * RG) * nstages;
     static bool configured = false;
-    if (!configured) { cudaFuncSetAttribute(k_expert_rows<DOWN, S, STALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
-    profile_launch(DOWN ? "k_expert_rows_down" : "k_expert_rows_gateup", st, [&] { return launch_pdl(pdl, k_expert_rows<DOWN, S, STALL>, dim3((unsigned)grid), XR_THREADS, smem, st, a, lg, nstages); });
+    if (!configured) { cudaFuncSetAttribute(k_expert_rows<DOWN, S, RG, STALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); configured = true; }
+    profile_launch(DOWN ? "k_expert_rows_down" : "k_expert_rows_gateup", st, [&] { return launch_pdl(pdl, k_expert_rows<DOWN, S, RG, STALL>, dim3((unsigned)grid), (xr_warps(RG) + 1) * 32, smem, st, a, lg, nstages); });
     return true;
+}
+// Blocks of 16 rows from a mean of more than 8 rows an expert: with fewer most blocks would be half empty, and the 16 warps that
+// two stages of 16 rows leave room for are slower than 24 (gate/up + down, 256 experts, 8 a row, evenly: 192 rows 121 us in blocks of 8,
+// 136 in blocks of 16, 256 rows 150 and 150, 320 rows 174 and 154, 512 rows 245 and 208).  For K = 4096 there is no room.
+template <bool DOWN, int S>
+static bool launch_expert_rows_s(const ExpertArgs& a, cudaStream_t st, bool pdl) {
+    if ((long)a.M * a.topk > 8l * a.E && !a.route_here && launch_expert_rows_t<DOWN, S, 2>(a, st, pdl)) return true;
+    return launch_expert_rows_t<DOWN, S, 1>(a, st, pdl);
 }
 template <bool DOWN>
 static bool launch_expert_rows_d(const ExpertArgs& a, cudaStream_t st, bool pdl) {
     switch (DOWN ? a.I : a.H) {
-        case 256: return launch_expert_rows_t<DOWN, 1>(a, st, pdl);
-        case 512: return !DOWN && a.stall ? launch_expert_rows_t<DOWN, 2, !DOWN>(a, st, pdl) : launch_expert_rows_t<DOWN, 2>(a, st, pdl);
-        case 1024: return launch_expert_rows_t<DOWN, 4>(a, st, pdl);
-        case 2048: return launch_expert_rows_t<DOWN, 8>(a, st, pdl);
-        case 4096: return launch_expert_rows_t<DOWN, 16>(a, st, pdl);
+        case 256: return launch_expert_rows_s<DOWN, 1>(a, st, pdl);
+        case 512: return !DOWN && a.stall ? launch_expert_rows_t<DOWN, 2, 1, !DOWN>(a, st, pdl) : launch_expert_rows_s<DOWN, 2>(a, st, pdl);
+        case 1024: return launch_expert_rows_s<DOWN, 4>(a, st, pdl);
+        case 2048: return launch_expert_rows_s<DOWN, 8>(a, st, pdl);
+        case 4096: return launch_expert_rows_t<DOWN, 16, 1>(a, st, pdl);
         default: return false;
     }
 }

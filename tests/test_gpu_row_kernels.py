@@ -88,6 +88,17 @@ def test_rows_routed_by_the_expert_kernels(engines, M):
     assert same(ha, hb) and np.array_equal(ba, bb) and same(oa, ob) and np.array_equal(ia, ib) and same(sa, sb)
 
 
+# expert blocks of 16 rows (a mean of more than 8 rows an expert): blocks of at most 8 rows among them, one and many blocks of an expert
+@pytest.mark.parametrize("M", [25, 30, 47, 66, 257, 512])
+def test_expert_blocks_of_sixteen_rows(engines, M):
+    import qwisp_b200 as Q
+    x = np.random.default_rng(M).standard_normal((M, MINI["hidden"])).astype(np.float16)
+    (oa, ia, sa), (ob, ib, sb) = (Q.ops.moe_block(e, 0, x) for e in engines)
+    counts = np.bincount(ia.ravel(), minlength=MINI["n_experts"])
+    assert M * MINI["top_k"] > 8 * MINI["n_experts"] and np.any(counts > 8) and np.any((counts - 1) % 16 < 8)
+    assert np.array_equal(ia, ib) and same(sa, sb) and same(oa, ob)
+
+
 # chunks of the state scan: a chunk less or more one row, remainders of its turns, behind a history
 @pytest.mark.parametrize("M", [3, 5, 47, 48, 49, 50, 97, 145])
 def test_state_scan_chunks(engines, M):

@@ -1370,7 +1370,10 @@ void launch_attn_prep(const AttnArgs& a, cudaStream_t st, bool pdl) {
 // Bound by latency: a warp has four keys of a 32-key split, and a CTA per split spent 2.4 us on descriptors, pages, two
 // keys in flight and the merge.  So: runs as long as the device stays full, the warp's next eight keys always in flight (a
 // ring in shared memory that every lane fills and reads for itself), and their rows looked up 32 at a time.  By events:
-// 512 rows of one stream 406 -> 278 us, 64 streams 87 -> 48, 17 rows at 1000 keys 64 -> 46.
+// 512 rows of one stream 406 -> 278 us, 64 streams 87 -> 48, 17 rows at 1000 keys 64 -> 46.  Of the 278 a third were the merges
+// of the warps: a thread now sums four dims of one head from quads without bank conflicts, with the factors that the warps
+// made for their own rows, and a chunk's longest rows start first: 235, 50 (a context of 192), 43 us.  Four keys side by side
+// in a warp, their latencies overlapped, were no faster (244, 52, 43.5: the other three warps of a scheduler cover them).
 __device__ __forceinline__ void af_cp16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
@@ -1379,12 +1382,12 @@ constexpr size_t AF_SMEM = (size_t)8 * 4 * ATT_D * 4 + (size_t)8 * AF_RING * ATT
 __global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, int fill, unsigned* counters) {
     extern __shared__ __align__(16) float sm_acc[];           // [8 warps][4 heads][256], then the rings
     constexpr int HG = 4;                                     // query heads of a CTA
-    __shared__ __align__(16) float sm_m[2][8][HG], sm_l[2][8][HG];
+    __shared__ __align__(16) float sm_m[2][8][HG], sm_l[2][8][HG], sm_f[8][HG];
     __shared__ __align__(16) __half sq[HG][ATT_D];
     __shared__ __align__(16) __half sk[ATT_D], sv[ATT_D];
     __shared__ int s_last;
     __shared__ float s_cs[32], s_sn[32];
-    const int kvh = blockIdx.y >> 1, h0 = blockIdx.y * HG, m = blockIdx.z;      // h0: first query head
+    const int kvh = blockIdx.y >> 1, h0 = blockIdx.y * HG, m = gridDim.z - 1 - blockIdx.z;      // h0: first query head; the longest rows of a chunk first
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Ahead of the programmatic-launch wait: everything that does not depend on this step's in-projection.
     // Stream lengths and page tables were written before the step; with prep != 0 every position below the
@@ -1493,28 +1496,30 @@ __global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, int
 #pragma unroll
         for (int g = 0; g < HG; ++g) {
             const float f = (mine[g] == -INFINITY) ? 0.f : __expf(mine[g] - gms[g]);
+            if (lane == g) sm_f[warp][g] = f;
             const f32x2 f2 = pk2(f, f);
-            float4* dst = reinterpret_cast<float4*>(sm_acc + ((size_t)warp * HG + g) * ATT_D + lane * 8);
+            float4* dst = reinterpret_cast<float4*>(sm_acc + ((size_t)warp * HG + g) * ATT_D);      // (quads swapped in pairs by the lane: no bank conflicts)
             const float2 a0 = unpk2(mul2(acc[g][0], f2)), a1 = unpk2(mul2(acc[g][1], f2)), a2 = unpk2(mul2(acc[g][2], f2)), a3 = unpk2(mul2(acc[g][3], f2));
-            dst[0] = make_float4(a0.x, a0.y, a1.x, a1.y);
-            dst[1] = make_float4(a2.x, a2.y, a3.x, a3.y);
+            dst[(2 * lane) ^ (lane >> 2 & 1)] = make_float4(a0.x, a0.y, a1.x, a1.y);
+            dst[(2 * lane + 1) ^ (lane >> 2 & 1)] = make_float4(a2.x, a2.y, a3.x, a3.y);
         }
         __syncthreads();
-        const int d = threadIdx.x;                            // 256 threads = 256 dims
-        float* po = a.part_o + (((size_t)m * a.NH + h0) * a.nsplit + sp) * ATT_D;
+        const int og = threadIdx.x >> 6, oq = threadIdx.x & 63;      // a thread: a quad of a head's dims
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int g = 0; g < HG; ++g) {
-            float o = 0.f;
-#pragma unroll
-            for (int w = 0; w < 8; ++w) o += sm_acc[((size_t)w * HG + g) * ATT_D + d];
-            po[(size_t)g * a.nsplit * ATT_D + d] = o;
+        for (int w = 0; w < 8; ++w) {
+            const float4 v = reinterpret_cast<const float4*>(sm_acc + ((size_t)w * HG + og) * ATT_D)[oq ^ (oq >> 3 & 1)];
+            o.x += v.x; o.y += v.y; o.z += v.z; o.w += v.w;
         }
+        *reinterpret_cast<float4*>(a.part_o + (((size_t)m * a.NH + h0 + og) * a.nsplit + sp) * ATT_D + oq * 4) = o;
         if (threadIdx.x < HG) {
             const int g = threadIdx.x;
-            float m8[8], l8[8];
-            for (int w = 0; w < 8; ++w) { m8[w] = sm_m[pb][w][g]; l8[w] = sm_l[pb][w][g]; }
-            const float gm = attn_warps_max(m8);
-            const float ls = attn_warps_lsum(m8, l8, gm);
+            float gm = -INFINITY, ls = 0.f;                   // attn_warps_max(), attn_warps_lsum() with the factors from above
+#pragma unroll
+            for (int w = 0; w < 8; ++w) {
+                gm = fmaxf(gm, sm_m[pb][w][g]);
+                ls = __fadd_rn(ls, __fmul_rn(sm_l[pb][w][g], sm_f[w][g]));
+            }
             float* pml = a.part_ml + (((size_t)m * a.NH + h0 + g) * a.nsplit + sp) * 2;
             pml[0] = gm; pml[1] = ls;
         }

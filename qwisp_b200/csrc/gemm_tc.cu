@@ -11,10 +11,10 @@
 // a fixed order, so results do not depend on how many rows share a call or on how a prompt is cut into calls.
 //
 // One kernel, k_tc, serves the dense projections (DenseWork) and the grouped experts (ExpertWork): persistent CTAs, one
-// per multiprocessor, walk a run of items of 128 weight rows x NT activation rows over the whole K, 128 inputs a stage.
+// per multiprocessor, each take their items of 128 weight rows x NT activation rows over the whole K, 128 inputs a stage.
 // The warps have roles and meet only at mbarriers:
-//   mma        1 warp: waits for a full stage, issues its eight MMAs (M=128, N=NT, K=16), commits them to the stage's
-//             "empty" barrier.  It is warp 0: the other warps keep the issue slots busy;
+//   mma        1 warp: waits for two full stages, issues their sixteen MMAs (M=128, N=NT, K=16), commits them to the stages'
+//             "empty" barriers.  It is warp 0: the other warps keep the issue slots busy;
 //   load       4 warps: the NT x 128 activations of the stage, 16-byte asynchronous copies that count themselves in at
 //             the stage's "full" barrier;
 //   dequant   16 warps: a warp owns 32 weight rows of the item (a lane a row: a lane of tensor memory is a row) and every
@@ -25,9 +25,10 @@
 // spent 2.5 us on a pair of groups whose MMAs take 0.3: every pair paid the latency of its weights and of its rows.
 // With roles but the A operand in shared memory, writing and reading it took most of that memory's bandwidth, and an MMA
 // warp that branched on its lane number needed 1200 cycles a stage to compute addresses: uniform code needs 700.
-// 1024-token chunk of the 2048 / 512 / 256-expert geometry (event times): experts 223 + 138 -> 158 + 109 us, dense
-// 105 -> 51; bound now by the issue of the expansion: counters of such a chunk give the ALU pipe 62 % of the active cycles
-// and the issue slots 67 %, the tensor pipe 47 % (dense 12352 x 2048), 26 % (gate/up) and 21 % (down).
+// 1024-token chunk of the 2048 / 512 / 256-expert geometry (alone, back to back, evenly routed): experts 101 + 70 us, dense
+// 12352 x 2048 54 us (0.95 PFLOP/s); 129 tokens: 77 + 47 and 18.6 us.  With a fragment of a row a lane, so that a quarter of the
+// warp had to exchange its words, the experts took 158 + 109.  The experts are bound by the issue of the expansion (129 tokens,
+// gate/up: issue slots 71 %, ALU 48 %, tensor pipe 22 % of the active cycles), the large dense products by rows and weights out of L2.
 #include "kernels.h"
 #include "gemv.cuh"
 

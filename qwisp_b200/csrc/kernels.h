@@ -84,8 +84,9 @@ struct ExpertArgs {
     __half* hbuf;                        // [(M*topk + M)][I]
     __half* dbuf;                        // [(M*topk + M)][H]
     int M, H, I, topk;
+    int E = 0;                           // experts of the model (of all ranks): a launch goes by the mean rows of an expert
     const __half* rlogits = nullptr;     // route_here: router logits [M][E]; every CTA routes from them itself (deterministic, so all CTAs
-    int E = 0; int route_here = 0;       //   agree) instead of waiting for a routing kernel or a routing tail in the router kernel
+    int route_here = 0;                  //   agree) instead of waiting for a routing kernel or a routing tail in the router kernel
     int* inds_out = nullptr; __half* scores_out = nullptr;   //   the result, published by one CTA (fused kernel) or one CTA per row
     int lg_slices2 = 0;                  // fused kernel: log2(I/256) of the down phase
     unsigned* slot_sync = nullptr;       // fused kernel: [2][top_k + 1] counters, zero between launches

@@ -873,6 +873,7 @@ static bool launch_expert_rows_t(const ExpertArgs& a, cudaStream_t st, bool pdl)
 // Blocks of 16 rows from a mean of more than 8 rows an expert: with fewer most blocks would be half empty, and the 16 warps that
 // two stages of 16 rows leave room for are slower than 24 (gate/up + down, 256 experts, 8 a row, evenly: 192 rows 121 us in blocks of 8,
 // 136 in blocks of 16, 256 rows 150 and 150, 320 rows 174 and 154, 512 rows 245 and 208).  For K = 4096 there is no room.
+// Expert-parallel calls too: their rows are those of all ranks, and the mean over all experts is that of the rank's own.
 template <bool DOWN, int S>
 static bool launch_expert_rows_s(const ExpertArgs& a, cudaStream_t st, bool pdl) {
     if ((long)a.M * a.topk > 8l * a.E && !a.route_here && launch_expert_rows_t<DOWN, S, 2>(a, st, pdl)) return true;

@@ -1,7 +1,7 @@
 // A stand-in for the CUDA runtime on the host, for tests of the library's host side without a GPU: preloaded in front of
 // libcudart, it gives "device" memory from the heap, runs copies at once and kernels not at all, and makes the calls fail that a
 // test asks it to fail.  Of the kernels only k_state_io is imitated: packing leaves each word's number, unpacking notes what
-// arrived for each word.
+// arrived for each word.  Found as libnccl.so.2 as well, it is that library for a rank whose peers do not exist.
 #include <cuda_runtime_api.h>
 #include <dlfcn.h>
 #include <errno.h>
@@ -19,6 +19,7 @@ namespace {
 std::mutex mu;
 std::map<std::string, long> counts;
 std::map<const void*, std::string> kernels;
+std::map<std::pair<std::string, unsigned>, long> launched;   // by kernel and threads of a block
 std::map<uint64_t, uint32_t> unpacked;
 const pthread_t main_thread = pthread_self();
 thread_local cudaError_t last = cudaSuccess;              // as the runtime keeps it: per host thread
@@ -41,11 +42,11 @@ cudaError_t alloc(const char* what, void** p, size_t n) {
     *p = calloc(1, n);
     return ret(*p ? cudaSuccess : cudaErrorMemoryAllocation);
 }
-cudaError_t launch(const void* f, void** args) {
+cudaError_t launch(const void* f, unsigned threads, void** args) {
     note("launches");
     if (launches_left.load() >= 0 && launches_left.fetch_sub(1) <= 0) return ret(cudaErrorLaunchOutOfResources);
     std::string name;
-    { std::lock_guard<std::mutex> l(mu); name = kernels[f]; }
+    { std::lock_guard<std::mutex> l(mu); name = kernels[f]; ++launched[{name, threads}]; }
     if (!capturing && name.find("k_state_io") != std::string::npos) {        // (StateIoArgs, first word, words, slot)
         const uint64_t w0 = *static_cast<uint64_t*>(args[1]);
         const unsigned n = *static_cast<unsigned*>(args[2]);
@@ -64,6 +65,12 @@ void fake_fail_alloc(size_t bytes) { fail_bytes = bytes; }                    //
 void fake_fail_threads(long after) { threads_left = after; }                  // thread starts fail after that many (-1: none)
 void fake_fail_launches(long after) { launches_left = after; }                // kernel launches fail after that many (-1: none)
 void fake_fail_graphs(int on) { fail_graphs = on != 0; }                      // no memory for graphs
+long fake_launched(const char* part, unsigned threads) {                      // launches of kernels with this in their name and blocks of so many threads
+    std::lock_guard<std::mutex> l(mu);
+    long n = 0;
+    for (auto& kv : launched) if (kv.first.second == threads && kv.first.first.find(part) != std::string::npos) n += kv.second;
+    return n;
+}
 long fake_unpacked(uint32_t* out, long n) {                                   // words that arrived, in order; -1 if one is missing
     std::lock_guard<std::mutex> l(mu);
     if ((long)unpacked.size() != n) return -1;
@@ -88,8 +95,8 @@ void __cudaRegisterFunction(void**, const char* host, char*, const char* name, i
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
 unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t s, void* st) { config = {g, b, s, st}; return 0; }
 cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* s, void* st) { *g = config.grid; *b = config.block; *s = config.smem; *static_cast<void**>(st) = config.stream; return cudaSuccess; }
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t, cudaStream_t) { return launch(f, args); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void* f, void** args) { return launch(f, args); }
+cudaError_t cudaLaunchKernel(const void* f, dim3, dim3 b, void** args, size_t, cudaStream_t) { return launch(f, b.x, args); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) { return launch(f, c->blockDim.x, args); }
 
 // ---- devices
 cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
@@ -114,9 +121,9 @@ cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { memcp
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { note("memcpy_async"); if (!capturing) memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemset(void* d, int v, size_t n) { memset(d, v, n); return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { if (!capturing) memset(d, v, n); return cudaSuccess; }
-cudaError_t cudaIpcGetMemHandle(cudaIpcMemHandle_t*, void*) { return ret(cudaErrorNotSupported); }
-cudaError_t cudaIpcOpenMemHandle(void**, cudaIpcMemHandle_t, unsigned) { return ret(cudaErrorNotSupported); }
-cudaError_t cudaIpcCloseMemHandle(void*) { return ret(cudaErrorNotSupported); }
+cudaError_t cudaIpcGetMemHandle(cudaIpcMemHandle_t* h, void*) { memset(h, 0, sizeof *h); return cudaSuccess; }
+cudaError_t cudaIpcOpenMemHandle(void** p, cudaIpcMemHandle_t, unsigned) { *p = calloc(1, 1 << 22); return ret(*p ? cudaSuccess : cudaErrorMemoryAllocation); }      // (a peer's memory, never written)
+cudaError_t cudaIpcCloseMemHandle(void* p) { free(p); return cudaSuccess; }
 
 // ---- streams, events, graphs
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = reinterpret_cast<cudaStream_t>(new char); return cudaSuccess; }
@@ -139,4 +146,15 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t, unsigned long 
 cudaError_t cudaGraphDestroy(cudaGraph_t g) { delete reinterpret_cast<char*>(g); return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t x) { note("graphs_dropped"); delete reinterpret_cast<char*>(x); return cudaSuccess; }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { note("graph_launches"); return cudaSuccess; }
+
+// ---- NCCL
+struct FakeNcclId { char bytes[128]; };
+int ncclGetUniqueId(FakeNcclId*) { return 0; }
+int ncclCommInitRank(void** c, int, FakeNcclId, int) { *c = new char; return 0; }
+int ncclCommDestroy(void* c) { delete static_cast<char*>(c); return 0; }
+int ncclAllGather(const void*, void*, size_t, int, void*, cudaStream_t) { return 0; }
+int ncclReduceScatter(const void*, void*, size_t, int, int, void*, cudaStream_t) { return 0; }
+int ncclGroupStart() { return 0; }
+int ncclGroupEnd() { return 0; }
+const char* ncclGetErrorString(int) { return "error of the stand-in"; }
 }

@@ -1,5 +1,5 @@
 """Host-side failures and host-side rules of the library, without a GPU: each test runs a child process in which a stand-in for the
-CUDA runtime (fake_cudart.cpp) is preloaded.  It gives memory, runs no kernels, and fails the calls it is told to fail."""
+CUDA runtime (fake_cudart.cpp) is preloaded, which also stands for NCCL.  It gives memory, runs no kernels, and fails the calls it is told to fail."""
 import os
 import subprocess
 import sys
@@ -20,6 +20,8 @@ F.fake_count.restype = C.c_long
 F.fake_unpacked.restype = C.c_long
 F.fake_fail_alloc.argtypes = [C.c_size_t]
 F.fake_fail_threads.argtypes = F.fake_fail_launches.argtypes = [C.c_long]
+F.fake_launched.restype = C.c_long
+F.fake_launched.argtypes = [C.c_char_p, C.c_uint]
 count = lambda what: F.fake_count(what.encode())
 GEOM = {TINY!r}
 
@@ -58,9 +60,11 @@ def fake(tmp_path_factory):
     so = str(tmp_path_factory.mktemp("fake") / "fake_cudart.so")
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I/usr/local/cuda/include", os.path.join(HERE, "fake_cudart.cpp"),
                     "-o", so, "-ldl", "-lpthread"], check=True, timeout=120)
+    os.symlink(so, os.path.join(os.path.dirname(so), "libnccl.so.2"))
+    env = dict(os.environ, LD_PRELOAD=so, LD_LIBRARY_PATH=os.path.dirname(so) + os.pathsep + os.environ.get("LD_LIBRARY_PATH", ""))
 
     def run(script):
-        out = subprocess.run([sys.executable, "-c", PRELUDE + script], env=dict(os.environ, LD_PRELOAD=so), capture_output=True, text=True, timeout=120)
+        out = subprocess.run([sys.executable, "-c", PRELUDE + script], env=env, capture_output=True, text=True, timeout=120)
         assert out.returncode == 0, out.stdout[-2000:] + out.stderr[-3000:]
     return run
 
@@ -222,4 +226,26 @@ for i, call in enumerate(calls):
     ran, counted = count("launches"), e.launch_count()
     call()
     assert count("launches") - ran == e.launch_count() - counted > 0, (i, count("launches") - ran, e.launch_count() - counted)
+""")
+
+
+@pytest.mark.parametrize("rows", [5, 13, 16, 17, 30])
+def test_expert_block_height_of_an_expert_parallel_step(fake, rows):
+    """Blocks of 8 rows (24 warps and the producer) up to a mean of 8 gathered rows an expert, of 16 rows (16 warps and the producer) from there
+    on, as in a plain call of as many rows: the rule goes by the experts of the model, in an expert-parallel step too."""
+    fake(f"rows = {rows}" + """
+blocks = lambda: [F.fake_launched(b"k_expert_rows", t) for t in (25 * 32, 17 * 32)]
+gathered, wide = 2 * rows, 2 * rows * GEOM["top_k"] > 8 * GEOM["n_experts"]
+ep = engine()
+ep.use_graphs(False)
+ep.ep_init(0, 2, np.zeros(128, np.uint8), rows)
+streams = [ep.stream(32) for _ in range(rows)]
+before = blocks()
+assert len(ep.batch_step_argmax(streams, [1] * rows)) == rows and F.fake_launched(b"k_ep_lists", 256) == GEOM["n_layers"]
+one = [b - a for a, b in zip(before, blocks())]
+assert one == [2 * GEOM["n_layers"] * (not wide), 2 * GEOM["n_layers"] * wide], one
+if gathered > 24:                                          # (shorter plain calls are routed by the expert kernels: always 8 rows)
+    s, before = ep.stream(128), blocks()
+    s.forward([1] * gathered)
+    assert [b - a for a, b in zip(before, blocks())] == one
 """)

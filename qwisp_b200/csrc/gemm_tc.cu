@@ -87,6 +87,8 @@ __device__ __forceinline__ void tc_arrive(uint64_t* b) { asm volatile("mbarrier.
 // Bounded wait of a role.  The first that runs out (a poll takes up to 4 us, so some 17 s) raises the CTA's abort word; every
 // later wait of the CTA then gives up after 256 polls.  The outcome is a lane's own, but what follows a wait needs whole warps:
 // a role goes on to the end of its item whatever its waits said (its results are discarded then) and leaves by tc_agree().
+// The lanes' polls, like every branch that is a lane's own (rows or tiles that only half a warp has), are behind a __syncwarp()
+// or a vote before the next tcgen05 instruction of the .sync.aligned kind, which a warp has to come to as one.
 // Warps need not agree: none waits for another but here and at the end of the kernel.
 template <int LIMIT>
 __device__ __forceinline__ bool tc_wait(uint64_t* b, uint32_t parity, volatile int* abort_word) {
@@ -171,6 +173,7 @@ struct DenseWork {
 #pragma unroll 1
         for (int c0 = 0; c0 < nt; c0 += 16) {
             uint32_t d[16];
+            __syncwarp();
             tmem_ld16(taddr + (uint32_t)c0, d);
             if (c0 + 16 >= nt) release();
             if (row < a.N) {
@@ -275,6 +278,7 @@ struct ExpertWork {
 #pragma unroll 1
         for (int c0 = 0; c0 < e.count; c0 += 16) {
             uint32_t d[16];
+            __syncwarp();
             tmem_ld16(taddr + (uint32_t)c0, d);
             if (c0 + 16 >= e.count) release();
             if (DOWN) {
@@ -323,6 +327,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
         mbar_fence_init();
     }
     if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&s_tmem)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -414,10 +419,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
             for (int u = 0; u < U; ++u) {
                 if (n < total) {
                     ok = tc_wait<LIMIT>(&s_empty[st], ph, &s_abort) && ok;
+                    __syncwarp();
                     tc_fence_after();                                       // (rows the matrix does not have are expanded too: their outputs are not stored)
                     tc_group_A(wv[u], sv[u][0], ta + st * 64);
                     tc_group_A(wv[u] + 4, sv[u][1], ta + st * 64 + 32);
                     fetch(wv[u], sv[u]);
+                    __syncwarp();                                           // (N % 32 == 16: only half of the warp has a tile)
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     tc_fence_before();
                     __syncwarp();
@@ -512,6 +519,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(typename W::Args a) {
     }
     tc_fence_before();
     __syncthreads();
+    __syncwarp();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512u) : "memory");
 }
 constexpr int TC_U = 2;

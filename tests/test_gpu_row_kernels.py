@@ -138,8 +138,8 @@ def test_batches_of_ragged_streams(engines, B):
         x.close(); y.close()
 
 
-# token tiles and weight-row groups of the tensor-core product
-@pytest.mark.parametrize("M,K,N", [(1, 512, 16), (31, 512, 128), (33, 512, 144), (65, 1024, 2064), (129, 4096, 272), (1000, 512, 144)])
+# token tiles and weight-row groups of the tensor-core product; runs of several items in which a warp's second tile comes and goes
+@pytest.mark.parametrize("M,K,N", [(1, 512, 16), (31, 512, 128), (33, 512, 144), (65, 1024, 2064), (129, 4096, 272), (1000, 512, 144), (20000, 512, 144), (6000, 512, 1040)])
 def test_tensor_core_tiles(M, K, N):
     from test_gpu_ops import test_tensor_core_gemm_matches_gemv_and_oracle as check
     check(M, K, N)

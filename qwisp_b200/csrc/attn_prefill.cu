@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(128) k_attn_prefill(AttnArgs a, int wave) {
             }
 #pragma unroll
             for (int rr = 0; rr < 2; ++rr) lrun[rr] = lrun[rr] * alpha[rr] + psum[rr];
-            if (alpha[0] != 1.f || alpha[1] != 1.f) {
+            if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {      // (as a warp: tensor-core steps follow)
 #pragma unroll
                 for (int i = 0; i < 32; ++i) { o[i][0] *= alpha[0]; o[i][1] *= alpha[0]; o[i][2] *= alpha[1]; o[i][3] *= alpha[1]; }
             }

@@ -93,7 +93,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* b, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait: gives up after 2^22 polls (up to 4 us each, so some 17 s) so a copy that never lands cannot hang the GPU;
-// the caller records the failure and carries on with whatever is in shared memory.
+// the caller records the failure and carries on with whatever is in shared memory.  The polls are a lane's own: a __syncwarp()
+// goes ahead of an mma or ldmatrix behind it, which a warp has to come to as one.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* b, uint32_t parity, int limit = 1 << 22) {
     for (int i = 0; i < limit; ++i) if (mbar_try_wait(b, parity)) return true;
     return false;

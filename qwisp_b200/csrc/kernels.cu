@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 2 : 1) k_gemv(DenseArgs a) 
         const int u = warp + NW * i;
         if (u < nvu) {
             if (!mbar_wait_bounded(ws.bar + (u >> 4), 0) && a.err && lane == 0) atomicOr(a.err, 1u);
+            __syncwarp();
             SliceRegs rg;
             load_slice_smem(rg, ws.w + (size_t)u * 128, ws.s + (size_t)u * 16, lane);
             float accS[4] = {0.f, 0.f, 0.f, 0.f}, accB[4] = {0.f, 0.f, 0.f, 0.f}, v[4];
@@ -214,6 +215,7 @@ __global__ void __launch_bounds__(256) k_head(DenseArgs a) {
     float best[2] = {-INFINITY, -INFINITY}; int besti[2] = {0x7fffffff, 0x7fffffff};
     while (have) {
         float tot[4] = {0.f, 0.f, 0.f, 0.f};
+        __syncwarp();                             // (behind the comparisons of the tile before, which are a lane's own)
         for (int sidx = 0; sidx < slices; ++sidx) {
             int ns = sidx + 1, ntile = tile;
             if (ns == slices) { ns = 0; ntile = tile + stride; }
@@ -873,6 +875,7 @@ __global__ void __launch_bounds__(512, 1) k_expert(ExpertArgs a) {
                 const int u = warp + 16 * i;
                 if (u < nvu) {
                     if (c0 == 0 && !mbar_wait_bounded(wsc.bar + i, parity) && a.err && lane == 0) atomicOr(a.err, 1u);
+                    __syncwarp();
                     SliceRegs rg;
                     load_slice_smem(rg, wsc.w + (size_t)u * 128, wsc.s + (size_t)u * 16, lane);
                     float accS[4] = {0.f, 0.f, 0.f, 0.f}, accB[4] = {0.f, 0.f, 0.f, 0.f}, v[4];
@@ -1045,6 +1048,7 @@ __global__ void __launch_bounds__(512, 1) k_expert_fused(ExpertArgs a) {
             const int u = warp + 16 * i;
             if (u < nvu1) {
                 if (!mbar_wait_bounded(ws1.bar + i, 0) && a.err && lane == 0) atomicOr(a.err, 1u);
+                __syncwarp();
                 SliceRegs rg;
                 load_slice_smem(rg, ws1.w + (size_t)u * 128, ws1.s + (size_t)u * 16, lane);
                 float accS[4] = {0.f, 0.f, 0.f, 0.f}, accB[4] = {0.f, 0.f, 0.f, 0.f}, v[4];
@@ -1110,6 +1114,7 @@ __global__ void __launch_bounds__(512, 1) k_expert_fused(ExpertArgs a) {
             const int u = warp + 16 * i;
             if (u < nvu2) {
                 if (!mbar_wait_bounded(ws2.bar + i, 0) && a.err && lane == 0) atomicOr(a.err, 1u);
+                __syncwarp();
                 SliceRegs rg;
                 load_slice_smem(rg, ws2.w + (size_t)u * 128, ws2.s + (size_t)u * 16, lane);
                 float accS[4] = {0.f, 0.f, 0.f, 0.f}, accB[4] = {0.f, 0.f, 0.f, 0.f}, v[4];

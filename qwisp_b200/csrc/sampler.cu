@@ -148,7 +148,9 @@ __global__ void __launch_bounds__(SAMP_T, 1) k_sample_rows(const __half* logits,
         for (int w = 0; w < 32; ++w) { const unsigned o = s_wsum[w]; total += o; if (w < warp) below += o; }
         cum += below;
         const unsigned target = (unsigned)__fmul_rn(top_p, (float)total);
-        if (cum >= target && (tid == 0 || cum - h < target)) s_bin = tid;     // the first bin that reaches the target
+        // the first bin that reaches the target.  (Counts wrap from 2^32 on, 524288 tokens as likely as the likeliest: then the sums
+        // may pass the target several times)
+        if (cum >= target && (tid == 0 || cum - h < target)) atomicMin(&s_bin, tid);
         __syncthreads();
         lthr = __fsub_rn(gmax, __fdiv_rn(__fmul_rn((float)(s_bin + 1), bin_w), invT));
     }

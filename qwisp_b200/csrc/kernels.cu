@@ -1500,7 +1500,7 @@ __global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, int
         const float gms[HG] = {gm4.x, gm4.y, gm4.z, gm4.w}, mine[HG] = {mine4.x, mine4.y, mine4.z, mine4.w};
 #pragma unroll
         for (int g = 0; g < HG; ++g) {
-            const float f = (mine[g] == -INFINITY) ? 0.f : __expf(mine[g] - gms[g]);
+            const float f = attn_warp_factor(mine[g], gms[g]);
             if (lane == g) sm_f[warp][g] = f;
             const f32x2 f2 = pk2(f, f);
             float4* dst = reinterpret_cast<float4*>(sm_acc + ((size_t)warp * HG + g) * ATT_D);      // (quads swapped in pairs by the lane: no bank conflicts)
@@ -1519,14 +1519,11 @@ __global__ void __launch_bounds__(256, 2) k_attn_fused(AttnArgs a, int prep, int
         *reinterpret_cast<float4*>(a.part_o + (((size_t)m * a.NH + h0 + og) * a.nsplit + sp) * ATT_D + oq * 4) = o;
         if (threadIdx.x < HG) {
             const int g = threadIdx.x;
-            float gm = -INFINITY, ls = 0.f;                   // attn_warps_max(), attn_warps_lsum() with the factors from above
+            float m8[8], l8[8], f8[8];
 #pragma unroll
-            for (int w = 0; w < 8; ++w) {
-                gm = fmaxf(gm, sm_m[pb][w][g]);
-                ls = __fadd_rn(ls, __fmul_rn(sm_l[pb][w][g], sm_f[w][g]));
-            }
+            for (int w = 0; w < 8; ++w) { m8[w] = sm_m[pb][w][g]; l8[w] = sm_l[pb][w][g]; f8[w] = sm_f[w][g]; }
             float* pml = a.part_ml + (((size_t)m * a.NH + h0 + g) * a.nsplit + sp) * 2;
-            pml[0] = gm; pml[1] = ls;
+            pml[0] = attn_warps_max(m8); pml[1] = attn_warps_lsum(l8, f8);
         }
     }
     // ---- the CTA that finishes last for this (row, four heads) merges the splits ----

@@ -174,9 +174,12 @@ __device__ __forceinline__ float attn_warps_max(const float m8[8]) {
     for (int w = 0; w < 8; ++w) gm = fmaxf(gm, m8[w]);
     return gm;
 }
-__device__ __forceinline__ float attn_warps_lsum(const float m8[8], const float l8[8], float gm) {
+// (f8: the warps' factors, attn_warp_factor(); no multiply-add, so that every kernel has the same bits)
+__device__ __forceinline__ float attn_warp_factor(float m, float gm) { return (m == -INFINITY) ? 0.f : __expf(m - gm); }
+__device__ __forceinline__ float attn_warps_lsum(const float l8[8], const float f8[8]) {
     float ls = 0.f;
-    for (int w = 0; w < 8; ++w) ls += (m8[w] == -INFINITY) ? 0.f : l8[w] * __expf(m8[w] - gm);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) ls = __fadd_rn(ls, __fmul_rn(l8[w], f8[w]));
     return ls;
 }
 // Merge of the splits of one (row, head): part_o [used][256] f32, part_ml [used][2] f32 (both read with the loaders the caller
@@ -196,7 +199,7 @@ __device__ __forceinline__ void attn_merge_splits(int used, int lane, const __ha
     gm = warp_max(gm);
     float tot = 0.f;
 #pragma unroll
-    for (int j = 0; j < 2; ++j) { fv[j] = (msv[j] == -INFINITY) ? 0.f : __expf(msv[j] - gm); tot += lsv[j] * fv[j]; }
+    for (int j = 0; j < 2; ++j) { fv[j] = attn_warp_factor(msv[j], gm); tot = fmaf(lsv[j], fv[j], tot); }
     tot = warp_sum(tot);
     float o[D];
 #pragma unroll

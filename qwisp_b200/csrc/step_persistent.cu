@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_step_persistent(PStepArgs a) 
 #pragma unroll
                         for (int x = 0; x < 8; ++x) m8[x] = sm.misc->sm_m[x][head];
                         const float gm = attn_warps_max(m8);
-                        const float f = (mx[hh] == -INFINITY) ? 0.f : __expf(mx[hh] - gm);
+                        const float f = attn_warp_factor(mx[hh], gm);
                         float4* dst = reinterpret_cast<float4*>(mbuf + ((size_t)kw * 2 + (warp >> 3)) * ATT_D + lane * 8);
                         dst[0] = make_float4(acc[hh][0] * f, acc[hh][1] * f, acc[hh][2] * f, acc[hh][3] * f);
                         dst[1] = make_float4(acc[hh][4] * f, acc[hh][5] * f, acc[hh][6] * f, acc[hh][7] * f);
@@ -758,11 +758,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_step_persistent(PStepArgs a) 
                             uint4* dstl = XP + ((size_t)hd * a.nsplit + split) * 129;
                             if ((d & 1) == 0) ll_store(dstl + (d >> 1), me, nb, seq);
                             if (d == 0) {
-                                float mm[8], ll8[8];
+                                float mm[8], ll8[8], ff8[8];
                                 const int hl = 4 * pass + 2 * which + hh;
                                 for (int x = 0; x < 8; ++x) { mm[x] = sm.misc->sm_m[x][hl]; ll8[x] = sm.misc->sm_l[x][hl]; }
                                 const float gm2 = attn_warps_max(mm);
-                                const float ls = attn_warps_lsum(mm, ll8, gm2);
+                                for (int x = 0; x < 8; ++x) ff8[x] = attn_warp_factor(mm[x], gm2);
+                                const float ls = attn_warps_lsum(ll8, ff8);
                                 ll_store(dstl + 128, __float_as_uint(gm2), __float_as_uint(ls), seq);
                             }
                         }

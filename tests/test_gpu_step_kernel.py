@@ -58,6 +58,25 @@ def test_step_kernel_equals_kernel_per_phase(geom_name, tiny_engine, mini_engine
         eng.use_persistent(False)
 
 
+# attention over part of a split of 32 keys, over one, over more than one, over several
+@pytest.mark.parametrize("context", [30, 40, 64, 150])
+def test_step_kernel_merges_of_several_splits(context, tiny_engine):
+    eng = tiny_engine
+    p = _prompt(TINY["vocab"], context + 1, "stepk.splits")
+    a, b = eng.stream(context + 8), eng.stream(context + 8)
+    for s in (a, b):
+        for i in range(0, context, 64):
+            s.forward(p[i:min(i + 64, context)], want_hidden=False)
+    try:
+        assert eng.use_persistent(True)
+        ta = a.chained_step_argmax(int(p[-1]), 4)
+    finally:
+        eng.use_persistent(False)
+    assert list(ta) == list(b.chained_step_argmax(int(p[-1]), 4))
+    assert np.array_equal(a.state_save(), b.state_save())
+    a.close(); b.close()
+
+
 def test_step_kernel_two_streams_interleaved(tiny_engine):
     """Two streams taking turns: the step kernel keeps nothing between launches except what is in the caches."""
     eng = tiny_engine

@@ -39,8 +39,8 @@ __device__ __forceinline__ __half hadd_rn(__half a, __half b) { return __hadd_rn
 __device__ __forceinline__ __half hsub_rn(__half a, __half b) { return __hsub_rn(a, b); }
 __device__ __forceinline__ __half hmul_rn(__half a, __half b) { return __hmul_rn(a, b); }
 __device__ __forceinline__ __half hdiv_rn(__half a, __half b) { return f2h(__fdiv_rn(h2f(a), h2f(b))); }     // (f32 carries >= 2*11+2 bits: rounding twice is rounding once)
-// 1 / a.  The last bit of the hardware's approximate reciprocal never reaches the fp16 result: equal to hdiv_rn(1, a) for every
-// half (all 65536 compared).  Without the branch of the exact form eight of them overlap.
+// 1 / a, equal to hdiv_rn(1, a) for every half: a quotient lies at least 2^-22 (relative) from where its fp16 rounding changes, and the
+// hardware's approximate reciprocal is at most 2^-23 off.  Without the branch of the exact form eight of them overlap.
 __device__ __forceinline__ __half hrcp_rn(__half a) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(h2f(a)));

@@ -495,3 +495,36 @@ def test_sampler_matches_golden():
             assert [f.tolist(), r.tolist(), a.tolist()] == g[name], name
     finally:
         eng.close()
+
+
+# the sigmoid's reciprocal is the hardware's approximate one rounded to fp16: the exact quotient's fp16 for every half
+def test_reciprocal_of_every_half(tmp_path):
+    import ctypes as C
+    import subprocess
+
+    from qwisp_b200 import build
+    src, so = tmp_path / "rcp.cu", str(tmp_path / "rcp.so")
+    src.write_text("""#include "common.cuh"
+__global__ void k_rcp(__half* out) {
+    const unsigned i = blockIdx.x * 256 + threadIdx.x;
+    out[i] = sl::hrcp_rn(__ushort_as_half((unsigned short)i));
+}
+extern "C" int rcp_of_every_half(void* host) {
+    __half* d = nullptr;
+    cudaError_t err = cudaMalloc(&d, 65536 * sizeof(__half));
+    if (err != cudaSuccess) return (int)err;
+    k_rcp<<<256, 256>>>(d);
+    err = cudaGetLastError();
+    if (err == cudaSuccess) err = cudaMemcpy(host, d, 65536 * sizeof(__half), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return (int)err;
+}
+""")
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    subprocess.run([nvcc] + build.NVCC_FLAGS + ["-shared", "-I", build.CSRC, str(src), "-o", so], check=True, timeout=300)
+    got = np.empty(65536, np.float16)
+    assert C.CDLL(so).rcp_of_every_half(C.c_void_p(got.ctypes.data)) == 0
+    with np.errstate(divide="ignore", invalid="ignore", over="ignore"):
+        ref = (1.0 / np.arange(65536, dtype=np.uint16).view(np.float16).astype(np.float64)).astype(np.float16)
+    nan = np.isnan(ref)
+    assert np.array_equal(np.isnan(got), nan) and np.array_equal(got.view(np.uint16)[~nan], ref.view(np.uint16)[~nan])

@@ -543,8 +543,11 @@ int launch_gemm_tc(const Q4R& q, int N, int K, int M, const __half* x, int ldx, 
     if (N % 16 || K % 256) return -1;
     GemmTcArgs a{q, N, K, M, x, ldx, y, ldy, add_to_y ? 1 : 0, err};
     // The token tile is a scheduling choice only (a token's column never interacts with another's).  An item's time is the
-    // larger of its MMAs and of the expansion of its weights (whatever the tile: about equal at 128 tokens), and a
-    // multiprocessor does ceil(items / multiprocessors) of them: the cheapest sum, the wider tile on a tie.
+    // larger of its MMAs and of the expansion of its weights (whatever the tile), and a multiprocessor does
+    // ceil(items / multiprocessors) of them: the cheapest sum, the wider tile on a tie.  Measured, K = 2048, weights from memory:
+    // 8.2, 5.7, 6.0 us an item of 128, 64, 32 tokens, the first with a start of about 8 more; the costs are those of the first (16.5, 13, 12.5).
+    // 20 row counts from 16 to 1024 of 12352 x 2048, 9216 x 2048 and 2048 x 4096: the chosen tile was the fastest or within 7 % of it,
+    // which is also what two runs of one tile differ by (129 rows of 12352: 23.1, 18.6, 24.9; 512: 33.0, 40.7, 59.6; 1024: 59.5, 70.0, 112).
     const long row_tiles = (N + TC_ROWS - 1) / TC_ROWS;
     const int nts[3] = {128, 64, 32}, cost[3] = {320, 260, 260};
     int best = 0; long best_cost = 0;

@@ -898,8 +898,8 @@ bool launch_expert_rows_down(const ExpertArgs& a, cudaStream_t st, bool pdl) { r
 //                 groups of 8, whose normed rows arrive in shared memory by cp.async two groups ahead of their use.
 //                 The dot product is the one of k_moe_router (lane l owns 8 consecutive inputs of every 256-wide block,
 //                 sequential f32 accumulate, butterfly over the lanes), so the logits are the same bits.
-// k_route_rows    one warp per row: top-k + gates (route_row_warp); the last CTA groups the (row, k) pairs by expert with
-//                 a parallel scan (or, expert-parallel, sends rows and indices to every rank).
+// k_route_rows    one warp per row: top-k + gates (route_row_warp), and the row's pairs go to their experts' places; the last CTA
+//                 lists the experts that have pairs.  (Expert-parallel: a CTA per row, which sends the indices to every rank.)
 // Input rows are already normed (k_final_norm), so no CTA repeats the norm.
 template <bool Q8>
 __global__ void __launch_bounds__(256, 2) k_router_rows(RouterArgs a) {

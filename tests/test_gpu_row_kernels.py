@@ -181,7 +181,7 @@ def test_sampler_vocabularies(vocab):
 def test_sampler_counts_wrap():
     import qwisp_b200 as Q
     from oracle import oracle as O
-    parts = ((366000, 0.0), (260000, -0.0625), (69200, -0.125))            # tokens, logit: bins 0, 1 and 3
+    parts = ((366000, 0.0), (169200, -0.0625), (92800, -3.921875))          # tokens, logit: bins 0, 1 and 100
     sums = np.cumsum([n * int(np.exp(np.float32(x)) * 8192) for n, x in parts]) % 2 ** 32
     assert sums[0] > 0.9 * sums[2] > sums[1] and sum(n for n, _ in parts) % 16 == 0
     row = np.concatenate([np.full(n, x, np.float16) for n, x in parts])
@@ -189,10 +189,11 @@ def test_sampler_counts_wrap():
     try:
         logits = np.stack([np.random.default_rng(i).permutation(row) for i in range(8)])
         draft = np.full(8, -1, dtype=np.int32)
-        got = Q.ops.sample_rows(e, logits, draft, 1.0, 0.9, 5, 6, 40)
-        ref = O.sample_rows(logits, draft, 1.0, 0.9, 5, 6, 40)
-        assert all(np.array_equal(g, r) for g, r in zip(got, ref)), (got, ref)
-        assert all(logits[i, t] == 0 for i, t in enumerate(ref[0]))
+        for pos in range(0, 160, 8):
+            got = Q.ops.sample_rows(e, logits, draft, 1.0, 0.9, 5, 6, pos)
+            ref = O.sample_rows(logits, draft, 1.0, 0.9, 5, 6, pos)
+            assert all(np.array_equal(g, r) for g, r in zip(got, ref)), (pos, got, ref)
+            assert all(logits[i, t] == 0 for i, t in enumerate(ref[0]))
     finally:
         e.close()
 
